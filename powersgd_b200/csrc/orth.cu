@@ -6,8 +6,8 @@
 // tall matrix exactly twice, whatever the rank:
 //
 //   G = X^T X        accumulated in float64, fixed summation order (bit-reproducible)
-//   G = R^T R        Cholesky in float64 by one warp; R^-1 by back substitution
-//   X <- X R^-1      rounded to float32 once
+//   G = R^T R        Cholesky in float64 by one warp
+//   X <- X R^-1      by forward substitution in float64, rounded to float32 once
 //
 // With a float64 Gram matrix one pass is as orthonormal as float32 can express for any X
 // that float32 can represent (error ~ 1e-16 * cond(X)^2 + 6e-8). A pivot below 1e-12 of its
@@ -18,19 +18,21 @@
 // Rank-1 units keep the reference's quirk: ONE Frobenius norm over the whole shape group
 // (all B matrices jointly), floored at 1e-16, divides every entry.
 //
-// Two launches. The first cuts every unit into row chunks, one CTA each: partial Gram matrices
-// (and partial cross products F_i^T X against earlier factors of the same side) go to scratch;
-// the CTA that arrives last at the unit's ticket adds the partials in chunk order, factorises,
-// and publishes R^-1 plus the cross products C_i = (F_i^T X) R^-1 = F_i^T X_hat that the product
-// kernels use to deflate algebraically. The second launch applies R^-1 to every row chunk. A long
-// factor (an embedding with 50 000 rows, rank 16) thus takes microseconds instead of the
-// hundreds that one CTA per unit needed.
+// Two launches, one CTA per row chunk of a unit in both. The first writes the chunk's partial Gram
+// matrix (and partial cross products F_i^T X against earlier factors of the same side). In the
+// second EVERY chunk adds the partials of its unit in chunk order, factorises the sum and solves
+// its own rows; one chunk per earlier factor also publishes the cross products
+// C_i = (F_i^T X) R^-1 = F_i^T X_hat that the product kernels use to deflate algebraically.
+// Both launches are bound by latency (a factor is tens of kilobytes), so what counts is the length
+// of the dependent chain: factorising redundantly takes the place of an arrival counter, a memory
+// fence, a lone last CTA and a second round trip through memory, and the second launch is
+// released early (programmatic dependent launch) so that only its wait remains.
 //
 // Multi-GPU: the factor to orthonormalise is the SUM over workers of what the previous product
 // launch pushed into this rank's slot arena. The first launch is then also the consumer of that
 // in-kernel all-reduce (powersgd/powersgd.py:205-209 in the reference is a blocking library
-// call): while staging its chunk every CTA polls the tagged words of the W slots, adds them in
-// rank order, and writes the sum to the factor buffer and to the copy the decompression reads.
+// call): every CTA polls the tagged words of its rows in the W slots, adds them in rank order, and
+// writes the sum to the factor buffer and to the copy the decompression reads.
 #include "psgd_bounds.cuh"
 #include "psgd_comm.cuh"
 
@@ -61,50 +63,124 @@ struct OrthArgs {
   const float* prev[PSGD_MAX_HIST];  // each laid out like x
   float* cmat[PSGD_MAX_HIST];        // out: [mat][r*r] blocks with stride PSGD_CMAT_STRIDE
   double* part;                      // scratch: [chunk][1 + nprev][RT*RT] partial sums
-  double* rinv;                      // scratch: [unit][RT*RT]  R^-1 (rank 1: [0] = the divisor)
-  int* dead;                         // scratch: [unit][RT]     column status (see sDead)
-  int* tickets;                      // [unit], zero between launches
+  float* head;                       // scratch: [unit][2*RT*RT] the unit's first 2r rows as they came in: what
+                                     // replacing a column needs of X while other chunks overwrite it in place
   const PsgdCommDev* comm;           // not null: x is first gathered from the channel's slots (see above)
   float* sum_out;                    // with comm: second destination of the gathered sum (laid out like x)
 };
 
 constexpr int ORTH_THREADS = 256;
-constexpr int ORTH_CHUNK_FLOATS = 2048;  // rows per chunk = 2048 / RT (8 KiB of the factor). The chunk
-                                         // is staged in shared memory as float64: conversions issue at
-                                         // a fraction of the FMA rate, so each value is converted once
-                                         // and not once per pair it takes part in
+constexpr int ORTH_WARPS = ORTH_THREADS / 32;
+constexpr int ORTH_STAGE_ROWS_X_RT = 2048;  // staged rows per pass at RT >= 8 = 2048 / RT, as float64: conversions
+                                            // issue at a fraction of the FMA rate, so each value is converted
+                                            // once and not once per pair it takes part in
 
-// Sum over the rows of a chunk of a[row][j] * b[row][k] for every pair (j, k), in float64 and in
-// a fixed order: row groups stride through the chunk, then the groups are added in order.
-// Result: out[j * RT + k] (global scratch), written by the threads with tid < RT * RT.
+// Rows of a chunk when the unit is short: two rows per thread of the second launch at RT <= 4, one
+// staging pass of the first launch above that.
 template <int RT>
-__device__ __forceinline__ void chunk_pairs(const double* sa, const double* sb, int rows, double* red, double* out, int tid) {
-  constexpr int NP = RT * RT;
-  constexpr int PP = NP > ORTH_THREADS ? NP / ORTH_THREADS : 1;     // pairs per thread
-  constexpr int NG = NP >= ORTH_THREADS ? 1 : ORTH_THREADS / NP;    // row groups
-  const int g = NP >= ORTH_THREADS ? 0 : tid / NP;
-  double acc[PP];
-#pragma unroll
-  for (int q = 0; q < PP; ++q) acc[q] = 0.0;
-  const int p0 = NP >= ORTH_THREADS ? tid : tid % NP;
-#pragma unroll 4
-  for (int row = g; row < rows; row += NG) {
-#pragma unroll
-    for (int q = 0; q < PP; ++q) {
-      const int p = p0 + q * ORTH_THREADS;
-      acc[q] = fma(sa[row * RT + p / RT], sb[row * RT + p % RT], acc[q]);
-    }
-  }
-  if (NG == 1) {
-#pragma unroll
-    for (int q = 0; q < PP; ++q) out[p0 + q * ORTH_THREADS] = acc[q];
+__host__ __device__ constexpr int orth_base_rows() { return RT <= 4 ? 512 : ORTH_STAGE_ROWS_X_RT / RT; }
+
+template <int RT>
+__device__ __forceinline__ void orth_load_row(const float* p, int r, double* v) {
+  if (RT == 4 && r == 4 && ((uintptr_t)p & 15u) == 0) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x; v[1 % RT] = q.y; v[2 % RT] = q.z; v[3 % RT] = q.w;
+  } else if (RT == 2 && r == 2 && ((uintptr_t)p & 7u) == 0) {
+    const float2 q = *reinterpret_cast<const float2*>(p);
+    v[0] = q.x; v[1 % RT] = q.y;
   } else {
-    red[tid] = acc[0];
+#pragma unroll
+    for (int c = 0; c < RT; ++c) v[c] = c < r ? (double)p[c] : 0.0;
+  }
+}
+
+// out[j * RT + k] = sum over the chunk's rows of a[row][j] * b[row][k], in float64 and in a fixed
+// order. a, b: first row of the chunk, r floats per row. `stage`: 2 * ORTH_STAGE_ROWS_X_RT doubles.
+template <int RT>
+__device__ __forceinline__ void chunk_pairs(const float* a, const float* b, int r, int rows, double* stage, double* out, int tid) {
+  constexpr int NP = RT * RT;
+  if (RT <= 4) {
+    // one row per thread, every pair in registers; lanes by shuffles, warps in index order
+    double acc[NP];
+#pragma unroll
+    for (int e = 0; e < NP; ++e) acc[e] = 0.0;
+#pragma unroll 2
+    for (int row = tid; row < rows; row += ORTH_THREADS) {
+      double va[RT], vb[RT];
+      orth_load_row<RT>(a + (long long)row * r, r, va);
+      orth_load_row<RT>(b + (long long)row * r, r, vb);
+#pragma unroll
+      for (int e = 0; e < NP; ++e) acc[e] = fma(va[e / RT], vb[e % RT], acc[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < NP; ++e) {
+      const double s = psgd_warp_sum(acc[e]);
+      if ((tid & 31) == 0) stage[(tid >> 5) * NP + e] = s;
+    }
     __syncthreads();
     if (tid < NP) {
       double s = 0.0;
-      for (int gg = 0; gg < NG; ++gg) s += red[gg * NP + tid];
+#pragma unroll
+      for (int w = 0; w < ORTH_WARPS; ++w) s += stage[w * NP + tid];
       out[tid] = s;
+    }
+    __syncthreads();
+  } else {
+    // rows staged as float64; every thread owns a 4 x 4 block of pairs and every NG-th row, so 8
+    // values read feed 16 multiply-adds; the row groups are added in index order at the end
+    constexpr int SR = ORTH_STAGE_ROWS_X_RT / RT;
+    constexpr int NB = RT / 4 < 1 ? 1 : RT / 4;
+    constexpr int NG = ORTH_THREADS / (NB * NB);
+    constexpr int PER = SR * RT / ORTH_THREADS;   // staged values per thread
+    double* sa = stage;
+    double* sb = stage + ORTH_STAGE_ROWS_X_RT;
+    const bool same = a == b;
+    const int blk = tid % (NB * NB), g = tid / (NB * NB);
+    const int j0 = blk / NB * 4, k0 = blk % NB * 4;
+    double acc[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+    float na[PER], nb[PER];
+    auto fetch = [&](int first) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int e = tid + i * ORTH_THREADS, row = first + e / RT, c = e % RT;
+        const bool in = row < rows && c < r;
+        na[i] = in ? a[(long long)row * r + c] : 0.f;
+        nb[i] = (in && !same) ? b[(long long)row * r + c] : 0.f;
+      }
+    };
+    fetch(0);
+    const double* rb = same ? sa : sb;
+    for (int first = 0; first < rows; first += SR) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        sa[tid + i * ORTH_THREADS] = (double)na[i];
+        if (!same) sb[tid + i * ORTH_THREADS] = (double)nb[i];
+      }
+      __syncthreads();
+      if (first + SR < rows) fetch(first + SR);  // lands while this pass is multiplied
+      const int n = min(SR, rows - first);
+#pragma unroll 2
+      for (int row = g; row < n; row += NG) {
+        const double2 a0 = *reinterpret_cast<const double2*>(sa + row * RT + j0), a1 = *reinterpret_cast<const double2*>(sa + row * RT + j0 + 2);
+        const double2 b0 = *reinterpret_cast<const double2*>(rb + row * RT + k0), b1 = *reinterpret_cast<const double2*>(rb + row * RT + k0 + 2);
+        const double va[4] = {a0.x, a0.y, a1.x, a1.y}, vb[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e] = fma(va[e >> 2], vb[e & 3], acc[e]);
+      }
+      __syncthreads();
+    }
+    // [NG][NP] group sums in the staging buffer (NG * NP = 16 * ORTH_THREADS doubles)
+    static_assert(NG * NP == 2 * ORTH_STAGE_ROWS_X_RT || RT < 8, "group sums must fill the staging buffer");
+#pragma unroll
+    for (int e = 0; e < 16; ++e) stage[g * NP + (j0 + (e >> 2)) * RT + k0 + (e & 3)] = acc[e];
+    __syncthreads();
+    for (int p = tid; p < NP; p += ORTH_THREADS) {
+      double s = 0.0;
+#pragma unroll 4
+      for (int gg = 0; gg < NG; ++gg) s += stage[gg * NP + p];
+      out[p] = s;
     }
     __syncthreads();
   }
@@ -117,45 +193,27 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_gram_kernel(OrthArgs a
   const PsgdOrthUnit u = a.units[ch.unit];
   const int r = u.r;
   const int tid = threadIdx.x;
-  const float* __restrict__ x = a.x + u.x_off;
+  __shared__ __align__(16) double stage[RT <= 4 ? ORTH_WARPS * NP : 2 * ORTH_STAGE_ROWS_X_RT];
+  psgd_launch_dependents();
+  psgd_wait_for_predecessor();
 #ifdef PSGD_BOUNDS_CHECK
   {
     bool ok = true;
     ok &= PSGD_BC(r >= 1 && r <= RT, 5, PSGD_BC_RANK, r, RT);
-    ok &= PSGD_BC(ch.row0 >= 0 && ch.rows > 0 && (long long)ch.row0 + ch.rows <= (long long)u.sub_len * u.nsub && ch.rows * RT <= ORTH_CHUNK_FLOATS,
+    ok &= PSGD_BC(ch.row0 >= 0 && ch.rows > 0 && (long long)ch.row0 + ch.rows <= (long long)u.sub_len * u.nsub,
                   5, PSGD_BC_CHUNK, (long long)ch.row0 + ch.rows, (long long)u.sub_len * u.nsub);
     ok &= PSGD_BC((int)blockIdx.x >= u.chunk0 && (int)blockIdx.x < u.chunk0 + u.nchunks, 5, PSGD_BC_CHUNK, blockIdx.x, u.chunk0 + u.nchunks);
     if (!ok) return;
   }
 #endif
-
-  __shared__ __align__(16) double sx[ORTH_CHUNK_FLOATS];
-  __shared__ __align__(16) double sf[ORTH_CHUNK_FLOATS];
-  __shared__ double red[ORTH_THREADS];
-  __shared__ double sG[NP];
-  __shared__ int sDead[RT];      // -1: alive; >= 0: row of the substituted basis vector; -2: dropped
-  __shared__ int s_last;
-  // used by the finishing CTA only, after the staging buffers are dead
-  static_assert(NP <= ORTH_CHUNK_FLOATS, "R must fit a staging buffer");
-  double* sR = sf;      // upper-triangular Cholesky factor
-  double* sRinv = sx;
-  __shared__ double sDiagInv[RT];                  // 1 / R[c][c]: float64 divisions and square roots
-                                                   // are long dependent instruction chains, so each
-                                                   // column pays for one and multiplies afterwards
-
-  // ---- partial sums of this chunk ---------------------------------------------------------
-  const int stride = 1 + a.nprev;
-  double* my_part = a.part + (long long)blockIdx.x * stride * NP;
+  const long long base = (long long)u.x_off + (long long)ch.row0 * r;
+  float* x = a.x + base;
   if (a.comm != nullptr) {
     // gather: this chunk is a contiguous run of rows * r words in every slot
     const PsgdCommDev& c = *a.comm;
     const int e1 = *c.epoch + 1;
-    const long long base = (long long)u.x_off + (long long)ch.row0 * r;
-    float* __restrict__ xw = a.x + base;
-    float* __restrict__ sw = a.sum_out + base;
+    float* sw = a.sum_out + base;
     const int n = ch.rows * r;
-    for (int e = tid; e < ch.rows * RT; e += ORTH_THREADS)
-      if (e % RT >= r) sx[e] = 0.0;
     bool ok = true;
     constexpr int NB = 4;
     for (int i0 = tid; i0 < n; i0 += NB * ORTH_THREADS) {
@@ -168,176 +226,162 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_gram_kernel(OrthArgs a
       for (int j = 0; j < NB; ++j) {
         const int i = i0 + j * ORTH_THREADS;
         if (i < n) {
-          xw[i] = v[j];
+          x[i] = v[j];
           sw[i] = v[j];
-          sx[(i / r) * RT + i % r] = (double)v[j];
         }
       }
     }
     psgd_comm_close_epoch(c, e1);  // (CTA barrier inside) every word of this chunk has been read
-  } else {
-    for (int e = tid; e < ch.rows * RT; e += ORTH_THREADS) {
-      const int row = e / RT, c = e % RT;
-      sx[e] = c < r ? (double)x[(long long)(ch.row0 + row) * r + c] : 0.0;
-    }
+    __syncthreads();               // and every element of x written
   }
-  __syncthreads();
-  chunk_pairs<RT>(sx, sx, ch.rows, red, my_part, tid);
-  for (int p = 0; p < a.nprev; ++p) {
-    const float* __restrict__ f = a.prev[p] + u.x_off;
-    __syncthreads();
-    for (int e = tid; e < ch.rows * RT; e += ORTH_THREADS) {
-      const int row = e / RT, c = e % RT;
-      sf[e] = c < r ? (double)f[(long long)(ch.row0 + row) * r + c] : 0.0;
-    }
-    __syncthreads();
-    chunk_pairs<RT>(sf, sx, ch.rows, red, my_part + (long long)(1 + p) * NP, tid);
-  }
+  const int stride = 1 + a.nprev;
+  double* my_part = a.part + (long long)blockIdx.x * stride * NP;
+  chunk_pairs<RT>(x, x, r, ch.rows, stage, my_part, tid);
+  for (int p = 0; p < a.nprev; ++p) chunk_pairs<RT>(a.prev[p] + base, x, r, ch.rows, stage, my_part + (long long)(1 + p) * NP, tid);
+  const int head_rows = min(2 * r - ch.row0, ch.rows);
+  float* head = a.head + (long long)ch.unit * 2 * NP + (long long)ch.row0 * r;
+  for (int e = tid; e < head_rows * r; e += ORTH_THREADS) head[e] = x[e];
+}
 
-  // ---- the chunk that arrives last finishes the unit ----------------------------------------
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = (psgd_atom_add_acqrel_gpu(a.tickets + ch.unit, 1) == u.nchunks - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const double* unit_part = a.part + (long long)u.chunk0 * stride * NP;
-  if (tid < NP) {
-    double s = 0.0;
-    for (int c = 0; c < u.nchunks; ++c) s += __ldcg(unit_part + (long long)c * stride * NP + tid);
-    sG[tid] = s;
-  }
-  __syncthreads();
-  double* rinv_out = a.rinv + (long long)ch.unit * NP;
-  int* dead_out = a.dead + (long long)ch.unit * RT;
-  const long long len = (long long)u.sub_len * u.nsub;
-
-  if (RT == 1 || r == 1) {
-    // joint Frobenius norm of the whole unit, float32 semantics of the division
-    const float d = fmaxf((float)sqrt(sG[0]), 1e-16f);
-    if (tid == 0) {
-      rinv_out[0] = (double)d;
-      dead_out[0] = -1;
-    }
-    // cross products per sub-matrix: (sum of f * x over the sub-matrix) / d
-    for (int e = tid; e < a.nprev * u.nsub; e += ORTH_THREADS) {
-      const int p = e / u.nsub, s = e % u.nsub;
-      double t = 0.0;
-      for (int c = 0; c < u.nchunks; ++c)
-        if (a.chunks[u.chunk0 + c].sub == s) t += __ldcg(unit_part + ((long long)c * stride + 1 + p) * NP);
-      a.cmat[p][(long long)(u.first_mat + s) * PSGD_CMAT_STRIDE] = (float)(t / (double)d);
-    }
-  } else {
-    // ---- Cholesky (one warp) with canonical-vector substitution -------------------------
-    if (tid < 32) {
-      const int lane = tid;
-      if (lane < RT) sDead[lane] = -1;
-      for (int e = lane; e < NP; e += 32) { sR[e] = 0.0; sRinv[e] = 0.0; }
+// ---- factorisation ---------------------------------------------------------------------------
+// R upper triangular with R^T R = G (row-major in sR, zero below the diagonal) and sDiagInv =
+// 1 / R[c][c], by one warp. What bounds it is the chain of r pivots, each a float64 reciprocal
+// square root followed by the update that the next pivot needs. So lane j keeps column j of the
+// trailing matrix in registers and every step updates all of it at once (right-looking); only the
+// row of R just finished goes through shared memory.
+// False when a pivot is not above the rounding noise of its column (or is not a number).
+template <int RT>
+__device__ __forceinline__ bool orth_cholesky(const double* sG, double* sR, double* sDiagInv, int r, int lane) {
+  double col[RT];
+#pragma unroll
+  for (int i = 0; i < RT; ++i) col[i] = lane < RT ? sG[i * RT + lane] : 0.0;
+  bool ok = true;
+#pragma unroll
+  for (int c = 0; c < RT; ++c) {
+    if (c < r && ok) {
+      const double s = __shfl_sync(0xffffffffu, col[c], c);
+      const double ref = sG[c * RT + c];
+      ok = (ref > 0.0) && (s > 1e-12 * ref);
+      const double inv = rsqrt(s);
+      const double v = lane >= c ? col[c] * inv : 0.0;
+      if (lane < RT) sR[c * RT + lane] = v;
+      if (lane == 0) sDiagInv[c] = inv;
       __syncwarp();
-      for (int c = 0; c < r; ++c) {
-        // pivot of column c
-        int attempt = 0;
-        double piv = 0.0, inv_piv = 0.0;
-        while (true) {
-          double s = sG[c * RT + c];
-          for (int i = 0; i < c; ++i) s -= sR[i * RT + c] * sR[i * RT + c];
-          const double ref = sG[c * RT + c];
-          const bool ok = (ref > 0.0) && (s > 1e-12 * ref);
-          if (ok) { inv_piv = rsqrt(s); piv = s * inv_piv; break; }
-          if (attempt == 2) { piv = 0.0; break; }
-          // substitute column c by the basis vector e_row; its Gram entries are matrix entries
-          const long long row = (attempt == 0 ? c : c + r) % len;
-          ++attempt;
-          __syncwarp();
-          if (lane < r) {
-            double g;
-            if (lane == c) g = 1.0;
-            else if (sDead[lane] >= 0) g = (sDead[lane] == (int)row) ? 1.0 : 0.0;
-            else if (sDead[lane] == -2) g = 0.0;
-            else g = (double)x[row * r + lane];
-            sG[c * RT + lane] = g;
-            sG[lane * RT + c] = g;
-          }
-          if (lane == 0) sDead[c] = (int)row;
-          __syncwarp();
-          // entries above the diagonal of column c were built from the old column: redo them
-          if (lane == 0) {
-            for (int i = 0; i < c; ++i) {
-              if (sDead[i] == -2) { sR[i * RT + c] = 0.0; continue; }
-              double t = sG[i * RT + c];
-              for (int l = 0; l < i; ++l) t -= sR[l * RT + i] * sR[l * RT + c];
-              sR[i * RT + c] = t * sDiagInv[i];
-            }
-          }
-          __syncwarp();
-        }
-        __syncwarp();
-        if (piv == 0.0) {
-          // could not be completed: drop the column (its output is zero)
-          if (lane == 0) {
-            sDead[c] = -2;
-            sR[c * RT + c] = 1.0;
-            sDiagInv[c] = 1.0;
-            for (int i = 0; i < c; ++i) sR[i * RT + c] = 0.0;
-          }
-          __syncwarp();
-          continue;  // row c of R stays zero right of the diagonal
-        }
-        if (lane == 0) {
-          sR[c * RT + c] = piv;
-          sDiagInv[c] = inv_piv;
-        }
-        // row c of R, right of the diagonal: one lane per column
-        for (int k = c + 1 + lane; k < r; k += 32) {
-          double t = sG[c * RT + k];
-          for (int i = 0; i < c; ++i) t -= sR[i * RT + c] * sR[i * RT + k];
-          sR[c * RT + k] = t * inv_piv;
-        }
-        __syncwarp();
-      }
-      // inverse of the upper-triangular R, one lane per column
-      for (int c = lane; c < r; c += 32) {
-        for (int i = c; i >= 0; --i) {
-          double t = (i == c) ? 1.0 : 0.0;
-          for (int k = i + 1; k <= c; ++k) t -= sR[i * RT + k] * sRinv[k * RT + c];
-          sRinv[i * RT + c] = t * sDiagInv[i];
-        }
-        if (sDead[c] == -2)
-          for (int i = 0; i <= c; ++i) sRinv[i * RT + c] = 0.0;
-      }
-    }
-    __syncthreads();
-    if (tid < NP) rinv_out[tid] = sRinv[tid];
-    if (tid < RT) dead_out[tid] = sDead[tid];
-    // ---- cross products: C_p = (F_p^T X') R^-1, X' = X with the substituted columns ----------
-    for (int p = 0; p < a.nprev; ++p) {
-      const float* __restrict__ f = a.prev[p] + u.x_off;
-      __syncthreads();
-      if (tid < NP) {
-        const int j = tid / RT, k = tid % RT;
-        double s = 0.0;
-        if (j < r && k < r) {
-          const int d = sDead[k];
-          if (d == -1) {
-            for (int c = 0; c < u.nchunks; ++c) s += __ldcg(unit_part + ((long long)c * stride + 1 + p) * NP + tid);
-          } else if (d >= 0) {
-            s = (double)f[(long long)d * r + j];  // column k of X' is the basis vector e_d
-          }
-        }
-        sG[tid] = s;
-      }
-      __syncthreads();
-      if (tid < NP) {
-        const int j = tid / RT, k = tid % RT;
-        if (j < r && k < r) {
-          double o = 0.0;
-          for (int l = 0; l <= k; ++l) o = fma(sG[j * RT + l], sRinv[l * RT + k], o);
-          a.cmat[p][(long long)u.first_mat * PSGD_CMAT_STRIDE + j * r + k] = (float)o;
-        }
-      }
+#pragma unroll
+      for (int i = c + 1; i < RT; ++i) col[i] = fma(-sR[c * RT + i], v, col[i]);
     }
   }
-  if (tid == 0) a.tickets[ch.unit] = 0;  // ready for the next launch
+  __syncwarp();
+  return ok;
+}
+
+// The same with canonical vectors in the place of columns that are noise: sDead[c] = -1 for a column
+// that stays, the row of the basis vector that replaces it, or -2 for one that could not be
+// completed (its output is zero). Rare (a factor that collapsed), so it is written for clarity.
+template <int RT>
+__device__ __noinline__ void orth_cholesky_substituting(double* sG, double* sR, double* sDiagInv, int* sDead, int r,
+                                                        const float* head, long long len, int lane) {
+  for (int e = lane; e < RT * RT; e += 32) sR[e] = 0.0;
+  __syncwarp();
+  for (int c = 0; c < r; ++c) {
+    int attempt = 0;
+    double piv = 0.0, inv_piv = 0.0;
+    while (true) {
+      double s = sG[c * RT + c];
+      for (int i = 0; i < c; ++i) s -= sR[i * RT + c] * sR[i * RT + c];
+      const double ref = sG[c * RT + c];
+      const bool ok = (ref > 0.0) && (s > 1e-12 * ref);
+      if (ok) { inv_piv = rsqrt(s); piv = s * inv_piv; break; }
+      if (attempt == 2) { piv = 0.0; break; }
+      // substitute column c by the basis vector e_row; its Gram entries are matrix entries
+      const long long row = (attempt == 0 ? c : c + r) % len;
+      ++attempt;
+      __syncwarp();
+      if (lane < r) {
+        double g;
+        if (lane == c) g = 1.0;
+        else if (sDead[lane] >= 0) g = (sDead[lane] == (int)row) ? 1.0 : 0.0;
+        else if (sDead[lane] == -2) g = 0.0;
+        else g = (double)head[row * r + lane];
+        sG[c * RT + lane] = g;
+        sG[lane * RT + c] = g;
+      }
+      if (lane == 0) sDead[c] = (int)row;
+      __syncwarp();
+      // entries above the diagonal of column c were built from the old column: redo them
+      if (lane == 0) {
+        for (int i = 0; i < c; ++i) {
+          if (sDead[i] == -2) { sR[i * RT + c] = 0.0; continue; }
+          double t = sG[i * RT + c];
+          for (int l = 0; l < i; ++l) t -= sR[l * RT + i] * sR[l * RT + c];
+          sR[i * RT + c] = t * sDiagInv[i];
+        }
+      }
+      __syncwarp();
+    }
+    __syncwarp();
+    if (piv == 0.0) {
+      // could not be completed: drop the column (its output is zero)
+      if (lane == 0) {
+        sDead[c] = -2;
+        sR[c * RT + c] = 1.0;
+        sDiagInv[c] = 1.0;
+        for (int i = 0; i < c; ++i) sR[i * RT + c] = 0.0;
+      }
+      __syncwarp();
+      continue;  // row c of R stays zero right of the diagonal
+    }
+    if (lane == 0) {
+      sR[c * RT + c] = piv;
+      sDiagInv[c] = inv_piv;
+    }
+    // row c of R, right of the diagonal: one lane per column
+    for (int k = c + 1 + lane; k < r; k += 32) {
+      double t = sG[c * RT + k];
+      for (int i = 0; i < c; ++i) t -= sR[i * RT + c] * sR[i * RT + k];
+      sR[c * RT + k] = t * inv_piv;
+    }
+    __syncwarp();
+  }
+}
+
+// v <- v R^-1 for one row of RT values (columns beyond r are zero and stay so).
+template <int RT>
+__device__ __forceinline__ void orth_solve_row(double* v, const double* sR, const double* sDiagInv, int r) {
+#pragma unroll
+  for (int k = 0; k < RT; ++k) {
+    if (k < r) {
+      v[k] *= sDiagInv[k];
+#pragma unroll
+      for (int c = k + 1; c < RT; ++c) v[c] = fma(-v[k], sR[k * RT + c], v[c]);
+    }
+  }
+}
+
+// Sum over the unit's chunks, in a fixed order, of the partial matrix at `first` (one every `stride`
+// doubles) into sOut[RT*RT]. Up to eight threads share one entry, each adding every eighth chunk.
+template <int RT>
+__device__ __forceinline__ void orth_sum_chunks(const double* first, long long stride, int nchunks, double* red, double* sOut, int tid) {
+  constexpr int NP = RT * RT;
+  constexpr int PARTS = NP * 8 <= ORTH_THREADS ? 8 : (NP < ORTH_THREADS ? ORTH_THREADS / NP : 1);
+  for (int p = tid; p < NP * PARTS; p += ORTH_THREADS) {
+    const int e = p % NP, part = p / NP;
+    double s = 0.0;
+#pragma unroll 8
+    for (int c = part; c < nchunks; c += PARTS) s += __ldcg(first + c * stride + e);
+    if (PARTS == 1) sOut[e] = s;
+    else red[p] = s;
+  }
+  __syncthreads();
+  if (PARTS > 1) {
+    if (tid < NP) {
+      double s = 0.0;
+#pragma unroll
+      for (int i = 0; i < PARTS; ++i) s += red[i * NP + tid];
+      sOut[tid] = s;
+    }
+    __syncthreads();
+  }
 }
 
 // Second launch: X <- X' R^-1 (rank 1: X / d) on every row chunk, optionally mirrored to copy_to.
@@ -348,74 +392,144 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs 
   const PsgdOrthUnit u = a.units[ch.unit];
   const int r = u.r;
   const int tid = threadIdx.x;
-  float* __restrict__ x = a.x + u.x_off;
-  float* __restrict__ x2 = a.copy_to ? a.copy_to + u.x_off : nullptr;
-  __shared__ double sRinv[NP];
+  __shared__ double sG[NP], sR[NP], sDiagInv[RT], red[ORTH_THREADS];
   __shared__ int sDead[RT];
-  if (tid < NP) sRinv[tid] = a.rinv[(long long)ch.unit * NP + tid];
-  if (tid < RT) sDead[tid] = a.dead[(long long)ch.unit * RT + tid];
-  __syncthreads();
+  float* x = a.x + u.x_off;
+  float* x2 = a.copy_to ? a.copy_to + u.x_off : nullptr;
+  const long long stride = (long long)(1 + a.nprev) * NP;
+  const double* unit_part = a.part + u.chunk0 * stride;
+  const int ci = (int)blockIdx.x - u.chunk0;   // this chunk's number inside its unit
+  psgd_launch_dependents();
+  psgd_wait_for_predecessor();
 
+  orth_sum_chunks<RT>(unit_part, stride, u.nchunks, red, sG, tid);
   if (RT == 1 || r == 1) {
-    const float d = (float)sRinv[0];
+    // joint Frobenius norm of the whole unit, float32 semantics of the division
+    const float d = fmaxf((float)sqrt(sG[0]), 1e-16f);
     for (int i = tid; i < ch.rows; i += ORTH_THREADS) {
       const float v = x[ch.row0 + i] / d;
       x[ch.row0 + i] = v;
       if (x2) x2[ch.row0 + i] = v;
     }
+    // cross products per sub-matrix: (sum of f * x over the sub-matrix) / d; every chunk has its share
+    for (int e = ci * ORTH_THREADS + tid; e < a.nprev * u.nsub; e += u.nchunks * ORTH_THREADS) {
+      const int p = e / u.nsub, s = e % u.nsub;
+      const int per = u.nchunks / u.nsub;   // every sub-matrix has the same number of chunks
+      double t = 0.0;
+#pragma unroll 4
+      for (int c = s * per; c < (s + 1) * per; ++c) t += __ldcg(unit_part + c * stride + (1 + p) * NP);
+      a.cmat[p][(long long)(u.first_mat + s) * PSGD_CMAT_STRIDE] = (float)(t / (double)d);
+    }
     return;
   }
+
+  // the first row's values travel while one warp factorises
+  const bool has = tid < ch.rows;
+  float* xr = x + (long long)(ch.row0 + tid) * r;
+  double v[RT];
+  if (has) orth_load_row<RT>(xr, r, v);
+  if (tid < 32) {
+    if (tid < RT) sDead[tid] = -1;
+    __syncwarp();
+    if (!orth_cholesky<RT>(sG, sR, sDiagInv, r, tid))
+      orth_cholesky_substituting<RT>(sG, sR, sDiagInv, sDead, r, a.head + (long long)ch.unit * 2 * NP, (long long)u.sub_len * u.nsub, tid);
+  }
+  __syncthreads();
   for (int lr = tid; lr < ch.rows; lr += ORTH_THREADS) {
-    const long long row = ch.row0 + lr;
-    float* xr = x + row * r;
-    double xin[RT];
+    const int row = ch.row0 + lr;
+    xr = x + (long long)row * r;
+    if (lr != tid) orth_load_row<RT>(xr, r, v);
 #pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      double v = 0.0;
-      if (k < r) {
-        const int d = sDead[k];
-        v = (d == -1) ? (double)xr[k] : ((d >= 0 && d == (int)row) ? 1.0 : 0.0);
-      }
-      xin[k] = v;
+    for (int k = 0; k < RT; ++k)
+      if (k < r && sDead[k] != -1) v[k] = sDead[k] == row ? 1.0 : 0.0;
+    orth_solve_row<RT>(v, sR, sDiagInv, r);
+    float* xr2 = x2 ? x2 + (long long)row * r : nullptr;
+    if (RT == 4 && r == 4 && (((uintptr_t)xr | (uintptr_t)xr2) & 15u) == 0) {
+      const float4 q = make_float4((float)v[0], (float)v[1 % RT], (float)v[2 % RT], (float)v[3 % RT]);
+      *reinterpret_cast<float4*>(xr) = q;
+      if (xr2) *reinterpret_cast<float4*>(xr2) = q;
+    } else if (RT == 2 && r == 2 && (((uintptr_t)xr | (uintptr_t)xr2) & 7u) == 0) {
+      const float2 q = make_float2((float)v[0], (float)v[1 % RT]);
+      *reinterpret_cast<float2*>(xr) = q;
+      if (xr2) *reinterpret_cast<float2*>(xr2) = q;
+    } else {
+#pragma unroll
+      for (int c = 0; c < RT; ++c)
+        if (c < r) {
+          xr[c] = (float)v[c];
+          if (xr2) xr2[c] = (float)v[c];
+        }
     }
+  }
+  // ---- cross products C_p = (F_p^T X') R^-1, X' = X with the substituted columns: chunk p of the unit
+  //      (modulo their number) has factor p ----
+  for (int p = ci; p < a.nprev; p += u.nchunks) {
+    const float* f = a.prev[p] + u.x_off;
+    __syncthreads();
+    orth_sum_chunks<RT>(unit_part + (long long)(1 + p) * NP, stride, u.nchunks, red, sG, tid);
+    if (tid < r) {
 #pragma unroll
-    for (int c = 0; c < RT; ++c) {
-      if (c < r) {
-        double o = 0.0;
-#pragma unroll
-        for (int k = 0; k <= c; ++k) o = fma(xin[k], sRinv[k * RT + c], o);
-        const float of = (float)o;
-        xr[c] = of;
-        if (x2) x2[row * r + c] = of;
+      for (int k = 0; k < RT; ++k) {
+        double s = 0.0;
+        if (k < r) {
+          const int d = sDead[k];
+          if (d == -1) s = sG[tid * RT + k];
+          else if (d >= 0) s = (double)f[(long long)d * r + tid];  // column k of X' is the basis vector e_d
+        }
+        v[k] = s;
       }
+      orth_solve_row<RT>(v, sR, sDiagInv, r);
+      float* cm = a.cmat[p] + (long long)u.first_mat * PSGD_CMAT_STRIDE + tid * r;
+#pragma unroll
+      for (int k = 0; k < RT; ++k)
+        if (k < r) cm[k] = (float)v[k];
     }
   }
 }
 
 template <int RT>
-static void orth_launch_rt(const OrthArgs& a, int nchunks, cudaStream_t stream) {
-  psgd_orth_gram_kernel<RT><<<nchunks, ORTH_THREADS, 0, stream>>>(a);
-  psgd_orth_apply_kernel<RT><<<nchunks, ORTH_THREADS, 0, stream>>>(a);
+static int orth_launch_rt(const OrthArgs& a, int nchunks, cudaStream_t stream) {
+  const int rc = psgd_launch(psgd_orth_gram_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, 0, a);
+  if (rc != 0) return rc;
+  return psgd_launch(psgd_orth_apply_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, 1, a);
 }
 
 // Template rank used for factors of rank max_r, and the rows of one chunk at that rank.
 PSGD_API int psgd_orth_template_rank(int max_r) {
   return max_r <= 1 ? 1 : max_r <= 2 ? 2 : max_r <= 4 ? 4 : max_r <= 8 ? 8 : max_r <= 16 ? 16 : 32;
 }
-PSGD_API int psgd_orth_chunk_rows(int max_r) { return ORTH_CHUNK_FLOATS / psgd_orth_template_rank(max_r); }
-// Scratch per chunk (doubles) for `nprev` earlier factors; per unit: RT*RT doubles and RT ints.
+// Rows of a chunk when the longest unit has `longest` rows. A short unit takes the base size. Every
+// chunk of the second launch reads the partial matrices of ALL chunks of its unit, so their number
+// is bounded: at the bound the partials are 32 to 400 KB per unit, read in as long as the chunk's own
+// rows take. (An embedding of 50257 rows at rank 16: 66 chunks instead of 393.)
+template <int RT>
+static int orth_chunk_rows(long long longest) {
+  const int base = orth_base_rows<RT>(), most = RT <= 4 ? 256 : RT == 8 ? 128 : RT == 16 ? 80 : 48;
+  const long long rows = (longest + most - 1) / most;
+  return (int)((rows + base - 1) / base > 1 ? (rows + base - 1) / base * base : base);
+}
+PSGD_API int psgd_orth_chunk_rows(int max_r, long long longest) {
+  switch (psgd_orth_template_rank(max_r)) {
+    case 1: return orth_chunk_rows<1>(longest);
+    case 2: return orth_chunk_rows<2>(longest);
+    case 4: return orth_chunk_rows<4>(longest);
+    case 8: return orth_chunk_rows<8>(longest);
+    case 16: return orth_chunk_rows<16>(longest);
+    default: return orth_chunk_rows<32>(longest);
+  }
+}
+// Scratch per chunk (doubles) for `nprev` earlier factors; per unit: 2 * RT*RT floats (`head`).
 PSGD_API int psgd_orth_part_doubles(int max_r, int nprev) {
   const int rt = psgd_orth_template_rank(max_r);
   return (1 + nprev) * rt * rt;
 }
 
 // units / chunks: device tables; all units of one call share the template rank RT >= max r.
-// part: nchunks * psgd_orth_part_doubles(max_r, nprev) doubles; rinv: nunits * RT*RT doubles;
-// dead: nunits * RT ints; tickets: nunits ints, zero (the kernel leaves them zero).
+// part: nchunks * psgd_orth_part_doubles(max_r, nprev) doubles; head: nunits * 2 * RT*RT floats.
 // comm / sum_out: see OrthArgs (null for a single worker or when x already holds the factor).
 PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks, int nchunks, int max_r, float* x,
                               float* copy_to, int nprev, const float* const* prev, float* const* cmat,
-                              double* part, double* rinv, int* dead, int* tickets, const void* comm,
+                              double* part, float* head, const void* comm,
                               float* sum_out, cudaStream_t stream) {
   if (nunits <= 0 || nchunks <= 0) return 0;
   if (max_r > PSGD_MAX_RANK || nprev > PSGD_MAX_HIST) {
@@ -433,9 +547,7 @@ PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks,
     a.cmat[i] = i < nprev ? cmat[i] : nullptr;
   }
   a.part = part;
-  a.rinv = rinv;
-  a.dead = dead;
-  a.tickets = tickets;
+  a.head = head;
   a.comm = (const PsgdCommDev*)comm;
   a.sum_out = sum_out;
   if (comm != nullptr && sum_out == nullptr) {
@@ -443,15 +555,13 @@ PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks,
     return -1;
   }
   switch (psgd_orth_template_rank(max_r)) {
-    case 1: orth_launch_rt<1>(a, nchunks, stream); break;
-    case 2: orth_launch_rt<2>(a, nchunks, stream); break;
-    case 4: orth_launch_rt<4>(a, nchunks, stream); break;
-    case 8: orth_launch_rt<8>(a, nchunks, stream); break;
-    case 16: orth_launch_rt<16>(a, nchunks, stream); break;
-    default: orth_launch_rt<32>(a, nchunks, stream); break;
+    case 1: return orth_launch_rt<1>(a, nchunks, stream);
+    case 2: return orth_launch_rt<2>(a, nchunks, stream);
+    case 4: return orth_launch_rt<4>(a, nchunks, stream);
+    case 8: return orth_launch_rt<8>(a, nchunks, stream);
+    case 16: return orth_launch_rt<16>(a, nchunks, stream);
+    default: return orth_launch_rt<32>(a, nchunks, stream);
   }
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
 }
 
 #ifdef PSGD_BOUNDS_CHECK

@@ -50,4 +50,38 @@ __device__ __forceinline__ int psgd_atom_add_acqrel_gpu(int* p, int v) {
   return old;
 }
 
+// ---- launches that overlap the end of their predecessor ----------------------------------------
+// A chain of short launches pays for each start: the grid is set up, descriptors are fetched, the
+// first loads take their latency. With programmatic dependent launch a kernel may start while its
+// predecessor in the stream still runs: the predecessor says so (psgd_launch_dependents, at its
+// very beginning here), and the successor does what does not depend on any launch of the chain
+// before it waits (psgd_wait_for_predecessor) for the predecessor to COMPLETE, memory included.
+// Every kernel launched with `early` != 0 executes that wait in every thread before it reads or
+// writes anything another launch of the chain writes; so completion stays transitive, and the
+// launch that opens a chain (`early` == 0) still waits for everything before it.
+__device__ __forceinline__ void psgd_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void psgd_wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Asks for the 128-byte line of L2 that holds *p. Only for addresses inside live allocations.
+__device__ __forceinline__ void psgd_prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// `early` != 0: the kernel contains the wait above and the launch directly before it in `stream` is
+// one of this library's.
+template <typename... Params, typename... Args>
+static inline int psgd_launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int early,
+                              Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  PSGD_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+  return 0;
+}
+
 static inline int psgd_ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -299,20 +299,19 @@ class NativeCompressor:
         self.h_loc = [torch.zeros(cap, **f32) for _ in range(self.T)]
         self.h_sum = [torch.zeros(cap, **f32) for _ in range(self.T)]
         self.cmat = [[torch.zeros(nm * layout.CMAT_STRIDE, **f32) for _ in range(t)] for t in range(self.T)]
-        chunk_rows = int(self.lib.psgd_orth_chunk_rows(self.tiles.max_r))
         rt = int(self.lib.psgd_orth_template_rank(self.tiles.max_r))
         self.units, self.chunks, self.n_units, self.n_chunks = {}, {}, {}, {}
         for s in ("p", "q"):
-            units, chunks = self.tiles.orth_units(s, chunk_rows)
+            longest = max(((g.n if s == "p" else g.m) * (g.batch if g.r == 1 else 1) for g in self.plan.groups), default=1)
+            units, chunks = self.tiles.orth_units(s, int(self.lib.psgd_orth_chunk_rows(self.tiles.max_r, longest)))
             self.units[s], self.chunks[s] = _to_device(units, self.device), _to_device(chunks, self.device)
             self.n_units[s], self.n_chunks[s] = len(units), len(chunks)
-        # scratch of the orthonormalisation: partial sums per chunk, R^-1 / column status / ticket per unit
+        # scratch of the orthonormalisation: partial sums per chunk; per unit the leading rows that its
+        # factor R falls back on when a column has to be replaced
         part_doubles = int(self.lib.psgd_orth_part_doubles(self.tiles.max_r, max(self.T - 1, 0)))
         max_units = max(max(self.n_units.values()), 1)
         self._orth_part = torch.zeros(max(max(self.n_chunks.values()), 1) * part_doubles, device=self.device, dtype=torch.float64)
-        self._orth_rinv = torch.zeros(max_units * rt * rt, device=self.device, dtype=torch.float64)
-        self._orth_dead = torch.zeros(max_units * rt, device=self.device, dtype=torch.int32)
-        self._orth_tickets = torch.zeros(max_units, device=self.device, dtype=torch.int32)
+        self._orth_rinv = torch.zeros(max_units * 2 * rt * rt, device=self.device, dtype=torch.float32)
         self._key = None
         self._out_arena: Optional[torch.Tensor] = None
         self._hyper_dev = _to_device(self._default_hyper(), self.device)
@@ -515,14 +514,12 @@ class NativeCompressor:
             ctypes.cast(_ptr_array(cm), ctypes.c_void_p),
             _ptr(self._orth_part),
             _ptr(self._orth_rinv),
-            _ptr(self._orth_dead),
-            _ptr(self._orth_tickets),
             self.comm.ptr if gather_to is not None else ctypes.c_void_p(0),
             _ptr(gather_to),
             _stream_ptr(),
         )
         native.check(code, "psgd_orth_launch")
-        self.launches += 2  # Gram + factorisation, then the application of R^-1
+        self.launches += 2  # partial Gram matrices, then factorisation + application of R^-1
 
     def _gemm(self, transposed: bool, fin: torch.Tensor, fout: torch.Tensor, corr_fac, corr_c,
               fout2: Optional[torch.Tensor] = None, part: str = "all"):
