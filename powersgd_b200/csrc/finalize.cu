@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(FIN_THREADS) psgd_finalize_kernel(FinalizeArgs
   __shared__ __align__(16) float sLs[FIN_KC][FIN_ROWS];
   __shared__ __align__(16) float sRl[FIN_KC][FIN_COLS];
   __shared__ __align__(16) float sRs[FIN_KC][FIN_COLS];
+  psgd_wait_for_predecessor();
   const PsgdTile whole = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[whole.mat];
   if (whole.vec == 4) finalize_general_tile<4, SAME>(a, whole, mt, sLl, sLs, sRl, sRs);
@@ -283,6 +284,41 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
     if (!ok) return;
   }
 #endif
+  const PsgdHyper hy = a.hyper[mt.hyper];
+  const bool sgd = a.fused_sgd != 0;
+  const bool mom = sgd && hy.has_momentum;
+  const bool global_res = (a.flags & 1) != 0;
+  float* const res_base = (a.flags & 2) ? mt.param : mt.grad;
+
+  // Global loads of a chunk of 32 rows; the rows of the chunk after it are asked into L2, so that
+  // their loads, which the registers have no room for yet, find them there.
+  __align__(16) float g4[4][4], p4[4][4], m4[4][4];
+  auto load = [&](int rc) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int lr = rc + warp * 4 + u;
+      const long long rowoff = (long long)(t.row0 + lr) * m + t.col0;
+#pragma unroll
+      for (int c4 = 0; c4 < 4; ++c4) g4[u][c4] = p4[u][c4] = m4[u][c4] = 0.f;
+      if (lr < t.rows) {
+        fin_load4<VEC>(mt.grad + rowoff, lane, t.cols, g4[u]);
+        if (sgd) fin_load4<VEC>(mt.param + rowoff, lane, t.cols, p4[u]);
+        if (mom) fin_load4<VEC>(mt.mom + rowoff, lane, t.cols, m4[u]);
+      }
+    }
+    const int next = rc + FIN_ROWS + warp * 4 + (lane >> 2), col = (lane & 3) * 32;
+    if (lane < 16 && next < t.rows && col < t.cols) {
+      const long long off = (long long)(t.row0 + next) * m + t.col0 + col;
+      psgd_prefetch_l2(mt.grad + off);
+      if (sgd) psgd_prefetch_l2(mt.param + off);
+      if (mom) psgd_prefetch_l2(mt.mom + off);
+    }
+  };
+  // gradients, parameters and momentum are written by no other launch of the chain: the first chunk
+  // is loaded ahead of the wait for the last product (with two accumulators the staging code that
+  // follows has no registers left for it, and several workers do not overlap launches)
+  if (SAME) load(0);
+  psgd_wait_for_predecessor();
   const bool gather = !SAME && a.comm != nullptr;
   int e1 = 0;
   bool ok = true;
@@ -337,29 +373,9 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   }
   if (gather) psgd_comm_close_epoch(*a.comm, e1);  // (CTA barrier inside) this strip has read its words
   __syncthreads();
-  const PsgdHyper hy = a.hyper[mt.hyper];
-  const bool sgd = a.fused_sgd != 0;
-  const bool mom = sgd && hy.has_momentum;
-  const bool global_res = (a.flags & 1) != 0;
-  float* const res_base = (a.flags & 2) ? mt.param : mt.grad;
 
   for (int rc = 0; rc < t.rows; rc += FIN_ROWS) {
-    // ---- global loads of this chunk first ----
-    __align__(16) float g4[4][4], p4[4][4], m4[4][4];
-    bool live[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int lr = rc + warp * 4 + u;
-      const long long rowoff = (long long)(t.row0 + lr) * m + t.col0;
-#pragma unroll
-      for (int c4 = 0; c4 < 4; ++c4) g4[u][c4] = p4[u][c4] = m4[u][c4] = 0.f;
-      live[u] = lr < t.rows;
-      if (live[u]) {
-        fin_load4<VEC>(mt.grad + rowoff, lane, t.cols, g4[u]);
-        if (sgd) fin_load4<VEC>(mt.param + rowoff, lane, t.cols, p4[u]);
-        if (mom) fin_load4<VEC>(mt.mom + rowoff, lane, t.cols, m4[u]);
-      }
-    }
+    if (rc || !SAME) load(rc);
     // ---- rank-K update from the staged panels ----
     float accE[4][4], accA[4][4];
 #pragma unroll
@@ -392,8 +408,8 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
     // ---- residual, mean update, optimizer ----
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (!live[u]) continue;
       const int lr = rc + warp * 4 + u;
+      if (lr >= t.rows) continue;
       const long long rowoff = (long long)(t.row0 + lr) * m + t.col0;
       __align__(16) float av[4];
 #pragma unroll
@@ -431,7 +447,7 @@ constexpr int FIN_SMEM_DEFAULT = 48 * 1024;
 constexpr int FIN_SMEM_OPT_IN = 96 * 1024;
 
 template <bool SAME>
-static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, cudaStream_t stream) {
+static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, int early, cudaStream_t stream) {
   const size_t smem = (size_t)(SAME ? 1 : 2) * kmax * (FIN_COLS + tile_rows) * sizeof(float);
   if (smem > (size_t)FIN_SMEM_DEFAULT) {
     static bool opted_in = false;   // per instantiation
@@ -440,8 +456,7 @@ static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_row
       opted_in = true;
     }
   }
-  psgd_finalize_strip_kernel<SAME><<<ntiles, FIN_THREADS, smem, stream>>>(a, tile_rows);
-  return 0;
+  return psgd_launch(psgd_finalize_strip_kernel<SAME>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
 }
 
 // Tallest strip (multiple of 32 rows, at most 256) whose panels fit the shared-memory budget.
@@ -470,12 +485,12 @@ PSGD_API int psgd_finalize_uses_strip(int nhist, int max_r, int tile_rows, int s
 // matrix in `mats`. With nhist * max_r <= 32 and panels that fit shared memory the strip kernel
 // runs, else the general one. Every tile carries its matrix's access width (`vec`).
 // comm / poll_left / sum_out1 / sum_out2 / flags / sum_scale: see FinalizeArgs (comm null: nothing
-// is gathered; flags 0 and sum_scale 1 for the library's own step).
+// is gathered; flags 0 and sum_scale 1 for the library's own step). early: see psgd_launch.
 PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntiles, int tile_rows, int max_r,
                                   const void* hyper, int nhist, const float* const* lloc, const float* const* rloc,
                                   const float* const* lsum, const float* const* rsum, float inv_world,
                                   int fused_sgd, const void* comm, int poll_left, float* sum_out1, float* sum_out2,
-                                  int flags, float sum_scale, cudaStream_t stream) {
+                                  int flags, float sum_scale, int early, cudaStream_t stream) {
   if (ntiles <= 0) return 0;
   if (tile_rows <= 0 || tile_rows % FIN_ROWS != 0 || max_r <= 0) {
     psgd_set_error("psgd_finalize_launch: tile_rows=%d must be a positive multiple of %d, max_r=%d positive", tile_rows, FIN_ROWS, max_r);
@@ -517,14 +532,10 @@ PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntile
   }
   if (strip) {
     const int kmax = nhist * max_r;
-    if (same) finalize_strip_launch<true>(a, ntiles, tile_rows, kmax, stream);
-    else finalize_strip_launch<false>(a, ntiles, tile_rows, kmax, stream);
-  } else {
-    if (same) psgd_finalize_kernel<true><<<ntiles, FIN_THREADS, 0, stream>>>(a);
-    else psgd_finalize_kernel<false><<<ntiles, FIN_THREADS, 0, stream>>>(a);
+    return same ? finalize_strip_launch<true>(a, ntiles, tile_rows, kmax, early, stream)
+                : finalize_strip_launch<false>(a, ntiles, tile_rows, kmax, early, stream);
   }
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
+  return psgd_launch(same ? psgd_finalize_kernel<true> : psgd_finalize_kernel<false>, ntiles, FIN_THREADS, 0, stream, early, a);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -630,6 +641,7 @@ __global__ void __launch_bounds__(FLAT_THREADS) psgd_flat_kernel(FlatArgs a) {
     }
   }
   if (uses_comm && mode >= 6) psgd_comm_close_epoch(c, e1);  // the last consumer CTA advances the channel
+  psgd_wait_for_predecessor();
 }
 
 // Streaming variant of the modes that move whole buffers (0-4, 12, 13): four elements per access.
@@ -750,22 +762,25 @@ __global__ void __launch_bounds__(FLAT_THREADS) psgd_flat_vec_kernel(FlatArgs a)
     }
   }
   if (MODE >= 12) psgd_comm_close_epoch(c, e1);
+  psgd_wait_for_predecessor();  // nothing above depends on it; whoever waits for this launch waits for that one too
 }
 
 PSGD_API int psgd_flat_block_elems() { return FLAT_PER_BLOCK; }
 
 template <int MODE>
-static void flat_vec_launch(const FlatArgs& a, int nblocks, cudaStream_t stream) {
-  psgd_flat_vec_kernel<MODE><<<nblocks, FLAT_THREADS, 0, stream>>>(a);
+static int flat_vec_launch(const FlatArgs& a, int nblocks, int early, cudaStream_t stream) {
+  return psgd_launch(psgd_flat_vec_kernel<MODE>, nblocks, FLAT_THREADS, 0, stream, early, a);
 }
 
 // vec != 0 promises 16-byte aligned grad / param / mom / out pointers and flat offsets that are
 // multiples of four floats; modes 5-7 (flag-in-data words) always run element-wise, and so do the
 // op-5 items of a mixed launch (mode 9), whose pointers need no alignment.
+// early (local modes 3, 4 and 8 only; else 0): the launch directly before this one in `stream` is one of
+// this library's and touches none of the listed tensors (see psgd_launch).
 // keep != 0: the packing modes (0, 3, 4, 5 and the op-5 items of mode 9) leave their inputs untouched.
 PSGD_API int psgd_flat_launch(int mode, int vec, const void* items, const int* block_item, const int* block_first,
                               int nblocks, const void* hyper, float* flat, float divisor, const void* comm,
-                              long long n_pad, int keep, cudaStream_t stream) {
+                              long long n_pad, int keep, int early, cudaStream_t stream) {
   if (nblocks <= 0) return 0;
   if (mode >= 5 && mode != 8 && comm == nullptr) {
     psgd_set_error("psgd_flat_launch: mode %d needs a communication channel", mode);
@@ -773,6 +788,10 @@ PSGD_API int psgd_flat_launch(int mode, int vec, const void* items, const int* b
   }
   if (!((mode >= 0 && mode <= 9) || mode == 12 || mode == 13)) {
     psgd_set_error("psgd_flat_launch: unknown mode %d", mode);
+    return -1;
+  }
+  if (early && mode != 3 && mode != 4 && mode != 8) {
+    psgd_set_error("psgd_flat_launch: mode %d cannot overlap its predecessor", mode);
     return -1;
   }
   FlatArgs a;
@@ -788,21 +807,18 @@ PSGD_API int psgd_flat_launch(int mode, int vec, const void* items, const int* b
   a.keep = keep;
   if (vec && !(mode >= 5 && mode <= 7)) {
     switch (mode) {
-      case 0: flat_vec_launch<0>(a, nblocks, stream); break;
-      case 1: flat_vec_launch<1>(a, nblocks, stream); break;
-      case 2: flat_vec_launch<2>(a, nblocks, stream); break;
-      case 3: flat_vec_launch<3>(a, nblocks, stream); break;
-      case 4: flat_vec_launch<4>(a, nblocks, stream); break;
-      case 8: flat_vec_launch<8>(a, nblocks, stream); break;
-      case 9: flat_vec_launch<9>(a, nblocks, stream); break;
-      case 12: flat_vec_launch<12>(a, nblocks, stream); break;
-      default: flat_vec_launch<13>(a, nblocks, stream); break;
+      case 0: return flat_vec_launch<0>(a, nblocks, early, stream);
+      case 1: return flat_vec_launch<1>(a, nblocks, early, stream);
+      case 2: return flat_vec_launch<2>(a, nblocks, early, stream);
+      case 3: return flat_vec_launch<3>(a, nblocks, early, stream);
+      case 4: return flat_vec_launch<4>(a, nblocks, early, stream);
+      case 8: return flat_vec_launch<8>(a, nblocks, early, stream);
+      case 9: return flat_vec_launch<9>(a, nblocks, early, stream);
+      case 12: return flat_vec_launch<12>(a, nblocks, early, stream);
+      default: return flat_vec_launch<13>(a, nblocks, early, stream);
     }
-  } else {
-    psgd_flat_kernel<<<nblocks, FLAT_THREADS, 0, stream>>>(a);
   }
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
+  return psgd_launch(psgd_flat_kernel, nblocks, FLAT_THREADS, 0, stream, early, a);
 }
 
 #ifdef PSGD_BOUNDS_CHECK

@@ -74,6 +74,12 @@ __device__ __forceinline__ bool product_tile_ok(const PsgdTile& t, const PsgdMat
 
 template <int RT>
 __host__ __device__ constexpr int nt_max_rows() { return RT <= 16 ? NT_MAX_ROWS : NT_MAX_ROWS / 2; }
+// Staging buffer of an NT tile: rows of P-hat, later (up to rank 8, 32 KiB) one sum per warp, so that
+// the warps' sums are added by all threads at once instead of one warp after another.
+template <int RT>
+__host__ __device__ constexpr int nt_stage_floats() {
+  return RT <= 8 && GEMM_WARPS * NT_TILE_COLS > nt_max_rows<RT>() ? GEMM_WARPS * NT_TILE_COLS * RT : nt_max_rows<RT>() * RT;
+}
 
 // A lane owns 4 of the 128 columns of a column block; which ones depends on the access width:
 // 4 adjacent (one 16-byte load), 2 + 2 adjacent (two 8-byte loads, 64 columns apart) or 4
@@ -131,8 +137,8 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   const int r = mt.r, m = mt.m;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-  float* sP = smem;                        // [rows][RT]
-  float* sSum = smem + nt_max_rows<RT>() * RT;   // [128][RT]
+  float* sP = smem;                        // [rows][RT], then the warps' sums [GEMM_WARPS][128][RT] (RT <= 8)
+  float* sSum = smem + nt_stage_floats<RT>();   // [128][RT]
   __shared__ int sLast;
 #ifdef PSGD_BOUNDS_CHECK
   if (!product_tile_ok<RT>(t, mt, 1, 1 << 30, NT_TILE_COLS, NT_TILE_COLS * RT)) return;
@@ -147,31 +153,51 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   const float* __restrict__ M = mt.grad;
   const int cend = t.col0 + t.cols;
   constexpr int MAXR = nt_max_rows<RT>();
+  constexpr int UR = 4;                       // rows of a warp in flight
+  constexpr int STEP = GEMM_WARPS * UR;
+
+  // The gradient does not depend on the launches before this one: the tile's first rows are loaded
+  // and the rest is asked into L2 while the basis is still being orthonormalised.
+  float v[UR][4];
+  auto load = [&](int row0, int rows, int i0) {
+#pragma unroll
+    for (int u = 0; u < UR; ++u) {
+      const int i = i0 + u * GEMM_WARPS;
+      const bool rok = i < rows;
+      load_lane_cols<VEC>(M + (long long)(row0 + (rok ? i : 0)) * m, t.col0, cend, lane, rok, v[u]);
+    }
+  };
+  load(t.row0, min(MAXR, t.rows), warp);
+  for (int e = tid + 4 * STEP; e < 4 * min(MAXR, t.rows); e += GEMM_THREADS)   // four lines of 128 bytes per row
+    if ((e & 3) * 32 < t.cols) psgd_prefetch_l2(M + (long long)(t.row0 + (e >> 2)) * m + t.col0 + (e & 3) * 32);
+  psgd_wait_for_predecessor();
 
   // a tall tile is walked in chunks of MAXR rows (what fits the staging buffer of P-hat); the
   // accumulators live across chunks, so a matrix with tens of thousands of rows needs tens of
   // partial tiles per column block, not hundreds
   for (int rb = 0; rb < t.rows; rb += MAXR) {
     const int rows = min(MAXR, t.rows - rb);
-    if (rb) __syncthreads();  // the previous chunk's rows of P-hat are no longer read
+    if (rb) {
+      load(t.row0 + rb, rows, warp);
+      __syncthreads();  // the previous chunk's rows of P-hat are no longer read
+    }
     // stage the chunk's rows of P-hat (zero padded to RT columns)
-    const float* __restrict__ pin = a.in + mt.p_off + (long long)(t.row0 + rb) * r;
+    const float* pin = a.in + mt.p_off + (long long)(t.row0 + rb) * r;
     for (int e = tid; e < rows * RT; e += GEMM_THREADS) {
       const int row = e / RT, k = e % RT;
       sP[e] = (k < r) ? pin[row * r + k] : 0.f;
     }
     __syncthreads();
 
-    for (int i0 = warp; i0 < rows; i0 += GEMM_WARPS * 4) {
-      float v[4][4];
+    for (int i0 = warp; i0 < rows; i0 += STEP) {
+      float cur[UR][4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * GEMM_WARPS;
-        const bool rok = i < rows;
-        load_lane_cols<VEC>(M + (long long)(t.row0 + rb + (rok ? i : 0)) * m, t.col0, cend, lane, rok, v[u]);
-      }
+      for (int u = 0; u < UR; ++u)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+        for (int c = 0; c < 4; ++c) cur[u][c] = v[u][c];
+      if (i0 + STEP < rows) load(t.row0 + rb, rows, i0 + STEP);  // the next rows travel while these are used
+#pragma unroll
+      for (int u = 0; u < UR; ++u) {
         const int i = i0 + u * GEMM_WARPS;
         if (i < rows) {
           const float* pr = sP + i * RT;
@@ -179,7 +205,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
           for (int k = 0; k < RT; ++k) {
             const float pk = pr[k];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[c][k] = fmaf(v[u][c], pk, acc[c][k]);
+            for (int c = 0; c < 4; ++c) acc[c][k] = fmaf(cur[u][c], pk, acc[c][k]);
           }
         }
       }
@@ -187,20 +213,36 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   }
   __syncthreads();
 
-  // deterministic cross-warp sum: warps add in index order
-  for (int w = 0; w < GEMM_WARPS; ++w) {
-    if (warp == w) {
+  // deterministic cross-warp sum: warps are added in index order
+  if (RT <= 8) {
+    float* mine = sP + warp * NT_TILE_COLS * RT;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int lc = lane_col<VEC>(lane, c);
+    for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int k = 0; k < RT; ++k) {
-          if (w == 0) sSum[lc * RT + k] = acc[c][k];
-          else sSum[lc * RT + k] += acc[c][k];
-        }
-      }
+      for (int k = 0; k < RT; ++k) mine[lane_col<VEC>(lane, c) * RT + k] = acc[c][k];
+    __syncthreads();
+    for (int e = tid; e < NT_TILE_COLS * RT; e += GEMM_THREADS) {
+      float s = sP[e];
+#pragma unroll
+      for (int w = 1; w < GEMM_WARPS; ++w) s += sP[w * NT_TILE_COLS * RT + e];
+      sSum[e] = s;
     }
     __syncthreads();
+  } else {
+    for (int w = 0; w < GEMM_WARPS; ++w) {
+      if (warp == w) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int lc = lane_col<VEC>(lane, c);
+#pragma unroll
+          for (int k = 0; k < RT; ++k) {
+            if (w == 0) sSum[lc * RT + k] = acc[c][k];
+            else sSum[lc * RT + k] += acc[c][k];
+          }
+        }
+      }
+      __syncthreads();
+    }
   }
 
   const int tile_elems = NT_TILE_COLS * RT;
@@ -252,6 +294,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
 template <int RT>
 __global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nt_kernel(GemmArgs a) {
   extern __shared__ float smem[];
+  psgd_launch_dependents();
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
   if (t.vec == 4) gemm_nt_tile<RT, 4>(a, t, mt, smem);
@@ -273,7 +316,7 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
 #endif
 
   const float* __restrict__ M = mt.grad;
-  const float* __restrict__ qin = a.in + mt.q_off;
+  const float* qin = a.in + mt.q_off;   // written by the launch before: plain loads, after the wait
 
   float acc[RPW][RT];
 #pragma unroll
@@ -291,10 +334,25 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
   }
 
   const int cend = t.col0 + t.cols;
-  for (int c0 = t.col0; c0 < cend; c0 += NN_CHUNK_COLS) {
-    float v[RPW][4];
+  // as in the NT tile: first loads and L2 prefetch ahead of the wait, then always one chunk ahead
+  float v[RPW][4];
 #pragma unroll
-    for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], c0, cend, lane, rok[u], v[u]);
+  for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], t.col0, cend, lane, rok[u], v[u]);
+#pragma unroll
+  for (int u = 0; u < RPW; ++u)
+    if (rok[u])
+      for (int c = t.col0 + NN_CHUNK_COLS + lane * 32; c < cend; c += 32 * 32) psgd_prefetch_l2(rowp[u] + c);
+  psgd_wait_for_predecessor();
+  for (int c0 = t.col0; c0 < cend; c0 += NN_CHUNK_COLS) {
+    float cur[RPW][4];
+#pragma unroll
+    for (int u = 0; u < RPW; ++u)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) cur[u][c] = v[u][c];
+    if (c0 + NN_CHUNK_COLS < cend) {
+#pragma unroll
+      for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], c0 + NN_CHUNK_COLS, cend, lane, rok[u], v[u]);
+    }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int col = c0 + lane_col<VEC>(lane, c);
@@ -302,9 +360,9 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
         const float* qr = qin + (long long)col * r;
 #pragma unroll
         for (int k = 0; k < RT; ++k) {
-          const float qk = (k < r) ? __ldg(qr + k) : 0.f;
+          const float qk = (k < r) ? qr[k] : 0.f;
 #pragma unroll
-          for (int u = 0; u < RPW; ++u) acc[u][k] = fmaf(v[u][c], qk, acc[u][k]);
+          for (int u = 0; u < RPW; ++u) acc[u][k] = fmaf(cur[u][c], qk, acc[u][k]);
         }
       }
     }
@@ -367,6 +425,7 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
 template <int RT, int RPW>
 __global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nn_kernel(GemmArgs a) {
   __shared__ float sSum[GEMM_WARPS * RPW * RT];
+  psgd_launch_dependents();
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
   if (t.vec == 4) gemm_nn_tile<RT, 4, RPW>(a, t, mt, sSum);
@@ -396,33 +455,29 @@ static void fill_args(GemmArgs& a, const void* mats, const void* tiles, const fl
 }
 
 template <int RT>
-static int launch_nt(const GemmArgs& a, int ntiles, cudaStream_t stream) {
-  const size_t smem = (size_t)(nt_max_rows<RT>() * RT + NT_TILE_COLS * RT) * sizeof(float);
+static int launch_nt(const GemmArgs& a, int ntiles, int early, cudaStream_t stream) {
+  const size_t smem = (size_t)(nt_stage_floats<RT>() + NT_TILE_COLS * RT) * sizeof(float);
   static bool configured = false;
   if (!configured && smem > 48 * 1024) {
     PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_gemm_nt_kernel<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  psgd_gemm_nt_kernel<RT><<<ntiles, GEMM_THREADS, smem, stream>>>(a);
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
+  return psgd_launch(psgd_gemm_nt_kernel<RT>, ntiles, GEMM_THREADS, smem, stream, early, a);
 }
 
 template <int RT>
-static int launch_nn(const GemmArgs& a, int ntiles, cudaStream_t stream) {
+static int launch_nn(const GemmArgs& a, int ntiles, int early, cudaStream_t stream) {
   constexpr int RPW = RT <= 8 ? 4 : (RT == 16 ? 2 : 1);
-  psgd_gemm_nn_kernel<RT, RPW><<<ntiles, GEMM_THREADS, 0, stream>>>(a);
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
+  return psgd_launch(psgd_gemm_nn_kernel<RT, RPW>, ntiles, GEMM_THREADS, 0, stream, early, a);
 }
 
 #define PSGD_DISPATCH_RT(FN)                                   \
-  if (max_r <= 1) return FN<1>(a, ntiles, stream);             \
-  if (max_r <= 2) return FN<2>(a, ntiles, stream);             \
-  if (max_r <= 4) return FN<4>(a, ntiles, stream);             \
-  if (max_r <= 8) return FN<8>(a, ntiles, stream);             \
-  if (max_r <= 16) return FN<16>(a, ntiles, stream);           \
-  return FN<32>(a, ntiles, stream);
+  if (max_r <= 1) return FN<1>(a, ntiles, early, stream);             \
+  if (max_r <= 2) return FN<2>(a, ntiles, early, stream);             \
+  if (max_r <= 4) return FN<4>(a, ntiles, early, stream);             \
+  if (max_r <= 8) return FN<8>(a, ntiles, early, stream);             \
+  if (max_r <= 16) return FN<16>(a, ntiles, early, stream);           \
+  return FN<32>(a, ntiles, early, stream);
 
 // Rows handled by one NN tile for the template rank that `max_r` selects (the planner needs it).
 PSGD_API int psgd_gemm_nn_tile_rows(int max_r) {
@@ -434,7 +489,8 @@ PSGD_API int psgd_gemm_template_rank(int max_r) {
   return max_r <= 1 ? 1 : max_r <= 2 ? 2 : max_r <= 4 ? 4 : max_r <= 8 ? 8 : max_r <= 16 ? 16 : 32;
 }
 
-// `transposed` != 0: NT (Q = M^T P); else NN (P = M Q). Every tile carries the access width of
+// `transposed` bit 0: NT (Q = M^T P), else NN (P = M Q); bit 1: the launch directly before this one in
+// `stream` is one of this library's that leaves the gradients alone (see psgd_launch). Every tile carries the access width of
 // its matrix (`vec`: 4 needs a 16-byte aligned base and m % 4 == 0; 2 an 8-byte aligned base and
 // an even m). `out2`, when not null, receives a second copy of the fresh factor.
 PSGD_API int psgd_gemm_ffma_launch(int transposed, int max_r, const void* mats, const void* tiles, int ntiles,
@@ -448,7 +504,8 @@ PSGD_API int psgd_gemm_ffma_launch(int transposed, int max_r, const void* mats, 
   }
   GemmArgs a;
   fill_args(a, mats, tiles, in, out, out2, ncorr, corr_fac, corr_c, partial, tickets, comm);
-  if (transposed) { PSGD_DISPATCH_RT(launch_nt) }
+  const int early = (transposed >> 1) & 1;
+  if (transposed & 1) { PSGD_DISPATCH_RT(launch_nt) }
   PSGD_DISPATCH_RT(launch_nn)
 }
 

@@ -230,6 +230,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_tmem;
   volatile int* abort_flag = &s_abort;
+  // Every CTA of this grid holds its tensor memory now, so a successor that starts early can only
+  // wait for it, never the other way round. The producer warp reads nothing but the gradient, which
+  // no launch of the chain before this one writes: it fills the ring while the basis is still being
+  // orthonormalised. Everybody else waits for that.
+  psgd_launch_dependents();
+  if (warp != 4) psgd_wait_for_predecessor();
   // warps 0-3: running FP32 sum of the finished segments of accumulator row (warp * 32 + lane)
   float sum[N2];
 #pragma unroll
@@ -270,6 +276,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
         }
       }
     }
+    psgd_wait_for_predecessor();   // this warp takes part in the epilogue
   } else if (warp == 5) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
@@ -309,7 +316,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
   } else {
     // ---------------- converters (then epilogue) ----------------
     const int ctid = warp < 4 ? tid : tid - 64;   // index among the converter threads
-    const float* __restrict__ fac = a.in + (TRANSPOSED ? mt.p_off : mt.q_off);
+    const float* fac = a.in + (TRANSPOSED ? mt.p_off : mt.q_off);   // written by the launch before: plain loads
     // each thread stages RP / 4 factor values per stage; they are fetched one stage ahead so
     // that their L2 latency hides behind the wait for the gradient tile
     constexpr int PER_THREAD = TC_BK * RP / TC_NCONV;
@@ -321,7 +328,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
         const int e = ctid + i * TC_NCONV;
         const int k = e / RP, n = e % RP;
         float v = 0.f;
-        if (kb < nk && n < r && k0 + k < k_limit && kb * TC_BK + k < k_len) v = __ldg(fac + (long long)(k0 + k) * r + n);
+        if (kb < nk && n < r && k0 + k < k_limit && kb * TC_BK + k < k_len) v = fac[(long long)(k0 + k) * r + n];
         pre[i] = v;
       }
     };
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
 }
 
 template <bool TRANSPOSED, int RP, bool SPLIT>
-int launch_tc(const TcArgs& a, int ntiles, cudaStream_t stream) {
+int launch_tc(const TcArgs& a, int ntiles, int early, cudaStream_t stream) {
   constexpr int N2 = ((SPLIT ? 2 : 1) * RP) < 16 ? 16 : ((SPLIT ? 2 : 1) * RP);
   const size_t smem = 1024 + (size_t)TC_STAGES * TC_A_BYTES + (size_t)TC_OP_STAGES * ((SPLIT ? TC_A_BYTES : 0) + N2 * 128);
   static bool configured = false;
@@ -450,16 +457,14 @@ int launch_tc(const TcArgs& a, int ntiles, cudaStream_t stream) {
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  psgd_gemm_tc_kernel<TRANSPOSED, RP, SPLIT><<<ntiles, TC_THREADS, smem, stream>>>(a);
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
+  return psgd_launch(psgd_gemm_tc_kernel<TRANSPOSED, RP, SPLIT>, ntiles, TC_THREADS, smem, stream, early, a);
 }
 
 template <bool TRANSPOSED, bool SPLIT>
-int dispatch_rank(const TcArgs& a, int max_r, int ntiles, cudaStream_t stream) {
-  if (max_r <= 8) return launch_tc<TRANSPOSED, 8, SPLIT>(a, ntiles, stream);
-  if (max_r <= 16) return launch_tc<TRANSPOSED, 16, SPLIT>(a, ntiles, stream);
-  return launch_tc<TRANSPOSED, 32, SPLIT>(a, ntiles, stream);
+int dispatch_rank(const TcArgs& a, int max_r, int ntiles, int early, cudaStream_t stream) {
+  if (max_r <= 8) return launch_tc<TRANSPOSED, 8, SPLIT>(a, ntiles, early, stream);
+  if (max_r <= 16) return launch_tc<TRANSPOSED, 16, SPLIT>(a, ntiles, early, stream);
+  return launch_tc<TRANSPOSED, 32, SPLIT>(a, ntiles, early, stream);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -517,7 +522,7 @@ PSGD_API int psgd_tma_encode_matrix(void* out, const float* base, int n, int m) 
   return 0;
 }
 
-// Same contract as psgd_gemm_ffma_launch; `maps` is a device array of tensor maps indexed like
+// Same contract as psgd_gemm_ffma_launch (both bits of `transposed` included); `maps` is a device array of tensor maps indexed like
 // `mats`; `split` selects split-precision TF32 (FP32-accurate) or plain TF32.
 PSGD_API int psgd_gemm_tc_launch(int transposed, int split, int max_r, const void* mats, const void* tiles, int ntiles,
                                  const void* maps, const float* in, float* out, float* out2, int ncorr,
@@ -544,6 +549,7 @@ PSGD_API int psgd_gemm_tc_launch(int transposed, int split, int max_r, const voi
   a.tickets = tickets;
   a.comm = (const PsgdCommDev*)comm;
   a.status = status;
-  if (transposed) return split ? dispatch_rank<true, true>(a, max_r, ntiles, stream) : dispatch_rank<true, false>(a, max_r, ntiles, stream);
-  return split ? dispatch_rank<false, true>(a, max_r, ntiles, stream) : dispatch_rank<false, false>(a, max_r, ntiles, stream);
+  const int early = (transposed >> 1) & 1;
+  if (transposed & 1) return split ? dispatch_rank<true, true>(a, max_r, ntiles, early, stream) : dispatch_rank<true, false>(a, max_r, ntiles, early, stream);
+  return split ? dispatch_rank<false, true>(a, max_r, ntiles, early, stream) : dispatch_rank<false, false>(a, max_r, ntiles, early, stream);
 }

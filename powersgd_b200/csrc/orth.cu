@@ -488,8 +488,8 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs 
 }
 
 template <int RT>
-static int orth_launch_rt(const OrthArgs& a, int nchunks, cudaStream_t stream) {
-  const int rc = psgd_launch(psgd_orth_gram_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, 0, a);
+static int orth_launch_rt(const OrthArgs& a, int nchunks, int early, cudaStream_t stream) {
+  const int rc = psgd_launch(psgd_orth_gram_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, early, a);
   if (rc != 0) return rc;
   return psgd_launch(psgd_orth_apply_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, 1, a);
 }
@@ -527,10 +527,11 @@ PSGD_API int psgd_orth_part_doubles(int max_r, int nprev) {
 // units / chunks: device tables; all units of one call share the template rank RT >= max r.
 // part: nchunks * psgd_orth_part_doubles(max_r, nprev) doubles; head: nunits * 2 * RT*RT floats.
 // comm / sum_out: see OrthArgs (null for a single worker or when x already holds the factor).
+// early: see psgd_launch (the second launch always follows the first that way).
 PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks, int nchunks, int max_r, float* x,
                               float* copy_to, int nprev, const float* const* prev, float* const* cmat,
                               double* part, float* head, const void* comm,
-                              float* sum_out, cudaStream_t stream) {
+                              float* sum_out, int early, cudaStream_t stream) {
   if (nunits <= 0 || nchunks <= 0) return 0;
   if (max_r > PSGD_MAX_RANK || nprev > PSGD_MAX_HIST) {
     psgd_set_error("psgd_orth_launch: rank %d or history %d beyond the compiled maximum", max_r, nprev);
@@ -555,12 +556,12 @@ PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks,
     return -1;
   }
   switch (psgd_orth_template_rank(max_r)) {
-    case 1: return orth_launch_rt<1>(a, nchunks, stream);
-    case 2: return orth_launch_rt<2>(a, nchunks, stream);
-    case 4: return orth_launch_rt<4>(a, nchunks, stream);
-    case 8: return orth_launch_rt<8>(a, nchunks, stream);
-    case 16: return orth_launch_rt<16>(a, nchunks, stream);
-    default: return orth_launch_rt<32>(a, nchunks, stream);
+    case 1: return orth_launch_rt<1>(a, nchunks, early, stream);
+    case 2: return orth_launch_rt<2>(a, nchunks, early, stream);
+    case 4: return orth_launch_rt<4>(a, nchunks, early, stream);
+    case 8: return orth_launch_rt<8>(a, nchunks, early, stream);
+    case 16: return orth_launch_rt<16>(a, nchunks, early, stream);
+    default: return orth_launch_rt<32>(a, nchunks, early, stream);
   }
 }
 

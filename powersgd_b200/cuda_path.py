@@ -497,10 +497,11 @@ class NativeCompressor:
 
     # -- phases ----------------------------------------------------------------------------
     def _orth(self, side: str, x: torch.Tensor, copy_to: torch.Tensor, prev: List[torch.Tensor], cm: List[torch.Tensor],
-              gather_to: Optional[torch.Tensor] = None):
+              gather_to: Optional[torch.Tensor] = None, early: bool = False):
         """Orthonormalise `x` in place (mirrored into `copy_to`). With `gather_to`, `x` is first
         filled with the sum over workers of the factor the previous product pushed (the sum is
-        also written to `gather_to`): the launch is the consumer of the in-kernel all-reduce."""
+        also written to `gather_to`): the launch is the consumer of the in-kernel all-reduce.
+        `early`: see `_chained`."""
         code = self.lib.psgd_orth_launch(
             _ptr(self.units[side]),
             self.n_units[side],
@@ -516,20 +517,29 @@ class NativeCompressor:
             _ptr(self._orth_rinv),
             self.comm.ptr if gather_to is not None else ctypes.c_void_p(0),
             _ptr(gather_to),
+            int(early),
             _stream_ptr(),
         )
         native.check(code, "psgd_orth_launch")
         self.launches += 2  # partial Gram matrices, then factorisation + application of R^-1
 
+    def _chained(self) -> bool:
+        """May a launch whose direct predecessor in the stream is a launch of the same step start
+        before that one has ended (csrc/psgd_common.cuh, psgd_launch)? One worker only: what several
+        workers exchange inside the kernels keeps the plain stream order."""
+        return self.comm is None and world_size() == 1
+
     def _gemm(self, transposed: bool, fin: torch.Tensor, fout: torch.Tensor, corr_fac, corr_c,
-              fout2: Optional[torch.Tensor] = None, part: str = "all"):
+              fout2: Optional[torch.Tensor] = None, part: str = "all", early: bool = False):
         """`part`: "all", or one half of a split launch - "early" (the CUDA-core tiles of the
-        matrices in the early bucket) / "late" (everything else); see `set_early_bucket`."""
+        matrices in the early bucket) / "late" (everything else); see `set_early_bucket`.
+        `early`: see `_chained`."""
         name = "nt" if transposed else "nn"
+        form = (1 if transposed else 0) | (2 if early else 0)
         tiles, count = self._tiles_dev[name]["tc"]
         if count and part != "early":
             code = self.lib.psgd_gemm_tc_launch(
-                1 if transposed else 0,
+                form,
                 1 if self._tc_split else 0,
                 self.tiles.max_r,
                 _ptr(self._mats_dev),
@@ -553,7 +563,7 @@ class NativeCompressor:
         tiles, count = self._tiles_dev[name]["f" if part == "all" else ("fA" if part == "early" else "fB")]
         if count:
             code = self.lib.psgd_gemm_ffma_launch(
-                1 if transposed else 0,
+                form,
                 self.tiles.max_r,
                 _ptr(self._mats_dev),
                 _ptr(tiles),
@@ -582,10 +592,11 @@ class NativeCompressor:
         return bool(self.lib.psgd_finalize_uses_strip(self.T, self.tiles.max_r, self.tiles.fin_rows, 0))
 
     def _finalize(self, sides: List[bool], fused_sgd: bool, workers: int, gather_state: Optional[torch.Tensor] = None,
-                  flags: int = 0):
+                  flags: int = 0, early: bool = False):
         """`gather_state`: the warm-start buffer that receives the summed factor of the last
         half-iteration when this launch is also its consumer (see `_gathers_in_finalize`).
-        `flags`: residual options of the strip / general kernels (csrc/finalize.cu, FinalizeArgs)."""
+        `flags`: residual options of the strip / general kernels (csrc/finalize.cu, FinalizeArgs).
+        `early`: see `_chained`."""
         if flags and self._tiles_dev["fin"]["tc"][1]:
             raise ValueError("residual options are not available with the tensor-core decompression kernel")
         lloc, rloc, lsum, rsum = [], [], [], []
@@ -640,6 +651,7 @@ class NativeCompressor:
                 _ptr(gather_state) if gather else ctypes.c_void_p(0),
                 int(flags),
                 1.0,
+                int(early and not self._tiles_dev["fin"]["tc"][1]),
                 _stream_ptr(),
             )
             native.check(code, "psgd_finalize_launch")
@@ -647,13 +659,15 @@ class NativeCompressor:
 
     def _half_iterations(self):
         """Runs the T half-iterations. Returns (sides, pending): `pending` is the warm-start buffer
-        whose summed factor the decompression launch still has to gather, or None."""
+        whose summed factor the decompression launch still has to gather, or None. `_follows` says
+        whether the last thing put on the stream was a launch of the step (see `_chained`)."""
         core = self.core
         workers = world_size()
         p2p = workers > 1 and self.comm is not None
         defer_last = p2p and self._gathers_in_finalize()
         sides: List[bool] = []
         pending: Optional[torch.Tensor] = None   # state buffer whose sum is still in the channel's slots
+        chained, self._follows = self._chained(), False
         for t in range(self.T):
             left = (core.step_counter * self.T + t) % 2 == 0
             sides.append(left)
@@ -681,16 +695,21 @@ class NativeCompressor:
                     if early_side != side:  # state changed under us (e.g. a checkpoint was loaded): redo
                         self._orth(side, state_in, self.h_in[t], same, self.cmat[t])
                 else:
-                    self._orth(side, state_in, self.h_in[t], same, self.cmat[t], gather_to)
+                    # the first launch of a step waits for all work before it (gradients, parameters)
+                    self._orth(side, state_in, self.h_in[t], same, self.cmat[t], gather_to, early=self._follows)
+                    self._follows = chained
             with _Range(f"psgd.iter{t}.product"):
                 # one worker: the product is final, so the kernel also writes the warm-start buffer
                 part = "all"
                 if t == 0 and self._early_product_done is not None:
                     part = "late"  # the early bucket's tiles were launched during backward
-                self._gemm(left, self.h_in[t], self.h_loc[t], other, self.cmat[t], state_out if workers == 1 else None, part=part)
+                self._gemm(left, self.h_in[t], self.h_loc[t], other, self.cmat[t], state_out if workers == 1 else None, part=part,
+                           early=self._follows)
+                self._follows = chained
                 if part == "late":
                     torch.cuda.current_stream().wait_event(self._early_product_done)
                     self._early_product_done = None
+                    self._follows = False
             total = state_out.numel()
             with _Range(f"psgd.iter{t}.reduce"):
                 if p2p and (t < self.T - 1 or defer_last):
@@ -761,7 +780,7 @@ class NativeCompressor:
         try:
             sides, pending = self._half_iterations()
             with _Range("psgd.finalize"):
-                self._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending)
+                self._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending, early=self._follows)
         finally:
             if workers == 1:
                 self.h_sum = saved
@@ -789,7 +808,7 @@ class NativeCompressor:
         try:
             sides, pending = self._half_iterations()
             with _Range("psgd.finalize+sgd"):
-                self._finalize(sides, fused_sgd=True, workers=workers, gather_state=pending)
+                self._finalize(sides, fused_sgd=True, workers=workers, gather_state=pending, early=self._follows)
         finally:
             self._hyper_dev = keep
             if workers == 1:
@@ -964,7 +983,7 @@ class NativeFlatAllReduce:
             self._nvls, self._nvls_failed = None, True
         return self._nvls
 
-    def _launch(self, mode: int, hyper_dev: torch.Tensor, divisor: float) -> None:
+    def _launch(self, mode: int, hyper_dev: torch.Tensor, divisor: float, early: bool = False) -> None:
         code = self.lib.psgd_flat_launch(
             mode,
             self._vec,
@@ -978,14 +997,15 @@ class NativeFlatAllReduce:
             self.comm.ptr if self.comm is not None else ctypes.c_void_p(0),
             ctypes.c_longlong(self.n_pad),
             1 if self._keep_inputs else 0,
+            int(early),
             _stream_ptr(),
         )
         native.check(code, "psgd_flat_launch")
         self.launches += 1
 
-    def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool) -> None:
+    def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool = False) -> None:
         if self.path == "local":
-            self._launch(4 if sgd else 3, hyper_dev, 1.0)
+            self._launch(4 if sgd else 3, hyper_dev, 1.0, early)
         elif self.path == "bulk":
             self._launch(0, hyper_dev, float(workers))
             code = self.lib.psgd_bulk_allreduce_launch(self.comm.ptr, ctypes.c_longlong(self.n_pad), workers, _stream_ptr())
@@ -1009,24 +1029,25 @@ class NativeFlatAllReduce:
             self._launch(2 if sgd else 1, hyper_dev, 1.0)
 
     def aggregate(self, gradients: List[torch.Tensor], outs: Optional[Sequence[torch.Tensor]] = None,
-                  keep_inputs: bool = False) -> List[torch.Tensor]:
+                  keep_inputs: bool = False, early: bool = False) -> List[torch.Tensor]:
         """Mean over workers. `outs`: caller-owned destination tensors (default: views of this
-        object's buffer, valid until the next call). `keep_inputs`: do not zero the inputs."""
+        object's buffer, valid until the next call). `keep_inputs`: do not zero the inputs. `early`:
+        the launch before this one is the decompression of other tensors, whose end it may overlap."""
         self.check()
         self.launches = 0
         self._bind(gradients, outs=outs)
         self._keep_inputs = bool(keep_inputs)
         try:
-            self._run(self._hyper_dev, world_size(), sgd=False)
+            self._run(self._hyper_dev, world_size(), sgd=False, early=early)
         finally:
             self._keep_inputs = False
         return list(self._views)
 
-    def aggregate_and_step(self, gradients, params, moms, hyper_index, hyper_dev) -> None:
+    def aggregate_and_step(self, gradients, params, moms, hyper_index, hyper_dev, early: bool = False) -> None:
         self.check()
         self.launches = 0
         self._bind(gradients, params, moms, hyper_index, need_out=False)
-        self._run(hyper_dev, world_size(), sgd=True)
+        self._run(hyper_dev, world_size(), sgd=True, early=early)
 
     def close(self) -> None:
         """Release the symmetric arena (collective across ranks)."""
@@ -1088,7 +1109,7 @@ class MultiTensorAccumulate:
         code = self.lib.psgd_flat_launch(
             8 if push is None else 9, self._vec, _ptr(self._items), _ptr(self._block_item), _ptr(self._block_first),
             self._nblocks, _ptr(self._hyper), ctypes.c_void_p(0), 1.0 if push is None else float(world_size()),
-            ctypes.c_void_p(0) if push is None else push.comm.ptr, ctypes.c_longlong(0), 0, _stream_ptr(),
+            ctypes.c_void_p(0) if push is None else push.comm.ptr, ctypes.c_longlong(0), 0, 0, _stream_ptr(),
         )
         native.check(code, "psgd_flat_launch")
         if push is not None:
@@ -1244,6 +1265,7 @@ class FusedSGDDriver:
             # after the low-rank path: a consumer that spins on its peers next to the product
             # kernels (tried as a parallel side-stream branch) cost more than it hid
             self._flat_plain.aggregate_and_step(
-                plain, pick(params, False), pick(moms, False), pick(index, False), hyper_dev
+                plain, pick(params, False), pick(moms, False), pick(index, False), hyper_dev,
+                early=bool(core.params) and core._native._chained(),
             )
             self.launches += self._flat_plain.launches

@@ -105,6 +105,7 @@ class NativeLowRank:
         self._bind(matrices)
         workers = world_size()
         p2p = workers > 1 and comp.comm is not None
+        chained = comp._chained()
         P, Q = core._ps_buffer, core._qs_buffer
         p_loc, q_loc, p_hat = comp.h_loc[0], comp.h_loc[1], comp.h_in[1]
         # p = M q; one worker: straight into the factor memory
@@ -113,9 +114,9 @@ class NativeLowRank:
             P.copy_(p_loc[: P.numel()])
             comp._allreduce_sum(P)
         # orthonormalise p in place (multi-GPU: the launch first gathers the pushed p's)
-        comp._orth("p", P, p_hat, [], [], comp.h_sum[0] if p2p else None)
+        comp._orth("p", P, p_hat, [], [], comp.h_sum[0] if p2p else None, early=chained)
         # q = M^T p
-        comp._gemm(True, p_hat, q_loc, [], [], Q if workers == 1 else None)
+        comp._gemm(True, p_hat, q_loc, [], [], Q if workers == 1 else None, early=chained)
         gather = p2p and comp._gathers_in_finalize()
         if p2p and not gather:
             code = comp.lib.psgd_factor_reduce_launch(
@@ -151,6 +152,7 @@ class NativeLowRank:
             _ptr(gather_state) if gather_state is not None else ctypes.c_void_p(0),
             3,  # residual = M - update, written to the `param` slot (the caller's memory tensor)
             1.0 / workers,
+            int(comp._chained()),
             _stream_ptr(),
         )
         native.check(code, "psgd_finalize_launch")
@@ -171,7 +173,7 @@ class NativeLowRank:
             saved, comp.h_sum = comp.h_sum, comp.h_loc
         try:
             sides, pending = comp._half_iterations()
-            comp._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending, flags=2)
+            comp._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending, flags=2, early=comp._follows)
         finally:
             if workers == 1:
                 comp.h_sum = saved
