@@ -26,6 +26,9 @@ constexpr int GEMM_WARPS = GEMM_THREADS / 32;
 constexpr int NT_TILE_COLS = 128;   // columns of M per NT tile
 constexpr int NT_MAX_ROWS = 256;    // rows of P-hat staged in smem at a time (128 at RT = 32); a tile may span several such chunks
 constexpr int NN_CHUNK_COLS = 128;  // columns consumed per inner iteration of an NN tile
+// Most columns of an NN tile: as many rows of Q-hat as fit 32 KiB of shared memory.
+template <int RT>
+__host__ __device__ constexpr int nn_max_cols() { return RT <= 8 ? 1024 : 8192 / RT; }
 
 struct GemmArgs {
   const PsgdMat* mats;
@@ -293,7 +296,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
 
 template <int RT>
 __global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nt_kernel(GemmArgs a) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   psgd_launch_dependents();
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
@@ -303,26 +306,52 @@ __global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nt_kernel(GemmArgs a) 
 }
 
 // ------------------------------------------------------------------------------------------
-// NN: each warp owns RPW rows; lanes stride across the columns and shuffle-reduce at the end.
+// NN: each warp owns RPW rows; lanes stride across the columns and reduce at the end.
 // ------------------------------------------------------------------------------------------
+// Sums of N values over the 32 lanes: value i ends up (complete) in the lanes whose top log2(N) bits
+// spell i. Every step halves what a lane still carries, so N values cost N - 1 + 5 - log2(N) shuffles
+// instead of 5 N; lanes are paired as in a butterfly (16, 8, 4, 2, 1), so the bits are the same.
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N], int lane) {
+  static_assert(N >= 1 && N <= 32 && (N & (N - 1)) == 0, "a power of two");
+  int off = 16;
+#pragma unroll
+  for (int n = N; n > 1; n >>= 1, off >>= 1) {
+    const bool upper = (lane & off) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if (i < n / 2) {
+        const float keep = upper ? v[i + n / 2] : v[i], send = upper ? v[i] : v[i + n / 2];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+  }
+  float s = v[0];
+  for (; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  return s;
+}
+
+// A tile is 8 * RPW rows by up to nn_max_cols columns. What bounds it: with few columns per tile the
+// chain load - multiply - reduce - hand over; with many, the loads of the gradient. So the rows of
+// Q-hat that the tile needs are staged in shared memory once, in the order the lanes read them (a lane
+// reads its 4 columns x RT values as RT 16-byte words: read straight from global memory they cost more
+// load instructions than the gradient itself), and the loop over 128-column chunks keeps one chunk of
+// the gradient in flight ahead of the one being multiplied.
 template <int RT, int VEC, int RPW>
-__device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& t, const PsgdMat& mt, float* sSum) {
+__device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& t, const PsgdMat& mt, float* sQ, float* sSum) {
   const int r = mt.r, m = mt.m;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int TILE_ROWS = GEMM_WARPS * RPW;
   __shared__ int sLast;
 #ifdef PSGD_BOUNDS_CHECK
-  if (!product_tile_ok<RT>(t, mt, 2, TILE_ROWS, 1 << 30, TILE_ROWS * RT)) return;
+  if (!product_tile_ok<RT>(t, mt, 2, TILE_ROWS, nn_max_cols<RT>(), TILE_ROWS * RT)) return;
 #endif
 
   const float* __restrict__ M = mt.grad;
-  const float* qin = a.in + mt.q_off;   // written by the launch before: plain loads, after the wait
 
-  float acc[RPW][RT];
+  float acc[RPW * RT];
 #pragma unroll
-  for (int u = 0; u < RPW; ++u)
-#pragma unroll
-    for (int k = 0; k < RT; ++k) acc[u][k] = 0.f;
+  for (int e = 0; e < RPW * RT; ++e) acc[e] = 0.f;
 
   const int rbase = warp * RPW;
   const float* rowp[RPW];
@@ -334,15 +363,33 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
   }
 
   const int cend = t.col0 + t.cols;
-  // as in the NT tile: first loads and L2 prefetch ahead of the wait, then always one chunk ahead
+  // as in the NT tile, the first loads go out ahead of the wait
   float v[RPW][4];
 #pragma unroll
   for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], t.col0, cend, lane, rok[u], v[u]);
-#pragma unroll
-  for (int u = 0; u < RPW; ++u)
-    if (rok[u])
-      for (int c = t.col0 + NN_CHUNK_COLS + lane * 32; c < cend; c += 32 * 32) psgd_prefetch_l2(rowp[u] + c);
   psgd_wait_for_predecessor();
+
+  // element (column lc of the tile, k): chunk of 128 columns, then word of 4 floats, then lane
+  const float* qin = a.in + mt.q_off + (long long)t.col0 * r;   // written by the launch before: plain loads
+  for (int e = tid; e < t.cols * r; e += GEMM_THREADS) {
+    const int lc = e / r, k = e - lc * r, b = lc & 127;
+    const int ln = VEC == 4 ? b >> 2 : VEC == 2 ? (b & 63) >> 1 : b & 31;
+    const int c = VEC == 4 ? b & 3 : VEC == 2 ? (b & 1) + 2 * (b >> 6) : b >> 5;
+    const int f = c * RT + k;
+    sQ[(((lc >> 7) * RT + (f >> 2)) * 32 + ln) * 4 + (f & 3)] = qin[e];
+  }
+  if (r < RT || (t.cols & 127) != 0) {
+    // the padding the loop reads: columns beyond the tile in its last chunk, values beyond the rank
+    const int chunks = (t.cols + 127) >> 7;
+    for (int e = tid; e < chunks * 128 * RT; e += GEMM_THREADS) {
+      const int word = e >> 7, ln = (e >> 2) & 31, f = (word % RT) * 4 + (e & 3);
+      const int c = f / RT, k = f % RT;
+      if (k >= r || (word / RT) * 128 + lane_col<VEC>(ln, c) >= t.cols) sQ[e] = 0.f;
+    }
+  }
+  __syncthreads();
+
+  const float4* q4 = reinterpret_cast<const float4*>(sQ) + lane;
   for (int c0 = t.col0; c0 < cend; c0 += NN_CHUNK_COLS) {
     float cur[RPW][4];
 #pragma unroll
@@ -354,27 +401,24 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
       for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], c0 + NN_CHUNK_COLS, cend, lane, rok[u], v[u]);
     }
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int col = c0 + lane_col<VEC>(lane, c);
-      if (col < cend) {
-        const float* qr = qin + (long long)col * r;
+    for (int w = 0; w < RT; ++w) {
+      const float4 q = q4[w * 32];
+      const float qv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int k = 0; k < RT; ++k) {
-          const float qk = (k < r) ? qr[k] : 0.f;
+      for (int i = 0; i < 4; ++i) {
+        const int c = (w * 4 + i) / RT, k = (w * 4 + i) % RT;
 #pragma unroll
-          for (int u = 0; u < RPW; ++u) acc[u][k] = fmaf(cur[u][c], qk, acc[u][k]);
-        }
+        for (int u = 0; u < RPW; ++u) acc[u * RT + k] = fmaf(cur[u][c], qv[i], acc[u * RT + k]);
       }
     }
+    q4 += RT * 32;
   }
 
-#pragma unroll
-  for (int u = 0; u < RPW; ++u)
-#pragma unroll
-    for (int k = 0; k < RT; ++k) {
-      const float s = psgd_warp_sum(acc[u][k]);
-      if (lane == 0) sSum[(rbase + u) * RT + k] = s;
-    }
+  if (RPW * RT <= 32) {
+    const float s = warp_sums<RPW * RT>(acc, lane);
+    constexpr int SPAN = 32 / (RPW * RT);   // lanes that hold the same sum
+    if (lane % SPAN == 0) sSum[rbase * RT + lane / SPAN] = s;
+  }
   __syncthreads();
 
   constexpr int tile_elems = TILE_ROWS * RT;
@@ -424,13 +468,14 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
 
 template <int RT, int RPW>
 __global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nn_kernel(GemmArgs a) {
+  extern __shared__ __align__(16) float smem[];   // staged rows of Q-hat
   __shared__ float sSum[GEMM_WARPS * RPW * RT];
   psgd_launch_dependents();
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
-  if (t.vec == 4) gemm_nn_tile<RT, 4, RPW>(a, t, mt, sSum);
-  else if (t.vec == 2) gemm_nn_tile<RT, 2, RPW>(a, t, mt, sSum);
-  else gemm_nn_tile<RT, 1, RPW>(a, t, mt, sSum);
+  if (t.vec == 4) gemm_nn_tile<RT, 4, RPW>(a, t, mt, smem, sSum);
+  else if (t.vec == 2) gemm_nn_tile<RT, 2, RPW>(a, t, mt, smem, sSum);
+  else gemm_nn_tile<RT, 1, RPW>(a, t, mt, smem, sSum);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -468,7 +513,8 @@ static int launch_nt(const GemmArgs& a, int ntiles, int early, cudaStream_t stre
 template <int RT>
 static int launch_nn(const GemmArgs& a, int ntiles, int early, cudaStream_t stream) {
   constexpr int RPW = RT <= 8 ? 4 : (RT == 16 ? 2 : 1);
-  return psgd_launch(psgd_gemm_nn_kernel<RT, RPW>, ntiles, GEMM_THREADS, 0, stream, early, a);
+  const size_t smem = (size_t)nn_max_cols<RT>() * RT * sizeof(float);
+  return psgd_launch(psgd_gemm_nn_kernel<RT, RPW>, ntiles, GEMM_THREADS, smem, stream, early, a);
 }
 
 #define PSGD_DISPATCH_RT(FN)                                   \
@@ -484,6 +530,8 @@ PSGD_API int psgd_gemm_nn_tile_rows(int max_r) {
   const int rt = max_r <= 1 ? 1 : max_r <= 2 ? 2 : max_r <= 4 ? 4 : max_r <= 8 ? 8 : max_r <= 16 ? 16 : 32;
   return GEMM_WARPS * (rt <= 8 ? 4 : (rt == 16 ? 2 : 1));
 }
+// Most columns of an NN tile (a multiple of 128).
+PSGD_API int psgd_gemm_nn_max_cols(int max_r) { return max_r <= 8 ? 1024 : max_r <= 16 ? nn_max_cols<16>() : nn_max_cols<32>(); }
 PSGD_API int psgd_gemm_nt_max_rows(int max_r) { return max_r <= 16 ? NT_MAX_ROWS : NT_MAX_ROWS / 2; }
 PSGD_API int psgd_gemm_template_rank(int max_r) {
   return max_r <= 1 ? 1 : max_r <= 2 ? 2 : max_r <= 4 ? 4 : max_r <= 8 ? 8 : max_r <= 16 ? 16 : 32;

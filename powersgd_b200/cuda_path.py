@@ -143,9 +143,14 @@ class TilePlan:
         self.rt = lib.psgd_gemm_template_rank(self.max_r)
         self.total_elems = sum(g.n * g.m * g.batch for g in plan.groups)
         nt_rows_cap = lib.psgd_gemm_nt_max_rows(self.max_r)
-        self.nt_rows = min(nt_rows_cap, 128 if self.total_elems < (64 << 20) else 256)
+        # rows of an NT tile: twice as many halve what a tile costs besides its loads (start, staging, the
+        # sum over the warps, the hand-over), as long as some 300 tiles are left for the 148 SMs. 128 / 256
+        # rows: ResNet-18 (11 M elements) 14.1 / 12.2 us, 3 x 1001x777 + 2 x 515x2049 (4 M) 12.4 / 13.7 us;
+        # matrices above 4096 rows, 256 / 512: the LSTM model (32 M) 52.8 / 49.0 us.
+        self.nt_rows = min(nt_rows_cap, 128 if self.total_elems < (8 << 20) else 256)
+        self.nt_tall_rows = 256 if self.total_elems < (16 << 20) else 512
         self.nn_rows = lib.psgd_gemm_nn_tile_rows(self.max_r)
-        self.nn_cols_cap = 1024
+        self.nn_cols_cap = lib.psgd_gemm_nn_max_cols(self.max_r)
         self.rp_tc = lib.psgd_gemm_tc_rank_pad(self.max_r)
         self.fin_tc_ok = False  # set by the compressor: (half-iterations x rank) fits the tensor-core finalize
         self.fin_rows = 32      # set by the compressor: height of a finalize strip (multiple of 32)
@@ -191,10 +196,10 @@ class TilePlan:
                     ticket += 1
                     tc_slots += len(col_blocks)
                 continue
-            # tall matrices: tiles of 256 rows (128 KiB: small enough that every SM holds several at
-            # any time, which is what hides the load latency) but never more than 160 partial tiles
+            # tall matrices: tiles of 256 or 512 rows (128 or 256 KiB: small enough that every SM gets several
+            # CTAs, which is what hides the load latency) but never more than 160 partial tiles
             # per column block (the kernel walks a taller tile in chunks of its staging buffer)
-            rows_per_tile = max(self.nt_rows if g.n <= 4096 else 256, -(-(-(-g.n // 160)) // 128) * 128)
+            rows_per_tile = max(self.nt_rows if g.n <= 4096 else self.nt_tall_rows, -(-(-(-g.n // 160)) // 128) * 128)
             row_blocks = _split_even(g.n, rows_per_tile, 1)
             for c0 in range(0, g.m, 128):
                 cols = min(128, g.m - c0)

@@ -18,6 +18,8 @@ def declare(lib) -> None:
 
     lib.psgd_gemm_nn_tile_rows.restype = i32
     lib.psgd_gemm_nn_tile_rows.argtypes = [i32]
+    lib.psgd_gemm_nn_max_cols.restype = i32
+    lib.psgd_gemm_nn_max_cols.argtypes = [i32]
     lib.psgd_gemm_nt_max_rows.restype = i32
     lib.psgd_gemm_nt_max_rows.argtypes = [i32]
     lib.psgd_gemm_template_rank.restype = i32
