@@ -242,6 +242,16 @@ __global__ void __launch_bounds__(FIN_THREADS) psgd_finalize_kernel(FinalizeArgs
 // once; the loop over 32-row chunks then runs without barriers, every chunk issuing its global
 // loads (gradient, parameter, momentum) before its FMA loop so that their latency overlaps it.
 constexpr int FIN_STRIP_KMAX = 32;
+// Floats between the panel rows of two factor columns: four more than their length. A factor is stored
+// row by row (r values together), so neighbouring threads of the staging loop write to neighbouring
+// panel rows; at a pitch of 128 or 256 floats all of them would meet in one shared-memory bank.
+constexpr int FIN_PANEL_PAD = 4;
+constexpr int FIN_RPITCH = FIN_COLS + FIN_PANEL_PAD;
+__host__ __device__ constexpr int fin_panel_floats(int tile_rows) { return FIN_RPITCH + tile_rows + FIN_PANEL_PAD; }  // per factor column
+
+// e / r for 0 <= e < 8192 and 2 <= r <= 32, with magic = ceil(2^20 / r): the product stays below 2^32 and
+// e * (magic * r - 2^20) below 2^20.
+__device__ __forceinline__ int fin_div(int e, int r, unsigned magic) { return r == 1 ? e : (int)(((unsigned)e * magic) >> 20); }
 
 // Gather `n` consecutive words starting at slot index `base` of this epoch (sum over ranks in
 // rank order) and hand each to `put(i, value)`.
@@ -260,23 +270,25 @@ __device__ __forceinline__ void fin_gather(const PsgdCommDev& c, int e1, long lo
   }
 }
 
-template <int VEC, bool SAME>
+template <int VEC, bool SAME, int RPW>
 __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const PsgdTile& t, const PsgdMat& mt,
                                                     int tile_rows, float* fin_smem) {
   const int r = mt.r, m = mt.m;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int K = a.nhist * r;
-  float* sRl = fin_smem;                         // [K][FIN_COLS]
-  float* sLl = sRl + K * FIN_COLS;               // [K][tile_rows]
-  float* sRs = SAME ? sRl : sLl + K * tile_rows;
-  float* sLs = SAME ? sLl : sRs + K * FIN_COLS;
+  const int lp = tile_rows + FIN_PANEL_PAD;
+  float* sRl = fin_smem;                         // [K][FIN_RPITCH]
+  float* sLl = sRl + K * FIN_RPITCH;             // [K][lp]
+  float* sRs = SAME ? sRl : sLl + K * lp;
+  float* sLs = SAME ? sLl : sRs + K * FIN_RPITCH;
+  const unsigned magic = ((1u << 20) + (unsigned)r - 1u) / (unsigned)r;
 
 #ifdef PSGD_BOUNDS_CHECK
   {
     bool ok = true;
     ok &= PSGD_BC(t.row0 >= 0 && t.rows > 0 && t.row0 + t.rows <= mt.n && t.rows <= tile_rows, 3, PSGD_BC_TILE_ROWS, t.row0 + t.rows, mt.n);
     ok &= PSGD_BC(t.col0 >= 0 && t.cols > 0 && t.col0 + t.cols <= mt.m && t.cols <= FIN_COLS, 3, PSGD_BC_TILE_COLS, t.col0 + t.cols, mt.m);
-    ok &= PSGD_BC(K >= 1 && K <= FIN_STRIP_KMAX && (SAME ? 1 : 2) * K * (FIN_COLS + tile_rows) * 4 <= 96 * 1024, 3, PSGD_BC_SMEM, K, FIN_STRIP_KMAX);
+    ok &= PSGD_BC(K >= 1 && K <= FIN_STRIP_KMAX && (SAME ? 1 : 2) * K * fin_panel_floats(tile_rows) * 4 <= 96 * 1024, 3, PSGD_BC_SMEM, K, FIN_STRIP_KMAX);
     const unsigned long long addr = (unsigned long long)mt.grad | (unsigned long long)mt.param | (unsigned long long)mt.mom | (unsigned long long)mt.out;
     ok &= PSGD_BC(t.vec == 1 || (t.vec == 2 && addr % 8 == 0 && mt.m % 2 == 0) || (t.vec == 4 && addr % 16 == 0 && mt.m % 4 == 0),
                   3, PSGD_BC_ALIGNMENT, addr % 16, t.vec);
@@ -292,22 +304,40 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
 
   // Global loads of a chunk of 32 rows; the rows of the chunk after it are asked into L2, so that
   // their loads, which the registers have no room for yet, find them there.
-  __align__(16) float g4[4][4], p4[4][4], m4[4][4];
+  // A warp has RPW rows of a chunk. With eight, parameters and momentum have no registers ahead of the
+  // multiplications either and are loaded after them (out of L2, where they were asked to go).
+  constexpr int CHUNK = 8 * RPW;
+  constexpr bool LATE = RPW > 4;
+  constexpr int PR = LATE ? 1 : RPW;
+  __align__(16) float g4[RPW][4], p4[PR][4], m4[PR][4];
+  auto load_state = [&](int lr, float* p, float* mo) {
+    const long long rowoff = (long long)(t.row0 + lr) * m + t.col0;
+#pragma unroll
+    for (int c4 = 0; c4 < 4; ++c4) p[c4] = mo[c4] = 0.f;
+    if (lr < t.rows) {
+      if (sgd) fin_load4<VEC>(mt.param + rowoff, lane, t.cols, p);
+      if (mom) fin_load4<VEC>(mt.mom + rowoff, lane, t.cols, mo);
+    }
+  };
   auto load = [&](int rc) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int lr = rc + warp * 4 + u;
-      const long long rowoff = (long long)(t.row0 + lr) * m + t.col0;
+    for (int u = 0; u < RPW; ++u) {
+      const int lr = rc + warp * RPW + u;
 #pragma unroll
-      for (int c4 = 0; c4 < 4; ++c4) g4[u][c4] = p4[u][c4] = m4[u][c4] = 0.f;
-      if (lr < t.rows) {
-        fin_load4<VEC>(mt.grad + rowoff, lane, t.cols, g4[u]);
-        if (sgd) fin_load4<VEC>(mt.param + rowoff, lane, t.cols, p4[u]);
-        if (mom) fin_load4<VEC>(mt.mom + rowoff, lane, t.cols, m4[u]);
+      for (int c4 = 0; c4 < 4; ++c4) g4[u][c4] = 0.f;
+      if (lr < t.rows) fin_load4<VEC>(mt.grad + (long long)(t.row0 + lr) * m + t.col0, lane, t.cols, g4[u]);
+      if (!LATE) load_state(lr, p4[u % PR], m4[u % PR]);
+    }
+    if (LATE && rc == 0 && sgd) {
+      const int now = warp * RPW + (lane >> 2), col = (lane & 3) * 32;
+      if (now < t.rows && col < t.cols) {
+        const long long off = (long long)(t.row0 + now) * m + t.col0 + col;
+        psgd_prefetch_l2(mt.param + off);
+        if (mom) psgd_prefetch_l2(mt.mom + off);
       }
     }
-    const int next = rc + FIN_ROWS + warp * 4 + (lane >> 2), col = (lane & 3) * 32;
-    if (lane < 16 && next < t.rows && col < t.cols) {
+    const int next = rc + CHUNK + warp * RPW + (lane >> 2), col = (lane & 3) * 32;
+    if (lane < 4 * RPW && next < t.rows && col < t.cols) {
       const long long off = (long long)(t.row0 + next) * m + t.col0 + col;
       psgd_prefetch_l2(mt.grad + off);
       if (sgd) psgd_prefetch_l2(mt.param + off);
@@ -331,16 +361,16 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
       const float* gs = a.rsum[h] + base;
       const bool poll = last && !a.poll_left;
       for (int e = tid; e < t.cols * r; e += FIN_THREADS) {
-        const int lc = e / r, j = e - lc * r;
+        const int lc = fin_div(e, r, magic), j = e - lc * r;
         const int pos = fin_panel_pos<VEC>(lc);
-        sRl[(h * r + j) * FIN_COLS + pos] = gl[e];
-        if (!SAME && !poll && gs != gl) sRs[(h * r + j) * FIN_COLS + pos] = gs[e];
+        sRl[(h * r + j) * FIN_RPITCH + pos] = gl[e];
+        if (!SAME && !poll && gs != gl) sRs[(h * r + j) * FIN_RPITCH + pos] = gs[e];
       }
       if (poll) {
         const bool writer = t.row0 == 0;
         fin_gather(*a.comm, e1, base, t.cols * r, ok, [&](int e, float v) {
-          const int lc = e / r, j = e - lc * r;
-          sRs[(h * r + j) * FIN_COLS + fin_panel_pos<VEC>(lc)] = v;
+          const int lc = fin_div(e, r, magic), j = e - lc * r;
+          sRs[(h * r + j) * FIN_RPITCH + fin_panel_pos<VEC>(lc)] = v;
           if (writer) {
             a.sum_out1[base + e] = v;
             if (a.sum_out2) a.sum_out2[base + e] = v * a.sum_scale;
@@ -354,15 +384,15 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
       const float* gs = a.lsum[h] + base;
       const bool poll = last && a.poll_left;
       for (int e = tid; e < t.rows * r; e += FIN_THREADS) {
-        const int lr = e / r, j = e - lr * r;
-        sLl[(h * r + j) * tile_rows + lr] = gl[e];
-        if (!SAME && !poll && gs != gl) sLs[(h * r + j) * tile_rows + lr] = gs[e];
+        const int lr = fin_div(e, r, magic), j = e - lr * r;
+        sLl[(h * r + j) * lp + lr] = gl[e];
+        if (!SAME && !poll && gs != gl) sLs[(h * r + j) * lp + lr] = gs[e];
       }
       if (poll) {
         const bool writer = t.col0 == 0;
         fin_gather(*a.comm, e1, base, t.rows * r, ok, [&](int e, float v) {
-          const int lr = e / r, j = e - lr * r;
-          sLs[(h * r + j) * tile_rows + lr] = v;
+          const int lr = fin_div(e, r, magic), j = e - lr * r;
+          sLs[(h * r + j) * lp + lr] = v;
           if (writer) {
             a.sum_out1[base + e] = v;
             if (a.sum_out2) a.sum_out2[base + e] = v * a.sum_scale;
@@ -374,12 +404,13 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   if (gather) psgd_comm_close_epoch(*a.comm, e1);  // (CTA barrier inside) this strip has read its words
   __syncthreads();
 
-  for (int rc = 0; rc < t.rows; rc += FIN_ROWS) {
+  for (int rc = 0; rc < t.rows; rc += CHUNK) {
+    if (rc + warp * RPW >= t.rows) break;   // this warp has no row left (and its panel entries would lie beyond the strip)
     if (rc || !SAME) load(rc);
     // ---- rank-K update from the staged panels ----
-    float accE[4][4], accA[4][4];
+    float accE[RPW][4], accA[RPW][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < RPW; ++u)
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) accE[u][c4] = accA[u][c4] = 0.f;
     for (int h = 0; h < a.nhist; ++h) {
@@ -390,14 +421,19 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
 #pragma unroll 4
       for (int j = 0; j < r; ++j) {
         const int k = h * r + j;
-        const float4 ll = *reinterpret_cast<const float4*>(sLl + k * tile_rows + rc + warp * 4);
-        const float4 rl = *reinterpret_cast<const float4*>(sRl + k * FIN_COLS + lane * 4);
-        const float4 ls = one_left ? ll : *reinterpret_cast<const float4*>(sLs + k * tile_rows + rc + warp * 4);
-        const float4 rs = one_right ? rl : *reinterpret_cast<const float4*>(sRs + k * FIN_COLS + lane * 4);
-        const float lv[4] = {ll.x, ll.y, ll.z, ll.w}, sv[4] = {ls.x, ls.y, ls.z, ls.w};
+        const float4 rl = *reinterpret_cast<const float4*>(sRl + k * FIN_RPITCH + lane * 4);
+        const float4 rs = one_right ? rl : *reinterpret_cast<const float4*>(sRs + k * FIN_RPITCH + lane * 4);
+        float lv[RPW], sv[RPW];
+#pragma unroll
+        for (int u = 0; u < RPW; u += 4) {
+          *reinterpret_cast<float4*>(lv + u) = *reinterpret_cast<const float4*>(sLl + k * lp + rc + warp * RPW + u);
+          if (!SAME)
+            *reinterpret_cast<float4*>(sv + u) = one_left ? *reinterpret_cast<const float4*>(lv + u)
+                                                          : *reinterpret_cast<const float4*>(sLs + k * lp + rc + warp * RPW + u);
+        }
         const float rlv[4] = {rl.x, rl.y, rl.z, rl.w}, rsv[4] = {rs.x, rs.y, rs.z, rs.w};
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < RPW; ++u)
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4) {
             accE[u][c4] = fmaf(lv[u], rlv[c4], accE[u][c4]);
@@ -407,21 +443,22 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
     }
     // ---- residual, mean update, optimizer ----
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int lr = rc + warp * 4 + u;
+    for (int u = 0; u < RPW; ++u) {
+      const int lr = rc + warp * RPW + u;
       if (lr >= t.rows) continue;
+      if (LATE) load_state(lr, p4[0], m4[0]);
       const long long rowoff = (long long)(t.row0 + lr) * m + t.col0;
       __align__(16) float av[4];
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) {
         av[c4] = (SAME ? accE[u][c4] : accA[u][c4]) * a.inv_world;
         g4[u][c4] -= global_res ? av[c4] : accE[u][c4];
-        if (sgd) psgd_sgd_update(av[c4], p4[u][c4], &m4[u][c4], hy);
+        if (sgd) psgd_sgd_update(av[c4], p4[u % PR][c4], &m4[u % PR][c4], hy);
       }
       fin_store4<VEC>(res_base + rowoff, lane, t.cols, g4[u]);
       if (sgd) {
-        fin_store4<VEC>(mt.param + rowoff, lane, t.cols, p4[u]);
-        if (mom) fin_store4<VEC>(mt.mom + rowoff, lane, t.cols, m4[u]);
+        fin_store4<VEC>(mt.param + rowoff, lane, t.cols, p4[u % PR]);
+        if (mom) fin_store4<VEC>(mt.mom + rowoff, lane, t.cols, m4[u % PR]);
       } else {
         fin_store4<VEC>(mt.out + rowoff, lane, t.cols, av);
       }
@@ -429,14 +466,14 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   }
 }
 
-template <bool SAME>
+template <bool SAME, int RPW>
 __global__ void __launch_bounds__(FIN_THREADS, 2) psgd_finalize_strip_kernel(FinalizeArgs a, int tile_rows) {
   extern __shared__ __align__(16) float fin_smem[];
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
-  if (t.vec == 4) finalize_strip_tile<4, SAME>(a, t, mt, tile_rows, fin_smem);
-  else if (t.vec == 2) finalize_strip_tile<2, SAME>(a, t, mt, tile_rows, fin_smem);
-  else finalize_strip_tile<1, SAME>(a, t, mt, tile_rows, fin_smem);
+  if (t.vec == 4) finalize_strip_tile<4, SAME, RPW>(a, t, mt, tile_rows, fin_smem);
+  else if (t.vec == 2) finalize_strip_tile<2, SAME, RPW>(a, t, mt, tile_rows, fin_smem);
+  else finalize_strip_tile<1, SAME, RPW>(a, t, mt, tile_rows, fin_smem);
 }
 
 // Shared-memory budgets of a strip CTA: the default carve-out serves the small ranks (several CTAs
@@ -446,32 +483,32 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) psgd_finalize_strip_kernel(Fin
 constexpr int FIN_SMEM_DEFAULT = 48 * 1024;
 constexpr int FIN_SMEM_OPT_IN = 96 * 1024;
 
-template <bool SAME>
+template <bool SAME, int RPW>
 static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, int early, cudaStream_t stream) {
-  const size_t smem = (size_t)(SAME ? 1 : 2) * kmax * (FIN_COLS + tile_rows) * sizeof(float);
+  const size_t smem = (size_t)(SAME ? 1 : 2) * kmax * fin_panel_floats(tile_rows) * sizeof(float);
   if (smem > (size_t)FIN_SMEM_DEFAULT) {
     static bool opted_in = false;   // per instantiation
     if (!opted_in) {
-      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
+      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME, RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
       opted_in = true;
     }
   }
-  return psgd_launch(psgd_finalize_strip_kernel<SAME>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
+  return psgd_launch(psgd_finalize_strip_kernel<SAME, RPW>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
 }
 
 // Tallest strip (multiple of 32 rows, at most 256) whose panels fit the shared-memory budget.
 PSGD_API int psgd_finalize_strip_rows(int kmax, int same) {
   if (kmax > FIN_STRIP_KMAX) return FIN_ROWS;  // general kernel: strips only save tile overhead
   const int per_row = (same ? 1 : 2) * kmax * (int)sizeof(float);
-  int rows = FIN_SMEM_DEFAULT / per_row - FIN_COLS;
-  if (rows < 256) rows = FIN_SMEM_OPT_IN / per_row - FIN_COLS;
+  int rows = FIN_SMEM_DEFAULT / per_row - fin_panel_floats(0);
+  if (rows < 256) rows = FIN_SMEM_OPT_IN / per_row - fin_panel_floats(0);
   rows = rows / FIN_ROWS * FIN_ROWS;
   return rows > 256 ? 256 : (rows < FIN_ROWS ? FIN_ROWS : rows);
 }
 
 static bool finalize_takes_strip(int nhist, int max_r, int tile_rows, bool same) {
   const int kmax = nhist * max_r;
-  const size_t strip_smem = (size_t)(same ? 1 : 2) * kmax * (FIN_COLS + tile_rows) * sizeof(float);
+  const size_t strip_smem = (size_t)(same ? 1 : 2) * kmax * fin_panel_floats(tile_rows) * sizeof(float);
   return kmax <= FIN_STRIP_KMAX && strip_smem <= (size_t)FIN_SMEM_OPT_IN;
 }
 
@@ -532,8 +569,9 @@ PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntile
   }
   if (strip) {
     const int kmax = nhist * max_r;
-    return same ? finalize_strip_launch<true>(a, ntiles, tile_rows, kmax, early, stream)
-                : finalize_strip_launch<false>(a, ntiles, tile_rows, kmax, early, stream);
+    if (!same) return finalize_strip_launch<false, 4>(a, ntiles, tile_rows, kmax, early, stream);
+    return kmax >= 16 ? finalize_strip_launch<true, 8>(a, ntiles, tile_rows, kmax, early, stream)
+                                : finalize_strip_launch<true, 4>(a, ntiles, tile_rows, kmax, early, stream);
   }
   return psgd_launch(same ? psgd_finalize_kernel<true> : psgd_finalize_kernel<false>, ntiles, FIN_THREADS, 0, stream, early, a);
 }

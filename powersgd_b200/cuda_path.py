@@ -293,9 +293,10 @@ class NativeCompressor:
         if self.T > layout.MAX_HIST:
             raise ValueError(f"num_iters_per_step {self.T} exceeds the compiled maximum {layout.MAX_HIST}")
         # finalize strips: as tall as the factor panels allow in shared memory, but short enough
-        # that a small model still spreads over ~6 strips per SM
+        # that a small model still spreads over ~3 strips per SM (a strip costs its panels and one start:
+        # ResNet-18's step takes 131 / 121.5 / 120 us with 12 / 6 / 3 strips per SM)
         strip_cap = int(self.lib.psgd_finalize_strip_rows(self.T * self.tiles.max_r, 1 if world_size() == 1 else 0))
-        want = self.tiles.total_elems // (128 * 148 * 6)
+        want = self.tiles.total_elems // (128 * 148 * 3)
         self.tiles.fin_rows = max(32, min(strip_cap, want // 32 * 32))
         nm = len(self.tiles.mats)
         cap = max(self.plan.p_total, self.plan.q_total, 1)

@@ -1,0 +1,46 @@
+"""The decompression with error feedback and update against float64 at the edges of its strips."""
+import pytest
+import torch
+
+from powersgd_b200 import Config, PowerSGD, optimizer_step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rank,iters", [(2, 1), (4, 2), (8, 2), (16, 1), (11, 2), (16, 2)])
+@pytest.mark.parametrize("momentum", [0.0, 0.9])
+def test_decompression_and_update_at_strip_edges(rank, iters, momentum):
+    """Residual and update of one step in float64 from the factors the launches used (at most 32 products
+    per entry, each side rounded to float32): off by at most about (K + 3) 2^-24 of the terms' sizes."""
+    shapes = [s for s in [(40, 66), (95, 130), (97, 129), (161, 512), (300, 260), (64, 257)]]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    draw = lambda s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    params = [torch.nn.Parameter(draw(s)) for s in shapes]
+    opt = torch.optim.SGD(params, lr=0.1, momentum=momentum)
+    for p in params:
+        p.grad = draw(p.shape)
+        if momentum:
+            opt.state[p]["momentum_buffer"] = draw(p.shape)
+    before = [(p.detach().double().clone(), p.grad.double().clone(), opt.state[p]["momentum_buffer"].double().clone() if momentum else None) for p in params]
+    agg = PowerSGD(params, Config(rank=rank, min_compression_rate=0.1, num_iters_per_step=iters, start_compressing_after_num_steps=0))
+    optimizer_step(opt, agg)
+    core, nat = agg._powersgd, agg._powersgd._native
+    for grp in core.plan.groups:
+        for pos, idx in enumerate(grp.members):
+            p0, q0 = grp.p_offset + pos * grp.n * grp.r, grp.q_offset + pos * grp.m * grp.r
+            cut = lambda buf, at, rows: buf[at : at + rows * grp.r].view(rows, grp.r).double()  # noqa: E731
+            update = size = 0.0
+            for t in range(iters):
+                left, right = (nat.h_in[t], nat.h_loc[t]) if t % 2 == 0 else (nat.h_loc[t], nat.h_in[t])
+                L, R = cut(left, p0, grp.n), cut(right, q0, grp.m)
+                update, size = update + L @ R.T, size + L.abs() @ R.abs().T
+            p, grad, mom = before[idx]
+            p, grad = p.view(grp.n, grp.m), grad.view(grp.n, grp.m)
+            eps = (grp.r * iters + 3) * 2.0 ** -24
+            now = params[idx]
+            assert ((now.grad.double().view_as(grad) - (grad - update)).abs() <= eps * (size + grad.abs())).all(), shapes[idx]
+            v = update if mom is None else momentum * mom.view_as(p) + update
+            bound = eps * (size + (0 if mom is None else mom.view_as(p).abs()))
+            if mom is not None:
+                assert ((opt.state[now]["momentum_buffer"].double().view_as(p) - v).abs() <= bound).all(), shapes[idx]
+            assert ((now.detach().double().view_as(p) - (p - 0.1 * v)).abs() <= bound + 2.0 ** -23 * (p.abs() + v.abs())).all(), shapes[idx]
