@@ -18,6 +18,8 @@ namespace {
 constexpr int TK_THREADS = 512;
 constexpr int TK_BINS0 = 2048, TK_BINS1 = 2048, TK_BINS2 = 512;
 
+constexpr int TK_FOUND = 1024;   // selected entries a block collects before it hands them out
+
 // workspace layout (ints): hist0[2048] hist1[2048] hist2[512] | cnt_gt, cnt_eq
 constexpr int TK_WS_INTS = TK_BINS0 + TK_BINS1 + TK_BINS2 + 8;
 
@@ -142,10 +144,10 @@ struct TopkItem {
 };
 
 // Block-wide: walks `bins` (<= 2048, TK_THREADS threads x 4 bins) from the top until `remain` entries are
-// covered; returns the bin in *bin_out and the number to take inside it in *remain_io. `scan` is
-// TK_THREADS ints of shared memory.
+// covered; returns the bin in *bin_out and the number to take inside it in *remain_io. `scan`: one
+// int per warp.
 __device__ void tk_choose_block(const int* __restrict__ hist, int bins, long long* remain_io, int* bin_out, int* scan) {
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   // thread t owns bins [4t, 4t + 4), counted from the TOP: bin index bins - 1 - j
   int c[4], local = 0;
 #pragma unroll
@@ -154,17 +156,20 @@ __device__ void tk_choose_block(const int* __restrict__ hist, int bins, long lon
     c[u] = j < bins ? hist[bins - 1 - j] : 0;
     local += c[u];
   }
-  scan[t] = local;
-  __syncthreads();
-  // inclusive prefix sum over the TK_THREADS partials (Hillis-Steele; 9 rounds)
-  for (int off = 1; off < TK_THREADS; off <<= 1) {
-    const int v = t >= off ? scan[t - off] : 0;
-    __syncthreads();
-    scan[t] += v;
-    __syncthreads();
+  // exclusive prefix sum: inside the warp by shuffles, then over the warps before this one
+  int upto = local;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, upto, off);
+    if (lane >= off) upto += v;
   }
+  if (lane == 31) scan[warp] = upto;
+  __syncthreads();
+  int base = 0;
+#pragma unroll
+  for (int w = 0; w < TK_THREADS / 32; ++w) base += w < warp ? scan[w] : 0;
   const long long remain = *remain_io;
-  const long long before = t == 0 ? 0 : scan[t - 1];   // entries in the bins above this thread's
+  const long long before = base + upto - local;   // entries in the bins above this thread's
   __syncthreads();
   if (before < remain && remain <= before + local) {    // exactly one thread
     long long left = remain - before;
@@ -179,6 +184,34 @@ __device__ void tk_choose_block(const int* __restrict__ hist, int bins, long lon
     }
   }
   __syncthreads();
+}
+
+// Calls f(value, index) for every entry of a block's part of a tensor (parts are interleaved in runs of
+// one block's accesses). 16-byte loads, four of a thread in flight, when the tensor allows them: a
+// pass is bound by the reads, which the L2 cache or HBM serve at TB/s only with that much under way.
+template <class F>
+__device__ __forceinline__ void tk_for_each(const float* __restrict__ x, long long n, int part, int parts, F f) {
+  const long long stride = (long long)parts * TK_THREADS;
+  long long i = (long long)part * TK_THREADS + threadIdx.x;
+  if (((uintptr_t)x & 15u) == 0) {
+    const float4* x4 = reinterpret_cast<const float4*>(x);
+    const long long n4 = n >> 2;
+    for (; i < n4; i += 4 * stride) {
+      float4 q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * stride < n4) q[u] = __ldg(x4 + i + u * stride);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * stride < n4) f(q[u], (i + u * stride) * 4, 4);
+    }
+    if (part == 0 && (long long)threadIdx.x < n - n4 * 4) {
+      const long long e = n4 * 4 + threadIdx.x;
+      f(make_float4(__ldg(x + e), 0.f, 0.f, 0.f), e, 1);
+    }
+  } else {
+    for (; i < n; i += stride) f(make_float4(__ldg(x + i), 0.f, 0.f, 0.f), i, 1);
+  }
 }
 
 // Digits chosen so far for one tensor (block-wide; result in shared `pick`).
@@ -211,8 +244,10 @@ __device__ void tk_derive_block(const int* ws, int upto, long long k, Pick* pick
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                           const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                           int* __restrict__ ws_all, int pass) {
-  __shared__ int sh[TK_BINS0];
-  __shared__ int scan[TK_THREADS];
+  // four copies of the histogram, by lane: the leading digit of a gradient takes a few dozen values,
+  // and lanes that meet on one address are served one after another
+  __shared__ __align__(16) int sh[TK_BINS0 * 4];
+  __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
   __shared__ long long remain_sh;
   __shared__ int bin_sh;
@@ -220,35 +255,47 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const T
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
   const int bins = pass == 2 ? TK_BINS2 : TK_BINS0;
-  for (int b = threadIdx.x; b < bins; b += TK_THREADS) sh[b] = 0;
+  for (int b = threadIdx.x; b < bins * 4; b += TK_THREADS) sh[b] = 0;
   tk_derive_block(ws, pass, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned prefix = pick.prefix;
   const unsigned mask = pass == 0 ? 0u : (pass == 1 ? 0x7FF00000u : 0x7FFFFE00u);
   const int shift = pass == 0 ? 20 : (pass == 1 ? 9 : 0);
   const unsigned digit_mask = pass == 2 ? 0x1FFu : 0x7FFu;
-  const long long stride = (long long)item_parts[it] * TK_THREADS;
-#pragma unroll 4
-  for (long long i = (long long)block_part[blockIdx.x] * TK_THREADS + threadIdx.x; i < item.n; i += stride) {
-    const unsigned key = tk_key(__ldg(item.x + i));
-    if ((key & mask) == prefix) atomicAdd(&sh[(key >> shift) & digit_mask], 1);
-  }
+  int* mine = sh + (threadIdx.x & 3);
+  tk_for_each(item.x, item.n, block_part[blockIdx.x], item_parts[it], [&](const float4& q, long long, int count) {
+    const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const unsigned key = tk_key(v[j]);
+      if (j < count && (key & mask) == prefix) atomicAdd(mine + 4 * ((key >> shift) & digit_mask), 1);
+    }
+  });
   __syncthreads();
   int* hist = ws + (pass == 0 ? 0 : (pass == 1 ? TK_BINS0 : TK_BINS0 + TK_BINS1));
-  for (int b = threadIdx.x; b < bins; b += TK_THREADS)
-    if (sh[b]) atomicAdd(hist + b, sh[b]);
+  for (int b = threadIdx.x; b < bins; b += TK_THREADS) {
+    const int4 c = reinterpret_cast<const int4*>(sh)[b];
+    const int total = c.x + c.y + c.z + c.w;
+    if (total) atomicAdd(hist + b, total);
+  }
 }
 
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                              const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                              int* __restrict__ ws_all, float* __restrict__ values,
                                                                              int* __restrict__ positions) {
-  __shared__ int scan[TK_THREADS];
+  __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
   __shared__ long long remain_sh;
   __shared__ int bin_sh;
+  // entries above the threshold are collected here and handed out with one addition to the tensor's
+  // counter per block: thousands of additions to one address would be served one after another
+  __shared__ float found_v[TK_FOUND];
+  __shared__ int found_p[TK_FOUND];
+  __shared__ int found, found_base;
   const int it = block_item[blockIdx.x];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
+  if (threadIdx.x == 0) found = 0;
   tk_derive_block(ws, 3, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned threshold = pick.prefix;
   const long long take_equal = pick.remain;
@@ -257,21 +304,54 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
   int* cnt_eq = cnt_gt + 1;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
-  const long long stride = (long long)item_parts[it] * TK_THREADS;
-  for (long long i = (long long)block_part[blockIdx.x] * TK_THREADS + threadIdx.x; i < item.n; i += stride) {
-    const float v = __ldg(item.x + i);
-    const unsigned key = tk_key(v);
-    long long slot = -1;
-    if (key > threshold) slot = atomicAdd(cnt_gt, 1);
-    else if (key == threshold) {
-      const long long e = atomicAdd(cnt_eq, 1);
-      if (e < take_equal) slot = base_equal + e;
+  const bool wide = ((uintptr_t)item.memory & 15u) == 0;
+  tk_for_each(item.x, item.n, block_part[blockIdx.x], item_parts[it], [&](const float4& q, long long first, int count) {
+    const float v[4] = {q.x, q.y, q.z, q.w};
+    float rest[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      rest[j] = v[j];
+      const unsigned key = tk_key(v[j]);
+      if (j < count && key >= threshold) {
+        const int i = (int)(first + j);
+        if (key > threshold) {
+          const int slot = atomicAdd(&found, 1);
+          if (slot < TK_FOUND) {
+            found_v[slot] = v[j];
+            found_p[slot] = i;
+          } else {
+            const int at = atomicAdd(cnt_gt, 1);
+            val[at] = v[j];
+            pos[at] = i;
+          }
+          rest[j] = 0.f;
+        } else {
+          const long long e = atomicAdd(cnt_eq, 1);
+          if (e < take_equal) {
+            val[base_equal + e] = v[j];
+            pos[base_equal + e] = i;
+            rest[j] = 0.f;
+          }
+        }
+      }
     }
-    if (slot >= 0) {
-      val[slot] = v;
-      pos[slot] = (int)i;
+    if (item.memory) {
+      if (count == 4 && wide) {
+        *reinterpret_cast<float4*>(item.memory + first) = make_float4(rest[0], rest[1], rest[2], rest[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < count) item.memory[first + j] = rest[j];
+      }
     }
-    if (item.memory) item.memory[i] = slot >= 0 ? 0.f : v;
+  });
+  __syncthreads();
+  const int mine = min(found, TK_FOUND);
+  if (threadIdx.x == 0 && mine) found_base = atomicAdd(cnt_gt, mine);
+  __syncthreads();
+  for (int e = threadIdx.x; e < mine; e += TK_THREADS) {
+    val[found_base + e] = found_v[e];
+    pos[found_base + e] = found_p[e];
   }
 }
 
@@ -337,15 +417,19 @@ __global__ void __launch_bounds__(SC_THREADS) psgd_sparse_combine_kernel(const f
                                                                           const int* __restrict__ positions, int workers,
                                                                           long long per_worker, const SparseSeg* __restrict__ segs,
                                                                           int nsegs, float divisor, unsigned* barrier, int* status) {
-  __shared__ long long ends[SC_MAX_SEGMENTS];
-  for (int s = threadIdx.x; s < nsegs; s += SC_THREADS) ends[s] = segs[s].end;
+  // the table travels to shared memory in one go: walked in global memory it costs the zero fill one
+  // dependent round trip per segment
+  __shared__ SparseSeg seg[SC_MAX_SEGMENTS];
+  for (int s = threadIdx.x; s < nsegs; s += SC_THREADS) seg[s] = segs[s];
   __syncthreads();
   const long long tid = (long long)blockIdx.x * SC_THREADS + threadIdx.x;
   const long long stride = (long long)gridDim.x * SC_THREADS;
   for (int s = 0; s < nsegs; ++s) {
-    float* out = segs[s].out;
-    const long long n = segs[s].numel;
-    for (long long i = tid; i < n; i += stride) out[i] = 0.f;
+    float* out = seg[s].out;
+    const long long n = seg[s].numel;
+    const long long n4 = ((uintptr_t)out & 15u) == 0 ? n >> 2 : 0;
+    for (long long i = tid; i < n4; i += stride) reinterpret_cast<float4*>(out)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long i = n4 * 4 + tid; i < n; i += stride) out[i] = 0.f;
   }
   // value * (1 / W) rounded, then added: what torch's division by a scalar followed by index_add_
   // computes on the GPU (no fused multiply-add), so the result matches that sequence bit for bit
@@ -362,10 +446,10 @@ __global__ void __launch_bounds__(SC_THREADS) psgd_sparse_combine_kernel(const f
       int lo = 0, hi = nsegs - 1;   // first segment whose end is above j
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (ends[mid] > j) hi = mid; else lo = mid + 1;
+        if (seg[mid].end > j) hi = mid; else lo = mid + 1;
       }
       const long long p = pos[j];
-      if (p >= 0 && p < segs[lo].numel) segs[lo].out[p] = __fadd_rn(segs[lo].out[p], __fmul_rn(val[j], inv));
+      if (p >= 0 && p < seg[lo].numel) seg[lo].out[p] = __fadd_rn(seg[lo].out[p], __fmul_rn(val[j], inv));
     }
   }
 }

@@ -87,14 +87,16 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
             raise RuntimeError("top-k item record out of sync with the native library")
         items = np.zeros(len(flats), dtype=dtype)
         block_item, block_part, parts = [], [], []
-        at = 0
+        at, total_n = 0, max(1, sum(f.numel() for f in flats))
         for i, (f, k, m) in enumerate(zip(flats, ks, mems)):
             n = f.numel()
             if not (0 < k <= n < (1 << 31)):
                 raise ValueError(f"topk_abs_many: need 0 < k <= n < 2^31 (k = {k}, n = {n})")
             items[i] = (f.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at)
             at += k
-            nparts = max(1, min(256, -(-n // (512 * 8))))   # <= 8 elements per thread and pass up to 1 Mi entries, then longer loops
+            # blocks of 512 threads with at least 16 elements each, some four per SM for the whole list:
+            # every block pays for its histogram (zeroing, choosing the digits so far, adding it up)
+            nparts = max(1, min(-(-n // (512 * 16)), -(-592 * n // total_n)))
             parts.append(nparts)
             block_item += [i] * nparts
             block_part += list(range(nparts))
