@@ -21,6 +21,7 @@ Factor bookkeeping for half-iteration t of a step (left = the P side is the inpu
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -75,22 +76,51 @@ def _ptr_array(tensors: Sequence[torch.Tensor]):
     return arr
 
 
-def _to_device(array: np.ndarray, device: torch.device) -> torch.Tensor:
-    """Upload a descriptor table. Staged through pinned memory with an async copy on the current
-    stream, so that it is legal during CUDA-graph capture (where it becomes a copy node that
-    re-reads the pinned buffer on every replay; the buffer is kept alive with the result)."""
-    raw = np.ascontiguousarray(array).view(np.uint8).reshape(-1)
-    pinned = torch.empty(max(raw.size, 1), dtype=torch.uint8).pin_memory()
-    pinned.numpy()[: raw.size] = raw
-    out = torch.empty(max(raw.size, 1), dtype=torch.uint8, device=device)
-    out.copy_(pinned, non_blocking=True)
-    out._psgd_pinned_src = pinned
+_upload_streams: Dict[torch.device, torch.cuda.Stream] = {}
+
+
+@contextlib.contextmanager
+def _outside_capture(device: torch.device):
+    """Runs its body at once, whether or not a CUDA graph is being recorded on the current stream: what
+    never changes (descriptor tables, cleared counters) is put in place once instead of by a node that
+    every replay of the graph pays for (eight copies of 1.3 us each in the step of a small perceptron).
+    Under capture the body gets a stream that is not part of it, so that its tensors come from the
+    ordinary pool - memory of the graph's own pool may be written by an earlier node of the same graph -
+    and is waited for."""
+    if not torch.cuda.is_current_stream_capturing():
+        yield
+        return
+    device = torch.device("cuda", torch.cuda.current_device()) if device.index is None else device
+    while True:
+        stream = _upload_streams.setdefault(device, torch.cuda.Stream(device=device))
+        with torch.cuda.stream(stream):
+            if torch.cuda.is_current_stream_capturing():   # streams are handed out in turn: this one was forked into the capture
+                del _upload_streams[device]
+                continue
+            yield
+            stream.synchronize()
+            return
+
+
+def _keep_with_graph(*tensors: torch.Tensor) -> None:
+    """Tensors whose addresses are being recorded must live as long as the graph does, whatever later
+    rebinding drops them from their owner. Inside a `capture_scope` the graph's owner keeps them; a
+    capture made without one parks them here for the life of the process."""
     if torch.cuda.is_current_stream_capturing():
-        # the recorded copy node reads `pinned` and writes `out` on every replay: both must
-        # outlive whatever later rebinding drops them from their owner, i.e. live as long as the
-        # graph does. Inside a `capture_scope` the graph's owner keeps them; a capture made
-        # without one parks them here for the life of the process.
-        (_capture_keep if _capture_keep is not None else _CAPTURED_TABLES).append((out, pinned))
+        (_capture_keep if _capture_keep is not None else _CAPTURED_TABLES).append(tensors)
+
+
+def _to_device(array: np.ndarray, device: torch.device) -> torch.Tensor:
+    """Upload a descriptor table: staged through pinned memory with an async copy on the current stream
+    (at once and outside the graph while one is being recorded)."""
+    raw = np.ascontiguousarray(array).view(np.uint8).reshape(-1)
+    with _outside_capture(device):
+        pinned = torch.empty(max(raw.size, 1), dtype=torch.uint8).pin_memory()
+        pinned.numpy()[: raw.size] = raw
+        out = torch.empty(max(raw.size, 1), dtype=torch.uint8, device=device)
+        out.copy_(pinned, non_blocking=True)
+        out._psgd_pinned_src = pinned
+    _keep_with_graph(out)
     return out
 
 
@@ -453,7 +483,9 @@ class NativeCompressor:
         self._split_tile_lists()
         self._partial = torch.empty(self.tiles.partial_floats, device=self.device, dtype=torch.float32)
         self._partial_tc = torch.empty(self.tiles.partial_tc_floats, device=self.device, dtype=torch.float32)
-        self._tickets = torch.zeros(self.tiles.n_tickets, device=self.device, dtype=torch.int32)
+        with _outside_capture(self.device):   # zero between launches: every launch leaves them so
+            self._tickets = torch.zeros(self.tiles.n_tickets, device=self.device, dtype=torch.int32)
+        _keep_with_graph(self._tickets)
         self._out_views = out_views
         self._key = key
 
@@ -866,7 +898,6 @@ class NativeFlatAllReduce:
         device = grads[0].device
         # every tensor starts at a multiple of four floats in the flat buffer (16-byte accesses)
         total = sum(-(-g.numel() // 4) * 4 for g in grads)
-        self._flat = torch.zeros(total, device=device, dtype=torch.float32)
         self._out = torch.empty(total, device=device, dtype=torch.float32) if (need_out and outs is None) else None
         items = np.zeros(len(grads), dtype=layout.FLAT_DTYPE)
         per_block = self.lib.psgd_flat_block_elems()
@@ -907,9 +938,9 @@ class NativeFlatAllReduce:
         self._views = views
         self._hyper_dev = _to_device(NativeCompressor._default_hyper(), device)
         self._key = key
-        self._choose_path(total, world_size())
+        self._choose_path(total, world_size(), device)
 
-    def _choose_path(self, total: int, workers: int) -> None:
+    def _choose_path(self, total: int, workers: int, device: torch.device) -> None:
         """local | oneshot (flag-in-data words to every peer) | bulk (two-shot, plain floats +
         chunk flags; the flat buffer lives in the symmetric arena; PSGD_B200_FLAT=bulk forces it
         for small buffers too) | nvls (PSGD_B200_FLAT=nvls: in-switch reduction of a buffer bound to
@@ -946,7 +977,11 @@ class NativeFlatAllReduce:
             from .parallel.symm import Channel
 
             self.comm = Channel(cap)
-        if path == "bulk":
+        if path in ("nccl", "oneshot"):
+            self._flat = torch.zeros(total, device=device, dtype=torch.float32)
+        elif path == "local":
+            self._flat = None   # one worker: nothing is packed
+        elif path == "bulk":
             # pack writes and unpack reads the arena's data region directly
             self._flat = self.comm.slots.tensor(0, self.n_pad)
         elif path == "nvls":

@@ -1,0 +1,36 @@
+"""Descriptor tables built while a CUDA graph is being recorded are put in place once, outside the graph:
+its replays must find them intact although the graph's own memory is written over and over."""
+import pytest
+import torch
+
+from powersgd_b200 import BasicConfig, BasicPowerSGD
+from powersgd_b200.cuda_path import capture_scope
+
+pytestmark = pytest.mark.gpu
+
+
+def test_tables_bound_under_capture_survive_replays():
+    shapes = [(96, 200), (300, 260), (64, 27)]
+    make = lambda: BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=2, num_iters_per_step=2), backend="native")  # noqa: E731
+    g = torch.Generator(device="cuda").manual_seed(0)
+    fresh = [torch.randn(s, generator=g, device="cuda") for s in shapes]
+    ours, plain = make(), make()
+    ours.aggregate([f.clone() for f in fresh])     # builds the native object; its tables are bound anew below
+    plain.aggregate([f.clone() for f in fresh])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with capture_scope() as keep, torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        for size in (64, 512, 4096, 1 << 16, 1 << 20):   # blocks of every size the tables could be given, written and let go
+            scratch = torch.full((size,), -1, dtype=torch.int32, device="cuda")
+            del scratch
+        grads = [f * 1.0 for f in fresh]
+        outs = ours.aggregate(grads)
+    assert keep
+    for step in range(3):
+        for f in fresh:
+            f.copy_(torch.randn(f.shape, generator=g, device="cuda"))
+        graph.replay()
+        want_grads = [f.clone() for f in fresh]
+        want = plain.aggregate(want_grads)
+        for a, b in zip(list(outs) + grads, list(want) + want_grads):
+            assert torch.equal(a, b), step
