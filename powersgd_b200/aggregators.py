@@ -169,19 +169,25 @@ class PowerSGD(Aggregator):
         # the fused path never calls optimizer.step(): registered step hooks would not fire
         if getattr(optimizer, "_optimizer_step_pre_hooks", None) or getattr(optimizer, "_optimizer_step_post_hooks", None):
             return False
+        # one pass over the parameters, with comparisons that stay inside the tensor library where the
+        # answer is the usual one: this runs before every step of an eager loop
+        state, f32 = optimizer.state, torch.float32
         for group in optimizer.param_groups:
             if group.get("maximize", False) or group.get("differentiable", False):
                 return False
-            seen = [("momentum_buffer" in optimizer.state.get(p, {})) and optimizer.state[p]["momentum_buffer"] is not None
-                    for p in group["params"]]
-            if any(seen) and not all(seen):
-                return False
+            buffers = 0
             for p in group["params"]:
-                if p.dtype != torch.float32 or p.grad is None or not is_dense(p) or not same_layout(p.grad, p):
+                grad = p.grad
+                if grad is None or p.dtype != f32 or not (p.is_contiguous() or is_dense(p)) or not same_layout(grad, p):
                     return False
-                buf = optimizer.state.get(p, {}).get("momentum_buffer")
-                if buf is not None and not same_layout(buf, p):
-                    return False
+                own = state.get(p)
+                buf = own.get("momentum_buffer") if own else None
+                if buf is not None:
+                    buffers += 1
+                    if not same_layout(buf, p):
+                        return False
+            if buffers and buffers != len(group["params"]):
+                return False
         return True
 
     def close(self) -> None:

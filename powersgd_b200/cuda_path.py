@@ -349,6 +349,8 @@ class NativeCompressor:
         self._orth_part = torch.zeros(max(max(self.n_chunks.values()), 1) * part_doubles, device=self.device, dtype=torch.float64)
         self._orth_rinv = torch.zeros(max_units * 2 * rt * rt, device=self.device, dtype=torch.float32)
         self._key = None
+        self._tape: Optional[list] = None
+        self._tapes: Dict[Tuple, list] = {}
         self._out_arena: Optional[torch.Tensor] = None
         self._hyper_dev = _to_device(self._default_hyper(), self.device)
         self.launches = 0  # kernels launched by the last aggregate()
@@ -487,6 +489,7 @@ class NativeCompressor:
             self._tickets = torch.zeros(self.tiles.n_tickets, device=self.device, dtype=torch.int32)
         _keep_with_graph(self._tickets)
         self._out_views = out_views
+        self._tapes.clear()
         self._key = key
 
     # -- early bucket ---------------------------------------------------------------------
@@ -533,6 +536,45 @@ class NativeCompressor:
         self._early_product_done = done
         return True
 
+    # -- launches --------------------------------------------------------------------------
+    def _call(self, name: str, *args) -> None:
+        """One launch of the library on the current stream, counted, and written down while a step is
+        being recorded (see `_taped`)."""
+        fn = getattr(self.lib, name)
+        native.check(fn(*args, _stream_ptr()), name)
+        launched = 2 if name == "psgd_orth_launch" else 1   # orthonormalisation: Gram matrices, then their use
+        self.launches += launched
+        if self._tape is not None:
+            self._tape.append((fn, name, args, launched))
+
+    def _taped(self, key: Tuple, body) -> None:
+        """Run `body`, which issues the launches of a step; from the second step of its kind on repeat
+        the same calls with the arguments they had, without working them out again (an eager loop over
+        a small model spends most of its step there). `key`: whatever the arguments depend on beyond
+        the bound tensors; a new binding drops all tapes. Only where a step is nothing but launches on
+        one stream: one worker, nothing launched ahead, no phase timing."""
+        plain = (world_size() == 1 and self.comm is None and self._early is None and self._early_product_done is None
+                 and not _Range.enabled and _Range.events is None)
+        if not plain:
+            body()
+            return
+        key = key + (self.core._ps_buffer.data_ptr(), self.core._qs_buffer.data_ptr())
+        tape = self._tapes.get(key)
+        if tape is None:
+            self._tape = []
+            try:
+                body()
+                self._tapes[key] = self._tape
+            finally:
+                self._tape = None
+            return
+        stream = _stream_ptr()
+        for fn, name, args, launched in tape:
+            code = fn(*args, stream)
+            if code != 0:
+                native.check(code, name)
+            self.launches += launched
+
     # -- phases ----------------------------------------------------------------------------
     def _orth(self, side: str, x: torch.Tensor, copy_to: torch.Tensor, prev: List[torch.Tensor], cm: List[torch.Tensor],
               gather_to: Optional[torch.Tensor] = None, early: bool = False):
@@ -540,7 +582,8 @@ class NativeCompressor:
         filled with the sum over workers of the factor the previous product pushed (the sum is
         also written to `gather_to`): the launch is the consumer of the in-kernel all-reduce.
         `early`: see `_chained`."""
-        code = self.lib.psgd_orth_launch(
+        self._call(
+            "psgd_orth_launch",
             _ptr(self.units[side]),
             self.n_units[side],
             _ptr(self.chunks[side]),
@@ -556,10 +599,7 @@ class NativeCompressor:
             self.comm.ptr if gather_to is not None else ctypes.c_void_p(0),
             _ptr(gather_to),
             int(early),
-            _stream_ptr(),
         )
-        native.check(code, "psgd_orth_launch")
-        self.launches += 2  # partial Gram matrices, then factorisation + application of R^-1
 
     def _chained(self) -> bool:
         """May a launch whose direct predecessor in the stream is a launch of the same step start
@@ -576,7 +616,8 @@ class NativeCompressor:
         form = (1 if transposed else 0) | (2 if early else 0)
         tiles, count = self._tiles_dev[name]["tc"]
         if count and part != "early":
-            code = self.lib.psgd_gemm_tc_launch(
+            self._call(
+                "psgd_gemm_tc_launch",
                 form,
                 1 if self._tc_split else 0,
                 self.tiles.max_r,
@@ -594,13 +635,11 @@ class NativeCompressor:
                 _ptr(self._tickets),
                 self.comm.ptr if self.comm is not None else ctypes.c_void_p(0),
                 self._status.dev_ptr,
-                _stream_ptr(),
             )
-            native.check(code, "psgd_gemm_tc_launch")
-            self.launches += 1
         tiles, count = self._tiles_dev[name]["f" if part == "all" else ("fA" if part == "early" else "fB")]
         if count:
-            code = self.lib.psgd_gemm_ffma_launch(
+            self._call(
+                "psgd_gemm_ffma_launch",
                 form,
                 self.tiles.max_r,
                 _ptr(self._mats_dev),
@@ -615,10 +654,7 @@ class NativeCompressor:
                 _ptr(self._partial),
                 _ptr(self._tickets),
                 self.comm.ptr if self.comm is not None else ctypes.c_void_p(0),
-                _stream_ptr(),
             )
-            native.check(code, "psgd_gemm_ffma_launch")
-            self.launches += 1
 
     def _gathers_in_finalize(self) -> bool:
         """Multi-GPU: can the decompression launch gather the last factor from the channel itself?
@@ -647,7 +683,8 @@ class NativeCompressor:
                 lloc.append(self.h_loc[t]); lsum.append(self.h_sum[t])
         tiles, count = self._tiles_dev["fin"]["tc"]
         if count:
-            code = self.lib.psgd_finalize_tc_launch(
+            self._call(
+                "psgd_finalize_tc_launch",
                 _ptr(self._mats_dev),
                 _ptr(tiles),
                 count,
@@ -662,14 +699,12 @@ class NativeCompressor:
                 1.0 / workers,
                 1 if fused_sgd else 0,
                 self._status.dev_ptr,
-                _stream_ptr(),
             )
-            native.check(code, "psgd_finalize_tc_launch")
-            self.launches += 1
         tiles, count = self._tiles_dev["fin"]["f"]
         if count:
             gather = gather_state is not None
-            code = self.lib.psgd_finalize_launch(
+            self._call(
+                "psgd_finalize_launch",
                 _ptr(self._mats_dev),
                 _ptr(tiles),
                 count,
@@ -690,10 +725,7 @@ class NativeCompressor:
                 int(flags),
                 1.0,
                 int(early and not self._tiles_dev["fin"]["tc"][1]),
-                _stream_ptr(),
             )
-            native.check(code, "psgd_finalize_launch")
-            self.launches += 1
 
     def _half_iterations(self):
         """Runs the T half-iterations. Returns (sides, pending): `pending` is the warm-start buffer
@@ -811,18 +843,24 @@ class NativeCompressor:
         self.check()
         self.launches = self._early_launches if self._early is not None else 0
         self._bind(gradients)
+        self._taped((self._first_left(), False), lambda: self._step(fused_sgd=False))
+        return list(self._out_views)
+
+    def _first_left(self) -> bool:
+        return (self.core.step_counter * self.T) % 2 == 0
+
+    def _step(self, fused_sgd: bool) -> None:
         workers = world_size()
         if workers == 1:
             saved = self.h_sum
             self.h_sum = self.h_loc
         try:
             sides, pending = self._half_iterations()
-            with _Range("psgd.finalize"):
-                self._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending, early=self._follows)
+            with _Range("psgd.finalize+sgd" if fused_sgd else "psgd.finalize"):
+                self._finalize(sides, fused_sgd=fused_sgd, workers=workers, gather_state=pending, early=self._follows)
         finally:
             if workers == 1:
                 self.h_sum = saved
-        return list(self._out_views)
 
     def aggregate_and_step(
         self,
@@ -837,20 +875,12 @@ class NativeCompressor:
         self.check()
         self.launches = self._early_launches if self._early is not None else 0
         self._bind(gradients, params, moms, hyper_index, need_out=False)
-        workers = world_size()
         keep = self._hyper_dev
         self._hyper_dev = hyper_dev
-        if workers == 1:
-            saved = self.h_sum
-            self.h_sum = self.h_loc
         try:
-            sides, pending = self._half_iterations()
-            with _Range("psgd.finalize+sgd"):
-                self._finalize(sides, fused_sgd=True, workers=workers, gather_state=pending, early=self._follows)
+            self._taped((self._first_left(), True, hyper_dev.data_ptr()), lambda: self._step(fused_sgd=True))
         finally:
             self._hyper_dev = keep
-            if workers == 1:
-                self.h_sum = saved
 
 
 class NativeFlatAllReduce:
@@ -1180,6 +1210,7 @@ class FusedSGDDriver:
         self._cursor = 0
         self._hyper_dev: Optional[torch.Tensor] = None
         self._cache_key = None
+        self._last_values = None   # what the device table holds
         self._flat_all = NativeFlatAllReduce()
         self._flat_plain = NativeFlatAllReduce()
         self.launches = 0
@@ -1208,6 +1239,11 @@ class FusedSGDDriver:
                     else:
                         moms.append(None)
             self._params, self._moms, self._index = params, moms, index
+            mask = self.agg.is_compressed_mask
+            if len(params) == len(mask):
+                # the same lists, compressed and uncompressed tensors apart (True / False)
+                self._split = {keep: tuple([x for x, k in zip(xs, mask) if k == keep] for xs in (params, moms, index))
+                               for keep in (True, False)}
             self._grads = [p.grad.data for p in params]
             self._cache_key = key
         return fresh_groups
@@ -1216,6 +1252,9 @@ class FusedSGDDriver:
         """Host side of a step: momentum buffers, hyper-parameter table, async upload."""
         fresh = self._collect(optimizer)
         groups = optimizer.param_groups
+        values = [(float(g["lr"]), float(g["momentum"]), float(g["dampening"]), float(g["weight_decay"]), bool(g["nesterov"])) for g in groups]
+        if not fresh and values == self._last_values:
+            return  # nothing changed since the last upload: the device table is already right
         table = np.zeros(len(groups), dtype=layout.HYPER_DTYPE)
         for gi, group in enumerate(groups):
             mu = float(group["momentum"])
@@ -1232,10 +1271,8 @@ class FusedSGDDriver:
             self._slots = [torch.empty(nbytes, dtype=torch.uint8).pin_memory() for _ in range(self.RING)]
             self._slot_events = [None] * self.RING
             self._hyper_dev = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        blob = table.tobytes()
-        if not fresh and blob == getattr(self, "_last_blob", None):
-            return  # nothing changed since the last upload: the device table is already right
-        self._last_blob = blob
+        # a fresh momentum buffer uploads a table for this step only
+        self._last_values = None if fresh else values
         i = self._cursor
         self._cursor = (i + 1) % self.RING
         if self._slot_events[i] is not None:
@@ -1278,8 +1315,9 @@ class FusedSGDDriver:
             self.prepare(optimizer)
         # the gradient tensors may have been replaced since the last step (dropped zero gradients
         # re-created by autograd, a loaded checkpoint): always bind what the parameters hold now
-        if any(p.grad.data_ptr() != g.data_ptr() for p, g in zip(self._params, self._grads)):
-            self._grads = [p.grad.data for p in self._params]
+        now = [p.grad for p in self._params]
+        if [g.data_ptr() for g in now] != [g.data_ptr() for g in self._grads]:
+            self._grads = [g.data for g in now]
         agg = self.agg
         hyper_dev, index, params, moms, grads = self._hyper_dev, self._index, self._params, self._moms, self._grads
         if len(grads) != len(agg.is_compressed_mask):
@@ -1290,23 +1328,20 @@ class FusedSGDDriver:
             self.launches = self._flat_all.launches
             return
         mask = agg.is_compressed_mask
-        pick = lambda xs, keep: [x for x, k in zip(xs, mask) if k == keep]  # noqa: E731
         core = agg._powersgd
         self.launches = 0
         if core.params:
             if core._native is None:
                 core._native = NativeCompressor(core)
-            core._native.aggregate_and_step(
-                pick(grads, True), pick(params, True), pick(moms, True), pick(index, True), hyper_dev
-            )
+            core._native.aggregate_and_step([g for g, k in zip(grads, mask) if k], *self._split[True], hyper_dev)
             core.step_counter += 1
             self.launches += core._native.launches
-        plain = pick(grads, False)
+        plain = [g for g, k in zip(grads, mask) if not k]
         if plain:
             # after the low-rank path: a consumer that spins on its peers next to the product
             # kernels (tried as a parallel side-stream branch) cost more than it hid
             self._flat_plain.aggregate_and_step(
-                plain, pick(params, False), pick(moms, False), pick(index, False), hyper_dev,
+                plain, *self._split[False], hyper_dev,
                 early=bool(core.params) and core._native._chained(),
             )
             self.launches += self._flat_plain.launches

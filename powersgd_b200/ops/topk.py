@@ -59,13 +59,13 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     the taken entries zeroed. Falls back to one `topk_abs` per tensor off the GPU."""
     ks = [int(k) for k in ks]
     total = sum(ks)
-    flats = [t.reshape(-1) for t in tensors]
-    mems = list(memories) if memories is not None else [None] * len(flats)
-    device = flats[0].device
+    tensors = list(tensors)
+    mems = list(memories) if memories is not None else [None] * len(tensors)
+    device, f32 = tensors[0].device, torch.float32
     native_ok = (
         device.type == "cuda" and native.use_for_cuda()
-        and all(t.dtype == torch.float32 and t.is_contiguous() for t in tensors)   # flats are then views
-        and all(m is None or (m.is_contiguous() and m.dtype == torch.float32) for m in mems)
+        and all(t.dtype == f32 and t.is_contiguous() for t in tensors)   # their memory is then the flattened tensor
+        and all(m is None or (m.is_contiguous() and m.dtype == f32) for m in mems)
     )
     if not native_ok:
         values = torch.empty(total, dtype=torch.float32, device=device)
@@ -79,20 +79,20 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     import numpy as np
 
     lib = native.lib()
-    key = (device, tuple(f.data_ptr() for f in flats), tuple(0 if m is None else m.data_ptr() for m in mems), tuple(f.numel() for f in flats), tuple(ks))
+    key = (device, tuple(t.data_ptr() for t in tensors), tuple(0 if m is None else m.data_ptr() for m in mems), tuple(t.numel() for t in tensors), tuple(ks))
     entry = _many_cache.get(key)
     if entry is None:
         dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64)])
         if dtype.itemsize != int(lib.psgd_topk_item_bytes()):
             raise RuntimeError("top-k item record out of sync with the native library")
-        items = np.zeros(len(flats), dtype=dtype)
+        items = np.zeros(len(tensors), dtype=dtype)
         block_item, block_part, parts = [], [], []
-        at, total_n = 0, max(1, sum(f.numel() for f in flats))
-        for i, (f, k, m) in enumerate(zip(flats, ks, mems)):
-            n = f.numel()
+        at, total_n = 0, max(1, sum(t.numel() for t in tensors))
+        for i, (t, k, m) in enumerate(zip(tensors, ks, mems)):
+            n = t.numel()
             if not (0 < k <= n < (1 << 31)):
                 raise ValueError(f"topk_abs_many: need 0 < k <= n < 2^31 (k = {k}, n = {n})")
-            items[i] = (f.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at)
+            items[i] = (t.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at)
             at += k
             # blocks of 512 threads with at least 16 elements each, some four per SM for the whole list:
             # every block pays for its histogram (zeroing, choosing the digits so far, adding it up)
@@ -105,7 +105,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
             "items": to_dev(items), "block_item": to_dev(np.asarray(block_item, dtype=np.int32)),
             "block_part": to_dev(np.asarray(block_part, dtype=np.int32)), "parts": to_dev(np.asarray(parts, dtype=np.int32)),
             "nblocks": len(block_item),
-            "ws": torch.zeros(len(flats) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
+            "ws": torch.zeros(len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
         }
         # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
         # valid for whatever tensors present the same addresses again, so no tensor is kept alive
@@ -116,7 +116,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     positions = torch.empty(total, dtype=torch.int32, device=device)
     vp = ctypes.c_void_p
     code = lib.psgd_topk_abs_many(
-        vp(entry["items"].data_ptr()), len(flats), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
+        vp(entry["items"].data_ptr()), len(tensors), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
         vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()),
         vp(torch.cuda.current_stream().cuda_stream),
     )
@@ -126,6 +126,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
 
 _SEG_DTYPE = None
 _combine_scratch = {}
+_segment_cache: dict = {}
 
 
 def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, ends, divisor: float) -> None:
@@ -157,19 +158,28 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
             scratch = torch.zeros(2, dtype=torch.int32, device=device)  # [grid barrier, status]
             _combine_scratch[device] = scratch
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        for first in range(0, len(outs), cap):
-            chunk = list(range(first, min(first + cap, len(outs))))
-            segs = np.zeros(len(chunk), dtype=_SEG_DTYPE)
-            base = ends[first - 1] if first else 0
-            for j, s in enumerate(chunk):
-                segs[j] = (outs[s].data_ptr(), outs[s].numel(), ends[s] - base)
-            segs_dev = torch.from_numpy(segs.view(np.uint8)).to(device, non_blocking=False)
-            width = ends[chunk[-1]] - base
+        # tables of addresses and lengths, kept by exactly those (as the selection's above): building and
+        # uploading one stalls the host until the selection has run
+        key = (device, tuple(o.data_ptr() for o in outs), tuple(o.numel() for o in outs), tuple(ends))
+        tables = _segment_cache.get(key)
+        if tables is None:
+            tables = []
+            for first in range(0, len(outs), cap):
+                chunk = list(range(first, min(first + cap, len(outs))))
+                segs = np.zeros(len(chunk), dtype=_SEG_DTYPE)
+                base = ends[first - 1] if first else 0
+                for j, s in enumerate(chunk):
+                    segs[j] = (outs[s].data_ptr(), outs[s].numel(), ends[s] - base)
+                tables.append((torch.from_numpy(segs.view(np.uint8)).to(device, non_blocking=False), len(chunk), base, ends[chunk[-1]] - base))
+            if len(_segment_cache) >= 4:
+                _segment_cache.clear()
+            _segment_cache[key] = tables
+        for segs_dev, count, base, width in tables:
             vals = all_values if (base == 0 and width == per_worker) else all_values[:, base : base + width].contiguous()
             poss = all_positions if (base == 0 and width == per_worker) else all_positions[:, base : base + width].contiguous()
             code = lib.psgd_sparse_combine_launch(
                 ctypes.c_void_p(vals.data_ptr()), ctypes.c_void_p(poss.data_ptr()), int(workers), ctypes.c_longlong(width),
-                ctypes.c_void_p(segs_dev.data_ptr()), len(chunk), ctypes.c_float(divisor),
+                ctypes.c_void_p(segs_dev.data_ptr()), count, ctypes.c_float(divisor),
                 ctypes.c_void_p(scratch.data_ptr()), ctypes.c_void_p(scratch.data_ptr() + 4), stream,
             )
             native.check(code, "psgd_sparse_combine_launch")

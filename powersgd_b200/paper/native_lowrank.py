@@ -57,7 +57,8 @@ class _Core:
 def usable(tensors: Sequence[torch.Tensor]) -> bool:
     """Native path: CUDA, float32, dense tensors, and the library present (its absence on a CUDA
     machine is an error unless PSGD_B200_ALLOW_FALLBACK=1)."""
-    if not tensors or not all(t.is_cuda and t.dtype == torch.float32 and is_dense(t) for t in tensors):
+    f32 = torch.float32
+    if not tensors or not all(t.is_cuda and t.dtype == f32 and (t.is_contiguous() or is_dense(t)) for t in tensors):
         return False
     return native.use_for_cuda()
 
@@ -99,10 +100,15 @@ class NativeLowRank:
     # ------------------------------------------------------------------------------------------
     def rank_k(self, matrices) -> None:
         """p = M q (q as it is), sum, orthonormalise, q = M^T p, mean, out = p q^T, memory = M - out."""
-        comp, core = self.comp, self.core
+        comp = self.comp
         comp.check()
         comp.launches = 0
         self._bind(matrices)
+        comp._taped(("rank_k",), self._rank_k)
+        self.launches += comp.launches
+
+    def _rank_k(self) -> None:
+        comp, core = self.comp, self.core
         workers = world_size()
         p2p = workers > 1 and comp.comm is not None
         chained = comp._chained()
@@ -132,7 +138,6 @@ class NativeLowRank:
             Q.div_(workers)  # the factor memory keeps the MEAN, which the next step starts from
         # out = p (sum q / W)^T, memory = M - out
         self._finalize_global(p_hat, q_loc, q_loc if workers == 1 else comp.h_sum[1], workers, Q if gather else None)
-        self.launches += comp.launches
 
     def _finalize_global(self, left: torch.Tensor, right_loc: torch.Tensor, right_sum: torch.Tensor, workers: int,
                          gather_state: Optional[torch.Tensor]) -> None:
@@ -142,7 +147,8 @@ class NativeLowRank:
         comp = self.comp
         tiles, count = comp._tiles_dev["fin"]["f"]
         one = [left]
-        code = comp.lib.psgd_finalize_launch(
+        comp._call(
+            "psgd_finalize_launch",
             _ptr(comp._mats_dev), _ptr(tiles), count, comp.tiles.fin_rows, comp.tiles.max_r, _ptr(comp._hyper_dev), 1,
             ctypes.cast(_ptr_array(one), ctypes.c_void_p), ctypes.cast(_ptr_array([right_loc]), ctypes.c_void_p),
             ctypes.cast(_ptr_array(one), ctypes.c_void_p), ctypes.cast(_ptr_array([right_sum]), ctypes.c_void_p),
@@ -153,10 +159,7 @@ class NativeLowRank:
             3,  # residual = M - update, written to the `param` slot (the caller's memory tensor)
             1.0 / workers,
             int(comp._chained()),
-            _stream_ptr(),
         )
-        native.check(code, "psgd_finalize_launch")
-        comp.launches += 1
 
     # ------------------------------------------------------------------------------------------
     def half_rank_k(self, matrices, compute_p: bool) -> None:
@@ -169,12 +172,16 @@ class NativeLowRank:
         # the library core multiplies with P as the basis on even parity
         core.step_counter = 1 if compute_p else 0
         workers = world_size()
-        if workers == 1:
-            saved, comp.h_sum = comp.h_sum, comp.h_loc
-        try:
-            sides, pending = comp._half_iterations()
-            comp._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending, flags=2, early=comp._follows)
-        finally:
+
+        def step() -> None:
             if workers == 1:
-                comp.h_sum = saved
+                saved, comp.h_sum = comp.h_sum, comp.h_loc
+            try:
+                sides, pending = comp._half_iterations()
+                comp._finalize(sides, fused_sgd=False, workers=workers, gather_state=pending, flags=2, early=comp._follows)
+            finally:
+                if workers == 1:
+                    comp.h_sum = saved
+
+        comp._taped(("half_rank_k", compute_p), step)
         self.launches += comp.launches

@@ -1,4 +1,5 @@
-"""Launches that overlap the end of their predecessor may not change a bit of what a step computes."""
+"""Launches that overlap the end of their predecessor, and steps repeated from their recorded calls:
+neither may change a bit of what a step computes."""
 import pytest
 import torch
 
@@ -26,20 +27,51 @@ def _aggregate(shapes, rank, iters, prepare=None):
 
 
 @pytest.mark.parametrize("rank,iters", [(1, 2), (2, 2), (4, 1), (4, 3), (16, 2)])
-def test_overlapped_launches_leave_the_bits_alone(rank, iters):
+def test_overlapped_and_repeated_launches_leave_the_bits_alone(rank, iters):
     usual, native = _aggregate(SHAPES, rank, iters)
-    assert native._chained()
-    apart, _ = _aggregate(SHAPES, rank, iters, lambda nat: setattr(nat, "_chained", lambda: False))
-    for a, b in zip(usual, apart):
-        assert torch.equal(a, b)
+    assert native._chained() and native._tapes
+    apart, _ = _aggregate(SHAPES, rank, iters, lambda nat: (setattr(nat, "_chained", lambda: False), nat._tapes.clear()))
+    again, _ = _aggregate(SHAPES, rank, iters, lambda nat: nat._tapes.clear())
+    for a, b, c in zip(usual, apart, again):
+        assert torch.equal(a, b) and torch.equal(a, c)
 
 
 def test_tensor_core_products_behind_an_overlapped_basis():
     shapes = [(1024, 1100), (2176, 900)]
     usual, native = _aggregate(shapes, 8, 2)
     assert native.uses_tensor_cores
-    apart, _ = _aggregate(shapes, 8, 2, lambda nat: setattr(nat, "_chained", lambda: False))
+    apart, _ = _aggregate(shapes, 8, 2, lambda nat: (setattr(nat, "_chained", lambda: False), nat._tapes.clear()))
     assert all(torch.equal(a, b) for a, b in zip(usual, apart))
+
+
+def test_new_gradients_new_rates_and_new_factors_are_seen():
+    """What a repeated step must not take from the step it repeats: the tensors, the learning rate, the
+    factors that a checkpoint put in place."""
+    def make():
+        g = torch.Generator(device="cuda").manual_seed(3)
+        params = [torch.nn.Parameter(torch.randn(s, generator=g, device="cuda")) for s in [(96, 200), (96, 200), (50, 40), (33,)]]
+        opt = torch.optim.SGD(params, lr=0.1, momentum=0.9)
+        return params, opt, PowerSGD(params, Config(rank=2, num_iters_per_step=2, start_compressing_after_num_steps=0))
+
+    (pa, oa, aa), (pb, ob, ab) = make(), make()
+    for step in range(8):
+        fresh = _gradients([tuple(p.shape) for p in pa], 40 + step)
+        for params, opt, agg in ((pa, oa, aa), (pb, ob, ab)):
+            if step in (0, 5):   # tensors of their own from here on
+                for p, f in zip(params, fresh):
+                    p.grad = f.clone() if p.grad is None else p.grad + f
+            else:
+                torch._foreach_add_([p.grad for p in params], fresh)
+            opt.param_groups[0]["lr"] = 0.1 / (1 + step // 3)
+            if step == 6:
+                for view in agg._powersgd._ps + agg._powersgd._qs:
+                    view.copy_(torch.ones_like(view).cumsum(1).sin())
+            if agg is ab and getattr(agg._powersgd, "_native", None) is not None:
+                agg._powersgd._native._tapes.clear()
+                agg._fused._last_values = None
+            optimizer_step(opt, agg)
+        for p, q in zip(pa, pb):
+            assert torch.equal(p, q) and torch.equal(p.grad, q.grad), step
 
 
 def test_recorded_in_a_graph_and_run_eagerly_agree():
