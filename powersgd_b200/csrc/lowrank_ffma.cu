@@ -161,8 +161,10 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
 
   // The gradient does not depend on the launches before this one: the tile's first rows are loaded
   // and the rest is asked into L2 while the basis is still being orthonormalised.
-  float v[UR][4];
-  auto load = [&](int row0, int rows, int i0) {
+  // Two batches of rows are under way at any time: one alone (16 KiB per CTA) leaves the memory system
+  // idle for most of its latency.
+  float v0[UR][4], v1[UR][4];
+  auto load = [&](float (&v)[UR][4], int row0, int rows, int i0) {
 #pragma unroll
     for (int u = 0; u < UR; ++u) {
       const int i = i0 + u * GEMM_WARPS;
@@ -170,8 +172,9 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
       load_lane_cols<VEC>(M + (long long)(row0 + (rok ? i : 0)) * m, t.col0, cend, lane, rok, v[u]);
     }
   };
-  load(t.row0, min(MAXR, t.rows), warp);
-  for (int e = tid + 4 * STEP; e < 4 * min(MAXR, t.rows); e += GEMM_THREADS)   // four lines of 128 bytes per row
+  load(v0, t.row0, min(MAXR, t.rows), warp);
+  load(v1, t.row0, min(MAXR, t.rows), warp + STEP);
+  for (int e = tid + 8 * STEP; e < 4 * min(MAXR, t.rows); e += GEMM_THREADS)   // four lines of 128 bytes per row
     if ((e & 3) * 32 < t.cols) psgd_prefetch_l2(M + (long long)(t.row0 + (e >> 2)) * m + t.col0 + (e & 3) * 32);
   psgd_wait_for_predecessor();
 
@@ -181,7 +184,8 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   for (int rb = 0; rb < t.rows; rb += MAXR) {
     const int rows = min(MAXR, t.rows - rb);
     if (rb) {
-      load(t.row0 + rb, rows, warp);
+      load(v0, t.row0 + rb, rows, warp);
+      load(v1, t.row0 + rb, rows, warp + STEP);
       __syncthreads();  // the previous chunk's rows of P-hat are no longer read
     }
     // stage the chunk's rows of P-hat (zero padded to RT columns)
@@ -192,13 +196,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
     }
     __syncthreads();
 
-    for (int i0 = warp; i0 < rows; i0 += STEP) {
-      float cur[UR][4];
-#pragma unroll
-      for (int u = 0; u < UR; ++u)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) cur[u][c] = v[u][c];
-      if (i0 + STEP < rows) load(t.row0 + rb, rows, i0 + STEP);  // the next rows travel while these are used
+    auto use = [&](const float (&v)[UR][4], int i0) {
 #pragma unroll
       for (int u = 0; u < UR; ++u) {
         const int i = i0 + u * GEMM_WARPS;
@@ -208,10 +206,16 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
           for (int k = 0; k < RT; ++k) {
             const float pk = pr[k];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[c][k] = fmaf(cur[u][c], pk, acc[c][k]);
+            for (int c = 0; c < 4; ++c) acc[c][k] = fmaf(v[u][c], pk, acc[c][k]);
           }
         }
       }
+    };
+    for (int i0 = warp; i0 < rows; i0 += 2 * STEP) {
+      use(v0, i0);
+      if (i0 + 2 * STEP < rows) load(v0, t.row0 + rb, rows, i0 + 2 * STEP);
+      use(v1, i0 + STEP);
+      if (i0 + 3 * STEP < rows) load(v1, t.row0 + rb, rows, i0 + 3 * STEP);
     }
   }
   __syncthreads();
@@ -295,7 +299,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
 }
 
 template <int RT>
-__global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nt_kernel(GemmArgs a) {
+__global__ void __launch_bounds__(GEMM_THREADS, RT <= 4 ? 3 : (RT <= 16 ? 2 : 1)) psgd_gemm_nt_kernel(GemmArgs a) {
   extern __shared__ __align__(16) float smem[];
   psgd_launch_dependents();
   const PsgdTile t = a.tiles[blockIdx.x];
@@ -335,8 +339,8 @@ __device__ __forceinline__ float warp_sums(float (&v)[N], int lane) {
 // chain load - multiply - reduce - hand over; with many, the loads of the gradient. So the rows of
 // Q-hat that the tile needs are staged in shared memory once, in the order the lanes read them (a lane
 // reads its 4 columns x RT values as RT 16-byte words: read straight from global memory they cost more
-// load instructions than the gradient itself), and the loop over 128-column chunks keeps one chunk of
-// the gradient in flight ahead of the one being multiplied.
+// load instructions than the gradient itself), and the loop over 128-column chunks keeps two chunks
+// of the gradient under way.
 template <int RT, int VEC, int RPW>
 __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& t, const PsgdMat& mt, float* sQ, float* sSum) {
   const int r = mt.r, m = mt.m;
@@ -364,9 +368,13 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
 
   const int cend = t.col0 + t.cols;
   // as in the NT tile, the first loads go out ahead of the wait
-  float v[RPW][4];
+  float v0[RPW][4], v1[RPW][4];
+  auto load = [&](float (&v)[RPW][4], int c0) {
 #pragma unroll
-  for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], t.col0, cend, lane, rok[u], v[u]);
+    for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], c0, cend, lane, rok[u], v[u]);
+  };
+  load(v0, t.col0);
+  load(v1, t.col0 + NN_CHUNK_COLS);   // (zeros where the tile has no such chunk)
   psgd_wait_for_predecessor();
 
   // element (column lc of the tile, k): chunk of 128 columns, then word of 4 floats, then lane
@@ -390,16 +398,7 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
   __syncthreads();
 
   const float4* q4 = reinterpret_cast<const float4*>(sQ) + lane;
-  for (int c0 = t.col0; c0 < cend; c0 += NN_CHUNK_COLS) {
-    float cur[RPW][4];
-#pragma unroll
-    for (int u = 0; u < RPW; ++u)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) cur[u][c] = v[u][c];
-    if (c0 + NN_CHUNK_COLS < cend) {
-#pragma unroll
-      for (int u = 0; u < RPW; ++u) load_lane_cols<VEC>(rowp[u], c0 + NN_CHUNK_COLS, cend, lane, rok[u], v[u]);
-    }
+  auto use = [&](const float (&v)[RPW][4]) {
 #pragma unroll
     for (int w = 0; w < RT; ++w) {
       const float4 q = q4[w * 32];
@@ -408,10 +407,18 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
       for (int i = 0; i < 4; ++i) {
         const int c = (w * 4 + i) / RT, k = (w * 4 + i) % RT;
 #pragma unroll
-        for (int u = 0; u < RPW; ++u) acc[u * RT + k] = fmaf(cur[u][c], qv[i], acc[u * RT + k]);
+        for (int u = 0; u < RPW; ++u) acc[u * RT + k] = fmaf(v[u][c], qv[i], acc[u * RT + k]);
       }
     }
     q4 += RT * 32;
+  };
+  for (int c0 = t.col0; c0 < cend; c0 += 2 * NN_CHUNK_COLS) {
+    use(v0);
+    if (c0 + 2 * NN_CHUNK_COLS < cend) load(v0, c0 + 2 * NN_CHUNK_COLS);
+    if (c0 + NN_CHUNK_COLS < cend) {
+      use(v1);
+      if (c0 + 3 * NN_CHUNK_COLS < cend) load(v1, c0 + 3 * NN_CHUNK_COLS);
+    }
   }
 
   if (RPW * RT <= 32) {
