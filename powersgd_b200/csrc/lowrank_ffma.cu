@@ -114,24 +114,6 @@ __device__ __forceinline__ void load_lane_cols(const float* __restrict__ rowp, i
   }
 }
 
-// Sum of element `e` over the `n` partial tiles of one output block, in split order (fixed, so the
-// result does not depend on which tile arrived last). Eight loads are in flight at a time: a tall
-// matrix has a hundred partial tiles per block, and one dependent L2 round trip per partial would
-// cost the last arriver tens of microseconds.
-__device__ __forceinline__ float sum_partials(const float* first, int tile_elems, int n) {
-  float s = 0.f;
-  int p = 0;
-  for (; p + 8 <= n; p += 8) {
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldcg(first + (long long)(p + j) * tile_elems);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s += v[j];
-  }
-  for (; p < n; ++p) s += __ldcg(first + (long long)p * tile_elems);
-  return s;
-}
-
 // ------------------------------------------------------------------------------------------
 // NT: each lane owns 4 columns, each warp strides over the tile's rows.
 // ------------------------------------------------------------------------------------------
@@ -252,7 +234,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
     }
   }
 
-  const int tile_elems = NT_TILE_COLS * RT;
+  constexpr int tile_elems = NT_TILE_COLS * RT;
   bool owner = true;  // does this CTA write the output rows?
   if (t.nsplit > 1) {
     float* mine = a.partial + (long long)(t.slot0 + t.split) * tile_elems;
@@ -264,7 +246,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
     owner = sLast != 0;
     if (owner) {
       __threadfence();
-      for (int e = tid; e < tile_elems; e += GEMM_THREADS) sSum[e] = sum_partials(a.partial + (long long)t.slot0 * tile_elems + e, tile_elems, t.nsplit);
+      psgd_sum_partials<tile_elems, GEMM_THREADS>(a.partial + (long long)t.slot0 * tile_elems, t.nsplit, sSum);
       if (tid == 0) a.tickets[t.ticket] = 0;  // ready for the next launch
       __syncthreads();
     }
@@ -440,7 +422,7 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
     owner = sLast != 0;
     if (owner) {
       __threadfence();
-      for (int e = tid; e < tile_elems; e += GEMM_THREADS) sSum[e] = sum_partials(a.partial + (long long)t.slot0 * tile_elems + e, tile_elems, t.nsplit);
+      psgd_sum_partials<tile_elems, GEMM_THREADS>(a.partial + (long long)t.slot0 * tile_elems, t.nsplit, sSum);
       if (tid == 0) a.tickets[t.ticket] = 0;
       __syncthreads();
     }

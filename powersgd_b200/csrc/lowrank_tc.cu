@@ -410,11 +410,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
     owner = s_last != 0;
     if (owner) {
       __threadfence();
-      for (int e = tid; e < tile_elems; e += TC_THREADS) {
-        float s = 0.f;
-        for (int p = 0; p < t.nsplit; ++p) s += __ldcg(a.partial + (long long)(t.slot0 + p) * tile_elems + e);
-        sSum[e] = s;
-      }
+      psgd_sum_partials<tile_elems, TC_THREADS>(a.partial + (long long)t.slot0 * tile_elems, t.nsplit, sSum);
       if (tid == 0) a.tickets[t.ticket] = 0;
       __syncthreads();
     }

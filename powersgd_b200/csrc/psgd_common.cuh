@@ -44,6 +44,50 @@ __device__ __forceinline__ double psgd_warp_sum(double v) {
   return v;
 }
 
+// Partial sums of a split tile: element e of partial p lies at first[p * tile_elems + e]. Writes the sums
+// over the `n` partials, in split order (fixed, so the result does not depend on which tile arrived last),
+// to out[0 .. TILE_ELEMS). One CTA does this at the end of a product while the rest of the GPU has
+// nothing left to do, and a tall matrix has tens of partials per block, so what counts is how many loads
+// are under way: every thread takes a vector of elements and eight or sixteen partials at a time.
+template <int TILE_ELEMS, int THREADS>
+__device__ __forceinline__ void psgd_sum_partials(const float* first, int n, float* out) {
+  constexpr int W = TILE_ELEMS >= 4 * THREADS / 2 ? 4 : (TILE_ELEMS >= 2 * THREADS ? 2 : 1);   // floats per thread and load
+  constexpr int B = W == 4 ? 8 : 16;                                                              // loads under way
+  static_assert(TILE_ELEMS % W == 0, "whole vectors");
+  for (int e = threadIdx.x * W; e < TILE_ELEMS; e += THREADS * W) {
+    float s[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) s[i] = 0.f;
+    for (int p = 0; p < n; p += B) {
+      float v[B][W];
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        if (p + j < n) {
+          const float* src = first + (long long)(p + j) * TILE_ELEMS + e;
+          if (W == 4) {
+            const float4 q = __ldcg(reinterpret_cast<const float4*>(src));
+            v[j][0] = q.x; v[j][1 % W] = q.y; v[j][2 % W] = q.z; v[j][3 % W] = q.w;
+          } else if (W == 2) {
+            const float2 q = __ldcg(reinterpret_cast<const float2*>(src));
+            v[j][0] = q.x; v[j][1 % W] = q.y;
+          } else {
+            v[j][0] = __ldcg(src);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        if (p + j < n) {
+#pragma unroll
+          for (int i = 0; i < W; ++i) s[i] += v[j][i];
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < W; ++i) out[e + i] = s[i];
+  }
+}
+
 __device__ __forceinline__ int psgd_atom_add_acqrel_gpu(int* p, int v) {
   int old;
   asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
