@@ -270,7 +270,7 @@ __device__ __forceinline__ void fin_gather(const PsgdCommDev& c, int e1, long lo
   }
 }
 
-template <int VEC, bool SAME, int RPW>
+template <int VEC, bool SAME, int RPW, bool OPT>
 __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const PsgdTile& t, const PsgdMat& mt,
                                                     int tile_rows, float* fin_smem) {
   const int r = mt.r, m = mt.m;
@@ -297,7 +297,7 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   }
 #endif
   const PsgdHyper hy = a.hyper[mt.hyper];
-  const bool sgd = a.fused_sgd != 0;
+  const bool sgd = OPT && a.fused_sgd != 0;
   const bool mom = sgd && hy.has_momentum;
   const bool global_res = (a.flags & 1) != 0;
   float* const res_base = (a.flags & 2) ? mt.param : mt.grad;
@@ -466,14 +466,19 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   }
 }
 
-template <bool SAME, int RPW>
-__global__ void __launch_bounds__(FIN_THREADS, 2) psgd_finalize_strip_kernel(FinalizeArgs a, int tile_rows) {
+// OPT = false: the variant without the optimizer step. A thread then holds a third of the operands, which
+// leaves room for a third CTA per SM: us per pass of 4 x 1024^2 61.4 -> 59.4, 4 x 4096^2 429.9 -> 421.7, 3 x
+// 1001x777 + 2 x 515x2049 118.8 -> 114.5. OPT = true decides at run time; fixing the optimizer step at compile
+// time as well, or eight rows without it, was slower (recorded ResNet-18 step 112.2 -> 115.0, LSTM step
+// 222.6 -> 225.5, 50257 x 1024 at rank 16 465.8 -> 469.2).
+template <bool SAME, int RPW, bool OPT>
+__global__ void __launch_bounds__(FIN_THREADS, OPT ? 2 : 3) psgd_finalize_strip_kernel(FinalizeArgs a, int tile_rows) {
   extern __shared__ __align__(16) float fin_smem[];
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
-  if (t.vec == 4) finalize_strip_tile<4, SAME, RPW>(a, t, mt, tile_rows, fin_smem);
-  else if (t.vec == 2) finalize_strip_tile<2, SAME, RPW>(a, t, mt, tile_rows, fin_smem);
-  else finalize_strip_tile<1, SAME, RPW>(a, t, mt, tile_rows, fin_smem);
+  if (t.vec == 4) finalize_strip_tile<4, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
+  else if (t.vec == 2) finalize_strip_tile<2, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
+  else finalize_strip_tile<1, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
 }
 
 // Shared-memory budgets of a strip CTA: the default carve-out serves the small ranks (several CTAs
@@ -483,17 +488,17 @@ __global__ void __launch_bounds__(FIN_THREADS, 2) psgd_finalize_strip_kernel(Fin
 constexpr int FIN_SMEM_DEFAULT = 48 * 1024;
 constexpr int FIN_SMEM_OPT_IN = 96 * 1024;
 
-template <bool SAME, int RPW>
+template <bool SAME, int RPW, bool OPT>
 static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, int early, cudaStream_t stream) {
   const size_t smem = (size_t)(SAME ? 1 : 2) * kmax * fin_panel_floats(tile_rows) * sizeof(float);
   if (smem > (size_t)FIN_SMEM_DEFAULT) {
     static bool opted_in = false;   // per instantiation
     if (!opted_in) {
-      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME, RPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
+      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME, RPW, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
       opted_in = true;
     }
   }
-  return psgd_launch(psgd_finalize_strip_kernel<SAME, RPW>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
+  return psgd_launch(psgd_finalize_strip_kernel<SAME, RPW, OPT>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
 }
 
 // Tallest strip (multiple of 32 rows, at most 256) whose panels fit the shared-memory budget.
@@ -569,9 +574,10 @@ PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntile
   }
   if (strip) {
     const int kmax = nhist * max_r;
-    if (!same) return finalize_strip_launch<false, 4>(a, ntiles, tile_rows, kmax, early, stream);
-    return kmax >= 16 ? finalize_strip_launch<true, 8>(a, ntiles, tile_rows, kmax, early, stream)
-                                : finalize_strip_launch<true, 4>(a, ntiles, tile_rows, kmax, early, stream);
+    if (!same) return finalize_strip_launch<false, 4, true>(a, ntiles, tile_rows, kmax, early, stream);
+    if (kmax >= 16) return finalize_strip_launch<true, 8, true>(a, ntiles, tile_rows, kmax, early, stream);
+    return fused_sgd ? finalize_strip_launch<true, 4, true>(a, ntiles, tile_rows, kmax, early, stream)
+                     : finalize_strip_launch<true, 4, false>(a, ntiles, tile_rows, kmax, early, stream);
   }
   return psgd_launch(same ? psgd_finalize_kernel<true> : psgd_finalize_kernel<false>, ntiles, FIN_THREADS, 0, stream, early, a);
 }
