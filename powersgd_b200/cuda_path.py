@@ -24,6 +24,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import os
+import weakref
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -310,7 +311,10 @@ class NativeCompressor:
     """Runs `BasicPowerSGD.aggregate` on the GPU with the in-tree kernels."""
 
     def __init__(self, core):
-        self.core = core
+        # the owner holds this object, not the other way round: both then go when the owner is dropped, and
+        # not whenever the cycle collector runs - which may be in the middle of a CUDA-graph capture,
+        # where giving back pinned memory ends the capture with an error
+        self.core = weakref.proxy(core)
         self.lib = native.lib()
         self.device = core.device
         self.plan = core.plan
@@ -1203,7 +1207,7 @@ class FusedSGDDriver:
     RING = 4
 
     def __init__(self, agg):
-        self.agg = agg
+        self.agg = weakref.proxy(agg)   # its owner, see NativeCompressor
         self.device = agg.device
         self._slots: List[torch.Tensor] = []
         self._slot_events: List[Optional[torch.cuda.Event]] = []

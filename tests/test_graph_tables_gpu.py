@@ -1,9 +1,12 @@
 """Descriptor tables built while a CUDA graph is being recorded are put in place once, outside the graph:
 its replays must find them intact although the graph's own memory is written over and over."""
+import gc
+import weakref
+
 import pytest
 import torch
 
-from powersgd_b200 import BasicConfig, BasicPowerSGD
+from powersgd_b200 import BasicConfig, BasicPowerSGD, Config, PowerSGD, optimizer_step
 from powersgd_b200.cuda_path import capture_scope
 
 pytestmark = pytest.mark.gpu
@@ -34,3 +37,22 @@ def test_tables_bound_under_capture_survive_replays():
         want = plain.aggregate(want_grads)
         for a, b in zip(list(outs) + grads, list(want) + want_grads):
             assert torch.equal(a, b), step
+
+
+def test_native_objects_go_with_their_aggregator():
+    """No reference cycle keeps pinned memory until the collector runs, which may be during a capture."""
+    params = [torch.nn.Parameter(torch.randn(s, device="cuda")) for s in [(96, 200), (33,)]]
+    for p in params:
+        p.grad = torch.randn_like(p)
+    opt = torch.optim.SGD(params, lr=0.1, momentum=0.9)
+    agg = PowerSGD(params, Config(rank=2, start_compressing_after_num_steps=0))
+    gc.collect()
+    gc.disable()
+    try:
+        for _ in range(3):
+            optimizer_step(opt, agg)
+        gone = [weakref.ref(agg._powersgd._native), weakref.ref(agg._fused)]
+        del agg
+        assert all(ref() is None for ref in gone)
+    finally:
+        gc.enable()
