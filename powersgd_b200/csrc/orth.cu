@@ -26,7 +26,8 @@
 // Both launches are bound by latency (a factor is tens of kilobytes), so what counts is the length
 // of the dependent chain: factorising redundantly takes the place of an arrival counter, a memory
 // fence, a lone last CTA and a second round trip through memory, and the second launch is
-// released early (programmatic dependent launch) so that only its wait remains.
+// released early (programmatic dependent launch) so that only its wait remains. Both launches
+// together, before and after: 21 factors of ResNet-18 at rank 2 12.3 / 9.3 us, 50257 x 16 43 / 24 us.
 //
 // Multi-GPU: the factor to orthonormalise is the SUM over workers of what the previous product
 // launch pushed into this rank's slot arena. The first launch is then also the consumer of that
@@ -501,7 +502,7 @@ PSGD_API int psgd_orth_template_rank(int max_r) {
 // Rows of a chunk when the longest unit has `longest` rows. A short unit takes the base size. Every
 // chunk of the second launch reads the partial matrices of ALL chunks of its unit, so their number
 // is bounded: at the bound the partials are 32 to 400 KB per unit, read in as long as the chunk's own
-// rows take. (An embedding of 50257 rows at rank 16: 66 chunks instead of 393.)
+// rows take. (An embedding of 50257 rows at rank 16: 79 chunks instead of 393.)
 template <int RT>
 static int orth_chunk_rows(long long longest) {
   const int base = orth_base_rows<RT>(), most = RT <= 4 ? 256 : RT == 8 ? 128 : RT == 16 ? 80 : 48;

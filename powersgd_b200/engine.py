@@ -365,7 +365,7 @@ class TrainStep:
         # capturing ran the host side of the step (counters) but not the kernels: rewind
         agg.step_counter, agg._powersgd.step_counter = saved
         self._graphs[parity] = graph
-        self._graph_keep[parity] = keep  # tables the graph's copy nodes read: same lifetime as the graph
+        self._graph_keep[parity] = keep  # tables whose addresses the graph holds: same lifetime as the graph
 
     def __call__(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         if not self._graphable_now():
