@@ -34,6 +34,17 @@ PSGD_API int psgd_device_info(int* sm_count, int* cc_major, int* cc_minor, int* 
   return 0;
 }
 
+// Exchanges the calling thread's capture mode (see cudaThreadExchangeStreamCaptureMode): *mode goes in, the
+// previous one comes out. In the relaxed mode (2) a thread that is recording one stream may allocate
+// memory and wait for others. Returns a CUDA error code.
+PSGD_API int psgd_capture_mode(int* mode) {
+  cudaStreamCaptureMode m = (cudaStreamCaptureMode)*mode;
+  const cudaError_t e = cudaThreadExchangeStreamCaptureMode(&m);
+  if (e != cudaSuccess) { psgd_set_error("cudaThreadExchangeStreamCaptureMode: %s", cudaGetErrorString(e)); return (int)e; }
+  *mode = (int)m;
+  return 0;
+}
+
 #ifdef PSGD_BOUNDS_CHECK
 extern "C" int psgd_bounds_read_products(int* out, int reset);
 extern "C" int psgd_bounds_read_finalize(int* out, int reset);

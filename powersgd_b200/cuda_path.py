@@ -87,20 +87,22 @@ def _outside_capture(device: torch.device):
     every replay of the graph pays for (eight copies of 1.3 us each in the step of a small perceptron).
     Under capture the body gets a stream that is not part of it, so that its tensors come from the
     ordinary pool - memory of the graph's own pool may be written by an earlier node of the same graph -
-    and is waited for."""
+    and is waited for; the thread is in the relaxed capture mode meanwhile, whatever mode the recording
+    was begun with (an allocation in the strict one ends it with an error)."""
     if not torch.cuda.is_current_stream_capturing():
         yield
         return
     device = torch.device("cuda", torch.cuda.current_device()) if device.index is None else device
-    while True:
-        stream = _upload_streams.setdefault(device, torch.cuda.Stream(device=device))
-        with torch.cuda.stream(stream):
-            if torch.cuda.is_current_stream_capturing():   # streams are handed out in turn: this one was forked into the capture
-                del _upload_streams[device]
-                continue
-            yield
-            stream.synchronize()
-            return
+    with native.relaxed_capture():
+        while True:
+            stream = _upload_streams.setdefault(device, torch.cuda.Stream(device=device))
+            with torch.cuda.stream(stream):
+                if torch.cuda.is_current_stream_capturing():   # streams are handed out in turn: this one was forked into the capture
+                    del _upload_streams[device]
+                    continue
+                yield
+                stream.synchronize()
+                return
 
 
 def _keep_with_graph(*tensors: torch.Tensor) -> None:

@@ -13,6 +13,9 @@ def declare(lib) -> None:
     lib.psgd_device_info.restype = i32
     lib.psgd_device_info.argtypes = [C.POINTER(i32)] * 4
 
+    lib.psgd_capture_mode.restype = i32
+    lib.psgd_capture_mode.argtypes = [C.POINTER(i32)]
+
     lib.psgd_orth_launch.restype = i32
     lib.psgd_orth_launch.argtypes = [vp, i32, vp, i32, i32, vp, vp, i32, vp, vp, vp, vp, vp, vp, i32, vp]
 

@@ -7,6 +7,7 @@ missing, and callers on a CUDA device treat that as fatal.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from typing import Optional
@@ -71,3 +72,15 @@ def check(code: int, what: str) -> None:
     if code != 0:
         msg = lib().psgd_last_error()
         raise RuntimeError(f"{what} failed (code {code}): {msg.decode() if msg else ''}")
+
+
+@contextlib.contextmanager
+def relaxed_capture():
+    """While this thread is recording a CUDA graph, calls that do not belong to the recording (allocations, a
+    wait for another stream) are refused and end it, unless the thread is in the relaxed capture mode."""
+    mode = ctypes.c_int(2)
+    check(lib().psgd_capture_mode(ctypes.byref(mode)), "psgd_capture_mode")
+    try:
+        yield
+    finally:
+        check(lib().psgd_capture_mode(ctypes.byref(mode)), "psgd_capture_mode")

@@ -56,3 +56,26 @@ def test_native_objects_go_with_their_aggregator():
         assert all(ref() is None for ref in gone)
     finally:
         gc.enable()
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_tables_can_be_bound_under_every_capture_mode(mode):
+    """New tensors bound for the first time inside a recording: the uploads allocate, which a strict recording
+    refuses on its own thread."""
+    shapes = [(96, 200), (64, 27)]
+    make = lambda: BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=2, num_iters_per_step=2), backend="native")  # noqa: E731
+    g = torch.Generator(device="cuda").manual_seed(0)
+    first, second = ([torch.randn(s, generator=g, device="cuda") for s in shapes] for _ in range(2))
+    ours, plain = make(), make()
+    before = [f.clone() for f in first]   # stays alive: the recorded call gets tensors at other addresses
+    ours.aggregate(before), plain.aggregate([f.clone() for f in first])
+    grads, want_grads = ([f.clone() for f in second] for _ in range(2))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with capture_scope() as keep, torch.cuda.graph(graph, capture_error_mode=mode):
+        outs = ours.aggregate(grads)
+    assert keep
+    graph.replay()
+    want = plain.aggregate(want_grads)
+    for a, b in zip(list(outs) + grads, list(want) + want_grads):
+        assert torch.equal(a, b)
