@@ -34,6 +34,17 @@ PSGD_API int psgd_device_info(int* sm_count, int* cc_major, int* cc_minor, int* 
   return 0;
 }
 
+// Which recording (CUDA-graph capture) `stream` is part of: an id of its own for every capture of the
+// process, 0 when the stream is not being recorded. Returns a CUDA error code.
+PSGD_API int psgd_capture_id(cudaStream_t stream, unsigned long long* id) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  *id = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo_v2(stream, &status, id, nullptr, nullptr, nullptr);
+  if (e != cudaSuccess) { psgd_set_error("cudaStreamGetCaptureInfo: %s", cudaGetErrorString(e)); return (int)e; }
+  if (status == cudaStreamCaptureStatusNone) *id = 0;
+  return 0;
+}
+
 // Exchanges the calling thread's capture mode (see cudaThreadExchangeStreamCaptureMode): *mode goes in, the
 // previous one comes out. In the relaxed mode (2) a thread that is recording one stream may allocate
 // memory and wait for others. Returns a CUDA error code.

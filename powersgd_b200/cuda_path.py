@@ -1201,9 +1201,11 @@ class FusedSGDDriver:
     every step (learning-rate schedules keep working), and follows torch's first-step rule
     that a fresh momentum buffer is the gradient itself.
 
-    The table travels through a ring of pinned host slots, one eager async copy per step, so
-    that a step recorded in a CUDA graph reads its hyper-parameters from device memory and
-    the host never overwrites a slot that a copy in flight still reads.
+    The table travels through a ring of pinned host slots, one async copy per step that changes
+    it, so that a step recorded in a CUDA graph reads its hyper-parameters from device memory and
+    the host never overwrites a slot that a copy in flight still reads. No copy is ever recorded:
+    a recorded step runs with what the device table holds when it is replayed (`prepare`, or any
+    eager step, brings it up to date).
     """
 
     RING = 4
@@ -1217,6 +1219,9 @@ class FusedSGDDriver:
         self._hyper_dev: Optional[torch.Tensor] = None
         self._cache_key = None
         self._last_values = None   # what the device table holds
+        self._stream: Optional[torch.cuda.Stream] = None   # of the last step that was not recorded
+        self._recorded_in = 0      # id of the recording that the last step was part of
+        self._fixed: Optional[torch.Tensor] = None   # table of the coming step alone, in place of the live one
         self._flat_all = NativeFlatAllReduce()
         self._flat_plain = NativeFlatAllReduce()
         self.launches = 0
@@ -1258,32 +1263,55 @@ class FusedSGDDriver:
         """Host side of a step: momentum buffers, hyper-parameter table, async upload."""
         fresh = self._collect(optimizer)
         groups = optimizer.param_groups
-        values = [(float(g["lr"]), float(g["momentum"]), float(g["dampening"]), float(g["weight_decay"]), bool(g["nesterov"])) for g in groups]
-        if not fresh and values == self._last_values:
+        # one row per group, as the kernels see it: a fresh momentum buffer is the gradient itself, whatever the dampening
+        values = [
+            (float(g["lr"]), float(g["momentum"]), 1.0 if gi in fresh else 1.0 - float(g["dampening"]), float(g["weight_decay"]), bool(g["nesterov"]))
+            for gi, g in enumerate(groups)
+        ]
+        recording = native.capture_id(torch.cuda.current_stream()) if torch.cuda.is_current_stream_capturing() else 0
+        joins = recording != 0 and recording == self._recorded_in   # an earlier step of this recording reads the live table
+        self._recorded_in = recording
+        self._fixed = None
+        if values == self._last_values:
+            if not recording:
+                self._stream = torch.cuda.current_stream()
             return  # nothing changed since the last upload: the device table is already right
         table = np.zeros(len(groups), dtype=layout.HYPER_DTYPE)
-        for gi, group in enumerate(groups):
-            mu = float(group["momentum"])
-            row = table[gi]
-            row["lr"] = group["lr"]
+        for row, (lr, mu, one_minus_dampening, decay, nesterov) in zip(table, values):
+            row["lr"] = lr
             row["momentum"] = mu
-            row["one_minus_dampening"] = 1.0 if gi in fresh else 1.0 - float(group["dampening"])
-            row["weight_decay"] = group["weight_decay"]
-            row["nesterov"] = 1 if group["nesterov"] else 0
+            row["one_minus_dampening"] = one_minus_dampening
+            row["weight_decay"] = decay
+            row["nesterov"] = 1 if nesterov else 0
             row["has_momentum"] = 1 if mu != 0.0 else 0
             row["grad_scale"] = 1.0
+        if joins or (recording and self._stream is not None and native.capture_id(self._stream)):
+            # The live table cannot change under a step that reads it already: one recorded before this in the
+            # same graph, or one that may still be running on a stream that is part of the recording and so
+            # cannot be waited for. This step keeps the values it was recorded with.
+            self._fixed = _to_device(table, self.device)
+            return
         nbytes = table.nbytes
         if self._hyper_dev is None or self._hyper_dev.numel() != nbytes:
-            self._slots = [torch.empty(nbytes, dtype=torch.uint8).pin_memory() for _ in range(self.RING)]
-            self._slot_events = [None] * self.RING
-            self._hyper_dev = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        # a fresh momentum buffer uploads a table for this step only
-        self._last_values = None if fresh else values
+            with _outside_capture(self.device):
+                self._slots = [torch.empty(nbytes, dtype=torch.uint8).pin_memory() for _ in range(self.RING)]
+                self._slot_events = [None] * self.RING
+                self._hyper_dev = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        self._last_values = values
+        raw = table.view(np.uint8).reshape(-1)
+        if recording:
+            # in place now, not by a copy that every replay would repeat over what later steps upload
+            with _outside_capture(self.device):
+                if self._stream is not None:
+                    self._stream.synchronize()   # the steps before this one have read the table
+                self._hyper_dev.copy_(torch.from_numpy(raw))
+            return
+        self._stream = torch.cuda.current_stream()
         i = self._cursor
         self._cursor = (i + 1) % self.RING
         if self._slot_events[i] is not None:
             self._slot_events[i].synchronize()
-        self._slots[i].numpy()[:] = table.view(np.uint8).reshape(-1)
+        self._slots[i].numpy()[:] = raw
         self._hyper_dev.copy_(self._slots[i], non_blocking=True)
         ev = torch.cuda.Event()
         ev.record()
@@ -1325,7 +1353,9 @@ class FusedSGDDriver:
         if [g.data_ptr() for g in now] != [g.data_ptr() for g in self._grads]:
             self._grads = [g.data for g in now]
         agg = self.agg
-        hyper_dev, index, params, moms, grads = self._hyper_dev, self._index, self._params, self._moms, self._grads
+        hyper_dev = self._hyper_dev if self._fixed is None else self._fixed
+        self._fixed = None
+        index, params, moms, grads = self._index, self._params, self._moms, self._grads
         if len(grads) != len(agg.is_compressed_mask):
             raise ValueError("optimizer parameters do not match the aggregator's parameter list")
         agg.step_counter += 1

@@ -13,6 +13,9 @@ def declare(lib) -> None:
     lib.psgd_device_info.restype = i32
     lib.psgd_device_info.argtypes = [C.POINTER(i32)] * 4
 
+    lib.psgd_capture_id.restype = i32
+    lib.psgd_capture_id.argtypes = [vp, C.POINTER(C.c_ulonglong)]
+
     lib.psgd_capture_mode.restype = i32
     lib.psgd_capture_mode.argtypes = [C.POINTER(i32)]
 

@@ -74,6 +74,13 @@ def check(code: int, what: str) -> None:
         raise RuntimeError(f"{what} failed (code {code}): {msg.decode() if msg else ''}")
 
 
+def capture_id(stream) -> int:
+    """Id of the CUDA-graph recording that `stream` is part of; 0 when it is not being recorded."""
+    out = ctypes.c_ulonglong(0)
+    check(lib().psgd_capture_id(ctypes.c_void_p(stream.cuda_stream), ctypes.byref(out)), "psgd_capture_id")
+    return int(out.value)
+
+
 @contextlib.contextmanager
 def relaxed_capture():
     """While this thread is recording a CUDA graph, calls that do not belong to the recording (allocations, a

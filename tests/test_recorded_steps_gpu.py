@@ -1,0 +1,113 @@
+"""Steps recorded in a CUDA graph by the program itself (`torch.cuda.graph` around `optimizer_step`): what
+happens between the recording and its replays - other learning rates, other tensors - must reach the
+replays exactly as it reaches eager steps, and must never pull memory away from under them."""
+import pytest
+import torch
+
+from powersgd_b200 import Config, PowerSGD, optimizer_step
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(128, 300), (70, 129), (33,)]
+
+
+def _tensors(shapes, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn(s, generator=g, device="cuda") for s in shapes]
+
+
+class _Program:
+    """A model's tensors, SGD with momentum, and a step that accumulates the same fresh gradients each time."""
+
+    def __init__(self, dampening=0.0):
+        self.params = [torch.nn.Parameter(x) for x in _tensors(SHAPES, 9)]
+        for p, x in zip(self.params, _tensors(SHAPES, 10)):
+            p.grad = x
+        self.optimizer = torch.optim.SGD(self.params, lr=0.1, momentum=0.9, dampening=dampening)
+        # two half-iterations per step: every step starts on the same side, so one graph serves them all
+        self.aggregator = PowerSGD(self.params, Config(rank=2, num_iters_per_step=2, start_compressing_after_num_steps=0))
+        self.fresh = _tensors(SHAPES, 11)
+
+    def step(self, rate=None):
+        if rate is not None:
+            self.optimizer.param_groups[0]["lr"] = rate
+        torch._foreach_add_([p.grad for p in self.params], self.fresh)
+        optimizer_step(self.optimizer, self.aggregator)
+
+    def record(self, *rates):
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for rate in rates:
+                self.step(rate)
+        return graph
+
+    def state(self):
+        torch.cuda.synchronize()
+        moms = [self.optimizer.state[p]["momentum_buffer"] for p in self.params]
+        return [t.clone() for p, m in zip(self.params, moms) for t in (p.detach(), p.grad, m)]
+
+
+def _same(a, b):
+    return all(torch.equal(x, y) for x, y in zip(a.state(), b.state()))
+
+
+@pytest.mark.parametrize("dampening", [0.0, 0.3])
+def test_replays_use_the_rate_of_the_last_prepared_step(dampening):
+    """A fresh optimizer, one eager step, the second step recorded; then more changes of the rate than the
+    table's ring has slots, eager steps and replays in turn."""
+    recorded, eager = _Program(dampening), _Program(dampening)
+    recorded.step(), eager.step()
+    if dampening:   # the first step's buffers take the whole gradient, the steps from here on do not
+        recorded.step(), eager.step()
+    graph = recorded.record(None)
+    rates = [0.05, 0.02, 0.2, 0.01, 0.3, 0.07, 0.15]
+    for i, rate in enumerate(rates):
+        recorded.step(rate), eager.step(rate)
+        for _ in range(2 if i == 0 else 1):
+            graph.replay()
+            eager.step()
+        assert _same(recorded, eager), i
+
+
+def test_rate_changed_for_the_recorded_step_itself():
+    recorded, eager = _Program(), _Program()
+    recorded.step(), eager.step()
+    graph = recorded.record(0.03)
+    for _ in range(2):
+        graph.replay()
+        eager.step(0.03)
+    assert _same(recorded, eager)
+    recorded.step(0.2), eager.step(0.2)
+    graph.replay()   # follows the eager step
+    eager.step()
+    assert _same(recorded, eager)
+
+
+def test_two_steps_of_one_recording_with_rates_of_their_own():
+    recorded, eager = _Program(), _Program()
+    recorded.step(), eager.step()
+    graph = recorded.record(0.03, 0.4)
+    for _ in range(3):
+        graph.replay()
+        eager.step(0.03), eager.step(0.4)
+    assert _same(recorded, eager)
+
+
+def test_first_step_recorded_on_the_stream_of_the_eager_ones():
+    """Recorded without waiting for the eager step before it, on the same stream: that step may still be
+    running and keeps its rate, the recorded one has its own."""
+    recorded, eager = _Program(), _Program()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        recorded.step(), recorded.step()
+        graph.capture_begin()
+        recorded.step(0.03)
+        graph.capture_end()
+        graph.replay()
+    torch.cuda.current_stream().wait_stream(stream)
+    for rate in (None, None, 0.03):
+        eager.step(rate)
+    assert _same(recorded, eager)
