@@ -1,8 +1,11 @@
 // Host-side odds and ends of the native library: last-error string, version, device query.
 #include <cuda_runtime.h>
 #include <stdarg.h>
+#include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <mutex>
+#include <vector>
 
 #define PSGD_API extern "C" __attribute__((visibility("default")))
 
@@ -54,6 +57,56 @@ PSGD_API int psgd_capture_mode(int* mode) {
   if (e != cudaSuccess) { psgd_set_error("cudaThreadExchangeStreamCaptureMode: %s", cudaGetErrorString(e)); return (int)e; }
   *mode = (int)m;
   return 0;
+}
+
+// ---- what lives as long as a recorded graph --------------------------------------------------
+// The caller numbers what a graph refers to and asks from time to time which numbers are free again. The
+// destructor of a user object may run on a thread of the driver and may call nothing of CUDA, so it only
+// notes the number. The list is never destroyed: graphs may go after the static objects of the process.
+struct Finished {
+  std::mutex lock;
+  std::vector<long long> numbers;
+};
+static Finished& finished() {
+  static Finished* f = new Finished;
+  return *f;
+}
+static void CUDART_CB note_finished(void* number) {
+  Finished& f = finished();
+  std::lock_guard<std::mutex> hold(f.lock);
+  f.numbers.push_back((long long)(intptr_t)number);
+}
+
+// Notes `number` as finished once the graph that `stream` is being recorded into, and every executable
+// instance of it, are destroyed. Returns a CUDA error code (-1: the stream is not being recorded).
+PSGD_API int psgd_graph_retain(long long number, cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  cudaError_t e = cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, &graph, nullptr, nullptr);
+  if (e == cudaSuccess && (status != cudaStreamCaptureStatusActive || graph == nullptr)) {
+    psgd_set_error("psgd_graph_retain: the stream is not being recorded");
+    return -1;
+  }
+  cudaUserObject_t object = nullptr;
+  if (e == cudaSuccess) e = cudaUserObjectCreate(&object, (void*)(intptr_t)number, note_finished, 1, cudaUserObjectNoDestructorSync);
+  if (e == cudaSuccess) {
+    e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
+  }
+  if (e != cudaSuccess) { psgd_set_error("psgd_graph_retain: %s", cudaGetErrorString(e)); return (int)e; }
+  return 0;
+}
+
+// Up to `most` finished numbers, each handed out once; returns how many.
+PSGD_API int psgd_graph_released(long long* numbers, int most) {
+  Finished& f = finished();
+  std::lock_guard<std::mutex> hold(f.lock);
+  int n = 0;
+  while (n < most && !f.numbers.empty()) {
+    numbers[n++] = f.numbers.back();
+    f.numbers.pop_back();
+  }
+  return n;
 }
 
 #ifdef PSGD_BOUNDS_CHECK

@@ -21,7 +21,6 @@ Factor bookkeeping for half-iteration t of a step (left = the P side is the inpu
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes
 import os
 import weakref
@@ -32,6 +31,8 @@ import torch
 import torch.distributed as dist
 
 from .ops import layout, native
+from .ops.recording import capture_scope, keep_with_graph, outside_capture  # noqa: F401  (capture_scope: for callers)
+from .ops.recording import to_device as _to_device
 from .utils import is_dense, like_strided, same_layout, world_size
 
 
@@ -75,75 +76,6 @@ def _ptr_array(tensors: Sequence[torch.Tensor]):
     for i, t in enumerate(tensors):
         arr[i] = t.data_ptr()
     return arr
-
-
-_upload_streams: Dict[torch.device, torch.cuda.Stream] = {}
-
-
-@contextlib.contextmanager
-def _outside_capture(device: torch.device):
-    """Runs its body at once, whether or not a CUDA graph is being recorded on the current stream: what
-    never changes (descriptor tables, cleared counters) is put in place once instead of by a node that
-    every replay of the graph pays for (eight copies of 1.3 us each in the step of a small perceptron).
-    Under capture the body gets a stream that is not part of it, so that its tensors come from the
-    ordinary pool - memory of the graph's own pool may be written by an earlier node of the same graph -
-    and is waited for; the thread is in the relaxed capture mode meanwhile, whatever mode the recording
-    was begun with (an allocation in the strict one ends it with an error)."""
-    if not torch.cuda.is_current_stream_capturing():
-        yield
-        return
-    device = torch.device("cuda", torch.cuda.current_device()) if device.index is None else device
-    with native.relaxed_capture():
-        while True:
-            stream = _upload_streams.setdefault(device, torch.cuda.Stream(device=device))
-            with torch.cuda.stream(stream):
-                if torch.cuda.is_current_stream_capturing():   # streams are handed out in turn: this one was forked into the capture
-                    del _upload_streams[device]
-                    continue
-                yield
-                stream.synchronize()
-                return
-
-
-def _keep_with_graph(*tensors: torch.Tensor) -> None:
-    """Tensors whose addresses are being recorded must live as long as the graph does, whatever later
-    rebinding drops them from their owner. Inside a `capture_scope` the graph's owner keeps them; a
-    capture made without one parks them here for the life of the process."""
-    if torch.cuda.is_current_stream_capturing():
-        (_capture_keep if _capture_keep is not None else _CAPTURED_TABLES).append(tensors)
-
-
-def _to_device(array: np.ndarray, device: torch.device) -> torch.Tensor:
-    """Upload a descriptor table: staged through pinned memory with an async copy on the current stream
-    (at once and outside the graph while one is being recorded)."""
-    raw = np.ascontiguousarray(array).view(np.uint8).reshape(-1)
-    with _outside_capture(device):
-        pinned = torch.empty(max(raw.size, 1), dtype=torch.uint8).pin_memory()
-        pinned.numpy()[: raw.size] = raw
-        out = torch.empty(max(raw.size, 1), dtype=torch.uint8, device=device)
-        out.copy_(pinned, non_blocking=True)
-        out._psgd_pinned_src = pinned
-    _keep_with_graph(out)
-    return out
-
-
-_CAPTURED_TABLES: list = []
-_capture_keep: Optional[list] = None
-
-
-class capture_scope:
-    """`with capture_scope() as keep:` around a CUDA-graph capture collects the descriptor tables
-    uploaded during it in `keep`; store `keep` next to the graph and drop both together."""
-
-    def __enter__(self) -> list:
-        global _capture_keep
-        self._outer = _capture_keep
-        _capture_keep = []
-        return _capture_keep
-
-    def __exit__(self, *exc):
-        global _capture_keep
-        _capture_keep = self._outer
 
 
 def _split_even(total: int, max_chunk: int, multiple: int) -> List[Tuple[int, int]]:
@@ -491,9 +423,8 @@ class NativeCompressor:
         self._split_tile_lists()
         self._partial = torch.empty(self.tiles.partial_floats, device=self.device, dtype=torch.float32)
         self._partial_tc = torch.empty(self.tiles.partial_tc_floats, device=self.device, dtype=torch.float32)
-        with _outside_capture(self.device):   # zero between launches: every launch leaves them so
+        with outside_capture(self.device):   # zero between launches: every launch leaves them so
             self._tickets = torch.zeros(self.tiles.n_tickets, device=self.device, dtype=torch.int32)
-        _keep_with_graph(self._tickets)
         self._out_views = out_views
         self._tapes.clear()
         self._key = key
@@ -559,6 +490,7 @@ class NativeCompressor:
         a small model spends most of its step there). `key`: whatever the arguments depend on beyond
         the bound tensors; a new binding drops all tapes. Only where a step is nothing but launches on
         one stream: one worker, nothing launched ahead, no phase timing."""
+        self._keep_recorded()
         plain = (world_size() == 1 and self.comm is None and self._early is None and self._early_product_done is None
                  and not _Range.enabled and _Range.events is None)
         if not plain:
@@ -580,6 +512,17 @@ class NativeCompressor:
             if code != 0:
                 native.check(code, name)
             self.launches += launched
+
+    def _keep_recorded(self) -> None:
+        """Everything a step addresses besides the caller's tensors stays alive with a graph that records
+        it: the next binding replaces the tables and the scratch, and the owner may go altogether."""
+        if torch.cuda.is_current_stream_capturing():
+            keep_with_graph(
+                self._mats_dev, self._maps_dev, [t for lists in self._tiles_dev.values() for t, _count in lists.values()],
+                self._partial, self._partial_tc, self._tickets, self._out_arena, self._hyper_dev, self._status,
+                self.units, self.chunks, self._orth_part, self._orth_rinv, self.h_in, self.h_loc, self.h_sum, self.cmat,
+                self.core._ps_buffer, self.core._qs_buffer,
+            )
 
     # -- phases ----------------------------------------------------------------------------
     def _orth(self, side: str, x: torch.Tensor, copy_to: torch.Tensor, prev: List[torch.Tensor], cm: List[torch.Tensor],
@@ -1081,6 +1024,7 @@ class NativeFlatAllReduce:
         self.launches += 1
 
     def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool = False) -> None:
+        keep_with_graph(self._items_dev, self._block_item, self._block_first, hyper_dev, self._flat, self._out)
         if self.path == "local":
             self._launch(4 if sgd else 3, hyper_dev, 1.0, early)
         elif self.path == "bulk":
@@ -1183,6 +1127,7 @@ class MultiTensorAccumulate:
             self._nblocks = len(block_item)
             self._hyper = _to_device(NativeCompressor._default_hyper(), device)
             self._key = key
+        keep_with_graph(self._items, self._block_item, self._block_first, self._hyper)
         code = self.lib.psgd_flat_launch(
             8 if push is None else 9, self._vec, _ptr(self._items), _ptr(self._block_item), _ptr(self._block_first),
             self._nblocks, _ptr(self._hyper), ctypes.c_void_p(0), 1.0 if push is None else float(world_size()),
@@ -1293,7 +1238,7 @@ class FusedSGDDriver:
             return
         nbytes = table.nbytes
         if self._hyper_dev is None or self._hyper_dev.numel() != nbytes:
-            with _outside_capture(self.device):
+            with outside_capture(self.device):
                 self._slots = [torch.empty(nbytes, dtype=torch.uint8).pin_memory() for _ in range(self.RING)]
                 self._slot_events = [None] * self.RING
                 self._hyper_dev = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
@@ -1301,7 +1246,7 @@ class FusedSGDDriver:
         raw = table.view(np.uint8).reshape(-1)
         if recording:
             # in place now, not by a copy that every replay would repeat over what later steps upload
-            with _outside_capture(self.device):
+            with outside_capture(self.device):
                 if self._stream is not None:
                     self._stream.synchronize()   # the steps before this one have read the table
                 self._hyper_dev.copy_(torch.from_numpy(raw))

@@ -19,6 +19,11 @@ def declare(lib) -> None:
     lib.psgd_capture_mode.restype = i32
     lib.psgd_capture_mode.argtypes = [C.POINTER(i32)]
 
+    lib.psgd_graph_retain.restype = i32
+    lib.psgd_graph_retain.argtypes = [C.c_longlong, vp]
+    lib.psgd_graph_released.restype = i32
+    lib.psgd_graph_released.argtypes = [C.POINTER(C.c_longlong), i32]
+
     lib.psgd_orth_launch.restype = i32
     lib.psgd_orth_launch.argtypes = [vp, i32, vp, i32, i32, vp, vp, i32, vp, vp, vp, vp, vp, vp, i32, vp]
 

@@ -1,10 +1,15 @@
 """Steps recorded in a CUDA graph by the program itself (`torch.cuda.graph` around `optimizer_step`): what
 happens between the recording and its replays - other learning rates, other tensors - must reach the
 replays exactly as it reaches eager steps, and must never pull memory away from under them."""
+import gc
+import time
+import weakref
+
 import pytest
 import torch
 
 from powersgd_b200 import Config, PowerSGD, optimizer_step
+from powersgd_b200.ops.recording import release_finished
 
 pytestmark = pytest.mark.gpu
 
@@ -111,3 +116,68 @@ def test_first_step_recorded_on_the_stream_of_the_eager_ones():
     for rate in (None, None, 0.03):
         eager.step(rate)
     assert _same(recorded, eager)
+
+
+def _write_over_free_memory():
+    """Blocks of every size the tables and the scratch of a step could have had, several of each, written."""
+    return [torch.full((size,), -1, dtype=torch.int32, device="cuda") for size in (8, 64, 128, 512, 2048, 8192, 1 << 15, 1 << 17) for _ in range(24)]
+
+
+def _step_on_other_gradients(program):
+    own = [p.grad for p in program.params]
+    other = _tensors(SHAPES, 77)
+    for p, x in zip(program.params, other):
+        p.grad = x
+    program.step()
+    for p, x in zip(program.params, own):
+        p.grad = x
+    return other
+
+
+def test_replay_after_other_tensors_were_bound():
+    """An eager step on other gradient tensors replaces the descriptor tables and the scratch; the graph
+    still refers to the old ones."""
+    recorded, eager = _Program(), _Program()
+    recorded.step(), eager.step()
+    graph = recorded.record(None)
+    others = _step_on_other_gradients(recorded), _step_on_other_gradients(eager)
+    junk = _write_over_free_memory()
+    for _ in range(2):
+        graph.replay()
+        eager.step()
+    assert _same(recorded, eager)
+    assert all(torch.equal(a, b) for a, b in zip(*others))
+    assert all(bool((j == -1).all()) for j in junk)
+
+
+def test_replay_after_the_aggregator_is_gone():
+    recorded, eager = _Program(), _Program()
+    recorded.step(), eager.step()
+    graph = recorded.record(None)
+    del recorded.aggregator
+    gc.collect()
+    junk = _write_over_free_memory()
+    graph.replay()
+    eager.step()
+    assert _same(recorded, eager)
+    assert all(bool((j == -1).all()) for j in junk)
+
+
+def test_what_a_graph_refers_to_goes_with_it():
+    recorded = _Program()
+    recorded.step()
+    graph = recorded.record(None)
+    native = recorded.aggregator._powersgd._native
+    refs = [weakref.ref(native._tickets), weakref.ref(native._partial), weakref.ref(native._mats_dev)]
+    del native
+    _step_on_other_gradients(recorded)
+    release_finished()
+    assert all(ref() is not None for ref in refs)
+    del graph
+    gc.collect()
+    torch.cuda.synchronize()
+    until = time.monotonic() + 20   # the graph says so on a thread of the driver
+    while any(ref() is not None for ref in refs) and time.monotonic() < until:
+        release_finished()
+        time.sleep(0.01)
+    assert all(ref() is None for ref in refs)
