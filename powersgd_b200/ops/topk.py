@@ -14,6 +14,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import native
+from .recording import keep_with_graph, outside_capture, release_finished
 
 _workspaces = {}
 
@@ -26,10 +27,14 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
         memory is None or (memory.is_contiguous() and memory.dtype == torch.float32)
     ):
         lib = native.lib()
-        ws = _workspaces.get(flat.device)
+        recorded = torch.cuda.is_current_stream_capturing()   # a graph gets counters of its own, see topk_abs_many
+        ws = None if recorded else _workspaces.get(flat.device)
         if ws is None:
             ws = torch.zeros(lib.psgd_topk_workspace_ints(), dtype=torch.int32, device=flat.device)
-            _workspaces[flat.device] = ws
+            if recorded:
+                keep_with_graph(ws)
+            else:
+                _workspaces[flat.device] = ws
         values = torch.empty(k, dtype=torch.float32, device=flat.device)
         positions = torch.empty(k, dtype=torch.int32, device=flat.device)
         code = lib.psgd_topk_abs(
@@ -80,8 +85,12 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
 
     lib = native.lib()
     key = (device, tuple(t.data_ptr() for t in tensors), tuple(0 if m is None else m.data_ptr() for m in mems), tuple(t.numel() for t in tensors), tuple(ks))
-    entry = _many_cache.get(key)
+    # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
+    # replay may run beside an eager call on the same tensors
+    recorded = torch.cuda.is_current_stream_capturing()
+    entry = None if recorded else _many_cache.get(key)
     if entry is None:
+        release_finished()
         dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64)])
         if dtype.itemsize != int(lib.psgd_topk_item_bytes()):
             raise RuntimeError("top-k item record out of sync with the native library")
@@ -101,17 +110,21 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
             block_item += [i] * nparts
             block_part += list(range(nparts))
         to_dev = lambda a: torch.from_numpy(a.view(np.uint8) if a.dtype.names else a).to(device)  # noqa: E731
-        entry = {
-            "items": to_dev(items), "block_item": to_dev(np.asarray(block_item, dtype=np.int32)),
-            "block_part": to_dev(np.asarray(block_part, dtype=np.int32)), "parts": to_dev(np.asarray(parts, dtype=np.int32)),
-            "nblocks": len(block_item),
-            "ws": torch.zeros(len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
-        }
-        # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
-        # valid for whatever tensors present the same addresses again, so no tensor is kept alive
-        if len(_many_cache) >= 4:
-            _many_cache.clear()
-        _many_cache[key] = entry
+        with outside_capture(device):
+            entry = {
+                "items": to_dev(items), "block_item": to_dev(np.asarray(block_item, dtype=np.int32)),
+                "block_part": to_dev(np.asarray(block_part, dtype=np.int32)), "parts": to_dev(np.asarray(parts, dtype=np.int32)),
+                "nblocks": len(block_item),
+                "ws": torch.zeros(len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
+            }
+        if recorded:
+            keep_with_graph(entry)
+        else:
+            # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
+            # valid for whatever tensors present the same addresses again, so no tensor is kept alive
+            if len(_many_cache) >= 4:
+                _many_cache.clear()
+            _many_cache[key] = entry
     values = torch.empty(total, dtype=torch.float32, device=device)
     positions = torch.empty(total, dtype=torch.int32, device=device)
     vp = ctypes.c_void_p
@@ -155,35 +168,46 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
         device = all_values.device
         scratch = _combine_scratch.get(device)
         if scratch is None:
-            scratch = torch.zeros(2, dtype=torch.int32, device=device)  # [grid barrier, status]
+            with outside_capture(device):
+                scratch = torch.zeros(2, dtype=torch.int32, device=device)  # [grid barrier, status]
             _combine_scratch[device] = scratch
+        barrier = scratch
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        # tables of addresses and lengths, kept by exactly those (as the selection's above): building and
-        # uploading one stalls the host until the selection has run
+        # tables of addresses and lengths, kept by exactly those (as the selection's above, recorded calls
+        # included): building and uploading one stalls the host until the selection has run
         key = (device, tuple(o.data_ptr() for o in outs), tuple(o.numel() for o in outs), tuple(ends))
-        tables = _segment_cache.get(key)
+        recorded = torch.cuda.is_current_stream_capturing()
+        tables = None if recorded else _segment_cache.get(key)
         if tables is None:
+            release_finished()
             tables = []
-            for first in range(0, len(outs), cap):
-                chunk = list(range(first, min(first + cap, len(outs))))
-                segs = np.zeros(len(chunk), dtype=_SEG_DTYPE)
-                base = ends[first - 1] if first else 0
-                for j, s in enumerate(chunk):
-                    segs[j] = (outs[s].data_ptr(), outs[s].numel(), ends[s] - base)
-                tables.append((torch.from_numpy(segs.view(np.uint8)).to(device, non_blocking=False), len(chunk), base, ends[chunk[-1]] - base))
-            if len(_segment_cache) >= 4:
-                _segment_cache.clear()
-            _segment_cache[key] = tables
+            with outside_capture(device):
+                for first in range(0, len(outs), cap):
+                    chunk = list(range(first, min(first + cap, len(outs))))
+                    segs = np.zeros(len(chunk), dtype=_SEG_DTYPE)
+                    base = ends[first - 1] if first else 0
+                    for j, s in enumerate(chunk):
+                        segs[j] = (outs[s].data_ptr(), outs[s].numel(), ends[s] - base)
+                    tables.append((torch.from_numpy(segs.view(np.uint8)).to(device, non_blocking=False), len(chunk), base, ends[chunk[-1]] - base))
+                if recorded:
+                    barrier = torch.zeros(1, dtype=torch.int32, device=device)
+            if recorded:
+                keep_with_graph(tables, barrier, scratch)
+            else:
+                if len(_segment_cache) >= 4:
+                    _segment_cache.clear()
+                _segment_cache[key] = tables
         for segs_dev, count, base, width in tables:
             vals = all_values if (base == 0 and width == per_worker) else all_values[:, base : base + width].contiguous()
             poss = all_positions if (base == 0 and width == per_worker) else all_positions[:, base : base + width].contiguous()
             code = lib.psgd_sparse_combine_launch(
                 ctypes.c_void_p(vals.data_ptr()), ctypes.c_void_p(poss.data_ptr()), int(workers), ctypes.c_longlong(width),
                 ctypes.c_void_p(segs_dev.data_ptr()), count, ctypes.c_float(divisor),
-                ctypes.c_void_p(scratch.data_ptr()), ctypes.c_void_p(scratch.data_ptr() + 4), stream,
+                ctypes.c_void_p(barrier.data_ptr()), ctypes.c_void_p(scratch.data_ptr() + 4), stream,
             )
             native.check(code, "psgd_sparse_combine_launch")
-            segs_dev.record_stream(torch.cuda.current_stream())
+            if not recorded:
+                segs_dev.record_stream(torch.cuda.current_stream())
         return
     start = 0
     for out, end in zip(outs, ends):

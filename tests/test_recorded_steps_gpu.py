@@ -181,3 +181,34 @@ def test_what_a_graph_refers_to_goes_with_it():
         release_finished()
         time.sleep(0.01)
     assert all(ref() is None for ref in refs)
+
+
+@pytest.mark.parametrize("reducer", ["TopKReducer", "GlobalTopKReducer"])
+@pytest.mark.parametrize("warm", [False, True])
+def test_recorded_topk_reduce_survives_other_tensor_sets(reducer, warm):
+    """The reducers keep tables for the last few sets of tensors; a recorded call must not depend on them."""
+    from powersgd_b200.paper import reducers
+
+    shapes = [(300, 200), (64, 27), (129,), (1,)]
+    red = getattr(reducers, reducer)(0, torch.device("cuda:0"), compression=1 / 16)
+    new = lambda seed: (_tensors(shapes, seed), [torch.full(s, 7.0, device="cuda") for s in shapes], [torch.full(s, 7.0, device="cuda") for s in shapes])  # noqa: E731
+    send, out, memory = new(0)
+    if warm:
+        red.reduce(send, out, memory)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        red.reduce(send, out, memory)
+    held = [new(seed) for seed in range(1, 7)]
+    for other in held:
+        red.reduce(*other)
+    junk = _write_over_free_memory()
+    for seed in (20, 21):
+        for x, fresh in zip(send, _tensors(shapes, seed)):
+            x.copy_(fresh)
+        graph.replay()
+        want = new(seed)
+        red.reduce(*want)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(out + memory, want[1] + want[2]))
+    assert all(bool((j == -1).all()) for j in junk)
