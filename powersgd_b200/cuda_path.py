@@ -107,13 +107,8 @@ class TilePlan:
             raise ValueError(f"rank {self.max_r} exceeds the compiled maximum {layout.MAX_RANK}")
         self.rt = lib.psgd_gemm_template_rank(self.max_r)
         self.total_elems = sum(g.n * g.m * g.batch for g in plan.groups)
-        nt_rows_cap = lib.psgd_gemm_nt_max_rows(self.max_r)
-        # rows of an NT tile: twice as many halve what a tile costs besides its loads (start, staging, the
-        # sum over the warps, the hand-over), as long as some 300 tiles are left for the 148 SMs. 128 / 256
-        # rows: ResNet-18 (11 M elements) 14.1 / 12.2 us, 3 x 1001x777 + 2 x 515x2049 (4 M) 12.4 / 13.7 us;
-        # matrices above 4096 rows, 256 / 512: the LSTM model (32 M) 52.8 / 49.0 us.
-        self.nt_rows = min(nt_rows_cap, 128 if self.total_elems < (8 << 20) else 256)
-        self.nt_tall_rows = 256 if self.total_elems < (16 << 20) else 512
+        self._nt_rows_cap = lib.psgd_gemm_nt_max_rows(self.max_r)
+        self.nt_rows, self.nt_tall_rows = min(self._nt_rows_cap, 128), 256   # chosen anew by every `build`
         self.nn_rows = lib.psgd_gemm_nn_tile_rows(self.max_r)
         self.nn_cols_cap = lib.psgd_gemm_nn_max_cols(self.max_r)
         self.rp_tc = lib.psgd_gemm_tc_rank_pad(self.max_r)
@@ -136,6 +131,7 @@ class TilePlan:
         tc_mats = [self.plan.groups[gi] for (gi, _p, _i), f in zip(self.mats, tc_flags) if f]
         tc_k_nt = self._pick_tc_k(tc_mats, transposed=True)
         tc_k_nn = self._pick_tc_k(tc_mats, transposed=False)
+        self._pick_nt_rows([self.plan.groups[gi] for (gi, _p, _i), f in zip(self.mats, tc_flags) if not f])
         for mi, (gi, _pos, _idx) in enumerate(self.mats):
             g = self.plan.groups[gi]
             v = int(vec_widths[mi])
@@ -161,11 +157,7 @@ class TilePlan:
                     ticket += 1
                     tc_slots += len(col_blocks)
                 continue
-            # tall matrices: tiles of 256 or 512 rows (128 or 256 KiB: small enough that every SM gets several
-            # CTAs, which is what hides the load latency) but never more than 160 partial tiles
-            # per column block (the kernel walks a taller tile in chunks of its staging buffer)
-            rows_per_tile = max(self.nt_rows if g.n <= 4096 else self.nt_tall_rows, -(-(-(-g.n // 160)) // 128) * 128)
-            row_blocks = _split_even(g.n, rows_per_tile, 1)
+            row_blocks = _split_even(g.n, self._nt_tile_rows(g.n), 1)
             for c0 in range(0, g.m, 128):
                 cols = min(128, g.m - c0)
                 for si, (r0, rows) in enumerate(row_blocks):
@@ -191,6 +183,31 @@ class TilePlan:
             "nn": {k: arr(v) for k, v in nn.items()},
             "fin": {k: arr(v) for k, v in fin.items()},
         }
+
+    NT_TILES = 250   # of the CUDA-core NT product, at least: some five for three of the 148 SMs
+
+    def _nt_tile_rows(self, n: int) -> int:
+        # tall matrices: never more than 160 partial tiles per column block (the kernel walks a tile that is
+        # taller than its staging buffer in chunks)
+        return max(self.nt_rows if n <= 4096 else self.nt_tall_rows, -(-(-(-n // 160)) // 128) * 128)
+
+    def _pick_nt_rows(self, groups) -> None:
+        """Rows of an NT tile (`groups`: the matrices of the CUDA-core launch, one entry each). Twice as many
+        halve what a tile costs besides its loads (start, staging, the sum over the warps, the hand-over),
+        as long as NT_TILES are left; only the tiles of this launch count, not the elements of the model, most of
+        which may be multiplied by the tensor cores. Measured (us per launch, data in L2, tiles at the larger
+        size): 128 / 256 rows: 192 tiles (6 x 1024x1001, rank 2) 8.1 / 9.8, 186 (3 x 1001x777 + 2 x 515x2049,
+        rank 3) 9.4 / 11.1, 240 (10 x 513x1001, rank 4) 9.3 / 10.1, 256 (8 x 1024x1001, rank 2) 11.9 / 9.8, 288 (9 of
+        them, rank 4) 14.5 / 12.5, 378 (ResNet-18) 12.8 / 10.9; 2 x 700x650 beside two matrices of 33 M elements:
+        6.0 / 8.1. Matrices above 4096 rows, 256 / 512: 204 (17000x650, rank 4) 17.7 / 18.8, 252 (21001x650) 26.3 /
+        19.5, 300 (2 x 7673x1255, rank 2) 19.5 / 17.0, 786 (the LSTM model) 46.2 / 43.1."""
+        def tiles(rows: int, tall_rows: int) -> int:
+            self.nt_rows, self.nt_tall_rows = min(self._nt_rows_cap, rows), tall_rows
+            return sum(-(-g.m // 128) * -(-g.n // self._nt_tile_rows(g.n)) for g in groups)
+
+        rows = 256 if tiles(256, 256) >= self.NT_TILES else 128
+        if tiles(rows, 512) < self.NT_TILES:
+            tiles(rows, 256)
 
     TC_CTAS_PER_SM = 2
     # prologue + epilogue of a tile (~4 us), in units of streamed K rows (~0.03 us each): measured

@@ -140,3 +140,34 @@ def test_in_switch_path_policy(monkeypatch):
     assert wants("nvls", 2) and not wants("bulk", 8)
     monkeypatch.setenv("NCCL_NVLS_ENABLE", "0")
     assert not wants("auto", 8) and wants("nvls", 8)
+
+
+def _nt_rows(shapes, rank, tc=lambda shape: False):
+    """Tallest CUDA-core NT tile of every matrix shape."""
+    from powersgd_b200.cuda_path import TilePlan
+
+    plan = CompressionPlan.build(shapes, rank=rank)
+    tiles = TilePlan(plan, _lib())
+    flags = [tc((plan.groups[gi].n, plan.groups[gi].m)) for gi, _p, _i in tiles.mats]
+    nt = tiles.build([4 if plan.groups[gi].m % 4 == 0 else 1 for gi, _p, _i in tiles.mats], flags)["nt"]["f"]
+    rows = {}
+    for t in nt:
+        group = plan.groups[tiles.mats[int(t["mat"])][0]]
+        rows[(group.n, group.m)] = max(rows.get((group.n, group.m), 0), int(t["rows"]))
+    return rows, len(nt)
+
+
+@pytest.mark.parametrize("rank", [1, 4, 16])
+def test_nt_tile_height_leaves_enough_tiles_of_its_own_launch(rank):
+    """Taller tiles only where they leave the launch some 250 tiles; matrices that the tensor cores multiply are
+    not part of it, however large they are."""
+    from powersgd_b200.cuda_path import TilePlan
+
+    large = [(8192, 4096)] * 2
+    for small in ([(513, 1001)] * 6, [(700, 650)] * 2, [(1024, 1001)] * 6):
+        alone, _ = _nt_rows(small, rank)
+        beside, count = _nt_rows(large + small, rank, tc=lambda shape: shape == (8192, 4096))
+        assert alone == beside and max(beside.values()) <= 128 and count < 2 * TilePlan.NT_TILES
+    assert max(_nt_rows([(1024, 1001)] * 9, rank)[0].values()) == 256
+    assert _nt_rows([(21001, 650)], rank)[0][(21001, 650)] > 256
+    assert _nt_rows([(17000, 650)], rank)[0][(17000, 650)] <= 256
