@@ -490,9 +490,9 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs 
 
 template <int RT>
 static int orth_launch_rt(const OrthArgs& a, int nchunks, int early, cudaStream_t stream) {
-  const int rc = psgd_launch(psgd_orth_gram_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, early, a);
+  const int rc = psgd_launch(psgd_orth_gram_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, early & 1, a);
   if (rc != 0) return rc;
-  return psgd_launch(psgd_orth_apply_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, 1, a);
+  return psgd_launch(psgd_orth_apply_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, (early >> 1) & 1, a);
 }
 
 // Template rank used for factors of rank max_r, and the rows of one chunk at that rank.
@@ -528,7 +528,9 @@ PSGD_API int psgd_orth_part_doubles(int max_r, int nprev) {
 // units / chunks: device tables; all units of one call share the template rank RT >= max r.
 // part: nchunks * psgd_orth_part_doubles(max_r, nprev) doubles; head: nunits * 2 * RT*RT floats.
 // comm / sum_out: see OrthArgs (null for a single worker or when x already holds the factor).
-// early: see psgd_launch (the second launch always follows the first that way).
+// early: see psgd_launch; bit 0 for the first launch, bit 1 for the second, which follows it. Both are off with
+// several workers: the first launch then waits for peers, and the CTAs of an early successor would hold
+// their places on the SMs meanwhile.
 PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks, int nchunks, int max_r, float* x,
                               float* copy_to, int nprev, const float* const* prev, float* const* cmat,
                               double* part, float* head, const void* comm,

@@ -564,7 +564,7 @@ class NativeCompressor:
             _ptr(self._orth_rinv),
             self.comm.ptr if gather_to is not None else ctypes.c_void_p(0),
             _ptr(gather_to),
-            int(early),
+            (1 if early else 0) | (2 if self._chained() else 0),   # the second launch follows the first
         )
 
     def _chained(self) -> bool:

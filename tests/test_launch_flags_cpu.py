@@ -1,0 +1,32 @@
+"""Which launches may start before their predecessor has ended (host code only, no GPU)."""
+import ctypes
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from powersgd_b200.cuda_path import NativeCompressor
+
+
+def _orth_flags(comm, early, gather):
+    nat = object.__new__(NativeCompressor)
+    buf = torch.zeros(4)
+    nat.units, nat.chunks, nat.n_units, nat.n_chunks = {"p": buf}, {"p": buf}, {"p": 1}, {"p": 1}
+    nat.tiles, nat._orth_part, nat._orth_rinv, nat.comm = SimpleNamespace(max_r=2), buf, buf, comm
+    calls = []
+    nat._call = lambda name, *args: calls.append((name, args))
+    nat._orth("p", buf, buf, [], [], buf if gather else None, early=early)
+    (name, args), = calls
+    assert name == "psgd_orth_launch"
+    return args[-1]
+
+
+def test_orthonormalisation_overlaps_on_one_worker():
+    assert _orth_flags(None, early=False, gather=False) == 2
+    assert _orth_flags(None, early=True, gather=False) == 3
+
+
+@pytest.mark.parametrize("gather", [False, True])
+def test_orthonormalisation_keeps_the_plain_order_with_several_workers(gather):
+    """A first launch that waits for peers must not have the second one's CTAs resident beside it."""
+    assert _orth_flags(SimpleNamespace(ptr=ctypes.c_void_p(8)), early=False, gather=gather) == 0
