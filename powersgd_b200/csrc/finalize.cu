@@ -251,6 +251,15 @@ constexpr int FIN_PANEL_PAD = 4;
 constexpr int FIN_RPITCH = FIN_COLS + FIN_PANEL_PAD;
 __host__ __device__ constexpr int fin_panel_floats(int tile_rows) { return FIN_RPITCH + tile_rows + FIN_PANEL_PAD; }  // per factor column
 
+// Shared-memory budgets of a strip CTA: the default carve-out serves the small ranks (several CTAs
+// stay resident per SM); when the panels of a 256-row strip do not fit it (K = 32, or K >= 16 with
+// separate local and summed factors), the kernel opts in to what the largest of them takes, 98 KiB: that
+// still leaves two CTAs per SM. Taller strips matter there: every strip re-stages 128 + rows panel
+// entries per K.
+constexpr int FIN_SMEM_DEFAULT = 48 * 1024;
+constexpr int FIN_SMEM_OPT_IN = 2 * FIN_STRIP_KMAX * fin_panel_floats(256) * (int)sizeof(float);
+static_assert(2 * (FIN_SMEM_OPT_IN + 1024) <= 227 * 1024, "two CTAs per SM");
+
 // e / r for 0 <= e < 8192 and 2 <= r <= 32, with magic = ceil(2^20 / r): the product stays below 2^32 and
 // e * (magic * r - 2^20) below 2^20.
 __device__ __forceinline__ int fin_div(int e, int r, unsigned magic) { return r == 1 ? e : (int)(((unsigned)e * magic) >> 20); }
@@ -290,7 +299,7 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
     bool ok = true;
     ok &= PSGD_BC(t.row0 >= 0 && t.rows > 0 && t.row0 + t.rows <= mt.n && t.rows <= tile_rows, 3, PSGD_BC_TILE_ROWS, t.row0 + t.rows, mt.n);
     ok &= PSGD_BC(t.col0 >= 0 && t.cols > 0 && t.col0 + t.cols <= mt.m && t.cols <= FIN_COLS, 3, PSGD_BC_TILE_COLS, t.col0 + t.cols, mt.m);
-    ok &= PSGD_BC(K >= 1 && K <= FIN_STRIP_KMAX && (SAME ? 1 : 2) * K * fin_panel_floats(tile_rows) * 4 <= 96 * 1024, 3, PSGD_BC_SMEM, K, FIN_STRIP_KMAX);
+    ok &= PSGD_BC(K >= 1 && K <= FIN_STRIP_KMAX && (SAME ? 1 : 2) * K * fin_panel_floats(tile_rows) * 4 <= FIN_SMEM_OPT_IN, 3, PSGD_BC_SMEM, K, FIN_STRIP_KMAX);
     const unsigned long long addr = (unsigned long long)mt.grad | (unsigned long long)mt.param | (unsigned long long)mt.mom | (unsigned long long)mt.out;
     ok &= PSGD_BC(t.vec == 1 || (t.vec == 2 && addr % 8 == 0 && mt.m % 2 == 0) || (t.vec == 4 && addr % 16 == 0 && mt.m % 4 == 0),
                   3, PSGD_BC_ALIGNMENT, addr % 16, t.vec);
@@ -482,13 +491,6 @@ __global__ void __launch_bounds__(FIN_THREADS, OPT ? 2 : 3) psgd_finalize_strip_
   else if (t.vec == 2) finalize_strip_tile<2, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
   else finalize_strip_tile<1, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
 }
-
-// Shared-memory budgets of a strip CTA: the default carve-out serves the small ranks (several CTAs
-// stay resident per SM); when the panels of a 256-row strip do not fit it (K = 32, or K >= 16 with
-// separate local and summed factors), the kernel opts in to a budget that still leaves two CTAs
-// per SM. Taller strips matter there: every strip re-stages 128 + rows panel entries per K.
-constexpr int FIN_SMEM_DEFAULT = 48 * 1024;
-constexpr int FIN_SMEM_OPT_IN = 96 * 1024;
 
 template <bool SAME, int RPW, bool OPT>
 static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, int early, cudaStream_t stream) {

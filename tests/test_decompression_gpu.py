@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from powersgd_b200 import Config, PowerSGD, optimizer_step
+from powersgd_b200 import BasicConfig, BasicPowerSGD, Config, PowerSGD, optimizer_step
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +44,34 @@ def test_decompression_and_update_at_strip_edges(rank, iters, momentum):
             if mom is not None:
                 assert ((opt.state[now]["momentum_buffer"].double().view_as(p) - v).abs() <= bound).all(), shapes[idx]
             assert ((now.detach().double().view_as(p) - (p - 0.1 * v)).abs() <= bound + 2.0 ** -23 * (p.abs() + v.abs())).all(), shapes[idx]
+
+
+@pytest.mark.parametrize("rank,rows", [(8, 256), (16, 256), (16, 96)])
+def test_local_and_summed_factors_apart(rank, rows):
+    """What several workers run (there without a channel): the residual from the local factors, the update
+    from the summed ones, in strips up to the tallest. The same bound as above, per product."""
+    shapes, iters, workers = [(700, 300), (256, 129), (97, 66)], 2, 3
+    core = BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=rank, num_iters_per_step=iters), backend="native")
+    g = torch.Generator(device="cuda").manual_seed(rank)
+    draw = lambda s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    grads = [draw(s) for s in shapes]
+    core.aggregate(grads)
+    nat = core._native
+    assert int(nat.lib.psgd_finalize_strip_rows(iters * rank, 0)) == 256
+    nat.tiles.fin_rows, nat._key = rows, None
+    nat._bind(grads)
+    for buf in nat.h_in + nat.h_loc + nat.h_sum:
+        buf.copy_(draw(buf.shape))
+    before = [x.double().clone() for x in grads]
+    nat._finalize([True, False], False, workers)
+    for grp in core.plan.groups:
+        for pos, idx in enumerate(grp.members):
+            p0, q0 = grp.p_offset + pos * grp.n * grp.r, grp.q_offset + pos * grp.m * grp.r
+            cut = lambda buf, at, n: buf[at : at + n * grp.r].view(n, grp.r).double()  # noqa: E731
+            own = [(cut(nat.h_in[0], p0, grp.n), cut(nat.h_loc[0], q0, grp.m)), (cut(nat.h_loc[1], p0, grp.n), cut(nat.h_in[1], q0, grp.m))]
+            all_ = [(cut(nat.h_in[0], p0, grp.n), cut(nat.h_sum[0], q0, grp.m)), (cut(nat.h_sum[1], p0, grp.n), cut(nat.h_in[1], q0, grp.m))]
+            product = lambda pairs: (sum(l @ r.T for l, r in pairs), sum(l.abs() @ r.abs().T for l, r in pairs))  # noqa: E731
+            eps, was = (grp.r * iters + 3) * 2.0 ** -24, before[idx]
+            (mine, mine_size), (total, total_size) = product(own), product(all_)
+            assert ((grads[idx].double() - (was - mine)).abs() <= eps * (mine_size + was.abs())).all(), shapes[idx]
+            assert ((nat._out_views[idx].double() - total / workers).abs() <= eps * total_size / workers).all(), shapes[idx]

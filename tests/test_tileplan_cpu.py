@@ -171,3 +171,12 @@ def test_nt_tile_height_leaves_enough_tiles_of_its_own_launch(rank):
     assert max(_nt_rows([(1024, 1001)] * 9, rank)[0].values()) == 256
     assert _nt_rows([(21001, 650)], rank)[0][(21001, 650)] > 256
     assert _nt_rows([(17000, 650)], rank)[0][(17000, 650)] <= 256
+
+
+@pytest.mark.parametrize("same", [0, 1])
+def test_tallest_strip_at_every_column_count_of_the_strip_kernel(same):
+    """256 rows wherever they did fit before panels were padded: up to 32 columns, with one set of factors or two."""
+    lib = _lib()
+    for k in range(1, 33):
+        assert int(lib.psgd_finalize_strip_rows(k, same)) == 256, k
+        assert int(lib.psgd_finalize_uses_strip(1, k, 256, same)) == 1, k
