@@ -48,11 +48,13 @@ __device__ __forceinline__ double psgd_warp_sum(double v) {
 // over the `n` partials, in split order (fixed, so the result does not depend on which tile arrived last),
 // to out[0 .. TILE_ELEMS). One CTA does this at the end of a product while the rest of the GPU has
 // nothing left to do, and a tall matrix has tens of partials per block, so what counts is how many loads
-// are under way: every thread takes a vector of elements and eight or sixteen partials at a time.
+// are under way: every thread takes four elements and eight partials at a time (tensor-core tiles, M^T P on CUDA
+// cores above rank 2), or, where that would leave more than half of the threads without work, one element
+// and sixteen partials (M^T P at rank 1 and 2, M Q on CUDA cores: at most 256 elements, one per thread).
 template <int TILE_ELEMS, int THREADS>
 __device__ __forceinline__ void psgd_sum_partials(const float* first, int n, float* out) {
-  constexpr int W = TILE_ELEMS >= 4 * THREADS / 2 ? 4 : (TILE_ELEMS >= 2 * THREADS ? 2 : 1);   // floats per thread and load
-  constexpr int B = W == 4 ? 8 : 16;                                                              // loads under way
+  constexpr int W = TILE_ELEMS >= 2 * THREADS ? 4 : 1;   // floats per thread and load
+  constexpr int B = W == 4 ? 8 : 16;                     // loads under way
   static_assert(TILE_ELEMS % W == 0, "whole vectors");
   for (int e = threadIdx.x * W; e < TILE_ELEMS; e += THREADS * W) {
     float s[W];
@@ -67,9 +69,6 @@ __device__ __forceinline__ void psgd_sum_partials(const float* first, int n, flo
           if (W == 4) {
             const float4 q = __ldcg(reinterpret_cast<const float4*>(src));
             v[j][0] = q.x; v[j][1 % W] = q.y; v[j][2 % W] = q.z; v[j][3 % W] = q.w;
-          } else if (W == 2) {
-            const float2 q = __ldcg(reinterpret_cast<const float2*>(src));
-            v[j][0] = q.x; v[j][1 % W] = q.y;
           } else {
             v[j][0] = __ldcg(src);
           }
