@@ -1043,7 +1043,7 @@ class NativeFlatAllReduce:
     def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool = False) -> None:
         keep_with_graph(self._items_dev, self._block_item, self._block_first, hyper_dev, self._flat, self._out)
         if self.path == "local":
-            self._launch(4 if sgd else 3, hyper_dev, 1.0, early)
+            self._launch(4 if sgd else 3, hyper_dev, 1.0, early and sgd)
         elif self.path == "bulk":
             self._launch(0, hyper_dev, float(workers))
             code = self.lib.psgd_bulk_allreduce_launch(self.comm.ptr, ctypes.c_longlong(self.n_pad), workers, _stream_ptr())
@@ -1067,21 +1067,22 @@ class NativeFlatAllReduce:
             self._launch(2 if sgd else 1, hyper_dev, 1.0)
 
     def aggregate(self, gradients: List[torch.Tensor], outs: Optional[Sequence[torch.Tensor]] = None,
-                  keep_inputs: bool = False, early: bool = False) -> List[torch.Tensor]:
+                  keep_inputs: bool = False) -> List[torch.Tensor]:
         """Mean over workers. `outs`: caller-owned destination tensors (default: views of this
-        object's buffer, valid until the next call). `keep_inputs`: do not zero the inputs. `early`:
-        the launch before this one is the decompression of other tensors, whose end it may overlap."""
+        object's buffer, valid until the next call). `keep_inputs`: do not zero the inputs."""
         self.check()
         self.launches = 0
         self._bind(gradients, outs=outs)
         self._keep_inputs = bool(keep_inputs)
         try:
-            self._run(self._hyper_dev, world_size(), sgd=False, early=early)
+            self._run(self._hyper_dev, world_size(), sgd=False)
         finally:
             self._keep_inputs = False
         return list(self._views)
 
     def aggregate_and_step(self, gradients, params, moms, hyper_index, hyper_dev, early: bool = False) -> None:
+        """The mean and the optimizer step in one pass. `early`: the launch before this one is the
+        decompression of other tensors, whose end it may overlap (one worker)."""
         self.check()
         self.launches = 0
         self._bind(gradients, params, moms, hyper_index, need_out=False)
