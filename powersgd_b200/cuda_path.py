@@ -519,6 +519,8 @@ class NativeCompressor:
             self._tape = []
             try:
                 body()
+                if len(self._tapes) >= 16:   # recordings with tables of their own bring keys of their own
+                    self._tapes.clear()
                 self._tapes[key] = self._tape
             finally:
                 self._tape = None
