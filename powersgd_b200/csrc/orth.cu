@@ -500,9 +500,13 @@ PSGD_API int psgd_orth_template_rank(int max_r) {
   return max_r <= 1 ? 1 : max_r <= 2 ? 2 : max_r <= 4 ? 4 : max_r <= 8 ? 8 : max_r <= 16 ? 16 : 32;
 }
 // Rows of a chunk when the longest unit has `longest` rows. A short unit takes the base size. Every
-// chunk of the second launch reads the partial matrices of ALL chunks of its unit, so their number
-// is bounded: at the bound the partials are 32 to 400 KB per unit, read in as long as the chunk's own
-// rows take. (An embedding of 50257 rows at rank 16: 79 chunks instead of 393.)
+// chunk of the second launch reads the partial matrices of ALL chunks of its unit, so their number is
+// bounded for a long factor: at the bound the partial Gram matrices of a unit are 2, 8, 32, 64, 160 and
+// 384 KiB at template ranks 1 to 32 (as much again per earlier factor for the chunk that publishes its
+// cross products), read in as long as the chunk's own rows take. (An embedding of 50257 rows at rank 16: 79
+// chunks instead of 393.) Chunks do not straddle the members of a rank-1 group, so a group of many
+// matrices has at least one chunk per member, and their reads grow with the square of the members: 8 bytes
+// per pair of members, 8 MB out of L2 for a thousand.
 template <int RT>
 static int orth_chunk_rows(long long longest) {
   const int base = orth_base_rows<RT>(), most = RT <= 4 ? 256 : RT == 8 ? 128 : RT == 16 ? 80 : 48;

@@ -74,7 +74,8 @@ def test_collapsed_columns_are_replaced(rank, rows):
 
 
 def test_long_unit_has_a_bounded_number_of_chunks():
-    """Every chunk reads the partial sums of all chunks of its unit, so their number may not grow with it."""
+    """Every chunk reads the partial sums of all chunks of its unit, so their number may not grow with its
+    length. Chunks keep to one member of a rank-1 group: there it grows with the members, and only with them."""
     for rank, most in ((1, 256), (4, 256), (8, 128), (16, 80), (32, 48)):
         for rows in (1, 512, 513, 50257, 1_000_003):
             core = BasicPowerSGD([torch.zeros(rows, 40, device="cuda")], BasicConfig(rank=rank), backend="native")
@@ -82,3 +83,26 @@ def test_long_unit_has_a_bounded_number_of_chunks():
 
             nat = NativeCompressor(core)
             assert 1 <= nat.n_chunks["p"] <= most
+    for members in (2, 300, 700):
+        core = BasicPowerSGD([torch.zeros(64, 40, device="cuda")] * members, BasicConfig(rank=1), backend="native")
+        assert NativeCompressor(core).n_chunks["p"] == members
+    core = BasicPowerSGD([torch.zeros(5000, 40, device="cuda")] * 300, BasicConfig(rank=1), backend="native")
+    assert NativeCompressor(core).n_chunks["p"] <= 2 * 300
+
+
+def test_rank_one_group_of_many_members():
+    """More members than a long unit may have chunks: one joint norm, and cross products member by member,
+    under the bounds of the test above."""
+    members, rows = 700, 64
+    core, nat = _compressor([(rows, 40)] * members, 1)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    draw = lambda t: t.copy_(torch.randn(t.shape, generator=g, device="cuda"))  # noqa: E731
+    x = draw(core._ps_buffer)
+    was, prev = core._ps[0].double().clone(), [draw(nat.h_loc[0]), draw(nat.h_loc[1])]
+    nat._orth("p", x, nat.h_in[2], prev, nat.cmat[2])
+    q = core._ps[0].double()
+    assert (q - was / was.norm()).abs().max() <= 2.0 ** -22
+    for p, c in zip(prev, nat.cmat[2]):
+        f = p[: members * rows].view(members, rows).double()
+        got = c.view(-1, 1024)[:members, 0].double()
+        assert (got - (f * q.view(members, rows)).sum(1)).abs().max() <= 4 * 2.0 ** -24 * f.norm(dim=1).max()
