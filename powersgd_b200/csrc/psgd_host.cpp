@@ -59,6 +59,13 @@ PSGD_API int psgd_capture_mode(int* mode) {
   return 0;
 }
 
+// Returns once everything put on `stream` so far is done. Returns a CUDA error code.
+PSGD_API int psgd_stream_wait(cudaStream_t stream) {
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) { psgd_set_error("cudaStreamSynchronize: %s", cudaGetErrorString(e)); return (int)e; }
+  return 0;
+}
+
 // ---- what lives as long as a recorded graph --------------------------------------------------
 // The caller numbers what a graph refers to and asks from time to time which numbers are free again. The
 // destructor of a user object may run on a thread of the driver and may call nothing of CUDA, so it only

@@ -21,6 +21,7 @@ Factor bookkeeping for half-iteration t of a step (left = the P side is the inpu
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import weakref
@@ -258,7 +259,30 @@ class TilePlan:
         return np.array(units, dtype=layout.ORTH_UNIT_DTYPE), np.array(chunks, dtype=layout.ORTH_CHUNK_DTYPE)
 
 
-class NativeCompressor:
+class _Recordable:
+    """What an object keeps about launches that read its tables: the stream of the last ones that were not
+    recorded, and, for recorded ones, the recording and what it refers to."""
+
+    _stream: Optional[ctypes.c_void_p] = None
+    recorded_in = 0
+
+    def _owned(self) -> tuple:
+        raise NotImplementedError
+
+    @contextlib.contextmanager
+    def _being_recorded(self):
+        if not hasattr(self, "_kept"):
+            self._kept: dict = {}
+        keep_with_graph(self._kept, *self._owned())
+        self.recorded_in = native.capture_id(_stream_ptr())
+        before = self._stream
+        try:
+            yield
+        finally:
+            self._stream = before
+
+
+class NativeCompressor(_Recordable):
     """Runs `BasicPowerSGD.aggregate` on the GPU with the in-tree kernels."""
 
     def __init__(self, core):
@@ -495,7 +519,8 @@ class NativeCompressor:
         """One launch of the library on the current stream, counted, and written down while a step is
         being recorded (see `_taped`)."""
         fn = getattr(self.lib, name)
-        native.check(fn(*args, _stream_ptr()), name)
+        self._stream = _stream_ptr()
+        native.check(fn(*args, self._stream), name)
         launched = 2 if name == "psgd_orth_launch" else 1   # orthonormalisation: Gram matrices, then their use
         self.launches += launched
         if self._tape is not None:
@@ -507,7 +532,13 @@ class NativeCompressor:
         a small model spends most of its step there). `key`: whatever the arguments depend on beyond
         the bound tensors; a new binding drops all tapes. Only where a step is nothing but launches on
         one stream: one worker, nothing launched ahead, no phase timing."""
-        self._keep_recorded()
+        if torch.cuda.is_current_stream_capturing():
+            with self._being_recorded():
+                self._run_taped(key, body)
+        else:
+            self._run_taped(key, body)
+
+    def _run_taped(self, key: Tuple, body) -> None:
         plain = (world_size() == 1 and self.comm is None and self._early is None and self._early_product_done is None
                  and not _Range.enabled and _Range.events is None)
         if not plain:
@@ -525,23 +556,22 @@ class NativeCompressor:
             finally:
                 self._tape = None
             return
-        stream = _stream_ptr()
+        self._stream = stream = _stream_ptr()
         for fn, name, args, launched in tape:
             code = fn(*args, stream)
             if code != 0:
                 native.check(code, name)
             self.launches += launched
 
-    def _keep_recorded(self) -> None:
-        """Everything a step addresses besides the caller's tensors stays alive with a graph that records
-        it: the next binding replaces the tables and the scratch, and the owner may go altogether."""
-        if torch.cuda.is_current_stream_capturing():
-            keep_with_graph(
-                self._mats_dev, self._maps_dev, [t for lists in self._tiles_dev.values() for t, _count in lists.values()],
-                self._partial, self._partial_tc, self._tickets, self._out_arena, self._hyper_dev, self._status,
-                self.units, self.chunks, self._orth_part, self._orth_rinv, self.h_in, self.h_loc, self.h_sum, self.cmat,
-                self.core._ps_buffer, self.core._qs_buffer,
-            )
+    def _owned(self) -> tuple:
+        """Everything a step addresses besides the caller's tensors; the next binding replaces the tables and
+        the scratch."""
+        return (
+            self._mats_dev, self._maps_dev, *(t for lists in self._tiles_dev.values() for t, _count in lists.values()),
+            self._partial, self._partial_tc, self._tickets, self._out_arena, self._hyper_dev, self._status,
+            self.units, self.chunks, self._orth_part, self._orth_rinv, self.h_in, self.h_loc, self.h_sum, self.cmat,
+            self.core._ps_buffer, self.core._qs_buffer,
+        )
 
     # -- phases ----------------------------------------------------------------------------
     def _orth(self, side: str, x: torch.Tensor, copy_to: torch.Tensor, prev: List[torch.Tensor], cm: List[torch.Tensor],
@@ -851,7 +881,7 @@ class NativeCompressor:
             self._hyper_dev = keep
 
 
-class NativeFlatAllReduce:
+class NativeFlatAllReduce(_Recordable):
     """Mean of a list of float32 tensors through one flat buffer, with the packing, the 1/W
     scale, the zeroing of the inputs and (optionally) the SGD update done by one multi-tensor
     kernel on each side of the collective."""
@@ -1023,6 +1053,7 @@ class NativeFlatAllReduce:
         return self._nvls
 
     def _launch(self, mode: int, hyper_dev: torch.Tensor, divisor: float, early: bool = False) -> None:
+        self._stream = _stream_ptr()
         code = self.lib.psgd_flat_launch(
             mode,
             self._vec,
@@ -1037,13 +1068,23 @@ class NativeFlatAllReduce:
             ctypes.c_longlong(self.n_pad),
             1 if self._keep_inputs else 0,
             int(early),
-            _stream_ptr(),
+            self._stream,
         )
         native.check(code, "psgd_flat_launch")
         self.launches += 1
 
+    def _owned(self) -> tuple:
+        return self._items_dev, self._block_item, self._block_first, self._hyper_dev, self._flat, self._out
+
     def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool = False) -> None:
-        keep_with_graph(self._items_dev, self._block_item, self._block_first, hyper_dev, self._flat, self._out)
+        if torch.cuda.is_current_stream_capturing():
+            with self._being_recorded():
+                keep_with_graph(self._kept, hyper_dev)
+                self._run_now(hyper_dev, workers, sgd, early)
+        else:
+            self._run_now(hyper_dev, workers, sgd, early)
+
+    def _run_now(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool) -> None:
         if self.path == "local":
             self._launch(4 if sgd else 3, hyper_dev, 1.0, early and sgd)
         elif self.path == "bulk":
@@ -1117,6 +1158,7 @@ class MultiTensorAccumulate:
     def __init__(self):
         self.lib = native.lib()
         self._key = None
+        self._kept: dict = {}   # tables that recorded launches refer to
 
     def __call__(self, dst: Sequence[torch.Tensor], src: Sequence[torch.Tensor], push: "Optional[NativeFlatAllReduce]" = None) -> None:
         key = (tuple(t.data_ptr() for t in dst), tuple(t.data_ptr() for t in src), None if push is None else push._key)
@@ -1147,7 +1189,8 @@ class MultiTensorAccumulate:
             self._nblocks = len(block_item)
             self._hyper = _to_device(NativeCompressor._default_hyper(), device)
             self._key = key
-        keep_with_graph(self._items, self._block_item, self._block_first, self._hyper)
+        if torch.cuda.is_current_stream_capturing():
+            keep_with_graph(self._kept, self._items, self._block_item, self._block_first, self._hyper)
         code = self.lib.psgd_flat_launch(
             8 if push is None else 9, self._vec, _ptr(self._items), _ptr(self._block_item), _ptr(self._block_first),
             self._nblocks, _ptr(self._hyper), ctypes.c_void_p(0), 1.0 if push is None else float(world_size()),
@@ -1177,6 +1220,7 @@ class FusedSGDDriver:
 
     def __init__(self, agg):
         self.agg = weakref.proxy(agg)   # its owner, see NativeCompressor
+        self.lib = native.lib()
         self.device = agg.device
         self._slots: List[torch.Tensor] = []
         self._slot_events: List[Optional[torch.cuda.Event]] = []
@@ -1184,8 +1228,6 @@ class FusedSGDDriver:
         self._hyper_dev: Optional[torch.Tensor] = None
         self._cache_key = None
         self._last_values = None   # what the device table holds
-        self._stream: Optional[torch.cuda.Stream] = None   # of the last step that was not recorded
-        self._recorded_in = 0      # id of the recording that the last step was part of
         self._fixed: Optional[torch.Tensor] = None   # table of the coming step alone, in place of the live one
         self._flat_all = NativeFlatAllReduce()
         self._flat_plain = NativeFlatAllReduce()
@@ -1233,13 +1275,8 @@ class FusedSGDDriver:
             (float(g["lr"]), float(g["momentum"]), 1.0 if gi in fresh else 1.0 - float(g["dampening"]), float(g["weight_decay"]), bool(g["nesterov"]))
             for gi, g in enumerate(groups)
         ]
-        recording = native.capture_id(torch.cuda.current_stream()) if torch.cuda.is_current_stream_capturing() else 0
-        joins = recording != 0 and recording == self._recorded_in   # an earlier step of this recording reads the live table
-        self._recorded_in = recording
         self._fixed = None
         if values == self._last_values:
-            if not recording:
-                self._stream = torch.cuda.current_stream()
             return  # nothing changed since the last upload: the device table is already right
         table = np.zeros(len(groups), dtype=layout.HYPER_DTYPE)
         for row, (lr, mu, one_minus_dampening, decay, nesterov) in zip(table, values):
@@ -1250,7 +1287,10 @@ class FusedSGDDriver:
             row["nesterov"] = 1 if nesterov else 0
             row["has_momentum"] = 1 if mu != 0.0 else 0
             row["grad_scale"] = 1.0
-        if joins or (recording and self._stream is not None and native.capture_id(self._stream)):
+        recording = native.capture_id(_stream_ptr()) if torch.cuda.is_current_stream_capturing() else 0
+        readers = [r for r in (self.agg._powersgd._native, self._flat_all, self._flat_plain) if r is not None]
+        streams = [r._stream for r in readers if r._stream is not None]
+        if recording and (any(r.recorded_in == recording for r in readers) or any(native.capture_id(s) for s in streams)):
             # The live table cannot change under a step that reads it already: one recorded before this in the
             # same graph, or one that may still be running on a stream that is part of the recording and so
             # cannot be waited for. This step keeps the values it was recorded with.
@@ -1267,11 +1307,10 @@ class FusedSGDDriver:
         if recording:
             # in place now, not by a copy that every replay would repeat over what later steps upload
             with outside_capture(self.device):
-                if self._stream is not None:
-                    self._stream.synchronize()   # the steps before this one have read the table
+                for stream in streams:   # the steps before this one have read the table
+                    native.check(self.lib.psgd_stream_wait(stream), "psgd_stream_wait")
                 self._hyper_dev.copy_(torch.from_numpy(raw))
             return
-        self._stream = torch.cuda.current_stream()
         i = self._cursor
         self._cursor = (i + 1) % self.RING
         if self._slot_events[i] is not None:

@@ -19,6 +19,8 @@ def declare(lib) -> None:
     lib.psgd_capture_mode.restype = i32
     lib.psgd_capture_mode.argtypes = [C.POINTER(i32)]
 
+    lib.psgd_stream_wait.restype = i32
+    lib.psgd_stream_wait.argtypes = [vp]
     lib.psgd_graph_retain.restype = i32
     lib.psgd_graph_retain.argtypes = [C.c_longlong, vp]
     lib.psgd_graph_released.restype = i32

@@ -74,10 +74,10 @@ def check(code: int, what: str) -> None:
         raise RuntimeError(f"{what} failed (code {code}): {msg.decode() if msg else ''}")
 
 
-def capture_id(stream) -> int:
+def capture_id(stream: ctypes.c_void_p) -> int:
     """Id of the CUDA-graph recording that `stream` is part of; 0 when it is not being recorded."""
     out = ctypes.c_ulonglong(0)
-    check(lib().psgd_capture_id(ctypes.c_void_p(stream.cuda_stream), ctypes.byref(out)), "psgd_capture_id")
+    check(lib().psgd_capture_id(stream, ctypes.byref(out)), "psgd_capture_id")
     return int(out.value)
 
 

@@ -2,8 +2,8 @@
 
 A recorded launch holds raw addresses: descriptor tables, scratch, factors. Two things follow. What never
 changes is put in place at once, beside the recording, and not by a node that every replay would pay for
-(`outside_capture`, `to_device`). And everything whose address is recorded lives as long as the graph,
-whatever its owner binds or drops later (`keep_with_graph`).
+(`outside_capture`, `to_device`). And everything whose address is recorded is kept for the graph, whatever
+its owner binds later (`keep_with_graph`).
 """
 from __future__ import annotations
 
@@ -64,21 +64,24 @@ _numbers = itertools.count(1)
 _scope: Optional[list] = None
 
 
-def keep_with_graph(*objects) -> None:
-    """While a CUDA graph is being recorded: `objects` (tensors, or whatever owns memory) live at least as
-    long as the graph and every instance of it. The graph itself says when it is gone (a user object whose
-    destructor notes the number), so this holds for a recording made by anybody, and nothing stays behind
-    for the life of the process."""
-    if not torch.cuda.is_current_stream_capturing():
-        return
-    number = next(_numbers)
-    _kept[number] = objects
-    native.check(
-        native.lib().psgd_graph_retain(ctypes.c_longlong(number), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)),
-        "psgd_graph_retain",
-    )
+def keep_with_graph(holder: Optional[dict], *objects) -> None:
+    """While a CUDA graph is being recorded: `objects` (tensors, or whatever owns memory) stay alive for it.
+    Inside a `capture_scope` the program has them. Otherwise `holder` has them, a dict of the object whose
+    launches are being recorded (an aggregator must outlive the graphs recorded from it, as the parameters
+    must): what that object binds or drops later then takes nothing from under a replay. Without a holder
+    the graph itself says when it is gone (a user object whose destructor notes a number); a replay of
+    such a graph costs 2 us more."""
     if _scope is not None:
         _scope.append(objects)
+    elif holder is not None:
+        holder.update((id(o), o) for o in objects)
+    else:
+        number = next(_numbers)
+        _kept[number] = objects
+        native.check(
+            native.lib().psgd_graph_retain(ctypes.c_longlong(number), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)),
+            "psgd_graph_retain",
+        )
 
 
 def release_finished() -> None:
@@ -96,8 +99,10 @@ def release_finished() -> None:
 
 
 class capture_scope:
-    """`with capture_scope() as keep:` around a CUDA-graph capture also collects in `keep` what the graph
-    refers to, for a program that wants to look at it or keep it longer than the graph."""
+    """`with capture_scope() as keep:` around a CUDA-graph capture collects in `keep` what the graph refers to
+    besides the caller's own tensors; store `keep` next to the graph and drop both together. Without it,
+    what was recorded lives as long as the aggregator: a program that records again and again on new
+    tensors gives back what earlier recordings held by using a scope."""
 
     def __enter__(self) -> list:
         global _scope

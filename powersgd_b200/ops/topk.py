@@ -32,7 +32,7 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
         if ws is None:
             ws = torch.zeros(lib.psgd_topk_workspace_ints(), dtype=torch.int32, device=flat.device)
             if recorded:
-                keep_with_graph(ws)
+                keep_with_graph(None, ws)
             else:
                 _workspaces[flat.device] = ws
         values = torch.empty(k, dtype=torch.float32, device=flat.device)
@@ -118,7 +118,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
                 "ws": torch.zeros(len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
             }
         if recorded:
-            keep_with_graph(entry)
+            keep_with_graph(None, entry)
         else:
             # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
             # valid for whatever tensors present the same addresses again, so no tensor is kept alive
@@ -192,7 +192,7 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
                 if recorded:
                     barrier = torch.zeros(1, dtype=torch.int32, device=device)
             if recorded:
-                keep_with_graph(tables, barrier, scratch)
+                keep_with_graph(None, tables, barrier, scratch)
             else:
                 if len(_segment_cache) >= 4:
                     _segment_cache.clear()

@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from powersgd_b200 import Config, PowerSGD, optimizer_step
+from powersgd_b200.cuda_path import capture_scope
 from powersgd_b200.ops.recording import release_finished
 
 pytestmark = pytest.mark.gpu
@@ -150,37 +151,66 @@ def test_replay_after_other_tensors_were_bound():
     assert all(bool((j == -1).all()) for j in junk)
 
 
-def test_replay_after_the_aggregator_is_gone():
-    recorded, eager = _Program(), _Program()
-    recorded.step(), eager.step()
-    graph = recorded.record(None)
-    del recorded.aggregator
-    gc.collect()
-    junk = _write_over_free_memory()
-    graph.replay()
-    eager.step()
-    assert _same(recorded, eager)
-    assert all(bool((j == -1).all()) for j in junk)
+def _refs(native):
+    return [weakref.ref(t) for t in (native._tickets, native._partial, native._mats_dev)]
 
 
-def test_what_a_graph_refers_to_goes_with_it():
+def test_what_was_recorded_goes_with_the_aggregator():
+    """Other tensors bound again and again keep nothing; a recording keeps what it refers to, once, until
+    the aggregator goes."""
     recorded = _Program()
     recorded.step()
-    graph = recorded.record(None)
-    native = recorded.aggregator._powersgd._native
-    refs = [weakref.ref(native._tickets), weakref.ref(native._partial), weakref.ref(native._mats_dev)]
-    del native
+    unrecorded = _refs(recorded.aggregator._powersgd._native)
     _step_on_other_gradients(recorded)
-    release_finished()
+    assert all(ref() is None for ref in unrecorded)
+    recorded.step()
+    refs = _refs(recorded.aggregator._powersgd._native)
+    graphs = [recorded.record(None) for _ in range(3)]
+    count = len(recorded.aggregator._powersgd._native._kept)
+    graphs.append(recorded.record(None))
+    assert len(recorded.aggregator._powersgd._native._kept) == count
+    _step_on_other_gradients(recorded)
     assert all(ref() is not None for ref in refs)
+    del graphs, recorded
+    gc.collect()
+    assert all(ref() is None for ref in refs)
+
+
+def test_a_scope_has_what_was_recorded():
+    recorded = _Program()
+    recorded.step()
+    refs = _refs(recorded.aggregator._powersgd._native)
+    with capture_scope() as keep:
+        graph = recorded.record(None)
+    _step_on_other_gradients(recorded)
+    assert all(ref() is not None for ref in refs)
+    del graph, keep
+    assert all(ref() is None for ref in refs)
+
+
+def test_what_a_graph_alone_refers_to_goes_with_it():
+    """Functions without an object of their own (the top-k tables) leave it to the graph."""
+    from powersgd_b200.ops import recording
+    from powersgd_b200.ops.topk import topk_abs_many
+
+    x = torch.randn(4096, device="cuda")
+    topk_abs_many([x], [16])
+    before = set(recording._kept)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        topk_abs_many([x], [16])
+    mine = set(recording._kept) - before
+    release_finished()
+    assert mine and mine <= set(recording._kept)
     del graph
     gc.collect()
     torch.cuda.synchronize()
     until = time.monotonic() + 20   # the graph says so on a thread of the driver
-    while any(ref() is not None for ref in refs) and time.monotonic() < until:
+    while mine & set(recording._kept) and time.monotonic() < until:
         release_finished()
         time.sleep(0.01)
-    assert all(ref() is None for ref in refs)
+    assert not mine & set(recording._kept)
 
 
 @pytest.mark.parametrize("reducer", ["TopKReducer", "GlobalTopKReducer"])
