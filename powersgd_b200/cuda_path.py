@@ -185,29 +185,32 @@ class TilePlan:
             "fin": {k: arr(v) for k, v in fin.items()},
         }
 
-    NT_TILES = 250   # of the CUDA-core NT product, at least: some five for three of the 148 SMs
-
     def _nt_tile_rows(self, n: int) -> int:
         # tall matrices: never more than 160 partial tiles per column block (the kernel walks a tile that is
         # taller than its staging buffer in chunks)
         return max(self.nt_rows if n <= 4096 else self.nt_tall_rows, -(-(-(-n // 160)) // 128) * 128)
 
     def _pick_nt_rows(self, groups) -> None:
-        """Rows of an NT tile (`groups`: the matrices of the CUDA-core launch, one entry each). Twice as many
-        halve what a tile costs besides its loads (start, staging, the sum over the warps, the hand-over),
-        as long as NT_TILES are left; only the tiles of this launch count, not the elements of the model, most of
-        which may be multiplied by the tensor cores. Measured (us per launch, data in L2, tiles at the larger
-        size): 128 / 256 rows: 192 tiles (6 x 1024x1001, rank 2) 8.1 / 9.8, 186 (3 x 1001x777 + 2 x 515x2049,
-        rank 3) 9.4 / 11.1, 240 (10 x 513x1001, rank 4) 9.3 / 10.1, 256 (8 x 1024x1001, rank 2) 11.9 / 9.8, 288 (9 of
-        them, rank 4) 14.5 / 12.5, 378 (ResNet-18) 12.8 / 10.9; 2 x 700x650 beside two matrices of 33 M elements:
-        6.0 / 8.1. Matrices above 4096 rows, 256 / 512: 204 (17000x650, rank 4) 17.7 / 18.8, 252 (21001x650) 26.3 /
-        19.5, 300 (2 x 7673x1255, rank 2) 19.5 / 17.0, 786 (the LSTM model) 46.2 / 43.1."""
-        def tiles(rows: int, tall_rows: int) -> int:
-            self.nt_rows, self.nt_tall_rows = min(self._nt_rows_cap, rows), tall_rows
-            return sum(-(-g.m // 128) * -(-g.n // self._nt_tile_rows(g.n)) for g in groups)
+        """Rows of an NT tile (`groups`: the matrices of the CUDA-core launch, one entry each): 128 or 256, and
+        256 or 512 above 4096 rows. Twice as many halve what a tile costs besides its loads (start, staging,
+        the sum over the warps, the hand-over), as long as the launch still fills some half of the places that
+        the SMs have for its CTAs (three per SM up to template rank 4, two above); only its own tiles count,
+        not the elements of the model, most of which may go to the tensor cores. Of the tall matrices only
+        their own tiles count: among many short ones a few tall tiles end last. Measured (us per launch, data in
+        L2, tiles at the larger height), 128 / 256 rows: 186 (3 x 1001x777 + 2 x 515x2049, rank 3) 9.4 / 11.1, 192
+        (6 x 1024x1001, rank 2) 8.1 / 9.8, 256 (8 of them) 11.9 / 9.8, 378 (ResNet-18) 12.8 / 10.9; rank 8, 256: 16.1 /
+        13.4; 36 (2 x 700x650 beside two matrices of 33 M elements) 6.0 / 8.1. 256 / 512 rows: 204 (17000x650, rank
+        4) 17.7 / 18.8, 252 (21001x650) 26.3 / 19.5, 786 (the LSTM model) 46.2 / 43.1; 323 of which 44 tall 12.4 /
+        16.8. Over 200 random lists of matrices the choice is on average 2 % slower than the best of the four
+        (5 % when the elements of the model decided), at worst 27 %."""
+        enough, enough_tall = (250, 220) if self.rt <= 4 else (150, 80)
 
-        rows = 256 if tiles(256, 256) >= self.NT_TILES else 128
-        if tiles(rows, 512) < self.NT_TILES:
+        def tiles(rows: int, tall_rows: int, above: int = 0) -> int:
+            self.nt_rows, self.nt_tall_rows = min(self._nt_rows_cap, rows), tall_rows
+            return sum(-(-g.m // 128) * -(-g.n // self._nt_tile_rows(g.n)) for g in groups if g.n > above)
+
+        rows = 256 if tiles(256, 256) >= enough else 128
+        if tiles(rows, 512, above=4096) < enough_tall:
             tiles(rows, 256)
 
     TC_CTAS_PER_SM = 2

@@ -159,18 +159,18 @@ def _nt_rows(shapes, rank, tc=lambda shape: False):
 
 @pytest.mark.parametrize("rank", [1, 4, 16])
 def test_nt_tile_height_leaves_enough_tiles_of_its_own_launch(rank):
-    """Taller tiles only where they leave the launch some 250 tiles; matrices that the tensor cores multiply are
-    not part of it, however large they are."""
-    from powersgd_b200.cuda_path import TilePlan
-
+    """Taller tiles only where the launch keeps enough of them; matrices that the tensor cores multiply are no
+    part of it, however large they are, and short ones do not make up for few tall ones."""
     large = [(8192, 4096)] * 2
-    for small in ([(513, 1001)] * 6, [(700, 650)] * 2, [(1024, 1001)] * 6):
-        alone, _ = _nt_rows(small, rank)
-        beside, count = _nt_rows(large + small, rank, tc=lambda shape: shape == (8192, 4096))
-        assert alone == beside and max(beside.values()) <= 128 and count < 2 * TilePlan.NT_TILES
+    for small in ([(513, 1001)] * 6, [(700, 650)] * 2, [(1024, 1001)] * 4, [(1024, 1001)] * 9, [(21001, 650)]):
+        assert _nt_rows(small, rank) == _nt_rows(large + small, rank, tc=lambda shape: shape == (8192, 4096))
+    assert max(_nt_rows([(700, 650)] * 2, rank)[0].values()) <= 128
     assert max(_nt_rows([(1024, 1001)] * 9, rank)[0].values()) == 256
     assert _nt_rows([(21001, 650)], rank)[0][(21001, 650)] > 256
-    assert _nt_rows([(17000, 650)], rank)[0][(17000, 650)] <= 256
+    assert _nt_rows([(5321, 27)] * 4 + [(1024, 1001)] * 9, rank)[0][(5321, 27)] <= 256
+    if rank <= 4:
+        assert max(_nt_rows([(1024, 1001)] * 6, rank)[0].values()) <= 128
+        assert _nt_rows([(17000, 650)], rank)[0][(17000, 650)] <= 256
 
 
 @pytest.mark.parametrize("same", [0, 1])
