@@ -32,7 +32,7 @@ import torch
 import torch.distributed as dist
 
 from .ops import layout, native
-from .ops.recording import capture_scope, keep_with_graph, outside_capture  # noqa: F401  (capture_scope: for callers)
+from .ops.recording import capture_scope, is_recorded, keep_with_graph, outside_capture  # noqa: F401  (capture_scope: for callers)
 from .ops.recording import to_device as _to_device
 from .utils import is_dense, like_strided, same_layout, world_size
 
@@ -273,11 +273,11 @@ class _Recordable:
         raise NotImplementedError
 
     @contextlib.contextmanager
-    def _being_recorded(self):
+    def _being_recorded(self, stream: ctypes.c_void_p):
         if not hasattr(self, "_kept"):
             self._kept: dict = {}
         keep_with_graph(self._kept, *self._owned())
-        self.recorded_in = native.capture_id(_stream_ptr())
+        self.recorded_in = native.capture_id(stream)
         before = self._stream
         try:
             yield
@@ -529,19 +529,17 @@ class NativeCompressor(_Recordable):
         if self._tape is not None:
             self._tape.append((fn, name, args, launched))
 
-    def _taped(self, key: Tuple, body) -> None:
+    def _taped(self, key: Tuple, body, inside: bool = False) -> None:
         """Run `body`, which issues the launches of a step; from the second step of its kind on repeat
         the same calls with the arguments they had, without working them out again (an eager loop over
         a small model spends most of its step there). `key`: whatever the arguments depend on beyond
         the bound tensors; a new binding drops all tapes. Only where a step is nothing but launches on
         one stream: one worker, nothing launched ahead, no phase timing."""
-        if torch.cuda.is_current_stream_capturing():
-            with self._being_recorded():
-                self._run_taped(key, body)
-        else:
-            self._run_taped(key, body)
-
-    def _run_taped(self, key: Tuple, body) -> None:
+        stream = _stream_ptr()
+        if stream and not inside and is_recorded(stream):   # (0, the default stream: never)
+            with self._being_recorded(stream):
+                self._taped(key, body, inside=True)
+            return
         plain = (world_size() == 1 and self.comm is None and self._early is None and self._early_product_done is None
                  and not _Range.enabled and _Range.events is None)
         if not plain:
@@ -559,7 +557,7 @@ class NativeCompressor(_Recordable):
             finally:
                 self._tape = None
             return
-        self._stream = stream = _stream_ptr()
+        self._stream = stream
         for fn, name, args, launched in tape:
             code = fn(*args, stream)
             if code != 0:
@@ -1056,7 +1054,6 @@ class NativeFlatAllReduce(_Recordable):
         return self._nvls
 
     def _launch(self, mode: int, hyper_dev: torch.Tensor, divisor: float, early: bool = False) -> None:
-        self._stream = _stream_ptr()
         code = self.lib.psgd_flat_launch(
             mode,
             self._vec,
@@ -1079,15 +1076,14 @@ class NativeFlatAllReduce(_Recordable):
     def _owned(self) -> tuple:
         return self._items_dev, self._block_item, self._block_first, self._hyper_dev, self._flat, self._out
 
-    def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool = False) -> None:
-        if torch.cuda.is_current_stream_capturing():
-            with self._being_recorded():
+    def _run(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool = False, inside: bool = False) -> None:
+        stream = _stream_ptr()
+        if stream and not inside and is_recorded(stream):   # (0, the default stream: never)
+            with self._being_recorded(stream):
                 keep_with_graph(self._kept, hyper_dev)
-                self._run_now(hyper_dev, workers, sgd, early)
-        else:
-            self._run_now(hyper_dev, workers, sgd, early)
-
-    def _run_now(self, hyper_dev: torch.Tensor, workers: int, sgd: bool, early: bool) -> None:
+                self._run(hyper_dev, workers, sgd, early, inside=True)
+            return
+        self._stream = stream
         if self.path == "local":
             self._launch(4 if sgd else 3, hyper_dev, 1.0, early and sgd)
         elif self.path == "bulk":
@@ -1192,12 +1188,13 @@ class MultiTensorAccumulate:
             self._nblocks = len(block_item)
             self._hyper = _to_device(NativeCompressor._default_hyper(), device)
             self._key = key
-        if torch.cuda.is_current_stream_capturing():
+        stream = _stream_ptr()
+        if is_recorded(stream):
             keep_with_graph(self._kept, self._items, self._block_item, self._block_first, self._hyper)
         code = self.lib.psgd_flat_launch(
             8 if push is None else 9, self._vec, _ptr(self._items), _ptr(self._block_item), _ptr(self._block_first),
             self._nblocks, _ptr(self._hyper), ctypes.c_void_p(0), 1.0 if push is None else float(world_size()),
-            ctypes.c_void_p(0) if push is None else push.comm.ptr, ctypes.c_longlong(0), 0, 0, _stream_ptr(),
+            ctypes.c_void_p(0) if push is None else push.comm.ptr, ctypes.c_longlong(0), 0, 0, stream,
         )
         native.check(code, "psgd_flat_launch")
         if push is not None:
@@ -1290,7 +1287,8 @@ class FusedSGDDriver:
             row["nesterov"] = 1 if nesterov else 0
             row["has_momentum"] = 1 if mu != 0.0 else 0
             row["grad_scale"] = 1.0
-        recording = native.capture_id(_stream_ptr()) if torch.cuda.is_current_stream_capturing() else 0
+        stream = _stream_ptr()
+        recording = native.capture_id(stream) if is_recorded(stream) else 0
         readers = [r for r in (self.agg._powersgd._native, self._flat_all, self._flat_plain) if r is not None]
         streams = [r._stream for r in readers if r._stream is not None]
         if recording and (any(r.recorded_in == recording for r in readers) or any(native.capture_id(s) for s in streams)):

@@ -17,6 +17,14 @@ import torch
 
 from . import native
 
+
+
+def is_recorded(stream: ctypes.c_void_p) -> bool:
+    """Is the current stream, whose handle is `stream`, being recorded? The default stream (handle 0) cannot be,
+    so eager loops on it are spared the question, which takes the driver some 2 us while launches are under way."""
+    return bool(stream) and torch.cuda.is_current_stream_capturing()
+
+
 _upload_streams: Dict[torch.device, torch.cuda.Stream] = {}
 
 

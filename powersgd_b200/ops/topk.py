@@ -14,7 +14,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import native
-from .recording import keep_with_graph, outside_capture, release_finished
+from .recording import is_recorded, keep_with_graph, outside_capture, release_finished
 
 _workspaces = {}
 
@@ -27,7 +27,8 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
         memory is None or (memory.is_contiguous() and memory.dtype == torch.float32)
     ):
         lib = native.lib()
-        recorded = torch.cuda.is_current_stream_capturing()   # a graph gets counters of its own, see topk_abs_many
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        recorded = is_recorded(stream)   # a graph gets counters of its own, see topk_abs_many
         ws = None if recorded else _workspaces.get(flat.device)
         if ws is None:
             ws = torch.zeros(lib.psgd_topk_workspace_ints(), dtype=torch.int32, device=flat.device)
@@ -40,8 +41,7 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
         code = lib.psgd_topk_abs(
             ctypes.c_void_p(flat.data_ptr()), ctypes.c_longlong(n), ctypes.c_longlong(k), ctypes.c_void_p(ws.data_ptr()),
             ctypes.c_void_p(values.data_ptr()), ctypes.c_void_p(positions.data_ptr()),
-            ctypes.c_void_p(0 if memory is None else memory.data_ptr()),
-            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream),
+            ctypes.c_void_p(0 if memory is None else memory.data_ptr()), stream,
         )
         native.check(code, "psgd_topk_abs")
         return values, positions
@@ -87,7 +87,8 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     key = (device, tuple(t.data_ptr() for t in tensors), tuple(0 if m is None else m.data_ptr() for m in mems), tuple(t.numel() for t in tensors), tuple(ks))
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
-    recorded = torch.cuda.is_current_stream_capturing()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    recorded = is_recorded(stream)
     entry = None if recorded else _many_cache.get(key)
     if entry is None:
         release_finished()
@@ -130,8 +131,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     vp = ctypes.c_void_p
     code = lib.psgd_topk_abs_many(
         vp(entry["items"].data_ptr()), len(tensors), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
-        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()),
-        vp(torch.cuda.current_stream().cuda_stream),
+        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
     )
     native.check(code, "psgd_topk_abs_many")
     return values, positions
@@ -176,7 +176,7 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
         # tables of addresses and lengths, kept by exactly those (as the selection's above, recorded calls
         # included): building and uploading one stalls the host until the selection has run
         key = (device, tuple(o.data_ptr() for o in outs), tuple(o.numel() for o in outs), tuple(ends))
-        recorded = torch.cuda.is_current_stream_capturing()
+        recorded = is_recorded(stream)
         tables = None if recorded else _segment_cache.get(key)
         if tables is None:
             release_finished()
