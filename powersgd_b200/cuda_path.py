@@ -1237,9 +1237,10 @@ class FusedSGDDriver:
         groups = optimizer.param_groups
         key = (id(optimizer), tuple(len(g["params"]) for g in groups), tuple(float(g["momentum"]) != 0.0 for g in groups))
         fresh_groups = set()
+        # a group whose first buffer is missing or another tensor (a loaded optimizer checkpoint) is looked at anew
         if key != self._cache_key or any(
-            float(g["momentum"]) != 0.0 and optimizer.state[p].get("momentum_buffer") is None
-            for g in groups
+            float(g["momentum"]) != 0.0 and optimizer.state[p].get("momentum_buffer") is not first
+            for g, first in zip(groups, self._first_moms)
             for p in g["params"][:1]
         ):
             params, moms, index = [], [], []
@@ -1257,6 +1258,7 @@ class FusedSGDDriver:
                     else:
                         moms.append(None)
             self._params, self._moms, self._index = params, moms, index
+            self._first_moms = [optimizer.state.get(g["params"][0], {}).get("momentum_buffer") if g["params"] else None for g in groups]
             mask = self.agg.is_compressed_mask
             if len(params) == len(mask):
                 # the same lists, compressed and uncompressed tensors apart (True / False)

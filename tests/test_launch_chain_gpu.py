@@ -105,3 +105,28 @@ def test_recorded_in_a_graph_and_run_eagerly_agree():
 
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+def test_loaded_optimizer_state_is_used():
+    """`optimizer.load_state_dict` puts other momentum buffers in place; the steps after it update those."""
+    import copy
+
+    def run(new_driver):
+        params = [torch.nn.Parameter(x) for x in _gradients([(128, 300), (70, 129), (33,)], 9)]
+        opt = torch.optim.SGD([{"params": params[:1]}, {"params": params[1:], "lr": 0.05}], lr=0.1, momentum=0.9)
+        agg = PowerSGD(params, Config(rank=2, num_iters_per_step=2, start_compressing_after_num_steps=0))
+        saved = None
+        for i in range(6):
+            for p, x in zip(params, _gradients([tuple(p.shape) for p in params], 20 + i)):
+                p.grad = x if p.grad is None else p.grad.add_(x)
+            if i == 2:
+                saved = copy.deepcopy(opt.state_dict())
+            if i == 4:
+                opt.load_state_dict(saved)
+            if new_driver:
+                agg._fused = None
+            optimizer_step(opt, agg)
+        return [t.detach().clone() for p in params for t in (p, p.grad, opt.state[p]["momentum_buffer"])]
+
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
