@@ -65,6 +65,7 @@ class TrainStep:
         self._steps_done = 0
         self._graphs: Dict[int, torch.cuda.CUDAGraph] = {}
         self._graph_keep: Dict[int, list] = {}
+        self._graph_moms: Dict[int, list] = {}   # the momentum buffers each graph updates
         self._static_x: Optional[torch.Tensor] = None
         self._static_y: Optional[torch.Tensor] = None
         self._static_loss: Optional[torch.Tensor] = None
@@ -365,7 +366,8 @@ class TrainStep:
         # capturing ran the host side of the step (counters) but not the kernels: rewind
         agg.step_counter, agg._powersgd.step_counter = saved
         self._graphs[parity] = graph
-        self._graph_keep[parity] = keep  # tables whose addresses the graph holds: same lifetime as the graph
+        self._graph_keep[parity] = keep  # what the graph refers to besides the model's tensors: same lifetime as the graph
+        self._graph_moms[parity] = agg._fused._moms
 
     def __call__(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         if not self._graphable_now():
@@ -393,6 +395,8 @@ class TrainStep:
             raise type(exc)(f"training step {self._steps_done}: {exc}") from None
         # host-side refresh of what the graph reads from memory (learning rates etc.)
         fused.prepare(self.optimizer)
+        if self._graph_moms[parity] is not fused._moms:   # a loaded optimizer state: other buffers to update
+            self._capture(parity)
         self._graphs[parity].replay()
         self._agg_events = self._graph_events.get(parity)
         self._bump_counters()

@@ -242,3 +242,34 @@ def test_recorded_topk_reduce_survives_other_tensor_sets(reducer, warm):
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(out + memory, want[1] + want[2]))
     assert all(bool((j == -1).all()) for j in junk)
+
+
+def test_train_step_uses_a_loaded_optimizer_state():
+    """The graph of a TrainStep updates the buffers that were there when it was recorded; after
+    `optimizer.load_state_dict` there are others."""
+    import copy
+
+    from powersgd_b200.engine import TrainStep
+    from powersgd_b200.models.mlp import MLP
+
+    x, y = torch.randn(32, 64, device="cuda"), torch.randint(0, 10, (32,), device="cuda")
+
+    def run(cuda_graph):
+        torch.manual_seed(0)
+        model = MLP(64, 128, 10).cuda()
+        opt = torch.optim.SGD(model.parameters(), lr=0.05, momentum=0.9)
+        agg = PowerSGD(list(model.parameters()), Config(rank=1, num_iters_per_step=1, start_compressing_after_num_steps=0))
+        step = TrainStep(model, torch.nn.functional.cross_entropy, opt, agg, cuda_graph=cuda_graph)
+        saved, losses = None, []
+        for i in range(12):
+            if i == 3:
+                saved = copy.deepcopy(opt.state_dict())
+            if i in (7, 10):
+                opt.load_state_dict(saved)
+            losses.append(step(x, y).clone())
+        assert bool(step._graphs) == cuda_graph
+        torch.cuda.synchronize()
+        return losses + [t.detach().clone() for p in model.parameters() for t in (p, opt.state[p]["momentum_buffer"])]
+
+    for a, b in zip(run(True), run(False)):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-6)   # the library may choose other kernels under capture
