@@ -305,8 +305,11 @@ class NativeCompressor(_Recordable):
         if self.T > layout.MAX_HIST:
             raise ValueError(f"num_iters_per_step {self.T} exceeds the compiled maximum {layout.MAX_HIST}")
         # finalize strips: as tall as the factor panels allow in shared memory, but short enough
-        # that a small model still spreads over ~3 strips per SM (a strip costs its panels and one start:
-        # ResNet-18's step takes 131 / 121.5 / 120 us with 12 / 6 / 3 strips per SM)
+        # that a small model still spreads over ~3 strips per SM (a strip costs its panels and one start).
+        # 12 / 6 / 3 strips per SM, us per launch without the optimizer step, data in L2: ResNet-18 at 2 x 2 columns
+        # 28.4 / 22.9 / 23.6, 2 x 2048^2 at 4 x 2 20.0 / 17.3 / 17.4, 17000x650 at 4 x 2 35.4 / 29.2 / 29.4, 8 x 1024x1001
+        # at 16 x 2 45.7 / 35.1 / 31.0, 4 x 1024^2 at 8 x 1 and 3 x 1001x777 + 2 x 515x2049 at 3 x 3 alike within 8 %;
+        # ResNet-18's recorded step 131 / 121.5 / 120.
         strip_cap = int(self.lib.psgd_finalize_strip_rows(self.T * self.tiles.max_r, 1 if world_size() == 1 else 0))
         want = self.tiles.total_elems // (128 * 148 * 3)
         self.tiles.fin_rows = max(32, min(strip_cap, want // 32 * 32))
@@ -324,8 +327,8 @@ class NativeCompressor(_Recordable):
             units, chunks = self.tiles.orth_units(s, int(self.lib.psgd_orth_chunk_rows(self.tiles.max_r, longest)))
             self.units[s], self.chunks[s] = _to_device(units, self.device), _to_device(chunks, self.device)
             self.n_units[s], self.n_chunks[s] = len(units), len(chunks)
-        # scratch of the orthonormalisation: partial sums per chunk; per unit the leading rows that its
-        # factor R falls back on when a column has to be replaced
+        # scratch of the orthonormalisation: partial sums per chunk; per unit (`_orth_rinv`) the leading
+        # rows of the factor as they came in, which R falls back on when a column has to be replaced
         part_doubles = int(self.lib.psgd_orth_part_doubles(self.tiles.max_r, max(self.T - 1, 0)))
         max_units = max(max(self.n_units.values()), 1)
         self._orth_part = torch.zeros(max(max(self.n_chunks.values()), 1) * part_doubles, device=self.device, dtype=torch.float64)
