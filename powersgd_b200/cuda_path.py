@@ -1056,7 +1056,8 @@ class NativeFlatAllReduce(_Recordable):
             self._nvls, self._nvls_failed = None, True
         return self._nvls
 
-    def _launch(self, mode: int, hyper_dev: torch.Tensor, divisor: float, early: bool = False) -> None:
+    def _launch(self, mode: int, hyper_dev: torch.Tensor, divisor: float, early: bool = False,
+                stream: Optional[ctypes.c_void_p] = None) -> None:
         code = self.lib.psgd_flat_launch(
             mode,
             self._vec,
@@ -1071,7 +1072,7 @@ class NativeFlatAllReduce(_Recordable):
             ctypes.c_longlong(self.n_pad),
             1 if self._keep_inputs else 0,
             int(early),
-            self._stream,
+            _stream_ptr() if stream is None else stream,
         )
         native.check(code, "psgd_flat_launch")
         self.launches += 1
@@ -1088,28 +1089,28 @@ class NativeFlatAllReduce(_Recordable):
             return
         self._stream = stream
         if self.path == "local":
-            self._launch(4 if sgd else 3, hyper_dev, 1.0, early and sgd)
+            self._launch(4 if sgd else 3, hyper_dev, 1.0, early and sgd, stream=stream)
         elif self.path == "bulk":
-            self._launch(0, hyper_dev, float(workers))
+            self._launch(0, hyper_dev, float(workers), stream=stream)
             code = self.lib.psgd_bulk_allreduce_launch(self.comm.ptr, ctypes.c_longlong(self.n_pad), workers, _stream_ptr())
             native.check(code, "psgd_bulk_allreduce_launch")
             self.launches += 2
-            self._launch(13 if sgd else 12, hyper_dev, 1.0)
+            self._launch(13 if sgd else 12, hyper_dev, 1.0, stream=stream)
         elif self.path == "nvls":
-            self._launch(0, hyper_dev, float(workers))
+            self._launch(0, hyper_dev, float(workers), stream=stream)
             self._nvls.all_reduce_()
             self.launches += self._nvls.launches
-            self._launch(2 if sgd else 1, hyper_dev, 1.0)
+            self._launch(2 if sgd else 1, hyper_dev, 1.0, stream=stream)
         elif self.path == "oneshot":
             if self._pushed:
                 self._pushed = False
             else:
-                self._launch(5, hyper_dev, float(workers))
-            self._launch(7 if sgd else 6, hyper_dev, 1.0)
+                self._launch(5, hyper_dev, float(workers), stream=stream)
+            self._launch(7 if sgd else 6, hyper_dev, 1.0, stream=stream)
         else:
-            self._launch(0, hyper_dev, float(workers))
+            self._launch(0, hyper_dev, float(workers), stream=stream)
             dist.all_reduce(self._flat)
-            self._launch(2 if sgd else 1, hyper_dev, 1.0)
+            self._launch(2 if sgd else 1, hyper_dev, 1.0, stream=stream)
 
     def aggregate(self, gradients: List[torch.Tensor], outs: Optional[Sequence[torch.Tensor]] = None,
                   keep_inputs: bool = False) -> List[torch.Tensor]:
@@ -1296,7 +1297,7 @@ class FusedSGDDriver:
         recording = native.capture_id(stream) if is_recorded(stream) else 0
         readers = [r for r in (self.agg._powersgd._native, self._flat_all, self._flat_plain) if r is not None]
         streams = [r._stream for r in readers if r._stream is not None]
-        if recording and (any(r.recorded_in == recording for r in readers) or any(native.capture_id(s) for s in streams)):
+        if recording and (any(r.recorded_in == recording for r in readers) or any(s and native.capture_id(s) for s in streams)):
             # The live table cannot change under a step that reads it already: one recorded before this in the
             # same graph, or one that may still be running on a stream that is part of the recording and so
             # cannot be waited for. This step keeps the values it was recorded with.

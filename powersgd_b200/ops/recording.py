@@ -18,7 +18,6 @@ import torch
 from . import native
 
 
-
 def is_recorded(stream: ctypes.c_void_p) -> bool:
     """Is the current stream, whose handle is `stream`, being recorded? The default stream (handle 0) cannot be,
     so eager loops on it are spared the question, which takes the driver some 2 us while launches are under way."""
