@@ -237,6 +237,30 @@ class TilePlan:
                 best, best_score = k, score
         return best
 
+    def panel_segments(self, mats: Sequence[int], vec_widths: Sequence[int], rows_per_panel) -> Tuple[np.ndarray, np.ndarray]:
+        """Segments of whole rows of the matrices `mats` for the kernel that does the last product and the
+        decompression in one pass, and the first segment of every CTA. Each CTA gets the same share of the elements, in
+        quads of rows and in the order of the matrices. `rows_per_panel(m, rows)`: of a segment."""
+        quads = [-(-self.plan.groups[self.mats[mi][0]].n // 4) for mi in mats]
+        costs = [4 * self.plan.groups[self.mats[mi][0]].m for mi in mats]
+        total = sum(q * c for q, c in zip(quads, costs))
+        ctas = max(1, min(148, sum(quads)))
+        segs, starts, done, cta = [], [0], 0, 0
+        for mi, left, cost in zip(mats, quads, costs):
+            g, row = self.plan.groups[self.mats[mi][0]], 0
+            while left:
+                share = total * (cta + 1) / ctas - done
+                take = left if cta == ctas - 1 else min(left, int(share / cost + 0.5))
+                if take <= 0:
+                    cta += 1
+                    starts.append(len(segs))
+                    continue
+                rows = min(4 * take, g.n - row)
+                segs.append((mi, row, rows, 0, g.m, rows_per_panel(g.m, rows), 1, 0, 0, int(vec_widths[mi]), (0, 0)))
+                row, left, done = row + rows, left - take, done + take * cost
+        starts += [len(segs)] * (ctas + 1 - len(starts))
+        return np.array(segs, dtype=layout.TILE_DTYPE), np.array(starts, dtype=np.int32)
+
     def orth_units(self, side: str, chunk_rows: int) -> Tuple[np.ndarray, np.ndarray]:
         """Units (one per matrix; one per shape group at rank 1) and their row chunks of at most
         `chunk_rows` rows, which never straddle the sub-matrices of a rank-1 unit."""
@@ -467,6 +491,7 @@ class NativeCompressor(_Recordable):
             self._tiles_dev[name] = {
                 v: (_to_device(a, self.device) if len(a) else None, len(a)) for v, a in by_vec.items()
             }
+        self._plan_panels(vec, [grads[idx].data_ptr() for _gi, _pos, idx in self.tiles.mats], mode, need_out)
         self._split_tile_lists()
         self._partial = torch.empty(self.tiles.partial_floats, device=self.device, dtype=torch.float32)
         self._partial_tc = torch.empty(self.tiles.partial_tc_floats, device=self.device, dtype=torch.float32)
@@ -475,6 +500,25 @@ class NativeCompressor(_Recordable):
         self._out_views = out_views
         self._tapes.clear()
         self._key = key
+
+    PANEL_ELEMS = 1 << 20
+
+    def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str, need_out: bool) -> None:
+        """Which matrices finish a step whose last basis is on the Q side in one pass (csrc/panel.cu), and the tile
+        lists of the others. One worker, no optimizer step, no product kernel asked for by name."""
+        rows = lambda m, n: int(self.lib.psgd_panel_rows(self.tiles.max_r, self.T, m, n))  # noqa: E731
+        groups = [self.plan.groups[gi] for gi, _pos, _idx in self.tiles.mats]
+        mats = [mi for mi, (g, at) in enumerate(zip(groups, addresses)) if at % 16 == 0 and rows(g.m, g.n) > 0]
+        self._panel = None
+        if not need_out or world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok or sum(groups[mi].n * groups[mi].m for mi in mats) < max(1, self.PANEL_ELEMS):
+            return
+        segs, starts = self.tiles.panel_segments(mats, vec, rows)
+        self._panel = (_to_device(segs, self.device), _to_device(starts, self.device), len(starts) - 1)
+        for name in ("nn", "fin"):
+            for key in ("f", "tc"):
+                arr = self._tile_arrays[name][key]
+                rest = arr[~np.isin(arr["mat"], mats)] if len(arr) else arr
+                self._tiles_dev[name][key + "_rest"] = (_to_device(rest, self.device) if len(rest) else None, len(rest))
 
     # -- early bucket ---------------------------------------------------------------------
     def set_early_bucket(self, compressed_indices: Sequence[int]) -> None:
@@ -572,7 +616,7 @@ class NativeCompressor(_Recordable):
         the scratch."""
         return (
             self._mats_dev, self._maps_dev, *(t for lists in self._tiles_dev.values() for t, _count in lists.values()),
-            self._partial, self._partial_tc, self._tickets, self._out_arena, self._hyper_dev, self._status,
+            self._panel, self._partial, self._partial_tc, self._tickets, self._out_arena, self._hyper_dev, self._status,
             self.units, self.chunks, self._orth_part, self._orth_rinv, self.h_in, self.h_loc, self.h_sum, self.cmat,
             self.core._ps_buffer, self.core._qs_buffer,
         )
@@ -612,11 +656,11 @@ class NativeCompressor(_Recordable):
     def _gemm(self, transposed: bool, fin: torch.Tensor, fout: torch.Tensor, corr_fac, corr_c,
               fout2: Optional[torch.Tensor] = None, part: str = "all", early: bool = False):
         """`part`: "all", or one half of a split launch - "early" (the CUDA-core tiles of the
-        matrices in the early bucket) / "late" (everything else); see `set_early_bucket`.
-        `early`: see `_chained`."""
+        matrices in the early bucket) / "late" (everything else); see `set_early_bucket` -, or
+        "rest" (what the panel kernel leaves). `early`: see `_chained`."""
         name = "nt" if transposed else "nn"
         form = (1 if transposed else 0) | (2 if early else 0)
-        tiles, count = self._tiles_dev[name]["tc"]
+        tiles, count = self._tiles_dev[name]["tc_rest" if part == "rest" else "tc"]
         if count and part != "early":
             self._call(
                 "psgd_gemm_tc_launch",
@@ -638,7 +682,7 @@ class NativeCompressor(_Recordable):
                 self.comm.ptr if self.comm is not None else ctypes.c_void_p(0),
                 self._status.dev_ptr,
             )
-        tiles, count = self._tiles_dev[name]["f" if part == "all" else ("fA" if part == "early" else "fB")]
+        tiles, count = self._tiles_dev[name][{"all": "f", "early": "fA", "late": "fB", "rest": "f_rest"}[part]]
         if count:
             self._call(
                 "psgd_gemm_ffma_launch",
@@ -668,8 +712,8 @@ class NativeCompressor(_Recordable):
         return bool(self.lib.psgd_finalize_uses_strip(self.T, self.tiles.max_r, self.tiles.fin_rows, 0))
 
     def _finalize(self, sides: List[bool], fused_sgd: bool, workers: int, gather_state: Optional[torch.Tensor] = None,
-                  flags: int = 0, early: bool = False):
-        """`gather_state`: the warm-start buffer that receives the summed factor of the last
+                  flags: int = 0, early: bool = False, rest: bool = False):
+        """`rest`: only the matrices that the panel kernel leaves. `gather_state`: the warm-start buffer that receives the summed factor of the last
         half-iteration when this launch is also its consumer (see `_gathers_in_finalize`).
         `flags`: residual options of the strip / general kernels (csrc/finalize.cu, FinalizeArgs).
         `early`: see `_chained`."""
@@ -683,7 +727,7 @@ class NativeCompressor(_Recordable):
             else:
                 rloc.append(self.h_in[t]); rsum.append(self.h_in[t])
                 lloc.append(self.h_loc[t]); lsum.append(self.h_sum[t])
-        tiles, count = self._tiles_dev["fin"]["tc"]
+        tiles, count = self._tiles_dev["fin"]["tc_rest" if rest else "tc"]
         if count:
             self._call(
                 "psgd_finalize_tc_launch",
@@ -702,7 +746,7 @@ class NativeCompressor(_Recordable):
                 1 if fused_sgd else 0,
                 self._status.dev_ptr,
             )
-        tiles, count = self._tiles_dev["fin"]["f"]
+        tiles, count = self._tiles_dev["fin"]["f_rest" if rest else "f"]
         if count:
             gather = gather_state is not None
             self._call(
@@ -729,17 +773,33 @@ class NativeCompressor(_Recordable):
                 int(early and not self._tiles_dev["fin"]["tc"][1]),
             )
 
-    def _half_iterations(self):
+    def _finish_panels(self, sides: List[bool], state_out: torch.Tensor, early: bool) -> None:
+        """The last half-iteration (basis on the Q side) and the decompression of the matrices that take one
+        pass for both. `early`: see `_chained`."""
+        last = len(sides) - 1
+        left = [self.h_in[t] if sides[t] else self.h_loc[t] for t in range(last)]
+        right = [self.h_loc[t] if sides[t] else self.h_in[t] for t in range(last)]
+        segs, starts, ctas = self._panel
+        self._call(
+            "psgd_panel_launch",
+            _ptr(self._mats_dev), _ptr(segs), _ptr(starts), ctas, self.tiles.max_r, len(sides),
+            _ptr(self.h_in[last]), _ptr(self.h_loc[last]), _ptr(state_out),
+            ctypes.cast(_ptr_array(left), ctypes.c_void_p), ctypes.cast(_ptr_array(right), ctypes.c_void_p),
+            ctypes.cast(_ptr_array(self.cmat[last]), ctypes.c_void_p), self._status.dev_ptr, int(early),
+        )
+
+    def _half_iterations(self, finish: bool = False):
         """Runs the T half-iterations. Returns (sides, pending): `pending` is the warm-start buffer
         whose summed factor the decompression launch still has to gather, or None. `_follows` says
-        whether the last thing put on the stream was a launch of the step (see `_chained`)."""
+        whether the last thing put on the stream was a launch of the step (see `_chained`), `_finished` whether
+        the last one was also the decompression of the matrices that the panel kernel takes, which `finish` allows."""
         core = self.core
         workers = world_size()
         p2p = workers > 1 and self.comm is not None
         defer_last = p2p and self._gathers_in_finalize()
         sides: List[bool] = []
         pending: Optional[torch.Tensor] = None   # state buffer whose sum is still in the channel's slots
-        chained, self._follows = self._chained(), False
+        chained, self._follows, self._finished = self._chained(), False, False
         for t in range(self.T):
             left = (core.step_counter * self.T + t) % 2 == 0
             sides.append(left)
@@ -775,8 +835,12 @@ class NativeCompressor(_Recordable):
                 part = "all"
                 if t == 0 and self._early_product_done is not None:
                     part = "late"  # the early bucket's tiles were launched during backward
+                elif finish and t == self.T - 1 and not left and self._panel is not None:
+                    part, self._finished = "rest", True
                 self._gemm(left, self.h_in[t], self.h_loc[t], other, self.cmat[t], state_out if workers == 1 else None, part=part,
                            early=self._follows)
+                if part == "rest":
+                    self._finish_panels(sides, state_out, early=self._follows)
                 self._follows = chained
                 if part == "late":
                     torch.cuda.current_stream().wait_event(self._early_product_done)
@@ -857,9 +921,10 @@ class NativeCompressor(_Recordable):
             saved = self.h_sum
             self.h_sum = self.h_loc
         try:
-            sides, pending = self._half_iterations()
+            sides, pending = self._half_iterations(finish=not fused_sgd)
             with _Range("psgd.finalize+sgd" if fused_sgd else "psgd.finalize"):
-                self._finalize(sides, fused_sgd=fused_sgd, workers=workers, gather_state=pending, early=self._follows)
+                self._finalize(sides, fused_sgd=fused_sgd, workers=workers, gather_state=pending, early=self._follows,
+                               rest=self._finished)
         finally:
             if workers == 1:
                 self.h_sum = saved

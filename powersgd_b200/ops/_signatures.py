@@ -40,6 +40,11 @@ def declare(lib) -> None:
     lib.psgd_gemm_ffma_launch.restype = i32
     lib.psgd_gemm_ffma_launch.argtypes = [i32, i32, vp, vp, i32, vp, vp, vp, i32, vp, vp, vp, vp, vp, vp]
 
+    lib.psgd_panel_rows.restype = i32
+    lib.psgd_panel_rows.argtypes = [i32, i32, i32, i32]
+    lib.psgd_panel_launch.restype = i32
+    lib.psgd_panel_launch.argtypes = [vp, vp, vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp]
+
     lib.psgd_finalize_launch.restype = i32
     lib.psgd_finalize_launch.argtypes = [vp, vp, i32, i32, i32, vp, i32, vp, vp, vp, vp, f32, i32, vp, i32, vp, vp, i32, f32, i32, vp]
     lib.psgd_finalize_uses_strip.restype = i32
