@@ -241,25 +241,22 @@ class TilePlan:
         """Segments of whole rows of the matrices `mats` for the kernel that does the last product and the
         decompression in one pass, and the first segment of every CTA. Each CTA gets the same share of the elements, in
         quads of rows and in the order of the matrices. `rows_per_panel(m, rows)`: of a segment."""
-        quads = [-(-self.plan.groups[self.mats[mi][0]].n // 4) for mi in mats]
-        costs = [4 * self.plan.groups[self.mats[mi][0]].m for mi in mats]
-        total = sum(q * c for q, c in zip(quads, costs))
-        ctas = max(1, min(148, sum(quads)))
-        segs, starts, done, cta = [], [0], 0, 0
-        for mi, left, cost in zip(mats, quads, costs):
-            g, row = self.plan.groups[self.mats[mi][0]], 0
-            while left:
-                share = total * (cta + 1) / ctas - done
-                take = left if cta == ctas - 1 else min(left, int(share / cost + 0.5))
-                if take <= 0:
-                    cta += 1
-                    starts.append(len(segs))
-                    continue
-                rows = min(4 * take, g.n - row)
-                segs.append((mi, row, rows, 0, g.m, rows_per_panel(g.m, rows), 1, 0, 0, int(vec_widths[mi]), (0, 0)))
-                row, left, done = row + rows, left - take, done + take * cost
-        starts += [len(segs)] * (ctas + 1 - len(starts))
-        return np.array(segs, dtype=layout.TILE_DTYPE), np.array(starts, dtype=np.int32)
+        groups = [self.plan.groups[self.mats[mi][0]] for mi in mats]
+        n, m = np.array([g.n for g in groups]), np.array([g.m for g in groups])
+        first_quad = np.concatenate([[0], np.cumsum(-(-n // 4))])      # of every matrix, counted over all of them
+        cost = np.concatenate([[0], np.cumsum(-(-n // 4) * m)])
+        ctas = min(148, int(first_quad[-1]))
+        shares = cost[-1] * np.arange(ctas + 1) / ctas
+        of = np.clip(np.searchsorted(cost, shares, side="right") - 1, 0, len(mats) - 1)
+        bounds = first_quad[of] + ((shares - cost[of]) / m[of] + 0.5).astype(np.int64)   # where a CTA's share begins
+        cuts = np.union1d(bounds, first_quad)
+        of = np.searchsorted(first_quad, cuts[:-1], side="right") - 1
+        segs = np.zeros(len(cuts) - 1, dtype=layout.TILE_DTYPE)
+        segs["mat"], segs["vec"] = np.array(mats)[of], np.array(vec_widths)[np.array(mats)[of]]
+        segs["row0"], segs["cols"], segs["nsplit"] = 4 * (cuts[:-1] - first_quad[of]), m[of], 1
+        segs["rows"] = np.minimum(4 * (cuts[1:] - first_quad[of]), n[of]) - segs["row0"]
+        segs["split"] = [rows_per_panel(c, r) for c, r in zip(segs["cols"].tolist(), segs["rows"].tolist())]
+        return segs, np.searchsorted(cuts, bounds).astype(np.int32)
 
     def orth_units(self, side: str, chunk_rows: int) -> Tuple[np.ndarray, np.ndarray]:
         """Units (one per matrix; one per shape group at rank 1) and their row chunks of at most
@@ -506,18 +503,27 @@ class NativeCompressor(_Recordable):
     def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str, need_out: bool) -> None:
         """Which matrices finish a step whose last basis is on the Q side in one pass (csrc/panel.cu), and the tile
         lists of the others. One worker, no optimizer step, no product kernel asked for by name."""
-        rows = lambda m, n: int(self.lib.psgd_panel_rows(self.tiles.max_r, self.T, m, n))  # noqa: E731
+        self._panel = None
+        if not need_out or world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok:
+            return
+        known: Dict[Tuple[int, int], int] = {}
+
+        def rows(m: int, n: int) -> int:
+            if (m, n) not in known:
+                known[m, n] = int(self.lib.psgd_panel_rows(self.tiles.max_r, self.T, m, n))
+            return known[m, n]
+
         groups = [self.plan.groups[gi] for gi, _pos, _idx in self.tiles.mats]
         mats = [mi for mi, (g, at) in enumerate(zip(groups, addresses)) if at % 16 == 0 and rows(g.m, g.n) > 0]
-        self._panel = None
-        if not need_out or world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok or sum(groups[mi].n * groups[mi].m for mi in mats) < max(1, self.PANEL_ELEMS):
+        if sum(groups[mi].n * groups[mi].m for mi in mats) < max(1, self.PANEL_ELEMS):
             return
         segs, starts = self.tiles.panel_segments(mats, vec, rows)
-        self._panel = (_to_device(segs, self.device), _to_device(starts, self.device), len(starts) - 1)
+        table = _to_device(np.concatenate([segs.view(np.uint8), starts.view(np.uint8)]), self.device)
+        self._panel = (table, segs.nbytes, len(starts) - 1)
         for name in ("nn", "fin"):
             for key in ("f", "tc"):
                 arr = self._tile_arrays[name][key]
-                rest = arr[~np.isin(arr["mat"], mats)] if len(arr) else arr
+                rest = arr[~np.isin(arr["mat"], mats)] if len(arr) and len(mats) < len(groups) else arr[:0]
                 self._tiles_dev[name][key + "_rest"] = (_to_device(rest, self.device) if len(rest) else None, len(rest))
 
     # -- early bucket ---------------------------------------------------------------------
@@ -779,10 +785,10 @@ class NativeCompressor(_Recordable):
         last = len(sides) - 1
         left = [self.h_in[t] if sides[t] else self.h_loc[t] for t in range(last)]
         right = [self.h_loc[t] if sides[t] else self.h_in[t] for t in range(last)]
-        segs, starts, ctas = self._panel
+        table, segs_bytes, ctas = self._panel
         self._call(
             "psgd_panel_launch",
-            _ptr(self._mats_dev), _ptr(segs), _ptr(starts), ctas, self.tiles.max_r, len(sides),
+            _ptr(self._mats_dev), _ptr(table), ctypes.c_void_p(table.data_ptr() + segs_bytes), ctas, self.tiles.max_r, len(sides),
             _ptr(self.h_in[last]), _ptr(self.h_loc[last]), _ptr(state_out),
             ctypes.cast(_ptr_array(left), ctypes.c_void_p), ctypes.cast(_ptr_array(right), ctypes.c_void_p),
             ctypes.cast(_ptr_array(self.cmat[last]), ctypes.c_void_p), self._status.dev_ptr, int(early),
