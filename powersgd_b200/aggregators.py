@@ -24,7 +24,7 @@ import torch.distributed as dist
 
 from .orthogonalization import orthogonalize
 from .plan import CompressionPlan, avg_compressed_size, matrix_shape, should_compress
-from .utils import allreduce_average, is_dense, is_distributed, pack, same_layout, unpack, world_size
+from .utils import allreduce_average, is_dense, is_distributed, pack, unpack, world_size
 
 
 class Aggregator(ABC):
@@ -169,26 +169,9 @@ class PowerSGD(Aggregator):
         # the fused path never calls optimizer.step(): registered step hooks would not fire
         if getattr(optimizer, "_optimizer_step_pre_hooks", None) or getattr(optimizer, "_optimizer_step_post_hooks", None):
             return False
-        # one pass over the parameters, with comparisons that stay inside the tensor library where the
-        # answer is the usual one: this runs before every step of an eager loop
-        state, f32 = optimizer.state, torch.float32
-        for group in optimizer.param_groups:
-            if group.get("maximize", False) or group.get("differentiable", False):
-                return False
-            buffers = 0
-            for p in group["params"]:
-                grad = p.grad
-                if grad is None or p.dtype != f32 or not (p.is_contiguous() or is_dense(p)) or not same_layout(grad, p):
-                    return False
-                own = state.get(p)
-                buf = own.get("momentum_buffer") if own else None
-                if buf is not None:
-                    buffers += 1
-                    if not same_layout(buf, p):
-                        return False
-            if buffers and buffers != len(group["params"]):
-                return False
-        return True
+        from .ops import scan
+
+        return scan.step_fits(optimizer)
 
     def close(self) -> None:
         """Free multi-GPU resources (peer mappings, symmetric arenas). Call on every rank."""

@@ -63,8 +63,36 @@ def _compile_one(nvcc: str, src: str, verbose: bool, debug: bool = False) -> str
     return obj
 
 
+def _build_scan() -> None:
+    """The list checks (host/tensor_scan.cpp), a CPython extension for the PyTorch of this interpreter. Without
+    PyTorch's headers the package asks in Python."""
+    src, out = os.path.join(HERE, "host", "tensor_scan.cpp"), os.path.join(HERE, "_tensor_scan.so")
+    import sysconfig
+
+    import torch
+
+    stamp_path = os.path.join(OBJ_DIR, "scan_stamp.txt")
+    stamp = f"{_digest([src])} {torch.__version__} {sys.version}"
+    if os.path.exists(out) and os.path.exists(stamp_path):
+        with open(stamp_path) as fp:
+            if fp.read() == stamp:
+                return
+    base = os.path.dirname(os.path.abspath(torch.__file__))
+    includes = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-isystem{i}" for i in includes], src, "-o", out,
+           f"-L{os.path.join(base, 'lib')}", "-lc10", "-ltorch_cpu", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on {src}:\n{res.stdout}\n{res.stderr}")
+    with open(stamp_path, "w") as fp:
+        fp.write(stamp)
+
+
 def build(force: bool = False, verbose: bool = False, debug: bool = False) -> str:
     """`debug=True` builds the bounds-checked variant (libpsgd_b200_debug.so) instead."""
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    _build_scan()
     srcs = sources()
     headers = [os.path.join(HERE, f) for f in os.listdir(HERE) if f.endswith((".h", ".cuh"))]
     obj_dir, lib = (DEBUG_OBJ_DIR, DEBUG_LIB) if debug else (OBJ_DIR, LIB)

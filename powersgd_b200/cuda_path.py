@@ -31,7 +31,7 @@ import numpy as np
 import torch
 import torch.distributed as dist
 
-from .ops import layout, native
+from .ops import layout, native, scan
 from .ops.recording import capture_scope, is_recorded, keep_with_graph, outside_capture  # noqa: F401  (capture_scope: for callers)
 from .ops.recording import to_device as _to_device
 from .utils import is_dense, like_strided, same_layout, world_size
@@ -65,7 +65,7 @@ class _Range:
 
 
 def _stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
@@ -402,13 +402,7 @@ class NativeCompressor(_Recordable):
     ) -> None:
         """`outs`: caller-owned tensors (laid out like the gradients) that receive the averaged
         update instead of this object's own arena."""
-        key = (
-            tuple(g.data_ptr() for g in grads),
-            None if params is None else tuple(p.data_ptr() for p in params),
-            None if moms is None else tuple(0 if m is None else m.data_ptr() for m in moms),
-            need_out,
-            None if outs is None else tuple(o.data_ptr() for o in outs),
-        )
+        key = (scan.addresses(grads), scan.addresses(params), scan.addresses(moms), need_out, scan.addresses(outs))
         if key == self._key:
             return
         for g in grads:
@@ -989,13 +983,7 @@ class NativeFlatAllReduce(_Recordable):
             self._nvls.check()
 
     def _bind(self, grads, params=None, moms=None, hyper_index=None, need_out=True, outs=None):
-        key = (
-            tuple(g.data_ptr() for g in grads),
-            None if params is None else tuple(p.data_ptr() for p in params),
-            None if moms is None else tuple(0 if m is None else m.data_ptr() for m in moms),
-            need_out,
-            None if outs is None else tuple(o.data_ptr() for o in outs),
-        )
+        key = (scan.addresses(grads), scan.addresses(params), scan.addresses(moms), need_out, scan.addresses(outs))
         if key == self._key:
             return
         device = grads[0].device
@@ -1339,7 +1327,7 @@ class FusedSGDDriver:
                 # the same lists, compressed and uncompressed tensors apart (True / False)
                 self._split = {keep: tuple([x for x, k in zip(xs, mask) if k == keep] for xs in (params, moms, index))
                                for keep in (True, False)}
-            self._grads = [p.grad.data for p in params]
+            self._bound_grads = None
             self._cache_key = key
         return fresh_groups
 
@@ -1431,30 +1419,32 @@ class FusedSGDDriver:
             self.prepare(optimizer)
         # the gradient tensors may have been replaced since the last step (dropped zero gradients
         # re-created by autograd, a loaded checkpoint): always bind what the parameters hold now
-        now = [p.grad for p in self._params]
-        if [g.data_ptr() for g in now] != [g.data_ptr() for g in self._grads]:
-            self._grads = [g.data for g in now]
         agg = self.agg
+        mask = agg.is_compressed_mask
+        now = scan.grad_addresses(self._params)
+        if now != self._bound_grads:
+            self._grads = [p.grad.data for p in self._params]
+            self._split_grads = {keep: [g for g, k in zip(self._grads, mask) if k == keep] for keep in (True, False)}
+            self._bound_grads = now
         hyper_dev = self._hyper_dev if self._fixed is None else self._fixed
         self._fixed = None
         index, params, moms, grads = self._index, self._params, self._moms, self._grads
-        if len(grads) != len(agg.is_compressed_mask):
+        if len(grads) != len(mask):
             raise ValueError("optimizer parameters do not match the aggregator's parameter list")
         agg.step_counter += 1
         if agg.step_counter <= agg.config.start_compressing_after_num_steps:
             self._flat_all.aggregate_and_step(grads, params, moms, index, hyper_dev)
             self.launches = self._flat_all.launches
             return
-        mask = agg.is_compressed_mask
         core = agg._powersgd
         self.launches = 0
         if core.params:
             if core._native is None:
                 core._native = NativeCompressor(core)
-            core._native.aggregate_and_step([g for g, k in zip(grads, mask) if k], *self._split[True], hyper_dev)
+            core._native.aggregate_and_step(self._split_grads[True], *self._split[True], hyper_dev)
             core.step_counter += 1
             self.launches += core._native.launches
-        plain = [g for g, k in zip(grads, mask) if not k]
+        plain = self._split_grads[False]
         if plain:
             # after the low-rank path: a consumer that spins on its peers next to the product
             # kernels (tried as a parallel side-stream branch) cost more than it hid

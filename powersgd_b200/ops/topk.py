@@ -13,7 +13,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import native
+from . import native, scan
 from .recording import is_recorded, keep_with_graph, outside_capture, release_finished
 
 _workspaces = {}
@@ -27,7 +27,7 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
         memory is None or (memory.is_contiguous() and memory.dtype == torch.float32)
     ):
         lib = native.lib()
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
         recorded = is_recorded(stream)   # a graph gets counters of its own, see topk_abs_many
         ws = None if recorded else _workspaces.get(flat.device)
         if ws is None:
@@ -66,12 +66,9 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     total = sum(ks)
     tensors = list(tensors)
     mems = list(memories) if memories is not None else [None] * len(tensors)
-    device, f32 = tensors[0].device, torch.float32
-    native_ok = (
-        device.type == "cuda" and native.use_for_cuda()
-        and all(t.dtype == f32 and t.is_contiguous() for t in tensors)   # their memory is then the flattened tensor
-        and all(m is None or (m.is_contiguous() and m.dtype == f32) for m in mems)
-    )
+    device = tensors[0].device
+    # contiguous: their memory is then the flattened tensor
+    native_ok = device.type == "cuda" and native.use_for_cuda() and scan.usable(tensors, True) and scan.usable([m for m in mems if m is not None], True)
     if not native_ok:
         values = torch.empty(total, dtype=torch.float32, device=device)
         positions = torch.empty(total, dtype=torch.int32, device=device)
@@ -84,10 +81,10 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     import numpy as np
 
     lib = native.lib()
-    key = (device, tuple(t.data_ptr() for t in tensors), tuple(0 if m is None else m.data_ptr() for m in mems), tuple(t.numel() for t in tensors), tuple(ks))
+    key = (device, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks))
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     recorded = is_recorded(stream)
     entry = None if recorded else _many_cache.get(key)
     if entry is None:
@@ -156,7 +153,7 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
     use_native = (
         all_values.is_cuda and native.use_for_cuda() and all_values.dtype == torch.float32 and all_positions.dtype == torch.int32
         and all_values.is_contiguous() and all_positions.is_contiguous()
-        and all(o.is_contiguous() and o.dtype == torch.float32 for o in outs)
+        and scan.usable(outs, True)
     )
     if use_native:
         import numpy as np
@@ -172,10 +169,10 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
                 scratch = torch.zeros(2, dtype=torch.int32, device=device)  # [grid barrier, status]
             _combine_scratch[device] = scratch
         barrier = scratch
-        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
         # tables of addresses and lengths, kept by exactly those (as the selection's above, recorded calls
         # included): building and uploading one stalls the host until the selection has run
-        key = (device, tuple(o.data_ptr() for o in outs), tuple(o.numel() for o in outs), tuple(ends))
+        key = (device, scan.addresses(outs), scan.sizes(outs), tuple(ends))
         recorded = is_recorded(stream)
         tables = None if recorded else _segment_cache.get(key)
         if tables is None:

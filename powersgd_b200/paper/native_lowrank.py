@@ -25,9 +25,9 @@ import numpy as np
 import torch
 
 from ..cuda_path import NativeCompressor, NativeFlatAllReduce, _ptr, _ptr_array, _stream_ptr
-from ..ops import native
+from ..ops import native, scan
 from ..plan import CompressionPlan
-from ..utils import is_dense, world_size
+from ..utils import world_size
 
 
 class _Core:
@@ -57,8 +57,7 @@ class _Core:
 def usable(tensors: Sequence[torch.Tensor]) -> bool:
     """Native path: CUDA, float32, dense tensors, and the library present (its absence on a CUDA
     machine is an error unless PSGD_B200_ALLOW_FALLBACK=1)."""
-    f32 = torch.float32
-    if not tensors or not all(t.is_cuda and t.dtype == f32 and (t.is_contiguous() or is_dense(t)) for t in tensors):
+    if not tensors or not scan.usable(tensors):
         return False
     return native.use_for_cuda()
 

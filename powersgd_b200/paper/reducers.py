@@ -31,7 +31,7 @@ import torch
 import torch.distributed as dist
 
 from ..orthogonalization import gram_schmidt_
-from ..ops import signpack
+from ..ops import scan, signpack
 from ..ops.svd import svd_many
 from ..ops.topk import sparse_combine, topk_abs, topk_abs_many
 from ..utils import TensorBuffer, n_bits
@@ -86,6 +86,8 @@ def _rows(gathered: List[torch.Tensor]) -> torch.Tensor:
     """[workers, K] tensor over the per-worker results of `_gather_all` (no copy when they already
     are the rows of one gathered buffer, as the in-kernel all-gather returns them)."""
     first = gathered[0]
+    if len(gathered) == 1:
+        return first.reshape(1, -1)
     base = first._base if first._base is not None else None
     if base is not None and base.dim() == 2 and base.shape == (len(gathered), first.numel()) and all(
         g._base is base and g.data_ptr() == base.data_ptr() + r * first.numel() * first.element_size() for r, g in enumerate(gathered)
@@ -499,8 +501,9 @@ class TopKReducer(Reducer):
 
     def reduce(self, grad_in, grad_out, memory_out) -> int:
         with self.timer("reduce.flatpack", verbosity=2):
-            sizes = [_top_size(self.compression, t.nelement()) for t in grad_in]
-            ends = np.cumsum(sizes).tolist()
+            numels = np.frombuffer(scan.sizes(grad_in), dtype=np.uint64).astype(np.float64)
+            sizes = np.maximum(1, (0.5 * self.compression * numels).astype(np.int64))   # _top_size of all
+            ends, sizes = np.cumsum(sizes).tolist(), sizes.tolist()
         with self.timer("reduce.topk", verbosity=2):
             # selection, gather and the error-feedback write (memory = x with the taken entries
             # zeroed) are one fused operation over the whole list: four launches on CUDA
