@@ -127,14 +127,21 @@ PSGD_API int psgd_topk_abs(const float* x, long long n, long long k, int* worksp
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same selection for MANY tensors at once. The per-tensor reducer of the harness calls the
+// The same selection for MANY tensors at once, with two passes over them. The per-tensor reducer of the harness calls the
 // selection once per parameter (62 times for ResNet-18, paper-code/gradient_reducers.py:226-253),
-// which is launch-bound; here the three histogram passes and the compaction are four launches for
-// the whole list. Every block serves one (tensor, chunk) pair from a block table; every tensor has
-// its own histograms and counters in the workspace, and the digit is chosen by the whole block
-// with a parallel suffix scan instead of one thread walking the bins. Bound by the reads (L2 for a
-// model of this size) and by what a block costs besides them, so some four blocks per SM serve the whole
-// list: 62 tensors of ResNet-18 (45 MB), k = numel / 488: a histogram pass 29 -> 14 us, compaction 46 -> 23 us.
+// which is launch-bound; here a few launches serve the whole list. Every block serves one (tensor, chunk) pair
+// from a block table; every tensor has its own histograms and counters in the workspace, and a digit is chosen
+// by the whole block with a parallel suffix scan instead of one thread walking the bins:
+//   1. histogram of the leading digit (11 of the 31 bits of |x|): one read;
+//   2. every entry above the chosen digit is taken, every entry inside it becomes a candidate (a list of up to
+//      `cap` per tensor), and `memory` is written: one read and one write;
+//   3. one block per tensor finds the threshold among its candidates and takes those above it.
+// A tensor with more candidates than its list holds (many entries of nearly equal size) goes the long way
+// instead: histograms of the second and the third digit over all entries in launches 2 and 3, and a
+// compaction pass in launch 4, which has nothing to do for the others.
+// Bound by the reads (L2 for a model of this size) and by what a block costs besides them, so some four blocks
+// per SM serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: three histogram passes of 14.2 us and a
+// compaction of 23.9 before (67 us); 14.8, 21.6, 14.5 and 6.0 (57 us) now.
 namespace {
 
 struct TopkItem {
@@ -143,6 +150,8 @@ struct TopkItem {
   long long n;
   long long k;         // entries to take (1 <= k <= n)
   long long out_off;   // start of this tensor's k pairs in values / positions
+  long long cand_off;  // start of its candidates, and
+  long long cap;       // how many there may be
 };
 
 // Block-wide: walks `bins` (<= 2048, TK_THREADS threads x 4 bins) from the top until `remain` entries are
@@ -243,28 +252,16 @@ __device__ void tk_derive_block(const int* ws, int upto, long long k, Pick* pick
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
-                                                                          const int* __restrict__ block_part, const int* __restrict__ item_parts,
-                                                                          int* __restrict__ ws_all, int pass) {
-  // four copies of the histogram, by lane: the leading digit of a gradient takes a few dozen values,
-  // and lanes that meet on one address are served one after another
-  __shared__ __align__(16) int sh[TK_BINS0 * 4];
-  __shared__ int scan[TK_THREADS / 32];
-  __shared__ Pick pick;
-  __shared__ long long remain_sh;
-  __shared__ int bin_sh;
-  const int it = block_item[blockIdx.x];
-  const TopkItem item = items[it];
-  int* ws = ws_all + (long long)it * TK_WS_INTS;
+// Histogram of digit `pass` of the entries that agree with the digits chosen so far (block-wide).
+__device__ void tk_histogram(const TopkItem& item, int part, int parts, int* ws, int pass, unsigned prefix, int* sh) {
   const int bins = pass == 2 ? TK_BINS2 : TK_BINS0;
   for (int b = threadIdx.x; b < bins * 4; b += TK_THREADS) sh[b] = 0;
-  tk_derive_block(ws, pass, item.k, &pick, &remain_sh, &bin_sh, scan);
-  const unsigned prefix = pick.prefix;
+  __syncthreads();
   const unsigned mask = pass == 0 ? 0u : (pass == 1 ? 0x7FF00000u : 0x7FFFFE00u);
   const int shift = pass == 0 ? 20 : (pass == 1 ? 9 : 0);
   const unsigned digit_mask = pass == 2 ? 0x1FFu : 0x7FFu;
   int* mine = sh + (threadIdx.x & 3);
-  tk_for_each(item.x, item.n, block_part[blockIdx.x], item_parts[it], [&](const float4& q, long long, int count) {
+  tk_for_each(item.x, item.n, part, parts, [&](const float4& q, long long, int count) {
     const float v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -281,6 +278,169 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const T
   }
 }
 
+__global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
+                                                                          const int* __restrict__ block_part, const int* __restrict__ item_parts,
+                                                                          int* __restrict__ ws_all) {
+  // four copies of the histogram, by lane: the leading digit of a gradient takes a few dozen values,
+  // and lanes that meet on one address are served one after another
+  __shared__ __align__(16) int sh[TK_BINS0 * 4];
+  const int it = block_item[blockIdx.x];
+  tk_histogram(items[it], block_part[blockIdx.x], item_parts[it], ws_all + (long long)it * TK_WS_INTS, 0, 0u, sh);
+}
+
+// Entries a block has found, handed out with one addition to a counter of the tensor per block: thousands
+// of additions to one address would be served one after another.
+struct Found {
+  float v[TK_FOUND];
+  int p[TK_FOUND];
+  int count, base;
+};
+__device__ __forceinline__ void tk_put(Found& f, int* counter, float* val, int* pos, float v, int p) {
+  const int slot = atomicAdd(&f.count, 1);
+  if (slot < TK_FOUND) {
+    f.v[slot] = v;
+    f.p[slot] = p;
+  } else {
+    const int at = atomicAdd(counter, 1);
+    val[at] = v;
+    pos[at] = p;
+  }
+}
+__device__ void tk_hand_out(Found& f, int* counter, float* val, int* pos) {   // block-wide
+  __syncthreads();
+  const int mine = min(f.count, TK_FOUND);
+  if (threadIdx.x == 0 && mine) f.base = atomicAdd(counter, mine);
+  __syncthreads();
+  for (int e = threadIdx.x; e < mine; e += TK_THREADS) {
+    val[f.base + e] = f.v[e];
+    pos[f.base + e] = f.p[e];
+  }
+}
+
+// Launch 2: what lies above the leading digit is taken, what lies in it is listed; or the second histogram.
+// cand_v / cand_p: lists of candidates; counters of a tensor: [0] taken, [1] equal to the threshold, [2] candidates.
+__global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
+                                                                           const int* __restrict__ block_part, const int* __restrict__ item_parts,
+                                                                           int* __restrict__ ws_all, float* __restrict__ values,
+                                                                           int* __restrict__ positions, float* __restrict__ cand_v,
+                                                                           int* __restrict__ cand_p) {
+  __shared__ union {
+    int hist[TK_BINS0 * 4];
+    struct { Found above, inside; } found;
+  } sh;
+  __shared__ int scan[TK_THREADS / 32];
+  __shared__ Pick pick;
+  __shared__ long long remain_sh;
+  __shared__ int bin_sh;
+  const int it = block_item[blockIdx.x];
+  const TopkItem item = items[it];
+  int* ws = ws_all + (long long)it * TK_WS_INTS;
+  tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
+  const unsigned prefix = pick.prefix;
+  if (ws[prefix >> 20] > item.cap) {
+    tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 1, prefix, sh.hist);
+    return;
+  }
+  if (threadIdx.x == 0) sh.found.above.count = sh.found.inside.count = 0;
+  __syncthreads();
+  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
+  float* val = values + item.out_off;
+  int* pos = positions + item.out_off;
+  float* cv = cand_v + item.cand_off;
+  int* cp = cand_p + item.cand_off;
+  const bool wide = ((uintptr_t)item.memory & 15u) == 0;
+  tk_for_each(item.x, item.n, block_part[blockIdx.x], item_parts[it], [&](const float4& q, long long first, int count) {
+    const float v[4] = {q.x, q.y, q.z, q.w};
+    float rest[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      rest[j] = v[j];
+      const unsigned key = tk_key(v[j]);
+      if (j < count && key >= prefix) {
+        if ((key & 0x7FF00000u) == prefix) {
+          tk_put(sh.found.inside, counters + 2, cv, cp, v[j], (int)(first + j));
+        } else {
+          tk_put(sh.found.above, counters, val, pos, v[j], (int)(first + j));
+          rest[j] = 0.f;
+        }
+      }
+    }
+    if (item.memory) {
+      if (count == 4 && wide) {
+        *reinterpret_cast<float4*>(item.memory + first) = make_float4(rest[0], rest[1], rest[2], rest[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j < count) item.memory[first + j] = rest[j];
+      }
+    }
+  });
+  tk_hand_out(sh.found.above, counters, val, pos);
+  tk_hand_out(sh.found.inside, counters + 2, cv, cp);
+}
+
+// Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram.
+__global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
+                                                                            const int* __restrict__ block_part, const int* __restrict__ item_parts,
+                                                                            int* __restrict__ ws_all, float* __restrict__ values,
+                                                                            int* __restrict__ positions, const float* __restrict__ cand_v,
+                                                                            const int* __restrict__ cand_p) {
+  __shared__ __align__(16) int sh[TK_BINS0 * 4];
+  __shared__ int scan[TK_THREADS / 32];
+  __shared__ Pick pick;
+  __shared__ long long remain_sh;
+  __shared__ int bin_sh;
+  const int it = block_item[blockIdx.x];
+  const TopkItem item = items[it];
+  int* ws = ws_all + (long long)it * TK_WS_INTS;
+  tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
+  const int n = ws[pick.prefix >> 20];
+  if (n > item.cap) {
+    tk_derive_block(ws, 2, item.k, &pick, &remain_sh, &bin_sh, scan);
+    tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 2, pick.prefix, sh);
+    return;
+  }
+  if (block_part[blockIdx.x] != 0) return;
+  const float* cv = cand_v + item.cand_off;
+  const int* cp = cand_p + item.cand_off;
+  for (int digit = 1; digit <= 2; ++digit) {
+    const int bins = digit == 2 ? TK_BINS2 : TK_BINS1, shift = digit == 2 ? 0 : 9;
+    const unsigned mask = digit == 2 ? 0x7FFFFE00u : 0x7FF00000u, prefix = pick.prefix;
+    for (int b = threadIdx.x; b < bins; b += TK_THREADS) sh[b] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += TK_THREADS) {
+      const unsigned key = tk_key(cv[e]);
+      if ((key & mask) == prefix) atomicAdd(sh + ((key >> shift) & (unsigned)(bins - 1)), 1);
+    }
+    __syncthreads();
+    tk_choose_block(sh, bins, &remain_sh, &bin_sh, scan);
+    if (threadIdx.x == 0) pick.prefix = prefix | ((unsigned)bin_sh << shift);
+    __syncthreads();
+  }
+  const unsigned threshold = pick.prefix;
+  const long long take_equal = remain_sh, base_equal = item.k - take_equal;
+  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
+  float* val = values + item.out_off;
+  int* pos = positions + item.out_off;
+  for (int e = threadIdx.x; e < n; e += TK_THREADS) {
+    const float v = cv[e];
+    const unsigned key = tk_key(v);
+    if (key < threshold) continue;
+    long long slot;
+    if (key > threshold) {
+      slot = atomicAdd(counters, 1);
+    } else {
+      const long long eq = atomicAdd(counters + 1, 1);
+      if (eq >= take_equal) continue;
+      slot = base_equal + eq;
+    }
+    val[slot] = v;
+    pos[slot] = cp[e];
+    if (item.memory) item.memory[cp[e]] = 0.f;
+  }
+}
+
+// Launch 4: takes the k entries of a tensor with too many candidates.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                              const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                              int* __restrict__ ws_all, float* __restrict__ values,
@@ -289,21 +449,18 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
   __shared__ Pick pick;
   __shared__ long long remain_sh;
   __shared__ int bin_sh;
-  // entries above the threshold are collected here and handed out with one addition to the tensor's
-  // counter per block: thousands of additions to one address would be served one after another
-  __shared__ float found_v[TK_FOUND];
-  __shared__ int found_p[TK_FOUND];
-  __shared__ int found, found_base;
+  __shared__ Found found;
   const int it = block_item[blockIdx.x];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
-  if (threadIdx.x == 0) found = 0;
+  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
+  tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
+  if (ws[pick.prefix >> 20] <= item.cap) return;   // launch 3 took the rest
+  if (threadIdx.x == 0) found.count = 0;
   tk_derive_block(ws, 3, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned threshold = pick.prefix;
   const long long take_equal = pick.remain;
   const long long base_equal = item.k - take_equal;
-  int* cnt_gt = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
-  int* cnt_eq = cnt_gt + 1;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
   const bool wide = ((uintptr_t)item.memory & 15u) == 0;
@@ -317,18 +474,10 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
       if (j < count && key >= threshold) {
         const int i = (int)(first + j);
         if (key > threshold) {
-          const int slot = atomicAdd(&found, 1);
-          if (slot < TK_FOUND) {
-            found_v[slot] = v[j];
-            found_p[slot] = i;
-          } else {
-            const int at = atomicAdd(cnt_gt, 1);
-            val[at] = v[j];
-            pos[at] = i;
-          }
+          tk_put(found, counters, val, pos, v[j], i);
           rest[j] = 0.f;
         } else {
-          const long long e = atomicAdd(cnt_eq, 1);
+          const long long e = atomicAdd(counters + 1, 1);
           if (e < take_equal) {
             val[base_equal + e] = v[j];
             pos[base_equal + e] = i;
@@ -347,14 +496,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
       }
     }
   });
-  __syncthreads();
-  const int mine = min(found, TK_FOUND);
-  if (threadIdx.x == 0 && mine) found_base = atomicAdd(cnt_gt, mine);
-  __syncthreads();
-  for (int e = threadIdx.x; e < mine; e += TK_THREADS) {
-    val[found_base + e] = found_v[e];
-    pos[found_base + e] = found_p[e];
-  }
+  tk_hand_out(found, counters, val, pos);
 }
 
 }  // namespace
@@ -363,15 +505,16 @@ PSGD_API int psgd_topk_item_bytes() { return (int)sizeof(TopkItem); }
 
 // Top-k of |x| for `nitems` tensors in four launches. items: device array of TopkItem; block_item /
 // block_part: device tables of `nblocks` entries (which tensor a block serves and which of that
-// tensor's `item_parts[item]` interleaved parts); workspace: nitems * psgd_topk_workspace_ints() ints.
-// values / positions receive every tensor's k pairs at its `out_off`.
+// tensor's `item_parts[item]` interleaved parts); workspace: nitems * psgd_topk_workspace_ints() ints; cand_v / cand_p: room for
+// the candidates of all tensors (`cand_off`, `cap` of the items). values / positions receive every tensor's k pairs at its `out_off`.
 PSGD_API int psgd_topk_abs_many(const void* items, int nitems, const int* block_item, const int* block_part, const int* item_parts,
-                                int nblocks, int* workspace, float* values, int* positions, cudaStream_t stream) {
+                                int nblocks, int* workspace, float* cand_v, int* cand_p, float* values, int* positions, cudaStream_t stream) {
   if (nitems <= 0 || nblocks <= 0) return 0;
   PSGD_CUDA_OK(cudaMemsetAsync(workspace, 0, sizeof(int) * (size_t)TK_WS_INTS * nitems, stream));
   const TopkItem* it = (const TopkItem*)items;
-  for (int pass = 0; pass < 3; ++pass)
-    psgd_topk_many_hist_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, pass);
+  psgd_topk_many_hist_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace);
+  psgd_topk_many_split_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, values, positions, cand_v, cand_p);
+  psgd_topk_many_refine_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, values, positions, cand_v, cand_p);
   psgd_topk_many_compact_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, values, positions);
   PSGD_CUDA_OK(cudaGetLastError());
   return 0;

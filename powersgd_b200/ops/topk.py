@@ -54,6 +54,7 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
 
 
 _many_cache: dict = {}
+CANDIDATES = 4   # room for candidates, in multiples of the entries taken (0: none)
 
 
 def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -89,18 +90,22 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     entry = None if recorded else _many_cache.get(key)
     if entry is None:
         release_finished()
-        dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64)])
+        dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64),
+                          ("cand_off", np.int64), ("cap", np.int64)])
         if dtype.itemsize != int(lib.psgd_topk_item_bytes()):
             raise RuntimeError("top-k item record out of sync with the native library")
         items = np.zeros(len(tensors), dtype=dtype)
         block_item, block_part, parts = [], [], []
-        at, total_n = 0, max(1, sum(t.numel() for t in tensors))
+        at, room, total_n = 0, 0, max(1, sum(t.numel() for t in tensors))
         for i, (t, k, m) in enumerate(zip(tensors, ks, mems)):
             n = t.numel()
             if not (0 < k <= n < (1 << 31)):
                 raise ValueError(f"topk_abs_many: need 0 < k <= n < 2^31 (k = {k}, n = {n})")
-            items[i] = (t.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at)
-            at += k
+            # candidates: entries that agree with the threshold in their leading 11 bits (an eighth of an octave); some
+            # two k of a normal distribution's tail. A tensor with more goes the long way
+            cap = min(n, CANDIDATES * k + n // 16 + 1024) if CANDIDATES else 0
+            items[i] = (t.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at, room, cap)
+            at, room = at + k, room + cap
             # blocks of 512 threads with at least 16 elements each, some four per SM for the whole list:
             # every block pays for its histogram (zeroing, choosing the digits so far, adding it up)
             nparts = max(1, min(-(-n // (512 * 16)), -(-592 * n // total_n)))
@@ -113,6 +118,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
                 "items": to_dev(items), "block_item": to_dev(np.asarray(block_item, dtype=np.int32)),
                 "block_part": to_dev(np.asarray(block_part, dtype=np.int32)), "parts": to_dev(np.asarray(parts, dtype=np.int32)),
                 "nblocks": len(block_item),
+                "cand_v": torch.empty(max(room, 1), dtype=torch.float32, device=device), "cand_p": torch.empty(max(room, 1), dtype=torch.int32, device=device),
                 "ws": torch.zeros(len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
             }
         if recorded:
@@ -128,7 +134,7 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
     vp = ctypes.c_void_p
     code = lib.psgd_topk_abs_many(
         vp(entry["items"].data_ptr()), len(tensors), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
-        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
+        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
     )
     native.check(code, "psgd_topk_abs_many")
     return values, positions
