@@ -93,6 +93,14 @@ def _split_even(total: int, max_chunk: int, multiple: int) -> List[Tuple[int, in
     return out
 
 
+def _split_count(total: int, max_chunk: int, multiple: int) -> int:
+    """len(_split_even(total, max_chunk, multiple))"""
+    if total <= max_chunk:
+        return 1
+    size = -(-total // -(-total // max_chunk))
+    return -(-total // (-(-size // multiple) * multiple))
+
+
 class TilePlan:
     """Static tile lists (independent of tensor addresses) for one CompressionPlan."""
 
@@ -137,13 +145,9 @@ class TilePlan:
             g = self.plan.groups[gi]
             v = int(vec_widths[mi])
             if tc_flags[mi] and self.fin_tc_ok:
-                for r0 in range(0, g.n, 128):
-                    for c0 in range(0, g.m, 64):
-                        fin["tc"].append((mi, r0, min(128, g.n - r0), c0, min(64, g.m - c0), 0, 1, 0, 0, v, (0, 0)))
+                fin["tc"].append(self._grid(mi, g.n, 128, g.m, 64, v))
             else:
-                for r0 in range(0, g.n, self.fin_rows):
-                    for c0 in range(0, g.m, 128):
-                        fin["f"].append((mi, r0, min(self.fin_rows, g.n - r0), c0, min(128, g.m - c0), 0, 1, 0, 0, v, (0, 0)))
+                fin["f"].append(self._grid(mi, g.n, self.fin_rows, g.m, 128, v))
             if tc_flags[mi]:
                 row_blocks = _split_even(g.n, tc_k_nt, 32)
                 for c0 in range(0, g.m, 128):
@@ -182,8 +186,17 @@ class TilePlan:
         return {
             "nt": {k: arr(v) for k, v in nt.items()},
             "nn": {k: arr(v) for k, v in nn.items()},
-            "fin": {k: arr(v) for k, v in fin.items()},
+            "fin": {k: np.concatenate(v) if v else arr(v) for k, v in fin.items()},
         }
+
+    @staticmethod
+    def _grid(mi: int, n: int, rows: int, m: int, cols: int, vec: int) -> np.ndarray:
+        """Tiles of rows x cols over an n x m matrix, row by row."""
+        r0, c0 = (x.ravel() for x in np.meshgrid(np.arange(0, n, rows), np.arange(0, m, cols), indexing="ij"))
+        tiles = np.zeros(len(r0), dtype=layout.TILE_DTYPE)
+        tiles["mat"], tiles["row0"], tiles["rows"] = mi, r0, np.minimum(rows, n - r0)
+        tiles["col0"], tiles["cols"], tiles["nsplit"], tiles["vec"] = c0, np.minimum(cols, m - c0), 1, vec
+        return tiles
 
     def _nt_tile_rows(self, n: int) -> int:
         # tall matrices: never more than 160 partial tiles per column block (the kernel walks a tile that is
@@ -225,12 +238,13 @@ class TilePlan:
             return int(os.environ["PSGD_B200_TC_K"])  # tuning knob: fixed K extent (a multiple of 32)
         slots = 148 * self.TC_CTAS_PER_SM
         best, best_score = 512, -1.0
-        longest = max((g.n if transposed else g.m) for g in groups)
+        extents: Dict[int, int] = {}   # output blocks by length of their sums
+        for g in groups:
+            k_len, out_len = (g.n, g.m) if transposed else (g.m, g.n)
+            extents[k_len] = extents.get(k_len, 0) + -(-out_len // 128)
+        longest = max(extents)
         for k in range(256, max(256, min(8192, -(-longest // 32) * 32)) + 1, 32):
-            tiles = 0
-            for g in groups:
-                k_len, out_len = (g.n, g.m) if transposed else (g.m, g.n)
-                tiles += -(-out_len // 128) * len(_split_even(k_len, k, 32))
+            tiles = sum(blocks * _split_count(k_len, k, 32) for k_len, blocks in extents.items())
             waves = -(-tiles // slots)
             score = tiles / (waves * slots) * k / (k + self.TC_TILE_OVERHEAD_ROWS)
             if score > best_score + 1e-9:
@@ -492,13 +506,13 @@ class NativeCompressor(_Recordable):
         self._tapes.clear()
         self._key = key
 
-    PANEL_ELEMS = 1 << 20
+    PANEL_ELEMS = 1 << 20   # least size of the matrices together
 
     def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str, need_out: bool) -> None:
         """Which matrices finish a step whose last basis is on the Q side in one pass (csrc/panel.cu), and the tile
         lists of the others. One worker, no optimizer step, no product kernel asked for by name."""
         self._panel = None
-        if not need_out or world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok:
+        if not need_out or world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok or self.tiles.total_elems < self.PANEL_ELEMS:
             return
         known: Dict[Tuple[int, int], int] = {}
 
