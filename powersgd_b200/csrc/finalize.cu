@@ -281,7 +281,11 @@ __device__ __forceinline__ void fin_gather(const PsgdCommDev& c, int e1, long lo
   }
 }
 
-template <int VEC, bool SAME, int RPW, bool OPT>
+// ROWS: where the rank is a multiple of four, the left panel lies row by row, as in memory: staged by 16-byte copies
+// without index arithmetic, read four values of a row at a time. Staging, 48 single loads per thread and strip at 32
+// factor columns before, was a sixth of such a strip's time and a quarter of its instructions. 50257 x 1024 at rank
+// 16 x 2: 467.6 -> 448.1 us per pass.
+template <int VEC, bool SAME, int RPW, bool OPT, bool ROWS>
 __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const PsgdTile& t, const PsgdMat& mt,
                                                     int tile_rows, float* fin_smem) {
   const int r = mt.r, m = mt.m;
@@ -360,6 +364,7 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   // follows has no registers left for it, and several workers do not overlap launches)
   if (SAME) load(0);
   psgd_wait_for_predecessor();
+  const bool by_rows = ROWS && (r & 3) == 0;
   const bool gather = !SAME && a.comm != nullptr;
   int e1 = 0;
   bool ok = true;
@@ -371,7 +376,17 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
       const float* gl = a.rloc[h] + base;
       const float* gs = a.rsum[h] + base;
       const bool poll = last && !a.poll_left;
-      for (int e = tid; e < t.cols * r; e += FIN_THREADS) {
+      const bool wide = by_rows && ((uintptr_t)gl & 15u) == 0;
+      if (wide) {
+#pragma unroll 2
+        for (int e = 4 * tid; e < t.cols * r; e += 4 * FIN_THREADS) {
+          const float4 q = *reinterpret_cast<const float4*>(gl + e);
+          const int lc = fin_div(e, r, magic), j = e - lc * r;
+          float* dst = sRl + (h * r + j) * FIN_RPITCH + fin_panel_pos<VEC>(lc);
+          dst[0] = q.x; dst[FIN_RPITCH] = q.y; dst[2 * FIN_RPITCH] = q.z; dst[3 * FIN_RPITCH] = q.w;
+        }
+      }
+      for (int e = tid; !wide && e < t.cols * r; e += FIN_THREADS) {
         const int lc = fin_div(e, r, magic), j = e - lc * r;
         const int pos = fin_panel_pos<VEC>(lc);
         sRl[(h * r + j) * FIN_RPITCH + pos] = gl[e];
@@ -394,7 +409,17 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
       const float* gl = a.lloc[h] + base;
       const float* gs = a.lsum[h] + base;
       const bool poll = last && a.poll_left;
-      for (int e = tid; e < t.rows * r; e += FIN_THREADS) {
+      if (by_rows) {
+        float* dst = sLl + h * tile_rows * r;
+        if (((uintptr_t)gl & 15u) == 0) {
+#pragma unroll 4
+          for (int e = 4 * tid; e < t.rows * r; e += 4 * FIN_THREADS) *reinterpret_cast<float4*>(dst + e) = *reinterpret_cast<const float4*>(gl + e);
+        } else {
+#pragma unroll 4
+          for (int e = tid; e < t.rows * r; e += FIN_THREADS) dst[e] = gl[e];
+        }
+      }
+      for (int e = tid; !by_rows && e < t.rows * r; e += FIN_THREADS) {
         const int lr = fin_div(e, r, magic), j = e - lr * r;
         sLl[(h * r + j) * lp + lr] = gl[e];
         if (!SAME && !poll && gs != gl) sLs[(h * r + j) * lp + lr] = gs[e];
@@ -424,7 +449,27 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
     for (int u = 0; u < RPW; ++u)
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) accE[u][c4] = accA[u][c4] = 0.f;
-    for (int h = 0; h < a.nhist; ++h) {
+    if (by_rows) {
+      for (int h = 0; h < a.nhist; ++h) {
+        const float* right = sRl + h * r * FIN_RPITCH + lane * 4;
+        const float* left = sLl + (h * tile_rows + rc + warp * RPW) * r;
+        for (int j = 0; j < r; j += 4, right += 4 * FIN_RPITCH, left += 4) {
+          __align__(16) float rv[4][4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(rv[i]) = *reinterpret_cast<const float4*>(right + i * FIN_RPITCH);
+#pragma unroll
+          for (int u = 0; u < RPW; ++u) {
+            const float4 l = *reinterpret_cast<const float4*>(left + u * r);
+            const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int c4 = 0; c4 < 4; ++c4) accE[u][c4] = fmaf(lv[i], rv[i][c4], accE[u][c4]);
+          }
+        }
+      }
+    }
+    for (int h = 0; !by_rows && h < a.nhist; ++h) {
       // the basis side of a half-iteration is the same array for the local and the summed product:
       // its panel was staged once and is read once
       const bool one_left = SAME || a.lloc[h] == a.lsum[h];
@@ -482,27 +527,27 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
 // 1001x777 + 2 x 515x2049 118.8 -> 114.5. OPT = true decides at run time; fixing the optimizer step at compile
 // time as well, or eight rows without it, was slower (recorded ResNet-18 step 112.2 -> 115.0, LSTM step
 // 222.6 -> 225.5, 50257 x 1024 at rank 16 465.8 -> 469.2).
-template <bool SAME, int RPW, bool OPT>
+template <bool SAME, int RPW, bool OPT, bool ROWS>
 __global__ void __launch_bounds__(FIN_THREADS, OPT ? 2 : 3) psgd_finalize_strip_kernel(FinalizeArgs a, int tile_rows) {
   extern __shared__ __align__(16) float fin_smem[];
   const PsgdTile t = a.tiles[blockIdx.x];
   const PsgdMat mt = a.mats[t.mat];
-  if (t.vec == 4) finalize_strip_tile<4, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
-  else if (t.vec == 2) finalize_strip_tile<2, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
-  else finalize_strip_tile<1, SAME, RPW, OPT>(a, t, mt, tile_rows, fin_smem);
+  if (t.vec == 4) finalize_strip_tile<4, SAME, RPW, OPT, ROWS>(a, t, mt, tile_rows, fin_smem);
+  else if (t.vec == 2) finalize_strip_tile<2, SAME, RPW, OPT, ROWS>(a, t, mt, tile_rows, fin_smem);
+  else finalize_strip_tile<1, SAME, RPW, OPT, ROWS>(a, t, mt, tile_rows, fin_smem);
 }
 
-template <bool SAME, int RPW, bool OPT>
+template <bool SAME, int RPW, bool OPT, bool ROWS>
 static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, int early, cudaStream_t stream) {
   const size_t smem = (size_t)(SAME ? 1 : 2) * kmax * fin_panel_floats(tile_rows) * sizeof(float);
   if (smem > (size_t)FIN_SMEM_DEFAULT) {
     static bool opted_in = false;   // per instantiation
     if (!opted_in) {
-      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME, RPW, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
+      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME, RPW, OPT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
       opted_in = true;
     }
   }
-  return psgd_launch(psgd_finalize_strip_kernel<SAME, RPW, OPT>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
+  return psgd_launch(psgd_finalize_strip_kernel<SAME, RPW, OPT, ROWS>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
 }
 
 // Tallest strip (multiple of 32 rows, at most 256) whose panels fit the shared-memory budget.
@@ -578,10 +623,12 @@ PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntile
   }
   if (strip) {
     const int kmax = nhist * max_r;
-    if (!same) return finalize_strip_launch<false, 4, true>(a, ntiles, tile_rows, kmax, early, stream);
-    if (kmax >= 16) return finalize_strip_launch<true, 8, true>(a, ntiles, tile_rows, kmax, early, stream);
-    return fused_sgd ? finalize_strip_launch<true, 4, true>(a, ntiles, tile_rows, kmax, early, stream)
-                     : finalize_strip_launch<true, 4, false>(a, ntiles, tile_rows, kmax, early, stream);
+    if (!same) return finalize_strip_launch<false, 4, true, false>(a, ntiles, tile_rows, kmax, early, stream);
+    if (kmax >= 16)
+      return max_r % 4 == 0 ? finalize_strip_launch<true, 8, true, true>(a, ntiles, tile_rows, kmax, early, stream)
+                            : finalize_strip_launch<true, 8, true, false>(a, ntiles, tile_rows, kmax, early, stream);
+    return fused_sgd ? finalize_strip_launch<true, 4, true, false>(a, ntiles, tile_rows, kmax, early, stream)
+                     : finalize_strip_launch<true, 4, false, false>(a, ntiles, tile_rows, kmax, early, stream);
   }
   return psgd_launch(same ? psgd_finalize_kernel<true> : psgd_finalize_kernel<false>, ntiles, FIN_THREADS, 0, stream, early, a);
 }

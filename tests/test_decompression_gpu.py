@@ -75,3 +75,25 @@ def test_local_and_summed_factors_apart(rank, rows):
             (mine, mine_size), (total, total_size) = product(own), product(all_)
             assert ((grads[idx].double() - (was - mine)).abs() <= eps * (mine_size + was.abs())).all(), shapes[idx]
             assert ((nat._out_views[idx].double() - total / workers).abs() <= eps * total_size / workers).all(), shapes[idx]
+
+
+@pytest.mark.parametrize("rank,iters", [(8, 2), (8, 3), (12, 2), (16, 1), (16, 2)])
+@pytest.mark.parametrize("first", [(64, 48), (5, 9)])
+def test_left_panels_by_rows(rank, iters, first):
+    """From 16 factor columns on: factors on 16-byte boundaries and, behind a matrix of rank 5, not. The bound of the first test."""
+    shapes = [first, (97, 129), (300, 260), (257, 66), (520, 128)]
+    core = BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=rank, num_iters_per_step=iters), backend="native")
+    g = torch.Generator(device="cuda").manual_seed(rank)
+    grads = [torch.randn(s, generator=g, device="cuda") for s in shapes]
+    before = [x.double() for x in grads]
+    outs, nat = core.aggregate(grads), core._native
+    for grp in core.plan.groups:
+        for pos, idx in enumerate(grp.members):
+            p0, q0 = grp.p_offset + pos * grp.n * grp.r, grp.q_offset + pos * grp.m * grp.r
+            cut = lambda buf, at, n: buf[at : at + n * grp.r].view(n, grp.r).double()  # noqa: E731
+            pairs = [(cut(a, p0, grp.n), cut(b, q0, grp.m)) for a, b in
+                     ((nat.h_in[t], nat.h_loc[t]) if t % 2 == 0 else (nat.h_loc[t], nat.h_in[t]) for t in range(iters))]
+            update, size = sum(l @ r.T for l, r in pairs), sum(l.abs() @ r.abs().T for l, r in pairs)
+            eps = (grp.r * iters + 3) * 2.0 ** -24
+            assert ((outs[idx].double() - update).abs() <= eps * size).all(), shapes[idx]
+            assert ((grads[idx].double() - (before[idx] - update)).abs() <= eps * (size + before[idx].abs())).all(), shapes[idx]
