@@ -281,10 +281,12 @@ __device__ __forceinline__ void fin_gather(const PsgdCommDev& c, int e1, long lo
   }
 }
 
-// ROWS: where the rank is a multiple of four, the left panel lies row by row, as in memory: staged by 16-byte copies
+// ROWS: where the rank is a multiple of four and accesses take 16 bytes, the left panel lies row by row, as in memory: staged by 16-byte copies
 // without index arithmetic, read four values of a row at a time. Staging, 48 single loads per thread and strip at 32
 // factor columns before, was a sixth of such a strip's time and a quarter of its instructions. 50257 x 1024 at rank
-// 16 x 2: 467.6 -> 448.1 us per pass.
+// 16 x 2: 467.6 -> 448.1 us per pass. Launches alone, before / now: 6 x 2048^2 at 8 x 2 88 / 87, 12 x 2 105 / 100, 16 x 2 118 / 110;
+// with 4-byte accesses 4 x 3000x1001 at 8 x 2 46.8 / 50.8, 16 x 2 59.3 / 62.5, with 8-byte ones 3 x 9000x650 75.9 / 77.8 and 97.4 /
+// 94.1, so those keep the other form.
 template <int VEC, bool SAME, int RPW, bool OPT, bool ROWS>
 __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const PsgdTile& t, const PsgdMat& mt,
                                                     int tile_rows, float* fin_smem) {
@@ -364,7 +366,7 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
   // follows has no registers left for it, and several workers do not overlap launches)
   if (SAME) load(0);
   psgd_wait_for_predecessor();
-  const bool by_rows = ROWS && (r & 3) == 0;
+  const bool by_rows = ROWS && VEC == 4 && (r & 3) == 0;
   const bool gather = !SAME && a.comm != nullptr;
   int e1 = 0;
   bool ok = true;

@@ -17,6 +17,11 @@
 // ring of three to six panels per group, so loads run ahead while a group multiplies, adds up its warps' sums
 // and finishes its rows, and rows of 650 or 27 floats are loaded as fast as any. Other groups fill the SM
 // while one waits. Multiplications are packed in pairs of columns (fma.rn.f32x2: two IEEE operations).
+// Bound by HBM and by what four warps per scheduler find to do between two barriers: 4 x 4096^2 at rank 4 x 2 takes
+// 151 us (805 MB, 5.3 TB/s) where the product (tensor cores) and the decompression took 60 + 146; the pass 421 -> 377.
+// Above eight factor columns a thread owns four or two matrix columns only, and the sums over the lanes cost as much as
+// the products (50257 x 1024 at rank 16 x 2: 75 + 186 -> 380 us); with the optimizer step, parameters and momentum would come
+// through registers between the barriers (GPT-2 medium: 284 + 1315 -> 1661 us). Both stay with the launches apart.
 #include "psgd_async.cuh"
 #include "psgd_bounds.cuh"
 
