@@ -506,7 +506,13 @@ class NativeCompressor(_Recordable):
         self._tapes.clear()
         self._key = key
 
-    PANEL_ELEMS = 1 << 20   # least size of the matrices together
+    # Where the one-pass kernel takes over: at least so many elements together, three quarters of them in matrices of
+    # 512 columns and more (a narrow matrix leaves most lanes of a group without columns). us per pass (accumulation
+    # included), one pass / launches apart, at rank 1 x 2, 4 x 2, 8 x 1: 2 x 512^2 30.8 / 30.7, 45.1 / 39.2, 32.4 / 32.8; 2 x 512x1024 31.6 / 33.8,
+    # 46.2 / 43.5, 33.8 / 34.8; 4 x 700x650 34.8 / 39.0, 47.2 / 51.2, 35.7 / 36.9; 8 x 1024^2 56 / 66, 82.0 / 82.8, 62.3 / 62.4; 3 x 4096x1024 73 / 85,
+    # 98.5 / 102, 82 / 84.7; 2 x 24000x96 49.2 / 48.8, 71.9 / 67.3, 58.8 / 55.4.
+    PANEL_ELEMS = 3 << 19
+    PANEL_WIDE = 512
 
     def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str, need_out: bool) -> None:
         """Which matrices finish a step whose last basis is on the Q side in one pass (csrc/panel.cu), and the tile
@@ -523,7 +529,9 @@ class NativeCompressor(_Recordable):
 
         groups = [self.plan.groups[gi] for gi, _pos, _idx in self.tiles.mats]
         mats = [mi for mi, (g, at) in enumerate(zip(groups, addresses)) if at % 16 == 0 and rows(g.m, g.n) > 0]
-        if sum(groups[mi].n * groups[mi].m for mi in mats) < max(1, self.PANEL_ELEMS):
+        elems = sum(groups[mi].n * groups[mi].m for mi in mats)
+        wide = sum(groups[mi].n * groups[mi].m for mi in mats if groups[mi].m >= self.PANEL_WIDE)
+        if elems < max(1, self.PANEL_ELEMS) or 4 * wide < 3 * elems:
             return
         segs, starts = self.tiles.panel_segments(mats, vec, rows)
         table = _to_device(np.concatenate([segs.view(np.uint8), starts.view(np.uint8)]), self.device)
