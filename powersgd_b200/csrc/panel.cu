@@ -391,6 +391,9 @@ __global__ void __launch_bounds__(PN_THREADS, 1) psgd_panel_kernel(const __grid_
   if (threadIdx.x < PN_MAX_GROUPS) sg.phases[threadIdx.x] = 0;
   if (threadIdx.x < 4) reinterpret_cast<float*>(pn_smem + pn_zero_off())[threadIdx.x] = 0.f;
   for (int s = first; s < end; ++s) {
+    // panels of another height or groups of another width move the rings onto bytes that the segment before wrote
+    // by ordinary stores: row values, sums, cross products
+    psgd_fence_async_shared();
     __syncwarp();
     __syncthreads();   // every group has left the segment before
     if (*(volatile int*)&sg.abort) break;

@@ -49,6 +49,10 @@ __device__ __forceinline__ void psgd_let_copies_land() {
   while (psgd_globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
 }
 
+// Ordinary stores of this thread to shared memory come before asynchronous copies into it that are issued behind a
+// later barrier. A barrier alone does not order the two.
+__device__ __forceinline__ void psgd_fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // `bytes` (a multiple of 16) of global memory into shared memory, both on 16-byte boundaries.
 __device__ __forceinline__ void psgd_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(psgd_smem_u32(dst)),

@@ -1,4 +1,6 @@
 """Segments of the one-pass kernel for the last product and the decompression (host code; needs the built library)."""
+import os
+
 import numpy as np
 import pytest
 
@@ -44,3 +46,11 @@ def test_refused_shapes():
         assert lib.psgd_panel_rows(rank, iters, m, 1000) == 0
     for rank, iters, m in [(4, 2, 4096), (2, 2, 4608), (8, 1, 4096)]:
         assert lib.psgd_panel_rows(rank, iters, m, 1000) == 4
+
+
+def test_stores_of_a_segment_are_fenced_from_the_copies_of_the_next():
+    """Where the rings begin depends on the height of a panel, so the copies of one segment may land on bytes that the
+    one before stored (tests/test_panel_gpu.py, test_segments_of_unlike_matrices): every thread has to fence."""
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "powersgd_b200", "csrc", "panel.cu")) as fp:
+        loop = fp.read().split("for (int s = first; s < end; ++s) {")[1]
+    assert 0 < loop.find("psgd_fence_async_shared();") < loop.find("__syncthreads();") < loop.find("sg.tile = a.tiles[s];")

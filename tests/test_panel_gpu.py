@@ -11,13 +11,11 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(5, 23), (70, 27), (64, 576), (129, 650), (33, 1001), (300, 1024), (41, 514), (600, 64), (2500, 24)]
 
 
-@pytest.mark.parametrize("rank,iters", [(1, 1), (1, 2), (1, 3), (1, 4), (2, 1), (2, 2), (2, 3), (2, 4), (3, 2), (4, 1), (4, 2), (5, 1), (8, 1)])
-def test_one_pass_against_float64(rank, iters, monkeypatch):
+def _check(shapes, rank, iters, monkeypatch):
     """The fresh P, the update and the residual from the factors of the launches before. P sums m products in chains of
     at most 12 and a tree of at most 10 additions, less the corrections of r products each; an update sums K
     products: off by at most that many 2^-24 of the terms' sizes (each side rounds to float32)."""
     monkeypatch.setattr(NativeCompressor, "PANEL_ELEMS", 0)
-    shapes = SHAPES + [(37, 4608 if rank * iters <= 4 else 4096)]
     gen = torch.Generator(device="cuda").manual_seed(7)
     draw = lambda s: torch.randn(s, generator=gen, device="cuda")  # noqa: E731
     params = [torch.nn.Parameter(draw(s)) for s in shapes]
@@ -49,3 +47,16 @@ def test_one_pass_against_float64(rank, iters, monkeypatch):
             bound = (r * iters + 3) * eps
             assert ((grads[idx].double().view_as(grad) - (grad - update)).abs() <= bound * (size + grad.abs())).all(), ("residual", shapes[idx])
             assert ((outs[idx].double().view_as(grad) - update).abs() <= bound * size).all(), ("update", shapes[idx])
+
+
+@pytest.mark.parametrize("rank,iters", [(1, 1), (1, 2), (1, 3), (1, 4), (2, 1), (2, 2), (2, 3), (2, 4), (3, 2), (4, 1), (4, 2), (5, 1), (8, 1)])
+def test_one_pass_against_float64(rank, iters, monkeypatch):
+    _check(SHAPES + [(37, 4608 if rank * iters <= 4 else 4096)], rank, iters, monkeypatch)
+
+
+@pytest.mark.parametrize("rank,iters", [(2, 2), (4, 2), (8, 1)])
+def test_segments_of_unlike_matrices(rank, iters, monkeypatch):
+    """Two or three segments per block, in turn of one group and four rows per panel and of eight groups and up to
+    sixteen rows: the rings begin elsewhere in each of them."""
+    wide = 4608 if rank * iters <= 4 else 4096
+    _check([s for i in range(100) for s in [(9 + i % 3, wide - i), (260 + i, 17 + i // 2)]], rank, iters, monkeypatch)
