@@ -252,8 +252,16 @@ __device__ void tk_derive_block(const int* ws, int upto, long long k, Pick* pick
   __syncthreads();
 }
 
+// Four copies of a block's histogram, by lane: the leading digit of a gradient takes a few dozen values, and
+// lanes that meet on one address are served one after another. The copies of a bin are added up by one 16-byte
+// access, so whatever holds this has to have its alignment.
+struct alignas(16) Bins {
+  int c[TK_BINS0 * 4];
+};
+
 // Histogram of digit `pass` of the entries that agree with the digits chosen so far (block-wide).
-__device__ void tk_histogram(const TopkItem& item, int part, int parts, int* ws, int pass, unsigned prefix, int* sh) {
+__device__ void tk_histogram(const TopkItem& item, int part, int parts, int* ws, int pass, unsigned prefix, Bins& shared) {
+  int* sh = shared.c;
   const int bins = pass == 2 ? TK_BINS2 : TK_BINS0;
   for (int b = threadIdx.x; b < bins * 4; b += TK_THREADS) sh[b] = 0;
   __syncthreads();
@@ -281,9 +289,7 @@ __device__ void tk_histogram(const TopkItem& item, int part, int parts, int* ws,
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                           const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                           int* __restrict__ ws_all) {
-  // four copies of the histogram, by lane: the leading digit of a gradient takes a few dozen values,
-  // and lanes that meet on one address are served one after another
-  __shared__ __align__(16) int sh[TK_BINS0 * 4];
+  __shared__ Bins sh;
   const int it = block_item[blockIdx.x];
   tk_histogram(items[it], block_part[blockIdx.x], item_parts[it], ws_all + (long long)it * TK_WS_INTS, 0, 0u, sh);
 }
@@ -317,6 +323,12 @@ __device__ void tk_hand_out(Found& f, int* counter, float* val, int* pos) {   //
   }
 }
 
+union SplitScratch {
+  Bins hist;
+  struct { Found above, inside; } found;
+};
+static_assert(alignof(SplitScratch) % alignof(int4) == 0, "tk_histogram reads its bins by 16 bytes");
+
 // Launch 2: what lies above the leading digit is taken, what lies in it is listed; or the second histogram.
 // cand_v / cand_p: lists of candidates; counters of a tensor: [0] taken, [1] equal to the threshold, [2] candidates.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
@@ -324,10 +336,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const 
                                                                            int* __restrict__ ws_all, float* __restrict__ values,
                                                                            int* __restrict__ positions, float* __restrict__ cand_v,
                                                                            int* __restrict__ cand_p) {
-  __shared__ union {
-    int hist[TK_BINS0 * 4];
-    struct { Found above, inside; } found;
-  } sh;
+  __shared__ SplitScratch sh;
   __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
   __shared__ long long remain_sh;
@@ -385,7 +394,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
                                                                             int* __restrict__ ws_all, float* __restrict__ values,
                                                                             int* __restrict__ positions, const float* __restrict__ cand_v,
                                                                             const int* __restrict__ cand_p) {
-  __shared__ __align__(16) int sh[TK_BINS0 * 4];
+  __shared__ Bins bins_sh;
   __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
   __shared__ long long remain_sh;
@@ -397,10 +406,11 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   const int n = ws[pick.prefix >> 20];
   if (n > item.cap) {
     tk_derive_block(ws, 2, item.k, &pick, &remain_sh, &bin_sh, scan);
-    tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 2, pick.prefix, sh);
+    tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 2, pick.prefix, bins_sh);
     return;
   }
   if (block_part[blockIdx.x] != 0) return;
+  int* sh = bins_sh.c;
   const float* cv = cand_v + item.cand_off;
   const int* cp = cand_p + item.cand_off;
   for (int digit = 1; digit <= 2; ++digit) {
