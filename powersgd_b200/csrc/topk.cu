@@ -301,23 +301,26 @@ struct Found {
   int p[TK_FOUND];
   int count, base;
 };
-__device__ __forceinline__ void tk_put(Found& f, int* counter, float* val, int* pos, float v, int p) {
+// `room`: entries of val / pos. A tensor has no more than that unless something writes it during the call.
+__device__ __forceinline__ void tk_put(Found& f, int* counter, float* val, int* pos, long long room, float v, int p) {
   const int slot = atomicAdd(&f.count, 1);
   if (slot < TK_FOUND) {
     f.v[slot] = v;
     f.p[slot] = p;
   } else {
     const int at = atomicAdd(counter, 1);
-    val[at] = v;
-    pos[at] = p;
+    if (at < room) {
+      val[at] = v;
+      pos[at] = p;
+    }
   }
 }
-__device__ void tk_hand_out(Found& f, int* counter, float* val, int* pos) {   // block-wide
+__device__ void tk_hand_out(Found& f, int* counter, float* val, int* pos, long long room) {   // block-wide
   __syncthreads();
   const int mine = min(f.count, TK_FOUND);
   if (threadIdx.x == 0 && mine) f.base = atomicAdd(counter, mine);
   __syncthreads();
-  for (int e = threadIdx.x; e < mine; e += TK_THREADS) {
+  for (int e = threadIdx.x; e < mine && f.base + e < room; e += TK_THREADS) {
     val[f.base + e] = f.v[e];
     pos[f.base + e] = f.p[e];
   }
@@ -367,9 +370,9 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const 
       const unsigned key = tk_key(v[j]);
       if (j < count && key >= prefix) {
         if ((key & 0x7FF00000u) == prefix) {
-          tk_put(sh.found.inside, counters + 2, cv, cp, v[j], (int)(first + j));
+          tk_put(sh.found.inside, counters + 2, cv, cp, item.cap, v[j], (int)(first + j));
         } else {
-          tk_put(sh.found.above, counters, val, pos, v[j], (int)(first + j));
+          tk_put(sh.found.above, counters, val, pos, item.k, v[j], (int)(first + j));
           rest[j] = 0.f;
         }
       }
@@ -384,8 +387,8 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const 
       }
     }
   });
-  tk_hand_out(sh.found.above, counters, val, pos);
-  tk_hand_out(sh.found.inside, counters + 2, cv, cp);
+  tk_hand_out(sh.found.above, counters, val, pos, item.k);
+  tk_hand_out(sh.found.inside, counters + 2, cv, cp, item.cap);
 }
 
 // Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram.
@@ -403,13 +406,14 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
   tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
-  const int n = ws[pick.prefix >> 20];
-  if (n > item.cap) {
+  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
+  if (ws[pick.prefix >> 20] > item.cap) {
     tk_derive_block(ws, 2, item.k, &pick, &remain_sh, &bin_sh, scan);
     tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 2, pick.prefix, bins_sh);
     return;
   }
   if (block_part[blockIdx.x] != 0) return;
+  const int n = (int)min((long long)counters[2], item.cap);   // what launch 2 has listed
   int* sh = bins_sh.c;
   const float* cv = cand_v + item.cand_off;
   const int* cp = cand_p + item.cand_off;
@@ -429,7 +433,6 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   }
   const unsigned threshold = pick.prefix;
   const long long take_equal = remain_sh, base_equal = item.k - take_equal;
-  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
   for (int e = threadIdx.x; e < n; e += TK_THREADS) {
@@ -444,6 +447,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
       if (eq >= take_equal) continue;
       slot = base_equal + eq;
     }
+    if (slot >= item.k) continue;
     val[slot] = v;
     pos[slot] = cp[e];
     if (item.memory) item.memory[cp[e]] = 0.f;
@@ -484,7 +488,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
       if (j < count && key >= threshold) {
         const int i = (int)(first + j);
         if (key > threshold) {
-          tk_put(found, counters, val, pos, v[j], i);
+          tk_put(found, counters, val, pos, item.k, v[j], i);
           rest[j] = 0.f;
         } else {
           const long long e = atomicAdd(counters + 1, 1);
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
       }
     }
   });
-  tk_hand_out(found, counters, val, pos);
+  tk_hand_out(found, counters, val, pos, item.k);
 }
 
 }  // namespace

@@ -9,6 +9,7 @@ comes from `torch.topk` (gradient_reducers.py:240-253 is the reference sequence)
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -16,7 +17,26 @@ import torch
 from . import native, scan
 from .recording import is_recorded, keep_with_graph, outside_capture, release_finished
 
-_workspaces = {}
+# Scratch (histograms, counters, lists, a barrier word) belongs to one stream, whose order keeps the calls that
+# share it apart, and the launches of a call go onto it in one piece: two streams, or two threads on one stream, that
+# share counters would hand out places beyond the end of a list. What is dropped here goes back to the
+# allocator of the same stream, behind the launches that use it.
+_launching = threading.RLock()
+MOST_STREAMS = 64
+_workspaces: dict = {}
+
+
+def _current_stream() -> ctypes.c_void_p:
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+
+
+def _of_stream(pool: dict, device: torch.device, stream: ctypes.c_void_p, make) -> torch.Tensor:
+    key = (device, stream.value)
+    if key not in pool:
+        if len(pool) >= MOST_STREAMS:
+            del pool[next(iter(pool))]
+        pool[key] = make()
+    return pool[key]
 
 
 def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -27,22 +47,21 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
         memory is None or (memory.is_contiguous() and memory.dtype == torch.float32)
     ):
         lib = native.lib()
-        stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
-        recorded = is_recorded(stream)   # a graph gets counters of its own, see topk_abs_many
-        ws = None if recorded else _workspaces.get(flat.device)
-        if ws is None:
-            ws = torch.zeros(lib.psgd_topk_workspace_ints(), dtype=torch.int32, device=flat.device)
-            if recorded:
-                keep_with_graph(None, ws)
-            else:
-                _workspaces[flat.device] = ws
+        stream = _current_stream()
+        make = lambda: torch.zeros(lib.psgd_topk_workspace_ints(), dtype=torch.int32, device=flat.device)  # noqa: E731
         values = torch.empty(k, dtype=torch.float32, device=flat.device)
         positions = torch.empty(k, dtype=torch.int32, device=flat.device)
-        code = lib.psgd_topk_abs(
-            ctypes.c_void_p(flat.data_ptr()), ctypes.c_longlong(n), ctypes.c_longlong(k), ctypes.c_void_p(ws.data_ptr()),
-            ctypes.c_void_p(values.data_ptr()), ctypes.c_void_p(positions.data_ptr()),
-            ctypes.c_void_p(0 if memory is None else memory.data_ptr()), stream,
-        )
+        with _launching:
+            if is_recorded(stream):   # a graph gets counters of its own, see topk_abs_many
+                ws = make()
+                keep_with_graph(None, ws)
+            else:
+                ws = _of_stream(_workspaces, flat.device, stream, make)
+            code = lib.psgd_topk_abs(
+                ctypes.c_void_p(flat.data_ptr()), ctypes.c_longlong(n), ctypes.c_longlong(k), ctypes.c_void_p(ws.data_ptr()),
+                ctypes.c_void_p(values.data_ptr()), ctypes.c_void_p(positions.data_ptr()),
+                ctypes.c_void_p(0 if memory is None else memory.data_ptr()), stream,
+            )
         native.check(code, "psgd_topk_abs")
         return values, positions
     _, idx = torch.topk(flat.abs(), k, sorted=False)
@@ -54,6 +73,7 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
 
 
 _many_cache: dict = {}
+MOST_LISTS = 8   # of tensors, each on one stream, whose tables are kept
 CANDIDATES = 4   # room for candidates, in multiples of the entries taken (0: none)
 
 
@@ -79,13 +99,22 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
             values[at : at + k], positions[at : at + k] = v, p
             at += k
         return values, positions
+    values = torch.empty(total, dtype=torch.float32, device=device)
+    positions = torch.empty(total, dtype=torch.int32, device=device)
+    with _launching:
+        _select(tensors, ks, mems, values, positions)
+    return values, positions
+
+
+def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) -> None:
     import numpy as np
 
     lib = native.lib()
-    key = (device, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks))
+    device = tensors[0].device
+    stream = _current_stream()
+    key = (device, stream.value, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks))
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
-    stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     recorded = is_recorded(stream)
     entry = None if recorded else _many_cache.get(key)
     if entry is None:
@@ -126,18 +155,16 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
         else:
             # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
             # valid for whatever tensors present the same addresses again, so no tensor is kept alive
-            if len(_many_cache) >= 4:
+            if len(_many_cache) >= MOST_LISTS:
                 _many_cache.clear()
             _many_cache[key] = entry
-    values = torch.empty(total, dtype=torch.float32, device=device)
-    positions = torch.empty(total, dtype=torch.int32, device=device)
     vp = ctypes.c_void_p
     code = lib.psgd_topk_abs_many(
         vp(entry["items"].data_ptr()), len(tensors), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
-        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
+        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()),
+        vp(values.data_ptr()), vp(positions.data_ptr()), stream,
     )
     native.check(code, "psgd_topk_abs_many")
-    return values, positions
 
 
 _SEG_DTYPE = None
@@ -154,63 +181,15 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
     the outputs and applies the workers in rank order (csrc/topk.cu), so replicas stay
     bit-identical; elsewhere the same sum runs as one `index_add_` per worker
     (gradient_reducers.py:262-271)."""
-    global _SEG_DTYPE
-    workers, per_worker = all_values.shape
+    workers = all_values.shape[0]
     use_native = (
         all_values.is_cuda and native.use_for_cuda() and all_values.dtype == torch.float32 and all_positions.dtype == torch.int32
         and all_values.is_contiguous() and all_positions.is_contiguous()
         and scan.usable(outs, True)
     )
     if use_native:
-        import numpy as np
-
-        lib = native.lib()
-        cap = int(lib.psgd_sparse_combine_max_segments())
-        if _SEG_DTYPE is None:
-            _SEG_DTYPE = np.dtype([("out", np.uint64), ("numel", np.int64), ("end", np.int64)])
-        device = all_values.device
-        scratch = _combine_scratch.get(device)
-        if scratch is None:
-            with outside_capture(device):
-                scratch = torch.zeros(2, dtype=torch.int32, device=device)  # [grid barrier, status]
-            _combine_scratch[device] = scratch
-        barrier = scratch
-        stream = ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
-        # tables of addresses and lengths, kept by exactly those (as the selection's above, recorded calls
-        # included): building and uploading one stalls the host until the selection has run
-        key = (device, scan.addresses(outs), scan.sizes(outs), tuple(ends))
-        recorded = is_recorded(stream)
-        tables = None if recorded else _segment_cache.get(key)
-        if tables is None:
-            release_finished()
-            tables = []
-            with outside_capture(device):
-                for first in range(0, len(outs), cap):
-                    chunk = list(range(first, min(first + cap, len(outs))))
-                    segs = np.zeros(len(chunk), dtype=_SEG_DTYPE)
-                    base = ends[first - 1] if first else 0
-                    for j, s in enumerate(chunk):
-                        segs[j] = (outs[s].data_ptr(), outs[s].numel(), ends[s] - base)
-                    tables.append((torch.from_numpy(segs.view(np.uint8)).to(device, non_blocking=False), len(chunk), base, ends[chunk[-1]] - base))
-                if recorded:
-                    barrier = torch.zeros(1, dtype=torch.int32, device=device)
-            if recorded:
-                keep_with_graph(None, tables, barrier, scratch)
-            else:
-                if len(_segment_cache) >= 4:
-                    _segment_cache.clear()
-                _segment_cache[key] = tables
-        for segs_dev, count, base, width in tables:
-            vals = all_values if (base == 0 and width == per_worker) else all_values[:, base : base + width].contiguous()
-            poss = all_positions if (base == 0 and width == per_worker) else all_positions[:, base : base + width].contiguous()
-            code = lib.psgd_sparse_combine_launch(
-                ctypes.c_void_p(vals.data_ptr()), ctypes.c_void_p(poss.data_ptr()), int(workers), ctypes.c_longlong(width),
-                ctypes.c_void_p(segs_dev.data_ptr()), count, ctypes.c_float(divisor),
-                ctypes.c_void_p(barrier.data_ptr()), ctypes.c_void_p(scratch.data_ptr() + 4), stream,
-            )
-            native.check(code, "psgd_sparse_combine_launch")
-            if not recorded:
-                segs_dev.record_stream(torch.cuda.current_stream())
+        with _launching:
+            _combine(all_values, all_positions, outs, ends, divisor)
         return
     start = 0
     for out, end in zip(outs, ends):
@@ -221,7 +200,61 @@ def sparse_combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, 
         start = end
 
 
+def _combine(all_values: torch.Tensor, all_positions: torch.Tensor, outs, ends, divisor: float) -> None:
+    global _SEG_DTYPE
+    import numpy as np
+
+    workers, per_worker = all_values.shape
+    lib = native.lib()
+    cap = int(lib.psgd_sparse_combine_max_segments())
+    if _SEG_DTYPE is None:
+        _SEG_DTYPE = np.dtype([("out", np.uint64), ("numel", np.int64), ("end", np.int64)])
+    device = all_values.device
+    stream = _current_stream()
+
+    def words() -> torch.Tensor:   # [grid barrier, status]
+        with outside_capture(device):
+            return torch.zeros(2, dtype=torch.int32, device=device)
+
+    scratch = _of_stream(_combine_scratch, device, stream, words)
+    barrier = scratch
+    # tables of addresses and lengths, kept by exactly those (as the selection's above, recorded calls
+    # included): building and uploading one stalls the host until the selection has run
+    key = (device, scan.addresses(outs), scan.sizes(outs), tuple(ends))
+    recorded = is_recorded(stream)
+    tables = None if recorded else _segment_cache.get(key)
+    if tables is None:
+        release_finished()
+        tables = []
+        with outside_capture(device):
+            for first in range(0, len(outs), cap):
+                chunk = list(range(first, min(first + cap, len(outs))))
+                segs = np.zeros(len(chunk), dtype=_SEG_DTYPE)
+                base = ends[first - 1] if first else 0
+                for j, s in enumerate(chunk):
+                    segs[j] = (outs[s].data_ptr(), outs[s].numel(), ends[s] - base)
+                tables.append((torch.from_numpy(segs.view(np.uint8)).to(device, non_blocking=False), len(chunk), base, ends[chunk[-1]] - base))
+            if recorded:
+                barrier = torch.zeros(1, dtype=torch.int32, device=device)
+        if recorded:
+            keep_with_graph(None, tables, barrier, scratch)
+        else:
+            if len(_segment_cache) >= 4:
+                _segment_cache.clear()
+            _segment_cache[key] = tables
+    for segs_dev, count, base, width in tables:
+        vals = all_values if (base == 0 and width == per_worker) else all_values[:, base : base + width].contiguous()
+        poss = all_positions if (base == 0 and width == per_worker) else all_positions[:, base : base + width].contiguous()
+        code = lib.psgd_sparse_combine_launch(
+            ctypes.c_void_p(vals.data_ptr()), ctypes.c_void_p(poss.data_ptr()), int(workers), ctypes.c_longlong(width),
+            ctypes.c_void_p(segs_dev.data_ptr()), count, ctypes.c_float(divisor),
+            ctypes.c_void_p(barrier.data_ptr()), ctypes.c_void_p(scratch.data_ptr() + 4), stream,
+        )
+        native.check(code, "psgd_sparse_combine_launch")
+        if not recorded:
+            segs_dev.record_stream(torch.cuda.current_stream())
+
+
 def sparse_combine_status(device) -> int:
-    """0 unless a grid barrier of `sparse_combine` gave up on `device` (reads the device word: synchronises)."""
-    scratch = _combine_scratch.get(torch.device(device))
-    return 0 if scratch is None else int(scratch[1].item())
+    """0 unless a grid barrier of `sparse_combine` gave up on `device` (reads the device words: synchronises)."""
+    return max((int(words[1].item()) for (of, _stream), words in list(_combine_scratch.items()) if of == torch.device(device)), default=0)

@@ -1,4 +1,6 @@
 """The batched selection where its candidate lists suffice, where they do not, and where there are none."""
+import threading
+
 import pytest
 import torch
 
@@ -44,3 +46,59 @@ def test_selection(room, memory, monkeypatch):
             rest = x.clone()
             rest[p] = 0.0
             assert torch.equal(mems[i], rest), i
+
+
+def test_streams_and_threads_do_not_share_scratch():
+    """The same tensors selected from on two streams, by two threads each, while the others are under way."""
+    dev = torch.device("cuda:0")
+    topk._many_cache.clear()
+    tensors, ks = map(list, zip(*_tensors(dev)))
+    want = [torch.topk(x.abs(), k).values for x, k in zip(tensors, ks)]
+    torch.cuda.synchronize()
+    streams, wrong = [torch.cuda.Stream(), torch.cuda.Stream()], []
+
+    def work(stream):
+        try:
+            with torch.cuda.stream(stream):
+                seen = []
+                for _ in range(40):
+                    values, positions = topk.topk_abs_many(tensors, ks)
+                    one, _ = topk.topk_abs(tensors[1], ks[1])
+                    seen.append((values, positions, one))
+                stream.synchronize()
+                for values, positions, one in seen:
+                    at = 0
+                    for x, k, w in zip(tensors, ks, want):
+                        v, p = values[at : at + k], positions[at : at + k].long()
+                        at += k
+                        if not (torch.equal(v, x[p]) and torch.equal(v.abs().sort(descending=True).values, w)):
+                            wrong.append((x.numel(), k))
+                    if not torch.equal(one.abs().sort(descending=True).values, want[1]):
+                        wrong.append("one tensor")
+        except Exception as error:
+            wrong.append(error)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in streams * 2]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:3]
+    assert len({entry["ws"].data_ptr() for entry in topk._many_cache.values()}) == 2
+    topk._many_cache.clear()
+
+
+def test_combining_on_two_streams_does_not_share_a_barrier():
+    dev = torch.device("cuda:0")
+    x = torch.randn(5000, device=dev)
+    values, positions = topk.topk_abs(x, 50)
+    want = torch.zeros_like(x)
+    want[positions.long()] = values
+    for stream in (torch.cuda.Stream(), torch.cuda.Stream()):   # one after the other
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            out = torch.full_like(x, 7.0)
+            topk.sparse_combine(values.view(1, -1), positions.view(1, -1), [out], [50], 1.0)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and topk._combine_scratch[dev, stream.cuda_stream][1].item() == 0
+    assert topk.sparse_combine_status(dev) == 0
