@@ -136,12 +136,13 @@ PSGD_API int psgd_topk_abs(const float* x, long long n, long long k, int* worksp
 //   2. every entry above the chosen digit is taken, every entry inside it becomes a candidate (a list of up to
 //      `cap` per tensor), and `memory` is written: one read and one write;
 //   3. one block per tensor finds the threshold among its candidates and takes those above it.
-// A tensor with more candidates than its list holds (many entries of nearly equal size) goes the long way
-// instead: histograms of the second and the third digit over all entries in launches 2 and 3, and a
-// compaction pass in launch 4, which has nothing to do for the others.
+// A tensor with more candidates than its list holds (many entries of nearly equal size, or a large k) goes the long
+// way instead: histograms of the second and the third digit over all entries in launches 2 and 3, and a
+// compaction pass in launch 4, which has nothing to do for the others. How long a list one block should walk: ops/topk.py.
 // Bound by the reads (L2 for a model of this size) and by what a block costs besides them, so some four blocks
-// per SM serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: three histogram passes of 14.2 us and a
-// compaction of 23.9 before (67 us); 14.8, 21.6, 14.5 and 6.0 (57 us) now.
+// per SM serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: 68 us by three histogram passes and a
+// compaction, 54 us by lists; launch 3 took 14.5 us of it while a thread had one load of its list under way and the
+// entries that it takes were counted in global memory (the pass of the reducer 88.6 us then, 86.0 now).
 namespace {
 
 struct TopkItem {
@@ -225,25 +226,27 @@ __device__ __forceinline__ void tk_for_each(const float* __restrict__ x, long lo
   }
 }
 
-// Digits chosen so far for one tensor (block-wide; result in shared `pick`).
-__device__ void tk_derive_block(const int* ws, int upto, long long k, Pick* pick, long long* remain_sh, int* bin_sh, int* scan) {
+// Digits `from` to `upto` - 1 of one tensor's threshold (block-wide; result in shared `pick`, which has those before).
+__device__ void tk_derive_block(const int* ws, int from, int upto, long long k, Pick* pick, long long* remain_sh, int* bin_sh, int* scan) {
   if (threadIdx.x == 0) {
-    pick->prefix = 0u;
-    *remain_sh = k;
+    if (from == 0) {
+      pick->prefix = 0u;
+      *remain_sh = k;
+    }
     *bin_sh = 0;
   }
   __syncthreads();
-  if (upto >= 1) {
+  if (from < 1 && upto >= 1) {
     tk_choose_block(ws, TK_BINS0, remain_sh, bin_sh, scan);
     if (threadIdx.x == 0) pick->prefix |= (unsigned)(*bin_sh) << 20;
     __syncthreads();
   }
-  if (upto >= 2) {
+  if (from < 2 && upto >= 2) {
     tk_choose_block(ws + TK_BINS0, TK_BINS1, remain_sh, bin_sh, scan);
     if (threadIdx.x == 0) pick->prefix |= (unsigned)(*bin_sh) << 9;
     __syncthreads();
   }
-  if (upto >= 3) {
+  if (from < 3 && upto >= 3) {
     tk_choose_block(ws + TK_BINS0 + TK_BINS1, TK_BINS2, remain_sh, bin_sh, scan);
     if (threadIdx.x == 0) pick->prefix |= (unsigned)(*bin_sh);
     __syncthreads();
@@ -347,7 +350,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const 
   const int it = block_item[blockIdx.x];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
-  tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
+  tk_derive_block(ws, 0, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned prefix = pick.prefix;
   if (ws[prefix >> 20] > item.cap) {
     tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 1, prefix, sh.hist);
@@ -391,6 +394,21 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const 
   tk_hand_out(sh.found.inside, counters + 2, cv, cp, item.cap);
 }
 
+// f(value, index) for every entry of a list (block-wide), eight loads of a thread under way: one block walks a list
+// alone, so nothing else hides the latency of L2.
+template <class F>
+__device__ __forceinline__ void tk_walk(const float* __restrict__ list, int n, F f) {
+  for (int first = threadIdx.x; first < n; first += 8 * TK_THREADS) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (first + u * TK_THREADS < n) v[u] = list[first + u * TK_THREADS];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (first + u * TK_THREADS < n) f(v[u], first + u * TK_THREADS);
+  }
+}
+
 // Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                             const int* __restrict__ block_part, const int* __restrict__ item_parts,
@@ -401,14 +419,14 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
   __shared__ long long remain_sh;
-  __shared__ int bin_sh;
+  __shared__ int bin_sh, above_sh, equal_sh;
   const int it = block_item[blockIdx.x];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
-  tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
+  tk_derive_block(ws, 0, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
   int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
   if (ws[pick.prefix >> 20] > item.cap) {
-    tk_derive_block(ws, 2, item.k, &pick, &remain_sh, &bin_sh, scan);
+    tk_derive_block(ws, 1, 2, item.k, &pick, &remain_sh, &bin_sh, scan);
     tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 2, pick.prefix, bins_sh);
     return;
   }
@@ -422,10 +440,10 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
     const unsigned mask = digit == 2 ? 0x7FFFFE00u : 0x7FF00000u, prefix = pick.prefix;
     for (int b = threadIdx.x; b < bins; b += TK_THREADS) sh[b] = 0;
     __syncthreads();
-    for (int e = threadIdx.x; e < n; e += TK_THREADS) {
-      const unsigned key = tk_key(cv[e]);
+    tk_walk(cv, n, [&](float v, int) {
+      const unsigned key = tk_key(v);
       if ((key & mask) == prefix) atomicAdd(sh + ((key >> shift) & (unsigned)(bins - 1)), 1);
-    }
+    });
     __syncthreads();
     tk_choose_block(sh, bins, &remain_sh, &bin_sh, scan);
     if (threadIdx.x == 0) pick.prefix = prefix | ((unsigned)bin_sh << shift);
@@ -435,23 +453,28 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   const long long take_equal = remain_sh, base_equal = item.k - take_equal;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
-  for (int e = threadIdx.x; e < n; e += TK_THREADS) {
-    const float v = cv[e];
+  if (threadIdx.x == 0) {   // nobody else takes entries of this tensor any more
+    above_sh = counters[0];
+    equal_sh = 0;
+  }
+  __syncthreads();
+  tk_walk(cv, n, [&](float v, int e) {
     const unsigned key = tk_key(v);
-    if (key < threshold) continue;
+    if (key < threshold) return;
     long long slot;
     if (key > threshold) {
-      slot = atomicAdd(counters, 1);
+      slot = atomicAdd(&above_sh, 1);
     } else {
-      const long long eq = atomicAdd(counters + 1, 1);
-      if (eq >= take_equal) continue;
+      const long long eq = atomicAdd(&equal_sh, 1);
+      if (eq >= take_equal) return;
       slot = base_equal + eq;
     }
-    if (slot >= item.k) continue;
+    if (slot >= item.k) return;
+    const int p = cp[e];
     val[slot] = v;
-    pos[slot] = cp[e];
-    if (item.memory) item.memory[cp[e]] = 0.f;
-  }
+    pos[slot] = p;
+    if (item.memory) item.memory[p] = 0.f;
+  });
 }
 
 // Launch 4: takes the k entries of a tensor with too many candidates.
@@ -468,10 +491,10 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
   int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
-  tk_derive_block(ws, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
+  tk_derive_block(ws, 0, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
   if (ws[pick.prefix >> 20] <= item.cap) return;   // launch 3 took the rest
   if (threadIdx.x == 0) found.count = 0;
-  tk_derive_block(ws, 3, item.k, &pick, &remain_sh, &bin_sh, scan);
+  tk_derive_block(ws, 1, 3, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned threshold = pick.prefix;
   const long long take_equal = pick.remain;
   const long long base_equal = item.k - take_equal;

@@ -74,7 +74,7 @@ def topk_abs(x: torch.Tensor, k: int, memory: Optional[torch.Tensor] = None) -> 
 
 _many_cache: dict = {}
 MOST_LISTS = 8   # of tensors, each on one stream, whose tables are kept
-CANDIDATES = 4   # room for candidates, in multiples of the entries taken (0: none)
+CANDIDATES = 2048   # room for candidates per tensor, besides what the length of the list allows (0: none)
 
 
 def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -130,9 +130,13 @@ def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) ->
             n = t.numel()
             if not (0 < k <= n < (1 << 31)):
                 raise ValueError(f"topk_abs_many: need 0 < k <= n < 2^31 (k = {k}, n = {n})")
-            # candidates: entries that agree with the threshold in their leading 11 bits (an eighth of an octave); some
-            # two k of a normal distribution's tail. A tensor with more goes the long way
-            cap = min(n, CANDIDATES * k + n // 16 + 1024) if CANDIDATES else 0
+            # candidates: entries that agree with the threshold in their leading 11 bits (an eighth of an octave), some
+            # 0.75 k in a normal distribution's tail. One block walks a tensor's list, 1.2 us per 1000 entries; a tensor with
+            # more of them than that goes the long way, some 1.2 us per million entries of the whole list of tensors.
+            # Room for half of what would break even. us per replayed call, long way / lists: 1 M, 1 700 candidates 25 / 25,
+            # 12 600 26 / 38; 4 M, 3 800 43 / 38, 27 000 45 / 63; 16 M, 15 000 75 / 77, 820 000 (uniform) 76 / 849; 50 M, 47 000
+            # 203 / 197, 81 000 203 / 238; 62 tensors of 11 M, 3 900 in the largest 68 / 54, 33 000 73 / 91
+            cap = min(n, CANDIDATES + total_n // 2048) if CANDIDATES else 0
             items[i] = (t.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at, room, cap)
             at, room = at + k, room + cap
             # blocks of 512 threads with at least 16 elements each, some four per SM for the whole list:

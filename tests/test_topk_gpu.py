@@ -102,3 +102,24 @@ def test_combining_on_two_streams_does_not_share_a_barrier():
         torch.cuda.synchronize()
         assert torch.equal(out, want) and topk._combine_scratch[dev, stream.cuda_stream][1].item() == 0
     assert topk.sparse_combine_status(dev) == 0
+
+
+@pytest.mark.parametrize("beyond", [0, 1, 100_000])
+def test_a_list_longer_than_one_block_walks_goes_the_long_way(beyond):
+    """Entries in the threshold's eighth of an octave: as many as the list of a tensor of 1 M entries holds, or more."""
+    dev = torch.device("cuda:0")
+    topk._many_cache.clear()
+    g = torch.Generator(device=dev).manual_seed(3)
+    n, room = 1 << 20, topk.CANDIDATES + 512
+    x = torch.rand(n, generator=g, device=dev) * 0.5
+    at = torch.randperm(n, generator=g, device=dev)[: room + beyond]
+    x[at] = 1.0 + 0.124 * torch.rand(len(at), generator=g, device=dev)
+    memory = torch.full_like(x, 7.0)
+    values, positions = topk.topk_abs_many([x], [2000], [memory])
+    p = positions.long()
+    assert torch.equal(values.sort(descending=True).values, torch.topk(x, 2000).values) and torch.equal(values, x[p])
+    assert torch.equal(memory, x.index_fill(0, p, 0.0))
+    (entry,) = topk._many_cache.values()
+    listed = int(entry["ws"][2048 + 2048 + 512 + 2])
+    assert entry["cand_v"].numel() == room and listed == (0 if beyond else room)
+    topk._many_cache.clear()
