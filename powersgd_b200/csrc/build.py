@@ -21,6 +21,7 @@ OBJ_DIR = os.path.join(HERE, "build")
 # record violations instead of accessing memory; loaded through PSGD_B200_LIB by the checked tests
 DEBUG_LIB = os.path.join(HERE, "libpsgd_b200_debug.so")
 DEBUG_OBJ_DIR = os.path.join(HERE, "build_debug")
+SCAN_LIB = os.path.join(HERE, "_tensor_scan.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden", "--use_fast_math=false"]
 
@@ -63,24 +64,35 @@ def _compile_one(nvcc: str, src: str, verbose: bool, debug: bool = False) -> str
     return obj
 
 
+def scan_target() -> str:
+    """What the list checks are compiled for. They have PyTorch's tensor layout compiled in, so another build of
+    it must not load them, whether or not it has the symbols that they ask for."""
+    import platform
+
+    import torch
+
+    return f"torch {torch.__version__} {torch.version.git_version}, python {platform.python_version()}"
+
+
 def _build_scan() -> None:
     """The list checks (host/tensor_scan.cpp), a CPython extension for the PyTorch of this interpreter. Without
     PyTorch's headers the package asks in Python."""
-    src, out = os.path.join(HERE, "host", "tensor_scan.cpp"), os.path.join(HERE, "_tensor_scan.so")
+    src = os.path.join(HERE, "host", "tensor_scan.cpp")
     import sysconfig
 
     import torch
 
     stamp_path = os.path.join(OBJ_DIR, "scan_stamp.txt")
-    stamp = f"{_digest([src])} {torch.__version__} {sys.version}"
-    if os.path.exists(out) and os.path.exists(stamp_path):
+    stamp = f"{_digest([src])} {scan_target()}"
+    if os.path.exists(SCAN_LIB) and os.path.exists(stamp_path):
         with open(stamp_path) as fp:
             if fp.read() == stamp:
                 return
     base = os.path.dirname(os.path.abspath(torch.__file__))
     includes = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-isystem{i}" for i in includes], src, "-o", out,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DPSGD_SCAN_TARGET="{scan_target()}"',
+           *[f"-isystem{i}" for i in includes], src, "-o", SCAN_LIB,
            f"-L{os.path.join(base, 'lib')}", "-lc10", "-ltorch_cpu", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

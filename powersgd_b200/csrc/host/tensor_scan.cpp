@@ -190,4 +190,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_tensor_scan", nullptr, -1, method
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__tensor_scan() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__tensor_scan() {
+  PyObject* m = PyModule_Create(&module);
+  // what this was compiled for, which the loader compares (csrc/build.py, scan_target)
+  if (m != nullptr && PyModule_AddStringConstant(m, "target", PSGD_SCAN_TARGET) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

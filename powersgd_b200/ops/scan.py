@@ -9,20 +9,21 @@ from typing import Optional, Sequence
 import numpy as np
 import torch
 
+from ..csrc.build import SCAN_LIB, scan_target
 from ..utils import is_dense, same_layout
 
 
-def _load():
-    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "_tensor_scan.so")
+def _load(path: str = SCAN_LIB):
+    """The extension at `path`; None where there is none or it was compiled for another PyTorch or Python."""
     if not os.path.exists(path):
         return None
     try:
         spec = importlib.util.spec_from_file_location("_tensor_scan", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
-        return module
-    except ImportError:   # built against another PyTorch or Python
+    except ImportError:   # symbols that are not there
         return None
+    return module if getattr(module, "target", None) == scan_target() else None
 
 
 _native = _load()

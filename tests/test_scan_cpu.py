@@ -87,3 +87,15 @@ def test_optimizers(what, monkeypatch):
     monkeypatch.setattr(scan, "_native", None)
     assert here == scan.step_fits(opt)
     assert keys is None or keys == scan.grad_addresses(params)
+
+
+@pytest.mark.parametrize("target,taken", [("scan_target()", True), ("scan_target() + '0'", False), ("'torch 2.6.0, python 3.11.0'", False), (None, False)])
+def test_an_extension_for_another_pytorch_is_left_alone(target, taken, tmp_path):
+    path = tmp_path / "_tensor_scan.py"
+    path.write_text("from powersgd_b200.csrc.build import scan_target\n" + (f"target = {target}\n" if target else ""))
+    assert (scan._load(str(path)) is not None) == taken
+
+
+@native
+def test_the_extension_of_this_tree_says_what_it_was_compiled_for():
+    assert scan._load(str(scan.SCAN_LIB)).target == scan.scan_target()
