@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import warnings
 from typing import List
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -75,8 +76,7 @@ def scan_target() -> str:
 
 
 def _build_scan() -> None:
-    """The list checks (host/tensor_scan.cpp), a CPython extension for the PyTorch of this interpreter. Without
-    PyTorch's headers the package asks in Python."""
+    """The list checks (host/tensor_scan.cpp), a CPython extension for the PyTorch of this interpreter."""
     src = os.path.join(HERE, "host", "tensor_scan.cpp")
     import sysconfig
 
@@ -104,7 +104,12 @@ def _build_scan() -> None:
 def build(force: bool = False, verbose: bool = False, debug: bool = False) -> str:
     """`debug=True` builds the bounds-checked variant (libpsgd_b200_debug.so) instead."""
     os.makedirs(OBJ_DIR, exist_ok=True)
-    _build_scan()
+    try:
+        _build_scan()
+    except Exception as exc:   # no PyTorch, headers of Python or host compiler: the package asks in Python instead, more slowly
+        if os.path.exists(SCAN_LIB):
+            os.remove(SCAN_LIB)
+        warnings.warn(f"list checks not built ({exc})", stacklevel=2)
     srcs = sources()
     headers = [os.path.join(HERE, f) for f in os.listdir(HERE) if f.endswith((".h", ".cuh"))]
     obj_dir, lib = (DEBUG_OBJ_DIR, DEBUG_LIB) if debug else (OBJ_DIR, LIB)
