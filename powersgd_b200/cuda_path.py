@@ -413,9 +413,11 @@ class NativeCompressor(_Recordable):
         hyper_index: Optional[Sequence[int]] = None,
         need_out: bool = True,
         outs: Optional[Sequence[torch.Tensor]] = None,
+        finish: bool = False,
     ) -> None:
         """`outs`: caller-owned tensors (laid out like the gradients) that receive the averaged
-        update instead of this object's own arena."""
+        update instead of this object's own arena. `finish`: the caller's steps may end in the one-pass
+        kernel (see `_half_iterations`); an object is always bound with the same."""
         key = (scan.addresses(grads), scan.addresses(params), scan.addresses(moms), need_out, scan.addresses(outs))
         if key == self._key:
             return
@@ -496,7 +498,9 @@ class NativeCompressor(_Recordable):
             self._tiles_dev[name] = {
                 v: (_to_device(a, self.device) if len(a) else None, len(a)) for v, a in by_vec.items()
             }
-        self._plan_panels(vec, [grads[idx].data_ptr() for _gi, _pos, idx in self.tiles.mats], mode, need_out)
+        self._panel = None
+        if finish:
+            self._plan_panels(vec, [grads[idx].data_ptr() for _gi, _pos, idx in self.tiles.mats], mode)
         self._split_tile_lists()
         self._partial = torch.empty(self.tiles.partial_floats, device=self.device, dtype=torch.float32)
         self._partial_tc = torch.empty(self.tiles.partial_tc_floats, device=self.device, dtype=torch.float32)
@@ -514,11 +518,10 @@ class NativeCompressor(_Recordable):
     PANEL_ELEMS = 3 << 19
     PANEL_WIDE = 512
 
-    def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str, need_out: bool) -> None:
+    def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str) -> None:
         """Which matrices finish a step whose last basis is on the Q side in one pass (csrc/panel.cu), and the tile
         lists of the others. One worker, no optimizer step, no product kernel asked for by name."""
-        self._panel = None
-        if not need_out or world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok or self.tiles.total_elems < self.PANEL_ELEMS:
+        if world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok or self.tiles.total_elems < self.PANEL_ELEMS:
             return
         known: Dict[Tuple[int, int], int] = {}
 
@@ -930,7 +933,7 @@ class NativeCompressor(_Recordable):
     def aggregate(self, gradients: List[torch.Tensor]) -> List[torch.Tensor]:
         self.check()
         self.launches = self._early_launches if self._early is not None else 0
-        self._bind(gradients)
+        self._bind(gradients, finish=True)
         self._taped((self._first_left(), False), lambda: self._step(fused_sgd=False))
         return list(self._out_views)
 

@@ -60,3 +60,13 @@ def test_segments_of_unlike_matrices(rank, iters, monkeypatch):
     sixteen rows: the rings begin elsewhere in each of them."""
     wide = 4608 if rank * iters <= 4 else 4096
     _check([s for i in range(100) for s in [(9 + i % 3, wide - i), (260 + i, 17 + i // 2)]], rank, iters, monkeypatch)
+
+
+def test_callers_that_never_finish_in_one_pass_plan_none(monkeypatch):
+    from powersgd_b200.paper.reducers import RankKReducer
+
+    monkeypatch.setattr(NativeCompressor, "PANEL_ELEMS", 0)
+    send = [torch.randn(600, 1024, device="cuda"), torch.randn(64, 576, device="cuda")]
+    reducer = RankKReducer(0, send[0].device, reuse_query=True, rank=2)
+    reducer.reduce(send, [torch.empty_like(x) for x in send], [torch.empty_like(x) for x in send])
+    assert reducer._native.comp._panel is None
