@@ -145,9 +145,9 @@ class TilePlan:
             g = self.plan.groups[gi]
             v = int(vec_widths[mi])
             if tc_flags[mi] and self.fin_tc_ok:
-                fin["tc"].append(self._grid(mi, g.n, 128, g.m, 64, v))
+                fin["tc"].append((mi, g.n, 128, g.m, 64, v))
             else:
-                fin["f"].append(self._grid(mi, g.n, self.fin_rows, g.m, 128, v))
+                fin["f"].append((mi, g.n, self.fin_rows, g.m, 128, v))
             if tc_flags[mi]:
                 row_blocks = _split_even(g.n, tc_k_nt, 32)
                 for c0 in range(0, g.m, 128):
@@ -186,17 +186,25 @@ class TilePlan:
         return {
             "nt": {k: arr(v) for k, v in nt.items()},
             "nn": {k: arr(v) for k, v in nn.items()},
-            "fin": {k: np.concatenate(v) if v else arr(v) for k, v in fin.items()},
+            "fin": {k: self._grids(v) if v else arr(v) for k, v in fin.items()},
         }
 
     @staticmethod
-    def _grid(mi: int, n: int, rows: int, m: int, cols: int, vec: int) -> np.ndarray:
-        """Tiles of rows x cols over an n x m matrix, row by row."""
-        r0, c0 = (x.ravel() for x in np.meshgrid(np.arange(0, n, rows), np.arange(0, m, cols), indexing="ij"))
-        tiles = np.zeros(len(r0), dtype=layout.TILE_DTYPE)
-        tiles["mat"], tiles["row0"], tiles["rows"] = mi, r0, np.minimum(rows, n - r0)
-        tiles["col0"], tiles["cols"], tiles["nsplit"], tiles["vec"] = c0, np.minimum(cols, m - c0), 1, vec
-        return tiles
+    def _grids(matrices: Sequence[Tuple[int, int, int, int, int, int]]) -> np.ndarray:
+        """Tiles of `rows` x `cols` over every (index, n, rows, m, cols, access width) of a list, row by row. All matrices
+        at once, since an array operation costs as much as building some ten tiles one by one."""
+        mat, n, rows, m, cols, vec = np.array(matrices, dtype=np.int32).reshape(-1, 6).T
+        across = -(-m // cols)
+        count = -(-n // rows) * across
+        of = np.repeat(np.arange(len(count)), count)
+        at = np.arange(len(of), dtype=np.int32) - (np.cumsum(count) - count)[of]
+        down, right = np.divmod(at, across[of])
+        row0, col0 = down * rows[of], right * cols[of]
+        tiles = np.zeros((len(of), layout.TILE_DTYPE.itemsize // 4), dtype=np.int32)
+        for name, values in (("mat", mat[of]), ("row0", row0), ("rows", np.minimum(rows[of], n[of] - row0)), ("col0", col0),
+                             ("cols", np.minimum(cols[of], m[of] - col0)), ("nsplit", 1), ("vec", vec[of])):
+            tiles[:, layout.TILE_DTYPE.fields[name][1] // 4] = values
+        return tiles.view(layout.TILE_DTYPE).reshape(-1)
 
     def _nt_tile_rows(self, n: int) -> int:
         # tall matrices: never more than 160 partial tiles per column block (the kernel walks a tile that is
