@@ -464,6 +464,43 @@ PSGD_API int psgd_panel_rows(int max_r, int nhist, int m, int rows) {
   return n;
 }
 
+// Shares of the CTAs, in quads of rows and in the order of the matrices: matrix i has quads[i] of them, each of
+// which costs quad_cost[i], and a CTA that goes on to another matrix pays `start`. bounds[c] .. bounds[c + 1] (counted
+// over all matrices) is what CTA c gets. The dearest CTA is as cheap as it can be, up to a quad: shares are found in
+// fractions and rounded, so that neighbours differ by a quad here and there. Whole quads to the same limit are some per cent
+// slower from HBM (4 x 4096^2 377 -> 384 us, 4 x 2048^2 at rank 4 x 2 116 -> 124): all CTAs then read at one stride. Host code.
+PSGD_API void psgd_panel_shares(const long long* quads, const long long* quad_cost, int nmats, long long start, int ctas, long long* bounds) {
+  const auto fill = [&](double limit) {   // does it all fit when no CTA costs more?
+    int mat = 0;
+    double taken = 0;      // of this matrix
+    long long before = 0;  // quads of the matrices before
+    for (int c = 0; c < ctas; ++c) {
+      bounds[c] = before + (long long)(taken + 0.5);
+      double left = limit;
+      for (bool first = true; mat < nmats; first = false) {
+        if (!first) left -= (double)start;
+        const double fits = left / (double)quad_cost[mat], rest = (double)quads[mat] - taken;
+        if (fits < rest) {
+          if (first || fits >= 1) taken += fits;   // less of another matrix is not worth its start
+          break;
+        }
+        left -= rest * (double)quad_cost[mat];
+        before += quads[mat++];
+        taken = 0;
+      }
+    }
+    bounds[ctas] = before;
+    return mat == nmats;
+  };
+  double low = 0, high = 1;   // too little, enough
+  for (int i = 0; i < nmats; ++i) high += (double)start + (double)quads[i] * (double)quad_cost[i];
+  for (int step = 0; step < 60 && high - low > 1; ++step) {
+    const double limit = 0.5 * (low + high);
+    (fill(limit) ? high : low) = limit;
+  }
+  fill(high);
+}
+
 // The last half-iteration of a step (basis `in` on the Q side) with the decompression; one worker, no optimizer step. nhist:
 // half-iterations of the step; lprev / rprev / cmat: the nhist - 1 earlier factor pairs and their cross products with `in`. tiles:
 // segments with `split` = psgd_panel_rows(...) rows per panel, row0 a multiple of four, matrices on a 16-byte

@@ -105,7 +105,7 @@ class TilePlan:
     """Static tile lists (independent of tensor addresses) for one CompressionPlan."""
 
     def __init__(self, plan, lib):
-        self.plan = plan
+        self.plan, self._lib = plan, lib
         mats = []  # (group index, position, compressed-list index)
         for gi, g in enumerate(plan.groups):
             for pos, idx in enumerate(g.members):
@@ -259,18 +259,58 @@ class TilePlan:
                 best, best_score = k, score
         return best
 
-    def panel_segments(self, mats: Sequence[int], vec_widths: Sequence[int], rows_per_panel) -> Tuple[np.ndarray, np.ndarray]:
+    # What the one-pass kernel takes for a segment besides the bytes of its rows, in elements (some 3 per ns and CTA): its
+    # first loads, and the factor values of its columns. A row of few columns costs as much as one of 192, of 256 or 384
+    # where accesses take 8 or 4 bytes: a group's threads go through all columns they might have. Shares by elements
+    # alone left some CTAs with most of the segments: 8 x 1024^2 + 20 x 64^2 at rank 4 x 2 175 us per pass, 78 now, 84 by the
+    # launches apart; ResNet-18 at 2 x 2 92, 82 and 84; 3 x 512x1024 at 2 x 2 43, 39 and 41.
+    PANEL_START = (6144, 2304)   # and so many per factor column
+    PANEL_ROW = {4: 192, 2: 256, 1: 384}
+
+    def panel_costs(self, mats: Sequence[int], vec_widths: Sequence[int], columns: int) -> Tuple[np.ndarray, int]:
+        """(what a row of each of the matrices costs at least, what a segment costs besides its rows) at so many factor columns."""
+        return np.array([self.PANEL_ROW[int(vec_widths[mi])] for mi in mats]), self.PANEL_START[0] + self.PANEL_START[1] * columns
+
+    def panel_pays(self, mats: Sequence[int], vec_widths: Sequence[int], columns: int, tc_flags: Sequence[bool], least: int) -> bool:
+        """Is one pass over the matrices `mats` (and the launches apart for what is left) faster than the launches apart for
+        all? `least`: elements that it needs in the best case. Measured as us per pass, accumulation included, launches apart /
+        one pass, at rank 1 x 2, 2 x 2, 4 x 2, 8 x 1 (an odd number of half-iterations: per two passes, one of which ends on the
+        Q side); over 90 random lists at 4 settings each it is on for half of them and 7 % faster there."""
+        groups = [self.plan.groups[self.mats[mi][0]] for mi in mats]
+        n, m = np.array([g.n for g in groups], dtype=np.int64), np.array([g.m for g in groups], dtype=np.int64)
+        elems = int((n * m).sum())
+        # Starts and narrow rows may cost an eighth: 320 x 64x640 (a quarter to a half) 142 / 136, 144 / 144, 164 / 167, 322 / 325;
+        # 64 x 128x1024 (8, 12, 19 %) 65 / 58, 70 / 64, 82 / 79, 132 / 131; 4 x 24000x96 (double) 82 / 81, 90 / 95, 103 / 112, 175 / 184.
+        # Starts of up to 16 rows are exempt, and elements of up to 8 rows count twice below: the launches apart pay as much for
+        # tiles that are mostly empty (100 x 4x4096 67 / 46, 68 / 50, 99 / 78, 103 / 87).
+        row, start = self.panel_costs(mats, vec_widths, columns)
+        if 8 * int((n * np.maximum(m, row) + start * (n > 16)).sum()) > 9 * elems:
+            return False
+        tc_wide = int((n * m)[np.array([bool(tc_flags[mi]) for mi in mats]) & (m > 1024)].sum())
+        if len(mats) < len(self.mats):
+            # two more launches that fill the GPU badly: 8 x 2048^2 + 512x5000 227 / 236 ... 392 / 440, 4 x 4096^2 + 64x7000
+            # 413 / 375 ... 718 / 690, + 512x7000 423 / 432 ... 728 / 750; 12 x 4096^2 + 512x7000 1127 / 1043 ... 1950 / 1912
+            least *= 80 if 128 * (self.total_elems - elems) > elems else 28
+        elif self.rt == 8 and 2 * tc_wide > elems:
+            # the tensor cores make little of the product at rank 8, and rows of more than 1024 columns leave a CTA two
+            # groups or one: 2 x 976x2048 at 8 x 1 86 / 93, 2 x 1952x2048 124 / 127, 2 x 2928x2048 164 / 163, 4 x 2048^2 210 / 200
+            least *= 8
+        elif columns > 4:
+            # 6 x 512^2 44 / 48 at 4 x 2 (35 / 33 at 1 x 2, 39 / 39 at 2 x 2), 2 x 780x1024 45 / 47, 2 x 1024^2 47 / 47, 2 x 1220x1024 52 / 50
+            least = least * 4 // 3
+        return elems + int((n * m)[n <= 8].sum()) >= least
+
+    def panel_segments(self, mats: Sequence[int], vec_widths: Sequence[int], rows_per_panel, row=0, start: int = 0) -> Tuple[np.ndarray, np.ndarray]:
         """Segments of whole rows of the matrices `mats` for the kernel that does the last product and the
-        decompression in one pass, and the first segment of every CTA. Each CTA gets the same share of the elements, in
-        quads of rows and in the order of the matrices. `rows_per_panel(m, rows)`: of a segment."""
+        decompression in one pass, and the first segment of every CTA. Each CTA gets the same share of the work (`row`, `start`:
+        see `panel_costs`), in quads of rows and in the order of the matrices. `rows_per_panel(m, rows)`: of a segment."""
         groups = [self.plan.groups[self.mats[mi][0]] for mi in mats]
         n, m = np.array([g.n for g in groups]), np.array([g.m for g in groups])
-        first_quad = np.concatenate([[0], np.cumsum(-(-n // 4))])      # of every matrix, counted over all of them
-        cost = np.concatenate([[0], np.cumsum(-(-n // 4) * m)])
+        quads, costs = (-(-n // 4)).astype(np.int64), (4 * np.maximum(m, row)).astype(np.int64)
+        first_quad = np.concatenate([[0], np.cumsum(quads)])      # of every matrix, counted over all of them
         ctas = min(148, int(first_quad[-1]))
-        shares = cost[-1] * np.arange(ctas + 1) / ctas
-        of = np.clip(np.searchsorted(cost, shares, side="right") - 1, 0, len(mats) - 1)
-        bounds = first_quad[of] + ((shares - cost[of]) / m[of] + 0.5).astype(np.int64)   # where a CTA's share begins
+        bounds = np.zeros(ctas + 1, dtype=np.int64)   # where a CTA's share begins
+        self._lib.psgd_panel_shares(quads.ctypes.data, costs.ctypes.data, len(mats), start, ctas, bounds.ctypes.data)
         cuts = np.union1d(bounds, first_quad)
         of = np.searchsorted(first_quad, cuts[:-1], side="right") - 1
         segs = np.zeros(len(cuts) - 1, dtype=layout.TILE_DTYPE)
@@ -508,7 +548,7 @@ class NativeCompressor(_Recordable):
             }
         self._panel = None
         if finish:
-            self._plan_panels(vec, [grads[idx].data_ptr() for _gi, _pos, idx in self.tiles.mats], mode)
+            self._plan_panels(vec, [grads[idx].data_ptr() for _gi, _pos, idx in self.tiles.mats], mode, tc)
         self._split_tile_lists()
         self._partial = torch.empty(self.tiles.partial_floats, device=self.device, dtype=torch.float32)
         self._partial_tc = torch.empty(self.tiles.partial_tc_floats, device=self.device, dtype=torch.float32)
@@ -518,15 +558,11 @@ class NativeCompressor(_Recordable):
         self._tapes.clear()
         self._key = key
 
-    # Where the one-pass kernel takes over: at least so many elements together, three quarters of them in matrices of
-    # 512 columns and more (a narrow matrix leaves most lanes of a group without columns). us per pass (accumulation
-    # included), one pass / launches apart, at rank 1 x 2, 4 x 2, 8 x 1: 2 x 512^2 30.8 / 30.7, 45.1 / 39.2, 32.4 / 32.8; 2 x 512x1024 31.6 / 33.8,
-    # 46.2 / 43.5, 33.8 / 34.8; 4 x 700x650 34.8 / 39.0, 47.2 / 51.2, 35.7 / 36.9; 8 x 1024^2 56 / 66, 82.0 / 82.8, 62.3 / 62.4; 3 x 4096x1024 73 / 85,
-    # 98.5 / 102, 82 / 84.7; 2 x 24000x96 49.2 / 48.8, 71.9 / 67.3, 58.8 / 55.4.
+    # Elements from which on a step may end in the one-pass kernel (0: wherever it can), see `panel_pays`. At rank 1 x 2, launches
+    # apart / one pass: 2 x 512^2 30.7 / 30.8, 2 x 512x1024 33.8 / 31.6, 2 x 780x1024 37 / 33, 2 x 1952x1024 43 / 37, 4 x 2048^2 114 / 92 us.
     PANEL_ELEMS = 3 << 19
-    PANEL_WIDE = 512
 
-    def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str) -> None:
+    def _plan_panels(self, vec: Sequence[int], addresses: Sequence[int], mode: str, tc: Sequence[bool]) -> None:
         """Which matrices finish a step whose last basis is on the Q side in one pass (csrc/panel.cu), and the tile
         lists of the others. One worker, no optimizer step, no product kernel asked for by name."""
         if world_size() != 1 or mode != "auto" or self.tiles.fin_tc_ok or self.tiles.total_elems < self.PANEL_ELEMS:
@@ -540,11 +576,10 @@ class NativeCompressor(_Recordable):
 
         groups = [self.plan.groups[gi] for gi, _pos, _idx in self.tiles.mats]
         mats = [mi for mi, (g, at) in enumerate(zip(groups, addresses)) if at % 16 == 0 and rows(g.m, g.n) > 0]
-        elems = sum(groups[mi].n * groups[mi].m for mi in mats)
-        wide = sum(groups[mi].n * groups[mi].m for mi in mats if groups[mi].m >= self.PANEL_WIDE)
-        if elems < max(1, self.PANEL_ELEMS) or 4 * wide < 3 * elems:
+        columns = self.tiles.rt * self.T
+        if not mats or (self.PANEL_ELEMS and not self.tiles.panel_pays(mats, vec, columns, tc, self.PANEL_ELEMS)):
             return
-        segs, starts = self.tiles.panel_segments(mats, vec, rows)
+        segs, starts = self.tiles.panel_segments(mats, vec, rows, *self.tiles.panel_costs(mats, vec, columns))
         table = _to_device(np.concatenate([segs.view(np.uint8), starts.view(np.uint8)]), self.device)
         self._panel = (table, segs.nbytes, len(starts) - 1)
         for name in ("nn", "fin"):

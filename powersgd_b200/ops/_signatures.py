@@ -42,6 +42,8 @@ def declare(lib) -> None:
 
     lib.psgd_panel_rows.restype = i32
     lib.psgd_panel_rows.argtypes = [i32, i32, i32, i32]
+    lib.psgd_panel_shares.restype = None
+    lib.psgd_panel_shares.argtypes = [vp, vp, i32, i64, i32, vp]
     lib.psgd_panel_launch.restype = i32
     lib.psgd_panel_launch.argtypes = [vp, vp, vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i32, vp]
 

@@ -37,6 +37,68 @@ def test_segments_cover_every_row_once_and_fit_the_kernel(rank, iters):
     assert max(work) <= total / len(work) + 8 * 4608   # a quad of the widest matrix at either end
 
 
+def _plan(shapes, rank, iters):
+    """(the plan, matrices that the kernel takes, factor columns, rows per panel)"""
+    from powersgd_b200.cuda_path import TilePlan
+
+    try:
+        lib = native.lib()
+    except Exception as exc:
+        pytest.skip(f"native library unavailable: {exc}")
+    tiles = TilePlan(CompressionPlan.build(shapes, rank=rank), lib)
+    rows_of = lambda m, n: int(lib.psgd_panel_rows(tiles.max_r, iters, m, n))  # noqa: E731
+    size = [(tiles.plan.groups[gi].n, tiles.plan.groups[gi].m) for gi, _pos, _idx in tiles.mats]
+    return tiles, size, [mi for mi, (n, m) in enumerate(size) if rows_of(m, n)], tiles.rt * iters, rows_of
+
+
+def _widths(size):
+    return [4 if m % 4 == 0 else 2 if m % 2 == 0 else 1 for _n, m in size]
+
+
+MANY_SMALL = [(1024, 1024)] * 8 + [(64, 64)] * 20
+
+
+@pytest.mark.parametrize("rank,iters", [(1, 2), (2, 2), (4, 2), (8, 1)])
+@pytest.mark.parametrize("shapes", [MANY_SMALL, [(1024, 1024)] * 8 + [(8000, 24)], [(2048, 2048)] * 4 + [(1000, 131)] * 4, [(512, 1024)] * 3])
+def test_no_block_gets_most_of_the_small_segments(shapes, rank, iters):
+    """Starts and narrow rows count: the blocks' costs are alike up to a quad and a start at either end."""
+    tiles, size, mats, columns, rows_of = _plan(shapes, rank, iters)
+    row, start = tiles.panel_costs(mats, _widths(size), columns)
+    segs, starts = tiles.panel_segments(mats, _widths(size), rows_of, row, start)
+    rows = np.zeros(len(size), dtype=np.int64)
+    np.add.at(rows, segs["mat"], segs["rows"])
+    assert rows.tolist() == [n for n, _m in size] and starts[0] == 0 and starts[-1] == len(segs)
+    least = dict(zip(mats, row.tolist()))
+    cost = [sum(start + int(s["rows"]) * max(int(s["cols"]), least[int(s["mat"])]) for s in segs[a:b]) for a, b in zip(starts, starts[1:])]
+    widest = max(max(m, r) for (_n, m), r in zip(size, row))
+    total = sum(start + n * max(m, least[mi]) for mi, (n, m) in enumerate(size))
+    assert max(cost) <= total / len(cost) + 2 * start + 8 * widest
+
+
+@pytest.mark.parametrize("shapes,rank,iters,pays", [
+    ([(4096, 4096)] * 4, 4, 2, True),
+    (MANY_SMALL, 4, 2, True),
+    ([(1024, 1024)] * 8 + [(64, 64)] * 300, 2, 2, False),     # starts
+    ([(64, 64)] * 500, 1, 2, False),
+    ([(24000, 96)] * 4, 1, 2, False),                         # narrow rows
+    ([(512, 2304)] * 2 + [(1000, 131)] * 4, 1, 2, False),
+    ([(4, 4096)] * 100, 4, 2, True),                          # few rows
+    ([(700, 1024)] * 2, 1, 2, False),                         # too little
+    ([(780, 1024)] * 2, 1, 2, True),
+    ([(780, 1024)] * 2, 4, 2, False),                         # ... for eight factor columns
+    ([(2048, 2048)] * 2, 8, 1, False),                        # ... for a product of rank 8 on the tensor cores
+    ([(2048, 2048)] * 4, 8, 1, True),
+    ([(512, 4608)] * 3 + [(512, 2304)] * 8, 4, 2, False),     # some are too wide for the kernel
+    ([(512, 4608)] * 3 + [(512, 2304)] * 8, 2, 2, True),
+])
+def test_where_one_pass_pays(shapes, rank, iters, pays):
+    from powersgd_b200.cuda_path import NativeCompressor
+
+    tiles, size, mats, columns, _rows_of = _plan(shapes, rank, iters)
+    tc = [m % 4 == 0 and n >= 128 and m >= 128 and (rank >= 8 or sum(a * b for a, b in size) > 24 << 20) for n, m in size]
+    assert tiles.panel_pays(mats, _widths(size), columns, tc, NativeCompressor.PANEL_ELEMS) == pays
+
+
 def test_refused_shapes():
     try:
         lib = native.lib()
