@@ -286,7 +286,9 @@ __device__ __forceinline__ void fin_gather(const PsgdCommDev& c, int e1, long lo
 // factor columns before, was a sixth of such a strip's time and a quarter of its instructions. 50257 x 1024 at rank
 // 16 x 2: 467.6 -> 448.1 us per pass. Launches alone, before / now: 6 x 2048^2 at 8 x 2 88 / 87, 12 x 2 105 / 100, 16 x 2 118 / 110;
 // with 4-byte accesses 4 x 3000x1001 at 8 x 2 46.8 / 50.8, 16 x 2 59.3 / 62.5, with 8-byte ones 3 x 9000x650 75.9 / 77.8 and 97.4 /
-// 94.1, so those keep the other form.
+// 94.1, so those keep the other form. In the same kernel they are still 1 to 3 % slower per pass than in one without ROWS
+// (8 x 1024x1001 at 8 x 2 106.1 / 107.8, 4 x 3000x1001 at 16 x 1 285 / 289, 2 x 2048^2 + 4 x 1000x131 at 16 x 1 193 / 199), so a launch is
+// of the kind only when all but a few of its elements gain (flags & 4 of psgd_finalize_launch).
 template <int VEC, bool SAME, int RPW, bool OPT, bool ROWS>
 __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const PsgdTile& t, const PsgdMat& mt,
                                                     int tile_rows, float* fin_smem) {
@@ -578,7 +580,8 @@ PSGD_API int psgd_finalize_uses_strip(int nhist, int max_r, int tile_rows, int s
 // matrix in `mats`. With nhist * max_r <= 32 and panels that fit shared memory the strip kernel
 // runs, else the general one. Every tile carries its matrix's access width (`vec`).
 // comm / poll_left / sum_out1 / sum_out2 / flags / sum_scale: see FinalizeArgs (comm null: nothing
-// is gathered; flags 0 and sum_scale 1 for the library's own step). early: see psgd_launch.
+// is gathered; flags 0 or 4 and sum_scale 1 for the library's own step). flags & 4: all but a few elements are accessed by
+// 16 bytes (see ROWS of the strips). early: see psgd_launch.
 PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntiles, int tile_rows, int max_r,
                                   const void* hyper, int nhist, const float* const* lloc, const float* const* rloc,
                                   const float* const* lsum, const float* const* rsum, float inv_world,
@@ -610,6 +613,8 @@ PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntile
   a.poll_left = poll_left;
   a.sum_out1 = sum_out1;
   a.sum_out2 = sum_out2;
+  const bool by_16 = (flags & 4) != 0;
+  flags &= 3;
   a.flags = flags;
   a.sum_scale = sum_scale;
   if (flags != 0 && fused_sgd) {
@@ -627,7 +632,7 @@ PSGD_API int psgd_finalize_launch(const void* mats, const void* tiles, int ntile
     const int kmax = nhist * max_r;
     if (!same) return finalize_strip_launch<false, 4, true, false>(a, ntiles, tile_rows, kmax, early, stream);
     if (kmax >= 16)
-      return max_r % 4 == 0 ? finalize_strip_launch<true, 8, true, true>(a, ntiles, tile_rows, kmax, early, stream)
+      return by_16 && max_r % 4 == 0 ? finalize_strip_launch<true, 8, true, true>(a, ntiles, tile_rows, kmax, early, stream)
                             : finalize_strip_launch<true, 8, true, false>(a, ntiles, tile_rows, kmax, early, stream);
     return fused_sgd ? finalize_strip_launch<true, 4, true, false>(a, ntiles, tile_rows, kmax, early, stream)
                      : finalize_strip_launch<true, 4, false, false>(a, ntiles, tile_rows, kmax, early, stream);

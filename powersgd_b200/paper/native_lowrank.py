@@ -155,7 +155,7 @@ class NativeLowRank:
             comp.comm.ptr if gather_state is not None else ctypes.c_void_p(0), 0,
             _ptr(comp.h_sum[1]) if gather_state is not None else ctypes.c_void_p(0),
             _ptr(gather_state) if gather_state is not None else ctypes.c_void_p(0),
-            3,  # residual = M - update, written to the `param` slot (the caller's memory tensor)
+            3 | comp._strip_flags,  # residual = M - update, written to the `param` slot (the caller's memory tensor)
             1.0 / workers,
             int(comp._chained()),
         )

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from powersgd_b200 import BasicConfig, BasicPowerSGD, Config, PowerSGD, optimizer_step
+from powersgd_b200.cuda_path import NativeCompressor
 
 pytestmark = pytest.mark.gpu
 
@@ -79,8 +80,9 @@ def test_local_and_summed_factors_apart(rank, rows):
 
 @pytest.mark.parametrize("rank,iters", [(8, 2), (8, 3), (12, 2), (16, 1), (16, 2)])
 @pytest.mark.parametrize("first", [(64, 48), (5, 9)])
-def test_left_panels_by_rows(rank, iters, first):
+def test_left_panels_by_rows(rank, iters, first, monkeypatch):
     """From 16 factor columns on: factors on 16-byte boundaries and, behind a matrix of rank 5, not. The bound of the first test."""
+    monkeypatch.setattr(NativeCompressor, "STRIPS_BY_16", 0.0)
     shapes = [first, (97, 129), (300, 260), (257, 66), (520, 128)]
     core = BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=rank, num_iters_per_step=iters), backend="native")
     g = torch.Generator(device="cuda").manual_seed(rank)
@@ -97,3 +99,10 @@ def test_left_panels_by_rows(rank, iters, first):
             eps = (grp.r * iters + 3) * 2.0 ** -24
             assert ((outs[idx].double() - update).abs() <= eps * size).all(), shapes[idx]
             assert ((grads[idx].double() - (before[idx] - update)).abs() <= eps * (size + before[idx].abs())).all(), shapes[idx]
+
+
+@pytest.mark.parametrize("shapes,flags", [([(300, 260), (64, 48)], 4), ([(300, 260), (64, 49)], 0), ([(300, 261)], 0), ([(900, 1024), (64, 49)], 4)])
+def test_strips_by_rows_are_for_lists_that_gain(shapes, flags):
+    core = BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=8, num_iters_per_step=2), backend="native")
+    core.aggregate([torch.randn(s, device="cuda") for s in shapes])
+    assert core._native._strip_flags == flags
