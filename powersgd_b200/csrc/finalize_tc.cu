@@ -15,6 +15,7 @@
 // All mbarrier waits are bounded (status word + abort flag), as in lowrank_tc.cu.
 #include <cuda.h>
 
+#include "psgd_async.cuh"
 #include "psgd_comm.cuh"
 
 namespace {
@@ -24,7 +25,6 @@ constexpr int FT_ROWS = 128;
 constexpr int FT_COLS = 64;
 constexpr int FT_MAX_KP = 128;                      // padded 3K; 4 slabs of 32
 constexpr int FT_TILE_BYTES = FT_ROWS * FT_COLS * 4;  // 32 KiB
-constexpr uint64_t FT_WAIT_LIMIT_NS = 2000000000ull;
 
 struct FinTcArgs {
   const PsgdMat* mats;
@@ -41,33 +41,6 @@ struct FinTcArgs {
   int* status;
 };
 
-__device__ __forceinline__ uint32_t ft_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool ft_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(ft_smem(bar)), "r"(parity) : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool ft_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  if (ft_try_wait(bar, parity)) return true;
-  const uint64_t t0 = psgd_globaltimer_ns();
-  while (!ft_try_wait(bar, parity)) {
-    if (*abort_flag) return false;
-    if (psgd_globaltimer_ns() - t0 > FT_WAIT_LIMIT_NS) {
-      *abort_flag = 1;
-      if (status) {
-        // plain store: the word may live in mapped pinned host memory, which the host reads
-        *((volatile int*)status) = (int)PSGD_TIMEOUT_MBARRIER;
-        __threadfence_system();
-      }
-      return false;
-    }
-  }
-  return true;
-}
 __device__ __forceinline__ uint64_t ft_desc(uint32_t saddr) {  // K-major, 128-byte swizzle, 8-row groups 1 KiB apart
   uint64_t d = 0;
   d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
@@ -140,14 +113,14 @@ __global__ void __launch_bounds__(FT_THREADS) psgd_finalize_tc_kernel(const __gr
   __shared__ int s_abort;
 
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ft_smem(&bar_m)), "r"(1));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ft_smem(&bar_panels)), "r"(128));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ft_smem(&bar_mma)), "r"(1));
+    psgd_mbar_init(&bar_m, 1);
+    psgd_mbar_init(&bar_panels, 128);
+    psgd_mbar_init(&bar_mma, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 4) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ft_smem(&s_tmem)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(psgd_smem_u32(&s_tmem)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -159,18 +132,18 @@ __global__ void __launch_bounds__(FT_THREADS) psgd_finalize_tc_kernel(const __gr
   if (warp == 4) {
     if (lane == 0) {
       // gradient tile: 2 column slabs x 4 row boxes of 32 x 32 floats
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ft_smem(&bar_m)), "r"(FT_TILE_BYTES) : "memory");
+      psgd_mbar_expect_tx(&bar_m, FT_TILE_BYTES);
 #pragma unroll
       for (int cs = 0; cs < 2; ++cs)
 #pragma unroll
         for (int rb = 0; rb < 4; ++rb)
           asm volatile(
               "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-              ::"r"(ft_smem(sM + cs * (FT_ROWS * 128) + rb * 4096)), "l"(map), "r"(ft_smem(&bar_m)),
+              ::"r"(psgd_smem_u32(sM + cs * (FT_ROWS * 128) + rb * 4096)), "l"(map), "r"(psgd_smem_u32(&bar_m)),
                 "r"(t.col0 + 32 * cs), "r"(t.row0 + 32 * rb) : "memory");
-      if (ft_wait(&bar_panels, 0, abort_flag, a.status)) {
+      if (psgd_mbar_wait(&bar_panels, 0, abort_flag, a.status)) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t al = ft_smem(sAl), bl = ft_smem(sBl), as = ft_smem(sAs), bs = ft_smem(sBs);
+        const uint32_t al = psgd_smem_u32(sAl), bl = psgd_smem_u32(sBl), as = psgd_smem_u32(sAs), bs = psgd_smem_u32(sBs);
         for (int ks = 0; ks < Kp / 8; ++ks) {
           const uint32_t ao = (uint32_t)(ks >> 2) * 16384u + (uint32_t)(ks & 3) * 32u;
           const uint32_t bo = (uint32_t)(ks >> 2) * 8192u + (uint32_t)(ks & 3) * 32u;
@@ -186,7 +159,7 @@ __global__ void __launch_bounds__(FT_THREADS) psgd_finalize_tc_kernel(const __gr
                 ::"r"(tmem + 64), "l"(ft_desc(as + ao)), "l"(ft_desc(bs + bo)), "r"(IDESC), "r"(acc) : "memory");
         }
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(ft_smem(&bar_mma)) : "memory");
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(psgd_smem_u32(&bar_mma)) : "memory");
     }
   } else {
     // ---- stage the factor panels (split along K) ----
@@ -211,11 +184,11 @@ __global__ void __launch_bounds__(FT_THREADS) psgd_finalize_tc_kernel(const __gr
       stage(sAs, FT_ROWS, t.rows, a.lsum, poff, true);
       stage(sBs, FT_COLS, t.cols, a.rsum, qoff, false);
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ft_smem(&bar_panels)) : "memory");
+    psgd_fence_async_shared();
+    psgd_mbar_arrive(&bar_panels);
 
     // ---- one tile row per thread: residual = M - E into sM, update into sU ----
-    const bool ok = ft_wait(&bar_mma, 0, abort_flag, a.status) && ft_wait(&bar_m, 0, abort_flag, a.status);
+    const bool ok = psgd_mbar_wait(&bar_mma, 0, abort_flag, a.status) && psgd_mbar_wait(&bar_m, 0, abort_flag, a.status);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {
       const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
@@ -244,8 +217,7 @@ __global__ void __launch_bounds__(FT_THREADS) psgd_finalize_tc_kernel(const __gr
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
   if (s_abort) {
-    const uint64_t t0 = psgd_globaltimer_ns();
-    while (psgd_globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    psgd_let_copies_land();
     return;
   }
 

@@ -29,6 +29,7 @@
 #include <cuda.h>
 #include <string.h>
 
+#include "psgd_async.cuh"
 #include "psgd_comm.cuh"
 
 namespace {
@@ -48,7 +49,6 @@ constexpr int TC_SEG = 16;        // stages (512 K rows) accumulated in TMEM bef
                                   // product: 5e-7 relative for 512 rows, 1e-5 for 2048, 6e-5 for 6272). Two
                                   // accumulators alternate, so the MMA stream never waits for the hand-over.
 constexpr int TC_DRAIN_LAG = 2;   // stages converted into the next segment before the finished one is read
-constexpr uint64_t TC_WAIT_LIMIT_NS = 2000000000ull;  // 2 s
 
 struct TcArgs {
   const PsgdMat* mats;
@@ -67,52 +67,10 @@ struct TcArgs {
   int* status;               // word (device or mapped host memory) set on a wait that ran out
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait. Returns false (and raises the abort flag) when the limit expires or another
-// role already aborted.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = psgd_globaltimer_ns();
-  while (!mbar_try_wait(bar, parity)) {
-    if (*abort_flag) return false;
-    if (psgd_globaltimer_ns() - t0 > TC_WAIT_LIMIT_NS) {
-      *abort_flag = 1;
-      if (status) {
-        // plain store: the word may live in mapped pinned host memory, which the host reads
-        *((volatile int*)status) = (int)PSGD_TIMEOUT_MBARRIER;
-        __threadfence_system();
-      }
-      return false;
-    }
-  }
-  return true;
-}
-
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      ::"r"(psgd_smem_u32(dst)), "l"(map), "r"(psgd_smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
 
@@ -139,7 +97,7 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint6
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(psgd_smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ float tf32_hi(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFE000u); }
@@ -207,22 +165,22 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
 
   if (tid == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
-      mbar_init(&bar_full[s], 1);
-      mbar_init(&bar_empty[s], 1);
+      psgd_mbar_init(&bar_full[s], 1);
+      psgd_mbar_init(&bar_empty[s], 1);
     }
     for (int s = 0; s < TC_OP_STAGES; ++s) {
-      mbar_init(&bar_ready[s], TC_NCONV);
-      mbar_init(&bar_op_empty[s], 1);
+      psgd_mbar_init(&bar_ready[s], TC_NCONV);
+      psgd_mbar_init(&bar_op_empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&bar_seg[b], 1);
-      mbar_init(&bar_drained[b], 128);
+      psgd_mbar_init(&bar_seg[b], 1);
+      psgd_mbar_init(&bar_drained[b], 128);
     }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(psgd_smem_u32(&s_tmem)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -245,7 +203,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
   bool drain_ok = true;
   auto drain = [&](int g) {
     // segment g used accumulator (g & 1) for the (g >> 1)-th time
-    if (drain_ok) drain_ok = mbar_wait(&bar_seg[g & 1], (g >> 1) & 1, abort_flag, a.status);
+    if (drain_ok) drain_ok = psgd_mbar_wait(&bar_seg[g & 1], (g >> 1) & 1, abort_flag, a.status);
     if (drain_ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float d[N2];
@@ -254,7 +212,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
       for (int i = 0; i < N2; ++i) sum[i] += d[i];
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
-    mbar_arrive(&bar_drained[g & 1]);
+    psgd_mbar_arrive(&bar_drained[g & 1]);
   };
 
   if (warp == 4) {
@@ -263,8 +221,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
       for (int kb = 0; kb < nk; ++kb) {
         const int s = kb % TC_STAGES;
         const uint32_t ph = (kb / TC_STAGES) & 1;
-        if (!mbar_wait(&bar_empty[s], ph ^ 1, abort_flag, a.status)) break;
-        mbar_expect_tx(&bar_full[s], TC_A_BYTES);
+        if (!psgd_mbar_wait(&bar_empty[s], ph ^ 1, abort_flag, a.status)) break;
+        psgd_mbar_expect_tx(&bar_full[s], TC_A_BYTES);
         uint8_t* dst = sA + s * TC_A_BYTES;
         const int k0 = k_begin + kb * TC_BK;
 #pragma unroll
@@ -286,15 +244,15 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
         const int g = kb / TC_SEG;
         const bool seg_first = kb % TC_SEG == 0;
         // accumulator (g & 1) was last used by segment g - 2: wait until the converters have read it
-        if (seg_first && g >= 2) ok = mbar_wait(&bar_drained[g & 1], ((g >> 1) - 1) & 1, abort_flag, a.status);
+        if (seg_first && g >= 2) ok = psgd_mbar_wait(&bar_drained[g & 1], ((g >> 1) - 1) & 1, abort_flag, a.status);
         if (!ok) break;
-        ok = mbar_wait(&bar_ready[so], (kb / TC_OP_STAGES) & 1, abort_flag, a.status);
+        ok = psgd_mbar_wait(&bar_ready[so], (kb / TC_OP_STAGES) & 1, abort_flag, a.status);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + (uint32_t)((g & 1) * N2);
-        const uint32_t aaddr = smem_u32(sA + s * TC_A_BYTES);
-        const uint32_t laddr = smem_u32(sAlo + so * TC_A_BYTES);
-        const uint32_t baddr = smem_u32(sB + so * B_BYTES);
+        const uint32_t aaddr = psgd_smem_u32(sA + s * TC_A_BYTES);
+        const uint32_t laddr = psgd_smem_u32(sAlo + so * TC_A_BYTES);
+        const uint32_t baddr = psgd_smem_u32(sB + so * B_BYTES);
 #pragma unroll
         for (int ks = 0; ks < TC_BK / 8; ++ks) {
           // NT (MN-major A): a slab holds 32 K rows of 128 bytes (32 columns); 8 K rows = two
@@ -340,8 +298,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
 #pragma unroll
       for (int i = 0; i < PER_THREAD; ++i) cur[i] = pre[i];
       fetch(kb + 1);
-      if (!mbar_wait(&bar_full[s], ph, abort_flag, a.status)) break;
-      if (!mbar_wait(&bar_op_empty[so], ((kb / TC_OP_STAGES) & 1) ^ 1, abort_flag, a.status)) break;
+      if (!psgd_mbar_wait(&bar_full[s], ph, abort_flag, a.status)) break;
+      if (!psgd_mbar_wait(&bar_op_empty[so], ((kb / TC_OP_STAGES) & 1) ^ 1, abort_flag, a.status)) break;
       if (SPLIT) {
         const float4* src = reinterpret_cast<const float4*>(sA + s * TC_A_BYTES);
         float4* dst = reinterpret_cast<float4*>(sAlo + so * TC_A_BYTES);
@@ -368,8 +326,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
         for (int e = ctid; e < (N2 - (SPLIT ? 2 : 1) * RP) * 32; e += TC_NCONV)
           reinterpret_cast<float*>(bt + (SPLIT ? 2 : 1) * RP * 128)[e] = 0.f;
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(&bar_ready[so]);
+      psgd_fence_async_shared();
+      psgd_mbar_arrive(&bar_ready[so]);
       // a finished segment is read a couple of stages later, when its MMAs are certainly done
       while (warp < 4 && next_drain < nseg - 1 && kb >= (next_drain + 1) * TC_SEG - 1 + TC_DRAIN_LAG) drain(next_drain++);
     }
@@ -389,8 +347,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) psgd_gemm_tc_kernel(const __gri
   if (s_abort) {
     // a wait ran out: give copies that may still be in flight time to land before this CTA's
     // shared memory is handed to another one
-    const uint64_t t0 = psgd_globaltimer_ns();
-    while (psgd_globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    psgd_let_copies_land();
     __syncthreads();
   }
   if (warp == 5) {

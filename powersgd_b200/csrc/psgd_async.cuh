@@ -1,4 +1,5 @@
-// Shared-memory barriers with bounded waits, as kernels that fill rings by asynchronous copies use them.
+// Shared-memory barriers with bounded waits, as kernels that fill rings by asynchronous copies and those on the
+// tensor cores use them.
 #pragma once
 #include "psgd_common.cuh"
 
@@ -8,6 +9,9 @@ __device__ __forceinline__ uint32_t psgd_smem_u32(const void* p) { return (uint3
 
 __device__ __forceinline__ void psgd_mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(psgd_smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void psgd_mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(psgd_smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void psgd_mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(psgd_smem_u32(bar)), "r"(bytes) : "memory");
