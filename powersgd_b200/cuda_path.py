@@ -439,7 +439,7 @@ class NativeCompressor(_Recordable):
                 (self.plan.signature(), int(core.config.rank), int(self.T)), "PowerSGD compression plan"
             )
             self.comm = Channel(cap)
-        # status word of the tensor-core kernels' bounded waits: mapped pinned host memory, so the
+        # status word of the bounded waits of the tensor-core and the one-pass kernels: mapped pinned host memory, so the
         # host can look at it every step without touching the GPU
         from .parallel.symm import StatusWord
 
@@ -973,11 +973,11 @@ class NativeCompressor(_Recordable):
 
     def check(self) -> None:
         """Raise `PowerSGDCommTimeout` if a bounded device-side wait of an EARLIER launch gave up
-        (a peer that never pushed, a tensor-core pipeline that stalled). Plain host reads of
+        (a peer that never pushed, copies into shared memory or tensor-core work that never ended). Plain host reads of
         mapped pinned words: no synchronisation, cheap enough for every step."""
         if self.comm is not None:
             self.comm.check()
-        self._status.check("a tensor-core pipeline wait")
+        self._status.check("a wait inside a product, decompression or one-pass kernel")
 
     # -- public ----------------------------------------------------------------------------
     def aggregate(self, gradients: List[torch.Tensor]) -> List[torch.Tensor]:

@@ -30,3 +30,22 @@ def test_orthonormalisation_overlaps_on_one_worker():
 def test_orthonormalisation_keeps_the_plain_order_with_several_workers(gather):
     """A first launch that waits for peers must not have the second one's CTAs resident beside it."""
     assert _orth_flags(SimpleNamespace(ptr=ctypes.c_void_p(8)), early=False, gather=gather) == 0
+
+
+def test_a_wait_that_ran_out_is_not_put_down_to_the_tensor_cores():
+    """The one-pass kernel, which does not use them, reports through the same word."""
+    from powersgd_b200.parallel.symm import PowerSGDCommTimeout, StatusWord
+
+    class Word(StatusWord):   # without memory that a GPU can see
+        value = 3
+
+        def __init__(self):
+            self._host = None
+
+    nat = object.__new__(NativeCompressor)
+    nat.comm, nat._status = None, Word()
+    with pytest.raises(PowerSGDCommTimeout, match="one-pass kernel") as caught:
+        nat.check()
+    assert "tensor-core" not in str(caught.value)
+    Word.value = 0
+    nat.check()
