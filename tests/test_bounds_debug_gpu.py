@@ -2,11 +2,12 @@
 with -DPSGD_BOUNDS_CHECK validate every tile against its matrix, its access width and the scratch
 capacities, record the first violation in a status block and SKIP the access (no trap, no fault).
 
-Two checks, each in a child process that loads the debug library through PSGD_B200_LIB:
+Three checks, each in a child process that loads the debug library through PSGD_B200_LIB:
   * the ragged small-shape suite (row pitches 27 and 650, rank above a dimension, rank-1 groups,
     several half-iterations, fused SGD) runs without a single violation and matches the PyTorch path;
   * a tile list that lies about its matrix (rows beyond the end, a 16-byte access width on a pitch of
-    27 floats, a scratch slot beyond the arena) is caught: violations are recorded, nothing is written.
+    27 floats, a scratch slot beyond the arena) is caught: violations are recorded, nothing is written;
+  * the same of the one-pass kernel and its segments.
 """
 import os
 import subprocess
@@ -133,3 +134,58 @@ def test_inconsistent_tiles_are_recorded_and_skipped():
         """
     )
     assert "CAUGHT-OK" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
+
+
+def test_one_pass_kernel_on_the_checked_build():
+    res = _run(
+        """
+        import ctypes, numpy as np, torch
+        from powersgd_b200 import BasicConfig, BasicPowerSGD
+        from powersgd_b200.cuda_path import NativeCompressor, _to_device
+        from powersgd_b200.ops import layout, native
+        lib = native.lib()
+        lib.psgd_bounds_status.restype = ctypes.c_int
+        status = (ctypes.c_int * 24)()
+        dev = torch.device("cuda:0")
+        NativeCompressor.PANEL_ELEMS = 0
+        shapes = [(64, 27), (300, 1024), (129, 650), (33, 1001), (37, 4096), (600, 64), (9, 4095), (2500, 24), (5, 23), (40, 6300)]
+        g = torch.Generator().manual_seed(0)
+        for rank, iters in [(1, 2), (1, 4), (2, 2), (3, 2), (4, 2), (5, 1), (8, 1)]:
+            core = BasicPowerSGD([torch.zeros(s, device=dev) for s in shapes], BasicConfig(rank=rank, num_iters_per_step=iters), backend="native")
+            grads = [torch.randn(s, generator=g).to(dev) for s in shapes]
+            for step in range(2):
+                before = [x.clone() for x in grads]
+                outs = core.aggregate(grads)
+                torch.cuda.synchronize()
+                for x, y, b in zip(outs, grads, before):   # what is left and the update make up the gradient
+                    assert torch.allclose(x + y, b, atol=1e-4)
+            assert core._native._finished, (rank, iters)
+        total = lib.psgd_bounds_status(status, 1)
+        assert total == 0, list(status)
+
+        # segments that lie about their matrix: rows beyond its end, an access width that its pitch does not allow,
+        # panels higher than the row values have room for
+        core = BasicPowerSGD([torch.zeros(40, 650, device=dev)], BasicConfig(rank=4, num_iters_per_step=2), backend="native")
+        grad = torch.randn(40, 650, device=dev)
+        core.aggregate([grad])
+        nat = core._native
+        table, nbytes, ctas = nat._panel
+        raw = table.cpu().numpy().copy()
+        for what, edit in [(1, lambda s: s.__setitem__("rows", s["rows"] + 40)), (3, lambda s: s.__setitem__("vec", 4)),
+                           (8, lambda s: s.__setitem__("split", 32))]:
+            bad = raw.copy()
+            segs = bad[:nbytes].view(layout.TILE_DTYPE)
+            edit(segs)
+            nat._panel = (_to_device(bad, dev), nbytes, ctas)
+            nat._tapes.clear()
+            before = grad.clone()
+            nat._out_arena.fill_(7.0)
+            core.aggregate([grad])
+            torch.cuda.synchronize()
+            total = lib.psgd_bounds_status(status, 1)
+            assert total >= 1 and status[8 + 1] == 6 and status[8 + 2] == what, (what, total, list(status)[8:16])
+            assert torch.equal(grad, before) and bool((nat._out_arena == 7.0).all()), "a rejected segment must not write"
+        print("PANEL-OK")
+        """
+    )
+    assert "PANEL-OK" in res.stdout, res.stdout[-2000:] + res.stderr[-4000:]
