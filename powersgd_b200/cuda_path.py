@@ -191,8 +191,11 @@ class TilePlan:
 
     @staticmethod
     def _grids(matrices: Sequence[Tuple[int, int, int, int, int, int]]) -> np.ndarray:
-        """Tiles of `rows` x `cols` over every (index, n, rows, m, cols, access width) of a list, row by row. All matrices
-        at once, since an array operation costs as much as building some ten tiles one by one."""
+        """Tiles of `rows` x `cols` over every (index, n, rows, m, cols, access width) of a list, row by row. By array
+        operations over all matrices at once; one by one up to some 40 tiles, which the array operations cost alone."""
+        if sum(-(-n // rows) * -(-m // cols) for _mi, n, rows, m, cols, _v in matrices) <= 40:
+            return np.array([(mi, r0, min(rows, n - r0), c0, min(cols, m - c0), 0, 1, 0, 0, v, (0, 0))
+                             for mi, n, rows, m, cols, v in matrices for r0 in range(0, n, rows) for c0 in range(0, m, cols)], dtype=layout.TILE_DTYPE)
         mat, n, rows, m, cols, vec = np.array(matrices, dtype=np.int32).reshape(-1, 6).T
         across = -(-m // cols)
         count = -(-n // rows) * across
@@ -517,8 +520,7 @@ class NativeCompressor(_Recordable):
             else:
                 vec.append(1)
         assert where is not None
-        by_16 = descs[np.array(vec) == 4]
-        by_16 = int((by_16["n"].astype(np.int64) * by_16["m"]).sum())
+        by_16 = sum(g.n * g.m for g, v in zip((self.plan.groups[gi] for gi, _pos, _idx in self.tiles.mats), vec) if v == 4)
         self._strip_flags = 4 if by_16 >= self.STRIPS_BY_16 * self.tiles.total_elems else 0
         self._mats_dev = _to_device(descs, self.device)
         # tensor-core (TMA + tcgen05) path: matrices TMA can address and that are worth it

@@ -182,11 +182,12 @@ def test_tallest_strip_at_every_column_count_of_the_strip_kernel(same):
         assert int(lib.psgd_finalize_uses_strip(1, k, 256, same)) == 1, k
 
 
-def test_grids_of_several_matrices_are_the_tiles_of_each_in_turn():
+@pytest.mark.parametrize("times", [0, 1, 2, 3, 20])   # few tiles are built one by one
+def test_grids_of_several_matrices_are_the_tiles_of_each_in_turn(times):
     from powersgd_b200.cuda_path import TilePlan
     from powersgd_b200.ops import layout
 
-    matrices = [(3, 64, 32, 27, 128, 1), (0, 1, 256, 1, 64, 4), (7, 100, 96, 300, 128, 2), (8, 0, 32, 5, 128, 1), (2, 256, 128, 128, 64, 4)]
+    matrices = [(3, 64, 32, 27, 128, 1), (0, 1, 256, 1, 64, 4), (7, 100, 96, 300, 128, 2), (8, 0, 32, 5, 128, 1), (2, 256, 128, 128, 64, 4)] * times
     want = [(mi, r0, min(rows, n - r0), c0, min(cols, m - c0), 0, 1, 0, 0, v, (0, 0))
             for mi, n, rows, m, cols, v in matrices for r0 in range(0, n, rows) for c0 in range(0, m, cols)]
     assert np.array_equal(TilePlan._grids(matrices), np.array(want, dtype=layout.TILE_DTYPE))
