@@ -545,11 +545,8 @@ template <bool SAME, int RPW, bool OPT, bool ROWS>
 static int finalize_strip_launch(const FinalizeArgs& a, int ntiles, int tile_rows, int kmax, int early, cudaStream_t stream) {
   const size_t smem = (size_t)(SAME ? 1 : 2) * kmax * fin_panel_floats(tile_rows) * sizeof(float);
   if (smem > (size_t)FIN_SMEM_DEFAULT) {
-    static bool opted_in = false;   // per instantiation
-    if (!opted_in) {
-      PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_finalize_strip_kernel<SAME, RPW, OPT, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, FIN_SMEM_OPT_IN));
-      opted_in = true;
-    }
+    static unsigned long long devices = 0;   // per instantiation
+    if (const int code = psgd_allow_shared((const void*)psgd_finalize_strip_kernel<SAME, RPW, OPT, ROWS>, FIN_SMEM_OPT_IN, devices)) return code;
   }
   return psgd_launch(psgd_finalize_strip_kernel<SAME, RPW, OPT, ROWS>, ntiles, FIN_THREADS, smem, stream, early, a, tile_rows);
 }

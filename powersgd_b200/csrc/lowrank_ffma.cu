@@ -495,10 +495,9 @@ static void fill_args(GemmArgs& a, const void* mats, const void* tiles, const fl
 template <int RT>
 static int launch_nt(const GemmArgs& a, int ntiles, int early, cudaStream_t stream) {
   const size_t smem = (size_t)(nt_stage_floats<RT>() + NT_TILE_COLS * RT) * sizeof(float);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
-    PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_gemm_nt_kernel<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
+  if (smem > 48 * 1024) {
+    static unsigned long long devices = 0;   // per instantiation
+    if (const int code = psgd_allow_shared((const void*)psgd_gemm_nt_kernel<RT>, smem, devices)) return code;
   }
   return psgd_launch(psgd_gemm_nt_kernel<RT>, ntiles, GEMM_THREADS, smem, stream, early, a);
 }

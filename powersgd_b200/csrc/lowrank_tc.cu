@@ -404,12 +404,8 @@ template <bool TRANSPOSED, int RP, bool SPLIT>
 int launch_tc(const TcArgs& a, int ntiles, int early, cudaStream_t stream) {
   constexpr int N2 = ((SPLIT ? 2 : 1) * RP) < 16 ? 16 : ((SPLIT ? 2 : 1) * RP);
   const size_t smem = 1024 + (size_t)TC_STAGES * TC_A_BYTES + (size_t)TC_OP_STAGES * ((SPLIT ? TC_A_BYTES : 0) + N2 * 128);
-  static bool configured = false;
-  if (!configured) {
-    PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_gemm_tc_kernel<TRANSPOSED, RP, SPLIT>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  static unsigned long long devices = 0;   // per instantiation
+  if (const int code = psgd_allow_shared((const void*)psgd_gemm_tc_kernel<TRANSPOSED, RP, SPLIT>, smem, devices)) return code;
   return psgd_launch(psgd_gemm_tc_kernel<TRANSPOSED, RP, SPLIT>, ntiles, TC_THREADS, smem, stream, early, a);
 }
 

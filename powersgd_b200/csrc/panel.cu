@@ -437,11 +437,8 @@ __global__ void __launch_bounds__(PN_THREADS, 1) psgd_panel_kernel(const __grid_
 
 template <int RT, int NH>
 static int panel_launch(const PanelArgs& a, int ctas, int early, cudaStream_t stream) {
-  static bool configured = false;   // per instantiation
-  if (!configured) {
-    PSGD_CUDA_OK(cudaFuncSetAttribute(psgd_panel_kernel<RT, NH>, cudaFuncAttributeMaxDynamicSharedMemorySize, PN_SMEM));
-    configured = true;
-  }
+  static unsigned long long devices = 0;   // per instantiation
+  if (const int code = psgd_allow_shared((const void*)psgd_panel_kernel<RT, NH>, PN_SMEM, devices)) return code;
   return psgd_launch(psgd_panel_kernel<RT, NH>, ctas, PN_THREADS, PN_SMEM, stream, early, a);
 }
 

@@ -108,6 +108,18 @@ __device__ __forceinline__ void psgd_wait_for_predecessor() { asm volatile("grid
 // Asks for the 128-byte line of L2 that holds *p. Only for addresses inside live allocations.
 __device__ __forceinline__ void psgd_prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// More than 48 KiB of dynamic shared memory for a kernel: asked once per device, whose copy of the kernel the attribute belongs
+// to. `devices`: those that have it (one bit each), a static variable of the caller.
+static inline int psgd_allow_shared(const void* kernel, size_t bytes, unsigned long long& devices) {
+  int device = 0;
+  PSGD_CUDA_OK(cudaGetDevice(&device));
+  const unsigned long long bit = 1ull << (device & 63);
+  if (device < 64 && (devices & bit) != 0) return 0;
+  PSGD_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (device < 64) __atomic_fetch_or(&devices, bit, __ATOMIC_RELAXED);
+  return 0;
+}
+
 // `early` != 0: the kernel contains the wait above and the launch directly before it in `stream` is
 // one of this library's.
 template <typename... Params, typename... Args>

@@ -38,3 +38,19 @@ def test_two_gpu_training_step_raises_when_a_peer_stays_away():
     in-kernel collectives on plain peer stores."""
     res = run_scenario("train_step_timeout", nproc=2, timeout=600, env=dict(ENV, PSGD_B200_COMM_TIMEOUT_MS="300"))
     assert "SCENARIO-OK" in res.stdout, res.stdout[-3000:] + res.stderr[-6000:]
+
+
+@needs_two
+@pytest.mark.parametrize("rank,iters", [(1, 2), (4, 2), (8, 1), (16, 2)])
+def test_one_process_on_two_gpus_in_turn(rank, iters):
+    """Kernels with much shared memory ask each device for it."""
+    from powersgd_b200 import BasicConfig, BasicPowerSGD
+
+    seen = []
+    for device in range(2):
+        with torch.cuda.device(device):
+            gen = torch.Generator().manual_seed(1)
+            grads = [torch.randn(s, generator=gen).cuda() for s in [(2048, 1024), (700, 650)]]
+            core = BasicPowerSGD([torch.zeros_like(g) for g in grads], BasicConfig(rank=rank, num_iters_per_step=iters), backend="native")
+            seen.append([x.cpu() for _ in range(2) for x in core.aggregate(grads)])
+    assert all(torch.allclose(a, b, atol=1e-4) for a, b in zip(*seen))
