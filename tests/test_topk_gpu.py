@@ -14,8 +14,8 @@ def _tensors(dev):
     normal = lambda n: torch.randn(n, generator=g, device=dev)  # noqa: E731
     flat = normal(70001)
     yield flat[1:], 143                                                                # 4-byte aligned
-    yield normal(300000), 614                                                           # some 2 k candidates
-    yield torch.rand(200000, generator=g, device=dev), 400                              # an eighth of all are candidates
+    yield normal(300000), 614                                                           # some 480 candidates
+    yield torch.rand(200000, generator=g, device=dev), 400                              # a twentieth of all are candidates
     yield torch.full((150000,), -0.75, device=dev), 300                                 # all of them
     yield torch.where(torch.rand(90000, generator=g, device=dev) < 0.01, 1.5, 1.0), 1200    # ties at the threshold
     yield normal(9000).sign() * 2.0 ** torch.randint(-126, 120, (9000,), generator=g, device=dev), 77
@@ -25,7 +25,7 @@ def _tensors(dev):
     yield normal(600), 600
 
 
-@pytest.mark.parametrize("room", [0, 1, 4])
+@pytest.mark.parametrize("room", [0, 1, 4, topk.CANDIDATES])   # and 403 for the length of the list
 @pytest.mark.parametrize("memory", ["other", "none", "own"])
 def test_selection(room, memory, monkeypatch):
     monkeypatch.setattr(topk, "CANDIDATES", room)
