@@ -27,7 +27,9 @@
 // of the dependent chain: factorising redundantly takes the place of an arrival counter, a memory
 // fence, a lone last CTA and a second round trip through memory, and the second launch is
 // released early (programmatic dependent launch) so that only its wait remains. Both launches
-// together, before and after: 21 factors of ResNet-18 at rank 2 12.3 / 9.3 us, 50257 x 16 43 / 24 us.
+// together, before and after: 21 factors of ResNet-18 at rank 2 12.3 / 9.3 us, 50257 x 16 43 / 24 us; with the factorisation as
+// a loop, loads in batches and rows by way of shared memory 50257 x 1024 at rank 16 445 -> 433 us per pass, 4 x 1024^2 at rank 8
+// 57.8 -> 55.3.
 //
 // Multi-GPU: the factor to orthonormalise is the SUM over workers of what the previous product
 // launch pushed into this rank's slot arena. The first launch is then also the consumer of that
@@ -172,15 +174,34 @@ __device__ __forceinline__ void chunk_pairs(const float* a, const float* b, int 
       }
       __syncthreads();
     }
-    // [NG][NP] group sums in the staging buffer (NG * NP = 16 * ORTH_THREADS doubles)
-    static_assert(NG * NP == 2 * ORTH_STAGE_ROWS_X_RT || RT < 8, "group sums must fill the staging buffer");
+    // sums over the row groups of a warp (its lanes GW apart hold the same pairs), then over the warps
+    constexpr int GW = NB * NB < 32 ? NB * NB : 32;
+    constexpr int LEFT = 16 * GW / 32 < 1 ? 1 : 16 * GW / 32;   // values a lane ends up with
+    int off = 16;
 #pragma unroll
-    for (int e = 0; e < 16; ++e) stage[g * NP + (j0 + (e >> 2)) * RT + k0 + (e & 3)] = acc[e];
+    for (int n = 16; n > LEFT; n >>= 1, off >>= 1) {
+      const bool upper = (tid & off) != 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (i < n / 2) {
+          const double keep = upper ? acc[i + n / 2] : acc[i], send = upper ? acc[i] : acc[i + n / 2];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      }
+    }
+    const int e0 = GW < 32 ? (tid & 31) / GW * LEFT : 0;   // the first of them
+    constexpr int SETS = GW < 32 ? ORTH_WARPS : NG;        // (RT = 32: the groups are whole warps apart)
+    const int set = GW < 32 ? tid >> 5 : g;
+#pragma unroll
+    for (int i = 0; i < LEFT; ++i) {
+      const int e = e0 + i;
+      stage[set * NP + (j0 + (e >> 2)) * RT + k0 + (e & 3)] = acc[i];
+    }
     __syncthreads();
     for (int p = tid; p < NP; p += ORTH_THREADS) {
       double s = 0.0;
-#pragma unroll 4
-      for (int gg = 0; gg < NG; ++gg) s += stage[gg * NP + p];
+#pragma unroll
+      for (int w = 0; w < SETS; ++w) s += stage[w * NP + p];
       out[p] = s;
     }
     __syncthreads();
@@ -245,35 +266,56 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_gram_kernel(OrthArgs a
 }
 
 // ---- factorisation ---------------------------------------------------------------------------
-// R upper triangular with R^T R = G (row-major in sR, zero below the diagonal) and sDiagInv =
-// 1 / R[c][c], by one warp. What bounds it is the chain of r pivots, each a float64 reciprocal
-// square root followed by the update that the next pivot needs. So lane j keeps column j of the
-// trailing matrix in registers and every step updates all of it at once (right-looking); only the
-// row of R just finished goes through shared memory.
-// False when a pivot is not above the rounding noise of its column (or is not a number).
+// R upper triangular with R^T R = G (row-major in sR, zero below the diagonal) and sDiagInv = 1 / R[c][c]; by one warp up to
+// RT = 4, by the whole block above. A thread has one entry of the trailing matrix (four at RT = 32); a step hands the
+// row just finished round through shared memory, and the rows are scaled by their pivots' square roots together at the end.
+// What bounds it is not the chain of r pivots but fetching its code, which runs once per launch: with a column per lane
+// in registers the r steps have to be unrolled, some 1250 cycles for each of 16 columns, nearly all of them
+// instruction misses. As a loop: 5800 -> 1600 cycles at RT = 4, 12200 -> 2600 at 8, 24700 -> 4100 at 16.
+// False (in all threads that take part) when a pivot is not above the rounding noise of its column (or is not a number).
 template <int RT>
-__device__ __forceinline__ bool orth_cholesky(const double* sG, double* sR, double* sDiagInv, int r, int lane) {
-  double col[RT];
+__device__ __forceinline__ bool orth_cholesky(const double* sG, double* sR, double* sDiagInv, int r, int tid) {
+  constexpr int NP = RT * RT, PER = NP > ORTH_THREADS ? NP / ORTH_THREADS : 1;
+  auto sync = [] {
+    if (RT <= 4) __syncwarp();
+    else __syncthreads();
+  };
+  double v[PER];
 #pragma unroll
-  for (int i = 0; i < RT; ++i) col[i] = lane < RT ? sG[i * RT + lane] : 0.0;
-  bool ok = true;
+  for (int k = 0; k < PER; ++k) v[k] = tid + k * ORTH_THREADS < NP ? sG[tid + k * ORTH_THREADS] : 0.0;
+#pragma unroll 1
+  for (int c = 0; c < r; ++c) {
 #pragma unroll
-  for (int c = 0; c < RT; ++c) {
-    if (c < r && ok) {
-      const double s = __shfl_sync(0xffffffffu, col[c], c);
-      const double ref = sG[c * RT + c];
-      ok = (ref > 0.0) && (s > 1e-12 * ref);
-      const double inv = rsqrt(s);
-      const double v = lane >= c ? col[c] * inv : 0.0;
-      if (lane < RT) sR[c * RT + lane] = v;
-      if (lane == 0) sDiagInv[c] = inv;
-      __syncwarp();
+    for (int k = 0; k < PER; ++k) {
+      const int e = tid + k * ORTH_THREADS;
+      if (e / RT == c) sR[e] = v[k];
+    }
+    sync();
+    const double ref = sG[c * RT + c], piv = sR[c * RT + c];
+    if (!((ref > 0.0) && (piv > 1e-12 * ref))) return false;
+    const double inv = 1.0 / piv;
 #pragma unroll
-      for (int i = c + 1; i < RT; ++i) col[i] = fma(-sR[c * RT + i], v, col[i]);
+    for (int k = 0; k < PER; ++k) {
+      const int e = tid + k * ORTH_THREADS;
+      if (e < NP) v[k] = fma(-(sR[c * RT + e / RT] * inv), sR[c * RT + e % RT], v[k]);   // (rows up to c: of no use any more)
     }
   }
-  __syncwarp();
-  return ok;
+  sync();
+  double scale[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int e = tid + k * ORTH_THREADS, row = e / RT;
+    scale[k] = e < NP && row < r ? rsqrt(sR[row * RT + row]) : 0.0;
+    v[k] = e < NP && row < r && e % RT >= row ? sR[e] * scale[k] : 0.0;
+  }
+  sync();
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int e = tid + k * ORTH_THREADS;
+    if (e < NP) sR[e] = v[k];
+    if (e < NP && e / RT == e % RT && e / RT < r) sDiagInv[e / RT] = scale[k];
+  }
+  return true;
 }
 
 // The same with canonical vectors in the place of columns that are noise: sDead[c] = -1 for a column
@@ -346,6 +388,20 @@ __device__ __noinline__ void orth_cholesky_substituting(double* sG, double* sR, 
   }
 }
 
+// The two together, block-wide; sDead is set. Ends with a barrier.
+template <int RT>
+__device__ __forceinline__ void orth_factorise(double* sG, double* sR, double* sDiagInv, int* sDead, int r, const float* head, long long len, int tid) {
+  if (tid < RT) sDead[tid] = -1;
+  bool ok = true;
+  if (RT > 4 || tid < 32) ok = orth_cholesky<RT>(sG, sR, sDiagInv, r, tid);
+  if (!ok) {
+    if (RT > 4) __syncthreads();   // everybody has read the pivot that failed
+    __syncwarp();
+    if (tid < 32) orth_cholesky_substituting<RT>(sG, sR, sDiagInv, sDead, r, head, len, tid);
+  }
+  __syncthreads();
+}
+
 // v <- v R^-1 for one row of RT values (columns beyond r are zero and stay so).
 template <int RT>
 __device__ __forceinline__ void orth_solve_row(double* v, const double* sR, const double* sDiagInv, int r) {
@@ -368,8 +424,14 @@ __device__ __forceinline__ void orth_sum_chunks(const double* first, long long s
   for (int p = tid; p < NP * PARTS; p += ORTH_THREADS) {
     const int e = p % NP, part = p / NP;
     double s = 0.0;
-#pragma unroll 8
-    for (int c = part; c < nchunks; c += PARTS) s += __ldcg(first + c * stride + e);
+    constexpr int B = 16;   // loads under way
+    for (int c = part; c < nchunks; c += B * PARTS) {
+      double q[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) q[j] = c + j * PARTS < nchunks ? __ldcg(first + (c + j * PARTS) * stride + e) : 0.0;
+#pragma unroll
+      for (int j = 0; j < B; ++j) s += q[j];
+    }
     if (PARTS == 1) sOut[e] = s;
     else red[p] = s;
   }
@@ -385,6 +447,126 @@ __device__ __forceinline__ void orth_sum_chunks(const double* first, long long s
   }
 }
 
+// X <- X' R^-1 on the rows of a CTA at RT >= 8, one row per thread. The rows pass through shared memory (`tile`, orth_tile_rows
+// of them), so that global memory sees whole lines: a thread that reads and writes its own row of 16 floats by single
+// accesses touches a line with each (50257 x 16: 20 000 -> 13 400 cycles for the 640 rows of a chunk). As everywhere in these launches code that runs once or twice costs some 5 cycles per
+// instruction to be fetched: what is not the usual case (a rank below RT) is left to loops.
+template <int RT>
+__host__ __device__ constexpr int orth_tile_pitch() { return RT + 1; }   // odd: no two rows of a warp in one bank
+template <int RT>
+__host__ __device__ constexpr int orth_tile_rows() { return RT <= 16 ? ORTH_THREADS : ORTH_THREADS / 2; }
+template <int RT>
+__host__ __device__ constexpr int orth_tile_floats() { return orth_tile_rows<RT>() * orth_tile_pitch<RT>(); }
+// Values of a tile per thread; at r = RT they are fetched into registers, a tile ahead.
+template <int RT>
+__host__ __device__ constexpr int orth_tile_values() { return orth_tile_rows<RT>() * RT / ORTH_THREADS; }
+template <int RT>
+__device__ __forceinline__ void orth_tile_fetch(const float* x, int rows, int r, float* q, int tid) {
+  if (r != RT) return;
+#pragma unroll
+  for (int j = 0; j < orth_tile_values<RT>(); ++j) q[j] = tid + j * ORTH_THREADS < rows * RT ? x[tid + j * ORTH_THREADS] : 0.f;
+}
+template <int RT>
+__device__ __forceinline__ void orth_solve_rows(float* x, float* x2, int row0, int rows, int r, const double* sR, const double* sDiagInv,
+                                                const int* sDead, float* ahead, float* tile, int tid) {
+  constexpr int T = orth_tile_rows<RT>(), TP = orth_tile_pitch<RT>(), STEP = ORTH_THREADS / RT * TP;
+  float* mine = tile + tid / RT * TP + tid % RT;   // of the values that this thread moves at r = RT
+#pragma unroll 1
+  for (int first = 0; first < rows; first += T) {
+    const int n = min(T, rows - first);
+    float* to = x + (long long)first * r;
+    float* to2 = x2 ? x2 + (long long)first * r : nullptr;
+    if (r == RT) {
+#pragma unroll
+      for (int j = 0; j < orth_tile_values<RT>(); ++j) mine[j * STEP] = ahead[j];   // (zeros beyond the last row)
+      if (first + T < rows) orth_tile_fetch<RT>(to + T * RT, min(T, rows - first - T), r, ahead, tid);
+    } else {
+#pragma unroll 4
+      for (int e = tid; e < n * r; e += ORTH_THREADS) tile[e / r * TP + e % r] = to[e];
+    }
+    __syncthreads();
+    if (tid < n) {
+      float* row = tile + tid * TP;
+      double v[RT];
+#pragma unroll
+      for (int k = 0; k < RT; ++k) {
+        v[k] = k < r ? (double)row[k] : 0.0;
+        if (k < r && sDead[k] != -1) v[k] = sDead[k] == row0 + first + tid ? 1.0 : 0.0;
+      }
+      orth_solve_row<RT>(v, sR, sDiagInv, r);
+#pragma unroll
+      for (int k = 0; k < RT; ++k)
+        if (k < r) row[k] = (float)v[k];
+    }
+    __syncthreads();
+    if (r == RT) {
+#pragma unroll
+      for (int j = 0; j < orth_tile_values<RT>(); ++j) {
+        const int e = tid + j * ORTH_THREADS;
+        if (e < n * RT) {
+          const float q = mine[j * STEP];
+          to[e] = q;
+          if (to2) to2[e] = q;
+        }
+      }
+    } else {
+#pragma unroll 1
+      for (int e = tid; e < n * r; e += ORTH_THREADS) {
+        const float q = tile[e / r * TP + e % r];
+        to[e] = q;
+        if (to2) to2[e] = q;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The same at RT <= 4: a row that a thread holds already.
+template <int RT>
+__device__ __forceinline__ void orth_row_solve(double* v, float* xr, float* xr2, int row, int r, const double* sR, const double* sDiagInv,
+                                               const int* sDead) {
+#pragma unroll
+  for (int k = 0; k < RT; ++k)
+    if (k < r && sDead[k] != -1) v[k] = sDead[k] == row ? 1.0 : 0.0;
+  orth_solve_row<RT>(v, sR, sDiagInv, r);
+  if (RT == 4 && r == 4 && (((uintptr_t)xr | (uintptr_t)xr2) & 15u) == 0) {
+    const float4 q = make_float4((float)v[0], (float)v[1 % RT], (float)v[2 % RT], (float)v[3 % RT]);
+    *reinterpret_cast<float4*>(xr) = q;
+    if (xr2) *reinterpret_cast<float4*>(xr2) = q;
+  } else if (RT == 2 && r == 2 && (((uintptr_t)xr | (uintptr_t)xr2) & 7u) == 0) {
+    const float2 q = make_float2((float)v[0], (float)v[1 % RT]);
+    *reinterpret_cast<float2*>(xr) = q;
+    if (xr2) *reinterpret_cast<float2*>(xr2) = q;
+  } else {
+#pragma unroll
+    for (int c = 0; c < RT; ++c)
+      if (c < r) {
+        xr[c] = (float)v[c];
+        if (xr2) xr2[c] = (float)v[c];
+      }
+  }
+}
+
+// C = (F^T X') R^-1 from sG = F^T X, X' = X with the substituted columns; f: the unit's part of F.
+template <int RT>
+__device__ __forceinline__ void orth_publish(const double* sG, const float* f, float* cmat, int first_mat, int r, const double* sR,
+                                             const double* sDiagInv, const int* sDead, int tid) {
+  if (tid >= r) return;
+  const double* v = sG + tid * RT;
+  const auto value = [&](int k) {   // (column k of X' may be the basis vector e_d)
+    const int d = sDead[k];
+    return d == -1 ? v[k] : d >= 0 ? (double)f[(long long)d * r + tid] : 0.0;
+  };
+  double w[RT];
+#pragma unroll
+  for (int k = 0; k < RT; ++k) w[k] = k < r ? value(k) : 0.0;
+  orth_solve_row<RT>(w, sR, sDiagInv, r);
+  float* cm = cmat + (long long)first_mat * PSGD_CMAT_STRIDE + tid * r;
+#pragma unroll
+  for (int k = 0; k < RT; ++k)
+    if (k < r) cm[k] = (float)w[k];
+}
+
 // Second launch: X <- X' R^-1 (rank 1: X / d) on every row chunk, optionally mirrored to copy_to.
 template <int RT>
 __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs a) {
@@ -393,7 +575,7 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs 
   const PsgdOrthUnit u = a.units[ch.unit];
   const int r = u.r;
   const int tid = threadIdx.x;
-  __shared__ double sG[NP], sR[NP], sDiagInv[RT], red[ORTH_THREADS];
+  __shared__ __align__(16) double sG[NP], sR[NP], sDiagInv[RT], red[ORTH_THREADS];
   __shared__ int sDead[RT];
   float* x = a.x + u.x_off;
   float* x2 = a.copy_to ? a.copy_to + u.x_off : nullptr;
@@ -424,67 +606,32 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs 
     return;
   }
 
-  // the first row's values travel while one warp factorises
-  const bool has = tid < ch.rows;
-  float* xr = x + (long long)(ch.row0 + tid) * r;
-  double v[RT];
-  if (has) orth_load_row<RT>(xr, r, v);
-  if (tid < 32) {
-    if (tid < RT) sDead[tid] = -1;
-    __syncwarp();
-    if (!orth_cholesky<RT>(sG, sR, sDiagInv, r, tid))
-      orth_cholesky_substituting<RT>(sG, sR, sDiagInv, sDead, r, a.head + (long long)ch.unit * 2 * NP, (long long)u.sub_len * u.nsub, tid);
+  // the first rows travel while the sum is factorised
+  double v[RT <= 4 ? RT : 1];
+  __shared__ float tile[RT <= 4 ? 1 : orth_tile_floats<RT>()];
+  float ahead[RT <= 4 ? 1 : orth_tile_values<RT>()];
+  float* xc = x + (long long)ch.row0 * r;
+  float* xc2 = x2 ? x2 + (long long)ch.row0 * r : nullptr;
+  if constexpr (RT <= 4) {
+    if (tid < ch.rows) orth_load_row<RT>(xc + (long long)tid * r, r, v);
+  } else {
+    orth_tile_fetch<RT>(xc, min(orth_tile_rows<RT>(), ch.rows), r, ahead, tid);
   }
-  __syncthreads();
-  for (int lr = tid; lr < ch.rows; lr += ORTH_THREADS) {
-    const int row = ch.row0 + lr;
-    xr = x + (long long)row * r;
-    if (lr != tid) orth_load_row<RT>(xr, r, v);
-#pragma unroll
-    for (int k = 0; k < RT; ++k)
-      if (k < r && sDead[k] != -1) v[k] = sDead[k] == row ? 1.0 : 0.0;
-    orth_solve_row<RT>(v, sR, sDiagInv, r);
-    float* xr2 = x2 ? x2 + (long long)row * r : nullptr;
-    if (RT == 4 && r == 4 && (((uintptr_t)xr | (uintptr_t)xr2) & 15u) == 0) {
-      const float4 q = make_float4((float)v[0], (float)v[1 % RT], (float)v[2 % RT], (float)v[3 % RT]);
-      *reinterpret_cast<float4*>(xr) = q;
-      if (xr2) *reinterpret_cast<float4*>(xr2) = q;
-    } else if (RT == 2 && r == 2 && (((uintptr_t)xr | (uintptr_t)xr2) & 7u) == 0) {
-      const float2 q = make_float2((float)v[0], (float)v[1 % RT]);
-      *reinterpret_cast<float2*>(xr) = q;
-      if (xr2) *reinterpret_cast<float2*>(xr2) = q;
-    } else {
-#pragma unroll
-      for (int c = 0; c < RT; ++c)
-        if (c < r) {
-          xr[c] = (float)v[c];
-          if (xr2) xr2[c] = (float)v[c];
-        }
+  orth_factorise<RT>(sG, sR, sDiagInv, sDead, r, a.head + (long long)ch.unit * 2 * NP, (long long)u.sub_len * u.nsub, tid);
+  if constexpr (RT <= 4) {
+    for (int lr = tid; lr < ch.rows; lr += ORTH_THREADS) {
+      float* xr = xc + (long long)lr * r;
+      if (lr != tid) orth_load_row<RT>(xr, r, v);
+      orth_row_solve<RT>(v, xr, xc2 ? xc2 + (long long)lr * r : nullptr, ch.row0 + lr, r, sR, sDiagInv, sDead);
     }
+  } else {
+    orth_solve_rows<RT>(xc, xc2, ch.row0, ch.rows, r, sR, sDiagInv, sDead, ahead, tile, tid);
   }
-  // ---- cross products C_p = (F_p^T X') R^-1, X' = X with the substituted columns: chunk p of the unit
-  //      (modulo their number) has factor p ----
+  // ---- cross products: chunk p of the unit (modulo their number) has factor p ----
   for (int p = ci; p < a.nprev; p += u.nchunks) {
-    const float* f = a.prev[p] + u.x_off;
     __syncthreads();
     orth_sum_chunks<RT>(unit_part + (long long)(1 + p) * NP, stride, u.nchunks, red, sG, tid);
-    if (tid < r) {
-#pragma unroll
-      for (int k = 0; k < RT; ++k) {
-        double s = 0.0;
-        if (k < r) {
-          const int d = sDead[k];
-          if (d == -1) s = sG[tid * RT + k];
-          else if (d >= 0) s = (double)f[(long long)d * r + tid];  // column k of X' is the basis vector e_d
-        }
-        v[k] = s;
-      }
-      orth_solve_row<RT>(v, sR, sDiagInv, r);
-      float* cm = a.cmat[p] + (long long)u.first_mat * PSGD_CMAT_STRIDE + tid * r;
-#pragma unroll
-      for (int k = 0; k < RT; ++k)
-        if (k < r) cm[k] = (float)v[k];
-    }
+    orth_publish<RT>(sG, a.prev[p] + u.x_off, a.cmat[p], u.first_mat, r, sR, sDiagInv, sDead, tid);
   }
 }
 
