@@ -635,6 +635,293 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_apply_kernel(OrthArgs 
   }
 }
 
+// ---- one launch for both: a cluster of CTAs per unit -------------------------------------------
+// What the two launches above spend on a short factor is mostly not theirs: the second one's start, the way of
+// the partial sums through memory, and a second read of the rows. Here a cluster of ORTH_CLUSTER CTAs holds
+// a unit: every CTA multiplies its rows, puts its partial matrices into the shared memory of all (of the one that publishes,
+// for cross products), and after one cluster barrier everybody adds them in the order of the CTAs, factorises and
+// solves the rows that it still has in registers (RT <= 4) or in L2. One worker only; units as psgd_orth_takes_clusters
+// allows. Of the some 3 us that are left at RT = 4 a quarter each goes to the products, the exchange, the factorisation and the
+// solution. us per pass, two launches / one: 3 x 1001x777 + 2 x 515x2049 at rank 3 x 3 114.7 / 99.6, ResNet-18's recorded step
+// 112.5 / 108.4, 4 x 4096^2 at 4 x 2 378 / 369, 4 x 1024^2 at 8 x 1 55.3 / 54.2.
+// `same`: the last earlier factor holds what x holds on entry, so its cross products are the Gram matrix.
+constexpr int ORTH_CLUSTER = 8;
+
+__device__ __forceinline__ uint32_t orth_cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void orth_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void orth_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// *p = v in the shared memory of CTA `rank` of the cluster, where `p` is this CTA's address of it.
+__device__ __forceinline__ void orth_put(double* p, uint32_t rank, double v) {
+  uint32_t at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+
+// Sums of N doubles over the lanes, as warp_sums in lowrank_ffma.cu: value i ends up in the lanes whose top log2(N) bits spell i.
+template <int N>
+__device__ __forceinline__ double orth_warp_sums(double (&v)[N], int lane) {
+  int off = 16;
+#pragma unroll
+  for (int n = N; n > 1; n >>= 1, off >>= 1) {
+    const bool upper = (lane & off) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      if (i < n / 2) {
+        const double keep = upper ? v[i + n / 2] : v[i], send = upper ? v[i] : v[i + n / 2];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+    }
+  }
+  double s = v[0];
+#pragma unroll
+  for (; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  return s;
+}
+
+template <int RT>
+__host__ __device__ constexpr int orth_kept_rows() { return RT == 1 ? 8 : 4; }   // per thread, RT <= 4
+constexpr int ORTH_CLUSTER_SUBS = 64;   // cross products of whole sub-matrices that a CTA can have
+// Shared memory in doubles: stage of the products; partial matrices of this CTA's rows; slots of the cluster for the
+// Gram matrix and for the cross products that this CTA publishes; R and what belongs to it.
+template <int RT>
+__host__ __device__ constexpr int orth_stage_doubles() { return RT <= 4 ? ORTH_WARPS * RT * RT * PSGD_MAX_HIST : 2 * ORTH_STAGE_ROWS_X_RT; }
+template <int RT>
+__host__ __device__ constexpr int orth_cluster_doubles() {
+  return orth_stage_doubles<RT>() + (RT <= 4 ? 0 : PSGD_MAX_HIST * RT * RT) + 2 * ORTH_CLUSTER * RT * RT + 2 * RT * RT + RT + ORTH_CLUSTER_SUBS;
+}
+
+template <int RT>
+__global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_cluster_kernel(OrthArgs a, int same) {
+  constexpr int NP = RT * RT, CL = ORTH_CLUSTER;
+  extern __shared__ __align__(16) double orth_smem[];
+  double* stage = orth_smem;                                           // products; later the tile of rows (RT >= 8)
+  double* mine = stage + orth_stage_doubles<RT>();                     // [1 + nprev][NP] (RT >= 8)
+  double* slots = mine + (RT <= 4 ? 0 : PSGD_MAX_HIST * NP);           // [CL][NP]
+  double* cross = slots + CL * NP;                                     // [CL][NP]
+  double* sG = cross + CL * NP;
+  double* sR = sG + NP;
+  double* sDiagInv = sR + NP;
+  double* subs = sDiagInv + RT;                                        // [ORTH_CLUSTER_SUBS]
+  __shared__ int sDead[RT];
+  const int ui = (int)blockIdx.x / CL;
+  const PsgdOrthUnit u = a.units[ui];
+  const uint32_t rank = orth_cluster_rank();
+  const int r = u.r, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // rows of this CTA: a share of the unit; whole sub-matrices where there are several
+  const int len = u.sub_len * u.nsub;
+  const int per = u.nsub > 1 ? (u.nsub + CL - 1) / CL * u.sub_len : ((len + CL - 1) / CL + 3) / 4 * 4;
+  const int row0 = min((int)rank * per, len), rows = min(per, len - row0);
+  psgd_launch_dependents();
+#ifdef PSGD_BOUNDS_CHECK
+  {
+    bool ok = true;   // the same verdict in all CTAs of a cluster
+    ok &= PSGD_BC(r >= 1 && r <= RT, 5, PSGD_BC_RANK, r, RT);
+    ok &= PSGD_BC(u.sub_len > 0 && u.nsub > 0 && (u.nsub == 1 || (r == 1 && (u.nsub + CL - 1) / CL * a.nprev <= ORTH_CLUSTER_SUBS)), 5, PSGD_BC_CHUNK, u.nsub, CL);
+    ok &= PSGD_BC(a.nprev < CL, 5, PSGD_BC_CHUNK, a.nprev, CL);
+    if (!ok) return;
+  }
+#endif
+  orth_cluster_arrive();   // all CTAs run: their shared memory may be written
+  psgd_wait_for_predecessor();
+  float* x = a.x + u.x_off + (long long)row0 * r;
+  float* x2 = a.copy_to ? a.copy_to + u.x_off + (long long)row0 * r : nullptr;
+  const int crosses = a.nprev - same;   // products of their own
+  {
+    const int head_rows = min(2 * r - row0, rows);
+    float* head = a.head + (long long)ui * 2 * NP + (long long)row0 * r;
+    for (int e = tid; e < head_rows * r; e += ORTH_THREADS) head[e] = x[e];
+  }
+
+  if (u.nsub > 1) {
+    // cross products of whole sub-matrices (r = 1): one warp for each of them and each factor
+    for (int e = warp; e < rows / u.sub_len * a.nprev; e += ORTH_WARPS) {
+      const int s = e / a.nprev, p = e % a.nprev;
+      const float* f = a.prev[p] + u.x_off + row0 + s * u.sub_len;
+      const float* g = x + s * u.sub_len;
+      double t = 0.0;
+#pragma unroll 8
+      for (int i = lane; i < u.sub_len; i += 32) t = fma((double)f[i], (double)g[i], t);
+      t = psgd_warp_sum(t);
+      if (lane == 0) subs[e] = t;
+    }
+  }
+  constexpr int KEPT = RT <= 4 ? orth_kept_rows<RT>() : 1;
+  float kept[KEPT][RT <= 4 ? RT : 1];   // this thread's first rows of x
+  if constexpr (RT <= 4) {
+    const bool wide = (RT == 4 && r == 4 && ((uintptr_t)x & 15u) == 0) || (RT == 2 && r == 2 && ((uintptr_t)x & 7u) == 0);
+    auto row_of = [&](const float* base, bool aligned, int row, float* v) {
+      if (RT == 4 && aligned) {
+        const float4 q = *reinterpret_cast<const float4*>(base + (long long)row * 4);
+        v[0] = q.x; v[1 % RT] = q.y; v[2 % RT] = q.z; v[3 % RT] = q.w;
+      } else if (RT == 2 && aligned) {
+        const float2 q = *reinterpret_cast<const float2*>(base + (long long)row * 2);
+        v[0] = q.x; v[1 % RT] = q.y;
+      } else {
+#pragma unroll
+        for (int c = 0; c < RT; ++c) v[c] = c < r ? base[(long long)row * r + c] : 0.f;
+      }
+    };
+    double acc[NP];
+    auto add = [&](const float* f, const float* g) {
+#pragma unroll
+      for (int e = 0; e < NP; ++e) acc[e] = fma((double)f[e / RT], (double)g[e % RT], acc[e]);
+    };
+    auto close = [&](int p) {
+      const double s = orth_warp_sums<NP>(acc, lane);
+      if (lane % (32 / NP) == 0) stage[(p * ORTH_WARPS + warp) * NP + lane / (32 / NP)] = s;
+#pragma unroll
+      for (int e = 0; e < NP; ++e) acc[e] = 0.0;
+    };
+#pragma unroll
+    for (int e = 0; e < NP; ++e) acc[e] = 0.0;
+#pragma unroll
+    for (int i = 0; i < KEPT; ++i) {
+#pragma unroll
+      for (int c = 0; c < RT; ++c) kept[i][c] = 0.f;
+      if (tid + i * ORTH_THREADS < rows) row_of(x, wide, tid + i * ORTH_THREADS, kept[i]);
+    }
+    float first[KEPT][RT];   // the same rows of the first earlier factor travel beside them
+    if (crosses > 0 && u.nsub == 1) {
+      const float* f = a.prev[0] + u.x_off + (long long)row0 * r;
+#pragma unroll
+      for (int i = 0; i < KEPT; ++i) {
+#pragma unroll
+        for (int c = 0; c < RT; ++c) first[i][c] = 0.f;
+        if (tid + i * ORTH_THREADS < rows) row_of(f, false, tid + i * ORTH_THREADS, first[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < KEPT; ++i) add(kept[i], kept[i]);
+    for (int row = tid + KEPT * ORTH_THREADS; row < rows; row += ORTH_THREADS) {
+      float v[RT];
+      row_of(x, wide, row, v);
+      add(v, v);
+    }
+    close(0);
+    if (u.nsub == 1) {
+      for (int p = 0; p < crosses; ++p) {
+        const float* f = a.prev[p] + u.x_off + (long long)row0 * r;
+        if (p == 0) {
+#pragma unroll
+          for (int i = 0; i < KEPT; ++i) add(first[i], kept[i]);
+        }
+        for (int row = tid + (p == 0 ? KEPT * ORTH_THREADS : 0); row < rows; row += ORTH_THREADS) {
+          float v[RT], w[RT];
+          row_of(f, false, row, w);
+          row_of(x, wide, row, v);
+          add(w, v);
+        }
+        close(1 + p);
+      }
+    }
+    __syncthreads();
+    orth_cluster_wait();
+    if (tid < NP * CL) {
+      const int e = tid % NP;
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < ORTH_WARPS; ++w) s += stage[w * NP + e];
+      orth_put(slots + rank * NP + e, tid / NP, s);
+    }
+    if (u.nsub == 1) {
+      for (int e = tid; e < crosses * NP; e += ORTH_THREADS) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < ORTH_WARPS; ++w) s += stage[((1 + e / NP) * ORTH_WARPS + w) * NP + e % NP];
+        orth_put(cross + rank * NP + e % NP, e / NP, s);
+      }
+    }
+  } else {
+    chunk_pairs<RT>(x, x, r, max(rows, 0), stage, mine, tid);
+    for (int p = 0; p < crosses && u.nsub == 1; ++p)
+      chunk_pairs<RT>(a.prev[p] + u.x_off + (long long)row0 * r, x, r, max(rows, 0), stage, mine + (1 + p) * NP, tid);
+    orth_cluster_wait();
+    for (int e = tid; e < NP * CL; e += ORTH_THREADS) orth_put(slots + rank * NP + e % NP, e / NP, mine[e % NP]);
+    for (int e = tid; e < crosses * NP && u.nsub == 1; e += ORTH_THREADS) orth_put(cross + rank * NP + e % NP, e / NP, mine[NP + e]);
+  }
+  orth_cluster_arrive();
+  float ahead[RT <= 4 ? 1 : orth_tile_values<RT>()];
+  if constexpr (RT > 4) orth_tile_fetch<RT>(x, min(orth_tile_rows<RT>(), rows), r, ahead, tid);
+  orth_cluster_wait();   // every partial matrix is there, and every CTA has copied its rows of `head`
+  for (int e = tid; e < NP; e += ORTH_THREADS) {
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < CL; ++c) s += slots[c * NP + e];
+    sG[e] = s;
+  }
+  __syncthreads();
+
+  if (RT == 1 || r == 1) {
+    const float d = fmaxf((float)sqrt(sG[0]), 1e-16f);   // joint Frobenius norm, float32 semantics of the division
+    auto put = [&](int i, float q) {
+      q = q / d;
+      x[i] = q;
+      if (x2) x2[i] = q;
+    };
+    if constexpr (RT <= 4) {
+#pragma unroll
+      for (int i = 0; i < KEPT; ++i)
+        if (tid + i * ORTH_THREADS < rows) put(tid + i * ORTH_THREADS, kept[i][0]);
+    }
+    for (int i = tid + (RT <= 4 ? KEPT * ORTH_THREADS : 0); i < rows; i += ORTH_THREADS) put(i, x[i]);
+    if (u.nsub > 1) {
+      for (int e = tid; e < rows / u.sub_len * a.nprev; e += ORTH_THREADS)
+        a.cmat[e % a.nprev][(long long)(u.first_mat + row0 / u.sub_len + e / a.nprev) * PSGD_CMAT_STRIDE] = (float)(subs[e] / (double)d);
+    } else if ((int)rank < a.nprev && tid == 0) {
+      double t = 0.0;
+      for (int c = 0; c < CL; ++c) t += ((int)rank < crosses ? cross : slots)[c * NP];
+      a.cmat[rank][(long long)u.first_mat * PSGD_CMAT_STRIDE] = (float)(t / (double)d);
+    }
+    return;
+  }
+
+  orth_factorise<RT>(sG, sR, sDiagInv, sDead, r, a.head + (long long)ui * 2 * NP, len, tid);
+  if constexpr (RT <= 4) {
+    auto solve = [&](int lr, const float* q) {
+      double v[RT];
+#pragma unroll
+      for (int c = 0; c < RT; ++c) v[c] = (double)q[c];
+      orth_row_solve<RT>(v, x + (long long)lr * r, x2 ? x2 + (long long)lr * r : nullptr, row0 + lr, r, sR, sDiagInv, sDead);
+    };
+#pragma unroll
+    for (int i = 0; i < KEPT; ++i)
+      if (tid + i * ORTH_THREADS < rows) solve(tid + i * ORTH_THREADS, kept[i]);
+    for (int lr = tid + KEPT * ORTH_THREADS; lr < rows; lr += ORTH_THREADS) {
+      float q[RT];
+#pragma unroll
+      for (int c = 0; c < RT; ++c) q[c] = c < r ? x[(long long)lr * r + c] : 0.f;
+      solve(lr, q);
+    }
+  } else {
+    orth_solve_rows<RT>(x, x2, row0, rows, r, sR, sDiagInv, sDead, ahead, reinterpret_cast<float*>(stage), tid);
+  }
+  if ((int)rank < a.nprev) {
+    __syncthreads();   // nobody reads the Gram matrix any more
+    for (int e = tid; e < NP; e += ORTH_THREADS) {
+      double s = 0.0;
+#pragma unroll
+      for (int c = 0; c < CL; ++c) s += ((int)rank < crosses ? cross : slots)[c * NP + e];
+      sG[e] = s;
+    }
+    __syncthreads();
+    orth_publish<RT>(sG, a.prev[rank] + u.x_off, a.cmat[rank], u.first_mat, r, sR, sDiagInv, sDead, tid);
+  }
+}
+
+template <int RT>
+static int orth_cluster_launch(const OrthArgs& a, int nunits, int same, int early, cudaStream_t stream) {
+  const size_t smem = (size_t)orth_cluster_doubles<RT>() * sizeof(double);
+  if (smem > 48 * 1024) {
+    static unsigned long long devices = 0;   // per instantiation
+    if (const int code = psgd_allow_shared((const void*)psgd_orth_cluster_kernel<RT>, smem, devices)) return code;
+  }
+  return psgd_launch_clusters(psgd_orth_cluster_kernel<RT>, nunits * ORTH_CLUSTER, ORTH_THREADS, smem, stream, early, ORTH_CLUSTER, a, same);
+}
+
 template <int RT>
 static int orth_launch_rt(const OrthArgs& a, int nchunks, int early, cudaStream_t stream) {
   const int rc = psgd_launch(psgd_orth_gram_kernel<RT>, nchunks, ORTH_THREADS, 0, stream, early & 1, a);
@@ -670,6 +957,17 @@ PSGD_API int psgd_orth_chunk_rows(int max_r, long long longest) {
     default: return orth_chunk_rows<32>(longest);
   }
 }
+// Whether one launch with a cluster per unit is the faster one for a list whose longest unit has `longest` rows in at most `subs`
+// sub-matrices, with `nprev` earlier factors. A cluster has eight SMs for a unit however long it is, the two launches have
+// one per chunk. us, two launches / one, 1 and 24 units: rank 1, 4096 rows 3.9 / 2.4 and 4.8 / 2.8, 16384 4.3 / 2.7 and 5.9 / 3.2, 24000
+// 4.3 / 4.9; rank 2, 4096 4.7 / 3.0 and 5.9 / 3.4, 12288 5.0 / 4.4 and 6.3 / 5.5, 24000 5.1 / 7.1; rank 4, 1024 5.7 / 3.3 and 6.7 / 3.6, 12288
+// 6.3 / 5.5 and 10.4 / 6.9, 16384 6.4 / 6.8; rank 8, 1024 6.5 / 5.0 and 8.3 / 5.8, 2048 6.7 / 5.5 and 7.9 / 6.7, 4096 6.9 / 7.6 and 11.4 / 9.4;
+// rank 16, 1024 8.5 / 7.7 and 10.2 / 9.5, 2048 9.0 / 9.5 and 15.1 / 12.4.
+PSGD_API int psgd_orth_takes_clusters(int max_r, long long longest, int subs, int nprev) {
+  const int rt = psgd_orth_template_rank(max_r);
+  if (rt > 16 || nprev >= ORTH_CLUSTER || (subs > 1 && (subs + ORTH_CLUSTER - 1) / ORTH_CLUSTER * nprev > ORTH_CLUSTER_SUBS)) return 0;
+  return longest <= (rt == 1 ? 16384 : rt <= 4 ? 12288 : rt == 8 ? 3072 : 1536);
+}
 // Scratch per chunk (doubles) for `nprev` earlier factors; per unit: 2 * RT*RT floats (`head`).
 PSGD_API int psgd_orth_part_doubles(int max_r, int nprev) {
   const int rt = psgd_orth_template_rank(max_r);
@@ -679,7 +977,9 @@ PSGD_API int psgd_orth_part_doubles(int max_r, int nprev) {
 // units / chunks: device tables; all units of one call share the template rank RT >= max r.
 // part: nchunks * psgd_orth_part_doubles(max_r, nprev) doubles; head: nunits * 2 * RT*RT floats.
 // comm / sum_out: see OrthArgs (null for a single worker or when x already holds the factor).
-// early: see psgd_launch; bit 0 for the first launch, bit 1 for the second, which follows it. Both are off with
+// early: see psgd_launch; bit 0 for the first launch, bit 1 for the second, which follows it; bit 2: one launch for both, a cluster per
+// unit (lists for which psgd_orth_takes_clusters says so, no channel); bit 3, with bit 2: the last earlier factor holds the values of x.
+// Bits 0 and 1 are off with
 // several workers: the first launch then waits for peers, and the CTAs of an early successor would hold
 // their places on the SMs meanwhile.
 PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks, int nchunks, int max_r, float* x,
@@ -705,6 +1005,23 @@ PSGD_API int psgd_orth_launch(const void* units, int nunits, const void* chunks,
   a.head = head;
   a.comm = (const PsgdCommDev*)comm;
   a.sum_out = sum_out;
+  if ((early & 4) != 0) {
+    const int same = (early >> 3) & 1;
+    if (comm != nullptr || nprev >= ORTH_CLUSTER || (same && nprev == 0)) {
+      psgd_set_error("psgd_orth_launch: no cluster form for a channel, %d earlier factors (same: %d)", nprev, same);
+      return -1;
+    }
+    switch (psgd_orth_template_rank(max_r)) {
+      case 1: return orth_cluster_launch<1>(a, nunits, same, early & 1, stream);
+      case 2: return orth_cluster_launch<2>(a, nunits, same, early & 1, stream);
+      case 4: return orth_cluster_launch<4>(a, nunits, same, early & 1, stream);
+      case 8: return orth_cluster_launch<8>(a, nunits, same, early & 1, stream);
+      case 16: return orth_cluster_launch<16>(a, nunits, same, early & 1, stream);
+      default:
+        psgd_set_error("psgd_orth_launch: no cluster form at rank %d", max_r);
+        return -1;
+    }
+  }
   if (comm != nullptr && sum_out == nullptr) {
     psgd_set_error("psgd_orth_launch: a channel was given without a destination for the gathered sum");
     return -1;

@@ -123,20 +123,34 @@ static inline int psgd_allow_shared(const void* kernel, size_t bytes, unsigned l
 // `early` != 0: the kernel contains the wait above and the launch directly before it in `stream` is
 // one of this library's.
 template <typename... Params, typename... Args>
-static inline int psgd_launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int early,
-                              Args&&... args) {
+static inline int psgd_launch_clusters(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int early,
+                                       int cluster, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchAttribute attrs[2];
+  int n = 0;
+  if (early) {
+    attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attrs[n].id = cudaLaunchAttributeClusterDimension;
+    attrs[n].val.clusterDim.x = (unsigned)cluster;
+    attrs[n].val.clusterDim.y = attrs[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attrs;
+  cfg.numAttrs = n;
   PSGD_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
   return 0;
+}
+template <typename... Params, typename... Args>
+static inline int psgd_launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int early,
+                              Args&&... args) {
+  return psgd_launch_clusters(kernel, grid, block, smem, stream, early, 1, static_cast<Args&&>(args)...);
 }
 
 static inline int psgd_ceil_div(int a, int b) { return (a + b - 1) / b; }

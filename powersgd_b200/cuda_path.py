@@ -374,6 +374,15 @@ class _Recordable:
 class NativeCompressor(_Recordable):
     """Runs `BasicPowerSGD.aggregate` on the GPU with the in-tree kernels."""
 
+    # sides whose factors may be orthonormalised in one launch, a cluster per unit, and those of them where that is the rule
+    _orth_clusters: Dict[str, bool] = {}
+    _orth_by_rule: Dict[str, bool] = {}
+
+    # Rows of a list from which on one launch is the rule. Below, a replayed step gains 0 to 4 us of 30 to 45 at ranks 1 to 4 (two launches /
+    # one: 784x256 34.8 / 30.7, 4 x 256^2 33.0 / 33.1 at rank 2); such steps keep the number of launches that they
+    # report, except behind an orthonormalisation ahead of time (`begin_step`: a recorded training step 101.2 / 98.2 us).
+    ORTH_CLUSTER_ROWS = 2048
+
     def __init__(self, core):
         # the owner holds this object, not the other way round: both then go when the owner is dropped, and
         # not whenever the cycle collector runs - which may be in the middle of a CUDA-graph capture,
@@ -408,11 +417,17 @@ class NativeCompressor(_Recordable):
         self.cmat = [[torch.zeros(nm * layout.CMAT_STRIDE, **f32) for _ in range(t)] for t in range(self.T)]
         rt = int(self.lib.psgd_orth_template_rank(self.tiles.max_r))
         self.units, self.chunks, self.n_units, self.n_chunks = {}, {}, {}, {}
+        self._orth_clusters, self._orth_by_rule = {}, {}
         for s in ("p", "q"):
             longest = max(((g.n if s == "p" else g.m) * (g.batch if g.r == 1 else 1) for g in self.plan.groups), default=1)
             units, chunks = self.tiles.orth_units(s, int(self.lib.psgd_orth_chunk_rows(self.tiles.max_r, longest)))
             self.units[s], self.chunks[s] = _to_device(units, self.device), _to_device(chunks, self.device)
             self.n_units[s], self.n_chunks[s] = len(units), len(chunks)
+            if world_size() == 1:
+                members = max((g.batch for g in self.plan.groups if g.r == 1), default=1)
+                self._orth_clusters[s] = bool(self.lib.psgd_orth_takes_clusters(self.tiles.max_r, longest, members, max(self.T - 1, 0)))
+                rows = sum((g.n if s == "p" else g.m) * g.batch for g in self.plan.groups)
+                self._orth_by_rule[s] = self._orth_clusters[s] and rows >= self.ORTH_CLUSTER_ROWS
         # scratch of the orthonormalisation: partial sums per chunk; per unit (`_orth_rinv`) the leading
         # rows of the factor as they came in, which R falls back on when a column has to be replaced
         part_doubles = int(self.lib.psgd_orth_part_doubles(self.tiles.max_r, max(self.T - 1, 0)))
@@ -648,7 +663,7 @@ class NativeCompressor(_Recordable):
         fn = getattr(self.lib, name)
         self._stream = _stream_ptr()
         native.check(fn(*args, self._stream), name)
-        launched = 2 if name == "psgd_orth_launch" else 1   # orthonormalisation: Gram matrices, then their use
+        launched = 2 if name == "psgd_orth_launch" and not args[-1] & 4 else 1   # orthonormalisation: Gram matrices, then their use
         self.launches += launched
         if self._tape is not None:
             self._tape.append((fn, name, args, launched))
@@ -700,11 +715,14 @@ class NativeCompressor(_Recordable):
 
     # -- phases ----------------------------------------------------------------------------
     def _orth(self, side: str, x: torch.Tensor, copy_to: torch.Tensor, prev: List[torch.Tensor], cm: List[torch.Tensor],
-              gather_to: Optional[torch.Tensor] = None, early: bool = False):
+              gather_to: Optional[torch.Tensor] = None, early: bool = False, same: bool = False,
+              clusters: Optional[bool] = None):
         """Orthonormalise `x` in place (mirrored into `copy_to`). With `gather_to`, `x` is first
         filled with the sum over workers of the factor the previous product pushed (the sum is
         also written to `gather_to`): the launch is the consumer of the in-kernel all-reduce.
-        `early`: see `_chained`."""
+        `early`: see `_chained`. `same`: the last factor in `prev` is a copy of `x` as it comes in. `clusters`: one
+        launch where it can be (True), never (False), by the rule (None)."""
+        clusters = gather_to is None and clusters is not False and (self._orth_clusters if clusters else self._orth_by_rule).get(side, False)
         self._call(
             "psgd_orth_launch",
             _ptr(self.units[side]),
@@ -721,7 +739,7 @@ class NativeCompressor(_Recordable):
             _ptr(self._orth_rinv),
             self.comm.ptr if gather_to is not None else ctypes.c_void_p(0),
             _ptr(gather_to),
-            (1 if early else 0) | (2 if self._chained() else 0),   # the second launch follows the first
+            (1 if early else 0) | ((12 if same else 4) if clusters else 2 if self._chained() else 0),   # the second launch follows the first
         )
 
     def _chained(self) -> bool:
@@ -877,6 +895,7 @@ class NativeCompressor(_Recordable):
         sides: List[bool] = []
         pending: Optional[torch.Tensor] = None   # state buffer whose sum is still in the channel's slots
         chained, self._follows, self._finished = self._chained(), False, False
+        ahead = self._early is not None
         for t in range(self.T):
             left = (core.step_counter * self.T + t) % 2 == 0
             sides.append(left)
@@ -905,7 +924,8 @@ class NativeCompressor(_Recordable):
                         self._orth(side, state_in, self.h_in[t], same, self.cmat[t])
                 else:
                     # the first launch of a step waits for all work before it (gradients, parameters)
-                    self._orth(side, state_in, self.h_in[t], same, self.cmat[t], gather_to, early=self._follows)
+                    self._orth(side, state_in, self.h_in[t], same, self.cmat[t], gather_to, early=self._follows,
+                               same=t > 0 and workers == 1, clusters=ahead or None)
                     self._follows = chained
             with _Range(f"psgd.iter{t}.product"):
                 # one worker: the product is final, so the kernel also writes the warm-start buffer
@@ -961,7 +981,9 @@ class NativeCompressor(_Recordable):
         self._side_stream.wait_event(fork)
         with torch.cuda.stream(self._side_stream):
             before = self.launches
-            self._orth(side, state_in, self.h_in[0], [], self.cmat[0])
+            # two launches: as the first node of a graph's side branch a launch with clusters delays the whole graph, 101 -> 107 us
+            # for a recorded step of a small perceptron, and there is nothing to gain off the critical path
+            self._orth(side, state_in, self.h_in[0], [], self.cmat[0], clusters=False)
             self._early_launches = self.launches - before  # counted with the step that uses them
             done = torch.cuda.Event()
             done.record(self._side_stream)
