@@ -81,6 +81,10 @@ class AllReduce(Aggregator):
         self._native = None
 
     def aggregate(self, gradients: List[torch.Tensor]) -> List[torch.Tensor]:
+        return self._aggregate(gradients)
+
+    def _aggregate(self, gradients: List[torch.Tensor], early: bool = False) -> List[torch.Tensor]:
+        """`early`: the last thing on the stream is a native launch that leaves `gradients` alone."""
         if len(gradients) == 0:
             return []
         device = gradients[0].device
@@ -90,7 +94,7 @@ class AllReduce(Aggregator):
 
             if self._native is None:
                 self._native = NativeFlatAllReduce()
-            return self._native.aggregate(gradients)
+            return self._native.aggregate(gradients, early=early)
         flat, shapes = pack(gradients)
         allreduce_average(flat)
         outputs = unpack(flat, shapes)
@@ -151,7 +155,9 @@ class PowerSGD(Aggregator):
         if self.step_counter <= self.config.start_compressing_after_num_steps:
             return self._allreduce.aggregate(gradients)
         lowrank, plain = self._split(gradients)
-        return self._merge(self._powersgd.aggregate(lowrank), self._allreduce.aggregate(plain))
+        updates = self._powersgd.aggregate(lowrank)
+        native = self._powersgd._native
+        return self._merge(updates, self._allreduce._aggregate(plain, early=self._powersgd._ran_native and native._chained()))
 
     @property
     def compression_rate(self) -> float:
@@ -247,6 +253,7 @@ class BasicPowerSGD(Aggregator):
         self.step_counter = 0
         self._backend_request = backend
         self._native = None
+        self._ran_native = False   # did the last `aggregate` end in native launches?
 
         # Warm-start memory. One seeded generator draws every P group and then every Q group,
         # so replicas that build the object the same way start from identical factors.
@@ -282,6 +289,7 @@ class BasicPowerSGD(Aggregator):
     def aggregate(self, gradients: List[torch.Tensor]) -> List[torch.Tensor]:
         if len(gradients) != len(self.params):
             raise ValueError("gradient list does not match the compressed parameter list")
+        self._ran_native = False
         if len(gradients) == 0:
             self.step_counter += 1
             return []
@@ -292,6 +300,7 @@ class BasicPowerSGD(Aggregator):
             if self._native is None:
                 self._native = NativeCompressor(self)
             outputs = self._native.aggregate(gradients)
+            self._ran_native = True
         else:
             outputs = self._aggregate_torch(gradients)
         self.step_counter += 1

@@ -1247,7 +1247,7 @@ class NativeFlatAllReduce(_Recordable):
             return
         self._stream = stream
         if self.path == "local":
-            self._launch(4 if sgd else 3, hyper_dev, 1.0, early and sgd, stream=stream)
+            self._launch(4 if sgd else 3, hyper_dev, 1.0, early, stream=stream)
         elif self.path == "bulk":
             self._launch(0, hyper_dev, float(workers), stream=stream)
             code = self.lib.psgd_bulk_allreduce_launch(self.comm.ptr, ctypes.c_longlong(self.n_pad), workers, _stream_ptr())
@@ -1271,15 +1271,15 @@ class NativeFlatAllReduce(_Recordable):
             self._launch(2 if sgd else 1, hyper_dev, 1.0, stream=stream)
 
     def aggregate(self, gradients: List[torch.Tensor], outs: Optional[Sequence[torch.Tensor]] = None,
-                  keep_inputs: bool = False) -> List[torch.Tensor]:
+                  keep_inputs: bool = False, early: bool = False) -> List[torch.Tensor]:
         """Mean over workers. `outs`: caller-owned destination tensors (default: views of this
-        object's buffer, valid until the next call). `keep_inputs`: do not zero the inputs."""
+        object's buffer, valid until the next call). `keep_inputs`: do not zero the inputs. `early`: see `aggregate_and_step`."""
         self.check()
         self.launches = 0
         self._bind(gradients, outs=outs)
         self._keep_inputs = bool(keep_inputs)
         try:
-            self._run(self._hyper_dev, world_size(), sgd=False)
+            self._run(self._hyper_dev, world_size(), sgd=False, early=early)
         finally:
             self._keep_inputs = False
         return list(self._views)

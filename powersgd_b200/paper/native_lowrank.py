@@ -90,10 +90,12 @@ class NativeLowRank:
             outs=[o for _t, o, _m in matrices],
         )
 
-    def reduce_vectors(self, vectors) -> None:
-        """Mean over workers of the 1-D tensors, written into the caller's outputs (inputs kept)."""
+    def reduce_vectors(self, vectors, early: bool = False) -> None:
+        """Mean over workers of the 1-D tensors, written into the caller's outputs (inputs kept). `early`: the
+        last thing on the stream are this object's launches over the matrices."""
         if vectors:
-            self.flat.aggregate([t for t, _o, _m in vectors], outs=[o for _t, o, _m in vectors], keep_inputs=True)
+            self.flat.aggregate([t for t, _o, _m in vectors], outs=[o for _t, o, _m in vectors], keep_inputs=True,
+                                early=early and self.comp._chained())
             self.launches += self.flat.launches
 
     # ------------------------------------------------------------------------------------------

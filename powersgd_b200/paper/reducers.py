@@ -261,10 +261,14 @@ class RankKReducer(_LowRankBase):
             if fresh or not self.reuse_query:
                 for i in range(len(matrices)):
                     self.set_random(drv.core.q_view(i))
+        alone = self.n_workers == 1   # nothing to wait for: the vectors beside the end of the matrices
         with self.timer("reduce.rank1", verbosity=2):
-            drv.reduce_vectors(vectors)
+            if not alone:
+                drv.reduce_vectors(vectors)
         with self.timer("reduce.lowrank", verbosity=2):
             drv.rank_k(matrices)
+            if alone:
+                drv.reduce_vectors(vectors, early=True)
         self._native_launches_last = drv.launches
         return n_bits(self.p_memory) + n_bits(self.q_memory) + self._rank1_bits(vectors)
 
@@ -330,10 +334,14 @@ class HalfRankKReducer(_LowRankBase):
         if fresh:
             for i in range(len(matrices)):
                 self.set_random(drv.core.q_view(i))
+        alone = self.n_workers == 1   # nothing to wait for: the vectors beside the end of the matrices
         with self.timer("reduce.rank1", verbosity=2):
-            drv.reduce_vectors(vectors)
+            if not alone:
+                drv.reduce_vectors(vectors)
         with self.timer("reduce.lowrank", verbosity=2):
             drv.half_rank_k(matrices, compute_p)
+            if alone:
+                drv.reduce_vectors(vectors, early=True)
         self._native_launches_last = drv.launches
         return n_bits(self.p_memory if compute_p else self.q_memory) + self._rank1_bits(vectors)
 
