@@ -141,8 +141,10 @@ PSGD_API int psgd_topk_abs(const float* x, long long n, long long k, int* worksp
 // compaction pass in launch 4, which has nothing to do for the others. How long a list one block should walk: ops/topk.py.
 // Bound by the reads (L2 for a model of this size) and by what a block costs besides them, so some four blocks
 // per SM serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: 68 us by three histogram passes and a
-// compaction, 54 us by lists; launch 3 took 14.5 us of it while a thread had one load of its list under way and the
-// entries that it takes were counted in global memory (the pass of the reducer 88.6 us then, 86.0 now).
+// compaction, 54 us by lists. With one worker launch 2 writes the dense output beside the memory (TopkItem::out), so that nothing
+// is left to combine, every launch starts beside the end of the one before, and the workspace is cleared by the call
+// before: the pass of the reducer 86 -> 55 us, of which 12 go to launch 1 (45 MB from HBM and as many additions in shared
+// memory), 27 to launch 2 (135 MB), 8 to launch 3 and 2 to launch 4.
 namespace {
 
 struct TopkItem {
@@ -153,7 +155,12 @@ struct TopkItem {
   long long out_off;   // start of this tensor's k pairs in values / positions
   long long cand_off;  // start of its candidates, and
   long long cap;       // how many there may be
+  float* out;          // optional: the taken entries at their places, zeros elsewhere
 };
+
+// Counters of a tensor behind its histograms: what launch 2 leaves for the launches behind it, besides what it counts.
+enum TopkCounter { TK_TAKEN = 0, TK_EQUAL = 1, TK_LISTED = 2, TK_WAY = 3, TK_PREFIX = 4, TK_REMAIN = 5 };
+constexpr int TK_SHORT = 1, TK_LONG = 2;   // TK_WAY: by the list of candidates, or by two more histograms
 
 // Block-wide: walks `bins` (<= 2048, TK_THREADS threads x 4 bins) from the top until `remain` entries are
 // covered; returns the bin in *bin_out and the number to take inside it in *remain_io. `scan`: one
@@ -293,6 +300,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_hist_kernel(const T
                                                                           const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                           int* __restrict__ ws_all) {
   __shared__ Bins sh;
+  psgd_launch_dependents();
   const int it = block_item[blockIdx.x];
   tk_histogram(items[it], block_part[blockIdx.x], item_parts[it], ws_all + (long long)it * TK_WS_INTS, 0, 0u, sh);
 }
@@ -335,70 +343,88 @@ union SplitScratch {
 };
 static_assert(alignof(SplitScratch) % alignof(int4) == 0, "tk_histogram reads its bins by 16 bytes");
 
+// Four entries of a tensor, or the first `count` of them.
+__device__ __forceinline__ void tk_store(float* dst, bool wide, long long first, int count, const float* v) {
+  if (count == 4 && wide) {
+    *reinterpret_cast<float4*>(dst + first) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < count) dst[first + j] = v[j];
+  }
+}
+// What a taken entry leaves in `out`: value / 1 added to zero, as the combination of several workers' entries has it.
+__device__ __forceinline__ float tk_dense(float v) { return __fadd_rn(0.f, v); }
+
 // Launch 2: what lies above the leading digit is taken, what lies in it is listed; or the second histogram.
-// cand_v / cand_p: lists of candidates; counters of a tensor: [0] taken, [1] equal to the threshold, [2] candidates.
+// cand_v / cand_p: lists of candidates. ws_next: workspace of the call after this one, cleared here (a clearing of its own costs
+// a call 3.5 us), or null.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                            const int* __restrict__ block_part, const int* __restrict__ item_parts,
-                                                                           int* __restrict__ ws_all, float* __restrict__ values,
-                                                                           int* __restrict__ positions, float* __restrict__ cand_v,
-                                                                           int* __restrict__ cand_p) {
+                                                                           int* __restrict__ ws_all, int* __restrict__ ws_next,
+                                                                           float* __restrict__ values, int* __restrict__ positions,
+                                                                           float* __restrict__ cand_v, int* __restrict__ cand_p) {
   __shared__ SplitScratch sh;
   __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
   __shared__ long long remain_sh;
   __shared__ int bin_sh;
-  const int it = block_item[blockIdx.x];
+  psgd_launch_dependents();
+  const int it = block_item[blockIdx.x], part = block_part[blockIdx.x], parts = item_parts[it];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
+  psgd_wait_for_predecessor();
+  if (ws_next)
+    for (int e = part * TK_THREADS + threadIdx.x; e < TK_WS_INTS; e += parts * TK_THREADS) ws_next[(long long)it * TK_WS_INTS + e] = 0;
   tk_derive_block(ws, 0, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned prefix = pick.prefix;
-  if (ws[prefix >> 20] > item.cap) {
-    tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 1, prefix, sh.hist);
+  const bool lists = ws[prefix >> 20] <= item.cap;
+  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
+  if (part == 0 && threadIdx.x == 0) {
+    counters[TK_WAY] = lists ? TK_SHORT : TK_LONG;
+    counters[TK_PREFIX] = (int)prefix;
+    counters[TK_REMAIN] = (int)remain_sh;
+  }
+  if (!lists) {
+    tk_histogram(item, part, parts, ws, 1, prefix, sh.hist);
     return;
   }
   if (threadIdx.x == 0) sh.found.above.count = sh.found.inside.count = 0;
   __syncthreads();
-  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
   float* cv = cand_v + item.cand_off;
   int* cp = cand_p + item.cand_off;
-  const bool wide = ((uintptr_t)item.memory & 15u) == 0;
-  tk_for_each(item.x, item.n, block_part[blockIdx.x], item_parts[it], [&](const float4& q, long long first, int count) {
+  const bool wide_memory = ((uintptr_t)item.memory & 15u) == 0, wide_out = ((uintptr_t)item.out & 15u) == 0;
+  tk_for_each(item.x, item.n, part, parts, [&](const float4& q, long long first, int count) {
     const float v[4] = {q.x, q.y, q.z, q.w};
-    float rest[4];
+    float rest[4], dense[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       rest[j] = v[j];
+      dense[j] = 0.f;
       const unsigned key = tk_key(v[j]);
       if (j < count && key >= prefix) {
         if ((key & 0x7FF00000u) == prefix) {
-          tk_put(sh.found.inside, counters + 2, cv, cp, item.cap, v[j], (int)(first + j));
+          tk_put(sh.found.inside, counters + TK_LISTED, cv, cp, item.cap, v[j], (int)(first + j));
         } else {
-          tk_put(sh.found.above, counters, val, pos, item.k, v[j], (int)(first + j));
+          tk_put(sh.found.above, counters + TK_TAKEN, val, pos, item.k, v[j], (int)(first + j));
           rest[j] = 0.f;
+          dense[j] = tk_dense(v[j]);
         }
       }
     }
-    if (item.memory) {
-      if (count == 4 && wide) {
-        *reinterpret_cast<float4*>(item.memory + first) = make_float4(rest[0], rest[1], rest[2], rest[3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < count) item.memory[first + j] = rest[j];
-      }
-    }
+    if (item.memory) tk_store(item.memory, wide_memory, first, count, rest);
+    if (item.out) tk_store(item.out, wide_out, first, count, dense);
   });
-  tk_hand_out(sh.found.above, counters, val, pos, item.k);
-  tk_hand_out(sh.found.inside, counters + 2, cv, cp, item.cap);
+  tk_hand_out(sh.found.above, counters + TK_TAKEN, val, pos, item.k);
+  tk_hand_out(sh.found.inside, counters + TK_LISTED, cv, cp, item.cap);
 }
 
-// f(value, index) for every entry of a list (block-wide), eight loads of a thread under way: one block walks a list
-// alone, so nothing else hides the latency of L2.
+// f(value, index) for every entry of a list from `from` on (block-wide), eight loads of a thread under way.
 template <class F>
-__device__ __forceinline__ void tk_walk(const float* __restrict__ list, int n, F f) {
-  for (int first = threadIdx.x; first < n; first += 8 * TK_THREADS) {
+__device__ __forceinline__ void tk_walk(const float* __restrict__ list, int from, int n, F f) {
+  for (int first = from + threadIdx.x; first < n; first += 8 * TK_THREADS) {
     float v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
@@ -409,7 +435,8 @@ __device__ __forceinline__ void tk_walk(const float* __restrict__ list, int n, F
   }
 }
 
-// Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram.
+// Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram. One block walks a list alone,
+// three times over, so nothing but the loads under way hides a latency: the first 4096 entries stay in registers.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                             const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                             int* __restrict__ ws_all, float* __restrict__ values,
@@ -420,32 +447,52 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   __shared__ Pick pick;
   __shared__ long long remain_sh;
   __shared__ int bin_sh, above_sh, equal_sh;
+  psgd_launch_dependents();
   const int it = block_item[blockIdx.x];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
-  tk_derive_block(ws, 0, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
-  int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
-  if (ws[pick.prefix >> 20] > item.cap) {
+  const int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
+  int* sh = bins_sh.c;
+  for (int b = threadIdx.x; b < TK_BINS1 + TK_BINS2; b += TK_THREADS) sh[b] = 0;
+  psgd_wait_for_predecessor();
+  if (threadIdx.x == 0) {
+    pick.prefix = (unsigned)counters[TK_PREFIX];
+    remain_sh = counters[TK_REMAIN];
+    above_sh = counters[TK_TAKEN];   // (nobody else takes entries of this tensor any more)
+    equal_sh = 0;
+  }
+  const bool lists = counters[TK_WAY] == TK_SHORT;
+  __syncthreads();
+  if (!lists) {
     tk_derive_block(ws, 1, 2, item.k, &pick, &remain_sh, &bin_sh, scan);
     tk_histogram(item, block_part[blockIdx.x], item_parts[it], ws, 2, pick.prefix, bins_sh);
     return;
   }
   if (block_part[blockIdx.x] != 0) return;
-  const int n = (int)min((long long)counters[2], item.cap);   // what launch 2 has listed
-  int* sh = bins_sh.c;
+  const int n = (int)min((long long)counters[TK_LISTED], item.cap);   // what launch 2 has listed
   const float* cv = cand_v + item.cand_off;
   const int* cp = cand_p + item.cand_off;
+  constexpr int OWN = 8;
+  float own[OWN];
+#pragma unroll
+  for (int u = 0; u < OWN; ++u) own[u] = (int)threadIdx.x + u * TK_THREADS < n ? cv[threadIdx.x + u * TK_THREADS] : 0.f;
+  auto walk = [&](auto f) {
+#pragma unroll
+    for (int u = 0; u < OWN; ++u)
+      if ((int)threadIdx.x + u * TK_THREADS < n) f(own[u], (int)threadIdx.x + u * TK_THREADS);
+    tk_walk(cv, OWN * TK_THREADS, n, f);
+  };
+#pragma unroll 1
   for (int digit = 1; digit <= 2; ++digit) {
     const int bins = digit == 2 ? TK_BINS2 : TK_BINS1, shift = digit == 2 ? 0 : 9;
     const unsigned mask = digit == 2 ? 0x7FFFFE00u : 0x7FF00000u, prefix = pick.prefix;
-    for (int b = threadIdx.x; b < bins; b += TK_THREADS) sh[b] = 0;
-    __syncthreads();
-    tk_walk(cv, n, [&](float v, int) {
+    int* hist = sh + (digit == 2 ? TK_BINS1 : 0);
+    walk([&](float v, int) {
       const unsigned key = tk_key(v);
-      if ((key & mask) == prefix) atomicAdd(sh + ((key >> shift) & (unsigned)(bins - 1)), 1);
+      if ((key & mask) == prefix) atomicAdd(hist + ((key >> shift) & (unsigned)(bins - 1)), 1);
     });
     __syncthreads();
-    tk_choose_block(sh, bins, &remain_sh, &bin_sh, scan);
+    tk_choose_block(hist, bins, &remain_sh, &bin_sh, scan);
     if (threadIdx.x == 0) pick.prefix = prefix | ((unsigned)bin_sh << shift);
     __syncthreads();
   }
@@ -453,12 +500,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   const long long take_equal = remain_sh, base_equal = item.k - take_equal;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
-  if (threadIdx.x == 0) {   // nobody else takes entries of this tensor any more
-    above_sh = counters[0];
-    equal_sh = 0;
-  }
-  __syncthreads();
-  tk_walk(cv, n, [&](float v, int e) {
+  walk([&](float v, int e) {
     const unsigned key = tk_key(v);
     if (key < threshold) return;
     long long slot;
@@ -474,6 +516,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
     val[slot] = v;
     pos[slot] = p;
     if (item.memory) item.memory[p] = 0.f;
+    if (item.out) item.out[p] = tk_dense(v);
   });
 }
 
@@ -487,53 +530,54 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(cons
   __shared__ long long remain_sh;
   __shared__ int bin_sh;
   __shared__ Found found;
+  psgd_launch_dependents();
   const int it = block_item[blockIdx.x];
   const TopkItem item = items[it];
   int* ws = ws_all + (long long)it * TK_WS_INTS;
   int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
-  tk_derive_block(ws, 0, 1, item.k, &pick, &remain_sh, &bin_sh, scan);
-  if (ws[pick.prefix >> 20] <= item.cap) return;   // launch 3 took the rest
-  if (threadIdx.x == 0) found.count = 0;
+  psgd_wait_for_predecessor();
+  if (counters[TK_WAY] == TK_SHORT) return;   // launch 3 took the rest
+  if (threadIdx.x == 0) {
+    pick.prefix = (unsigned)counters[TK_PREFIX];
+    remain_sh = counters[TK_REMAIN];
+    found.count = 0;
+  }
+  __syncthreads();
   tk_derive_block(ws, 1, 3, item.k, &pick, &remain_sh, &bin_sh, scan);
   const unsigned threshold = pick.prefix;
   const long long take_equal = pick.remain;
   const long long base_equal = item.k - take_equal;
   float* val = values + item.out_off;
   int* pos = positions + item.out_off;
-  const bool wide = ((uintptr_t)item.memory & 15u) == 0;
+  const bool wide_memory = ((uintptr_t)item.memory & 15u) == 0, wide_out = ((uintptr_t)item.out & 15u) == 0;
   tk_for_each(item.x, item.n, block_part[blockIdx.x], item_parts[it], [&](const float4& q, long long first, int count) {
     const float v[4] = {q.x, q.y, q.z, q.w};
-    float rest[4];
+    float rest[4], dense[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      rest[j] = v[j];
       const unsigned key = tk_key(v[j]);
+      bool taken = false;
       if (j < count && key >= threshold) {
         const int i = (int)(first + j);
         if (key > threshold) {
-          tk_put(found, counters, val, pos, item.k, v[j], i);
-          rest[j] = 0.f;
+          tk_put(found, counters + TK_TAKEN, val, pos, item.k, v[j], i);
+          taken = true;
         } else {
-          const long long e = atomicAdd(counters + 1, 1);
+          const long long e = atomicAdd(counters + TK_EQUAL, 1);
           if (e < take_equal) {
             val[base_equal + e] = v[j];
             pos[base_equal + e] = i;
-            rest[j] = 0.f;
+            taken = true;
           }
         }
       }
+      rest[j] = taken ? 0.f : v[j];
+      dense[j] = taken ? tk_dense(v[j]) : 0.f;
     }
-    if (item.memory) {
-      if (count == 4 && wide) {
-        *reinterpret_cast<float4*>(item.memory + first) = make_float4(rest[0], rest[1], rest[2], rest[3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < count) item.memory[first + j] = rest[j];
-      }
-    }
+    if (item.memory) tk_store(item.memory, wide_memory, first, count, rest);
+    if (item.out) tk_store(item.out, wide_out, first, count, dense);
   });
-  tk_hand_out(found, counters, val, pos, item.k);
+  tk_hand_out(found, counters + TK_TAKEN, val, pos, item.k);
 }
 
 }  // namespace
@@ -542,19 +586,28 @@ PSGD_API int psgd_topk_item_bytes() { return (int)sizeof(TopkItem); }
 
 // Top-k of |x| for `nitems` tensors in four launches. items: device array of TopkItem; block_item /
 // block_part: device tables of `nblocks` entries (which tensor a block serves and which of that
-// tensor's `item_parts[item]` interleaved parts); workspace: nitems * psgd_topk_workspace_ints() ints; cand_v / cand_p: room for
-// the candidates of all tensors (`cand_off`, `cap` of the items). values / positions receive every tensor's k pairs at its `out_off`.
+// tensor's `item_parts[item]` interleaved parts); workspace: nitems * psgd_topk_workspace_ints() ints; next_workspace: null, or as
+// many ints again that this call clears for the one after it, whose `workspace` they have to be (as `workspace` was cleared by the call before);
+// cand_v / cand_p: room for the candidates of all tensors (`cand_off`, `cap` of the items). values / positions receive every
+// tensor's k pairs at its `out_off`.
 PSGD_API int psgd_topk_abs_many(const void* items, int nitems, const int* block_item, const int* block_part, const int* item_parts,
-                                int nblocks, int* workspace, float* cand_v, int* cand_p, float* values, int* positions, cudaStream_t stream) {
+                                int nblocks, int* workspace, int* next_workspace, float* cand_v, int* cand_p, float* values, int* positions,
+                                cudaStream_t stream) {
   if (nitems <= 0 || nblocks <= 0) return 0;
-  PSGD_CUDA_OK(cudaMemsetAsync(workspace, 0, sizeof(int) * (size_t)TK_WS_INTS * nitems, stream));
   const TopkItem* it = (const TopkItem*)items;
-  psgd_topk_many_hist_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace);
-  psgd_topk_many_split_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, values, positions, cand_v, cand_p);
-  psgd_topk_many_refine_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, values, positions, cand_v, cand_p);
-  psgd_topk_many_compact_kernel<<<nblocks, TK_THREADS, 0, stream>>>(it, block_item, block_part, item_parts, workspace, values, positions);
-  PSGD_CUDA_OK(cudaGetLastError());
-  return 0;
+  if (next_workspace == nullptr) PSGD_CUDA_OK(cudaMemsetAsync(workspace, 0, sizeof(int) * (size_t)TK_WS_INTS * nitems, stream));
+  int code = psgd_launch(psgd_topk_many_hist_kernel, nblocks, TK_THREADS, 0, stream, 0, it, block_item, block_part, item_parts, workspace);
+  // the others start beside the end of the one before and wait for it
+  if (code == 0)
+    code = psgd_launch(psgd_topk_many_split_kernel, nblocks, TK_THREADS, 0, stream, 1, it, block_item, block_part, item_parts, workspace,
+                       next_workspace, values, positions, cand_v, cand_p);
+  if (code == 0)
+    code = psgd_launch(psgd_topk_many_refine_kernel, nblocks, TK_THREADS, 0, stream, 1, it, block_item, block_part, item_parts, workspace,
+                       values, positions, cand_v, cand_p);
+  if (code == 0)
+    code = psgd_launch(psgd_topk_many_compact_kernel, nblocks, TK_THREADS, 0, stream, 1, it, block_item, block_part, item_parts, workspace,
+                       values, positions);
+  return code;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -77,12 +77,14 @@ MOST_LISTS = 8   # of tensors, each on one stream, whose tables are kept
 CANDIDATES = 2048   # room for candidates per tensor, besides what the length of the list allows (0: none)
 
 
-def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tensor]:
+def topk_abs_many(tensors, ks, memories=None, outs=None) -> Tuple[torch.Tensor, torch.Tensor]:
     """`topk_abs` for a list of tensors in four launches (csrc/topk.cu, psgd_topk_abs_many).
 
     Returns flat `(values, positions)`: tensor i's `ks[i]` pairs start at `sum(ks[:i])`; positions
     are int32 indices into the flattened tensor i. `memories[i]`, when given, receives tensor i with
-    the taken entries zeroed. Falls back to one `topk_abs` per tensor off the GPU."""
+    the taken entries zeroed. `outs[i]`, when given, receives the taken entries of tensor i at their places and
+    zeros elsewhere: what `sparse_combine` makes of one worker's pairs, without a pass of its own where `outs` lie apart
+    from what is read. Falls back to one `topk_abs` per tensor off the GPU."""
     ks = [int(k) for k in ks]
     total = sum(ks)
     tensors = list(tensors)
@@ -98,21 +100,54 @@ def topk_abs_many(tensors, ks, memories=None) -> Tuple[torch.Tensor, torch.Tenso
             v, p = topk_abs(t, k, memory=m)
             values[at : at + k], positions[at : at + k] = v, p
             at += k
+        if outs is not None:
+            _combine_own(values, positions, ks, list(outs))
         return values, positions
     values = torch.empty(total, dtype=torch.float32, device=device)
     positions = torch.empty(total, dtype=torch.int32, device=device)
+    outs = None if outs is None else list(outs)
+    dense = outs is not None and scan.usable(outs, True)
     with _launching:
-        _select(tensors, ks, mems, values, positions)
+        dense = _select(tensors, ks, mems, outs if dense else None, values, positions) and dense
+    if outs is not None and not dense:
+        _combine_own(values, positions, ks, outs)
     return values, positions
 
 
-def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) -> None:
+def _combine_own(values: torch.Tensor, positions: torch.Tensor, ks, outs) -> None:
+    ends, at = [], 0
+    for k in ks:
+        at += k
+        ends.append(at)
+    sparse_combine(values.view(1, -1), positions.view(1, -1), outs, ends, 1.0)
+
+
+def _apart(outs, sizes, read) -> bool:
+    """Do the tensors `outs` have the numbers of elements `sizes`, and no byte in common with each other or with the tensors `read`?
+    A launch may write one tensor's part of `outs` while another's is still to be read."""
+    import numpy as np
+
+    if any(o.numel() != n for o, n in zip(outs, sizes)):
+        return False
+    start = np.array([o.data_ptr() for o in outs], dtype=np.uint64)
+    order = np.argsort(start, kind="stable")
+    start, end = start[order], (start + 4 * np.array(sizes, dtype=np.uint64))[order]
+    if (end[:-1] > start[1:]).any():
+        return False
+    first = np.array([t.data_ptr() for t in read], dtype=np.uint64)
+    last = first + 4 * np.array([t.numel() for t in read], dtype=np.uint64)
+    before = np.searchsorted(start, last, side="left")   # how many begin before the end of what is read; the last of them ends last
+    return not ((before > 0) & (end[np.maximum(before, 1) - 1] > first)).any()
+
+
+def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tensor) -> bool:
+    """The launches; are `outs` written as well?"""
     import numpy as np
 
     lib = native.lib()
     device = tensors[0].device
     stream = _current_stream()
-    key = (device, stream.value, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks))
+    key = (device, stream.value, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks), scan.addresses(outs))
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
     recorded = is_recorded(stream)
@@ -120,12 +155,13 @@ def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) ->
     if entry is None:
         release_finished()
         dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64),
-                          ("cand_off", np.int64), ("cap", np.int64)])
+                          ("cand_off", np.int64), ("cap", np.int64), ("out", np.uint64)])
         if dtype.itemsize != int(lib.psgd_topk_item_bytes()):
             raise RuntimeError("top-k item record out of sync with the native library")
         items = np.zeros(len(tensors), dtype=dtype)
         block_item, block_part, parts = [], [], []
         at, room, total_n = 0, 0, max(1, sum(t.numel() for t in tensors))
+        dense = outs is not None and _apart(outs, [t.numel() for t in tensors], tensors + [m for m in mems if m is not None])
         for i, (t, k, m) in enumerate(zip(tensors, ks, mems)):
             n = t.numel()
             if not (0 < k <= n < (1 << 31)):
@@ -137,7 +173,7 @@ def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) ->
             # 12 600 26 / 38; 4 M, 3 800 43 / 38, 27 000 45 / 63; 16 M, 15 000 75 / 77, 820 000 (uniform) 76 / 849; 50 M, 47 000
             # 203 / 197, 81 000 203 / 238; 62 tensors of 11 M, 3 900 in the largest 68 / 54, 33 000 73 / 91
             cap = min(n, CANDIDATES + total_n // 2048) if CANDIDATES else 0
-            items[i] = (t.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at, room, cap)
+            items[i] = (t.data_ptr(), 0 if m is None else m.data_ptr(), n, k, at, room, cap, outs[i].data_ptr() if dense else 0)
             at, room = at + k, room + cap
             # blocks of 512 threads with at least 16 elements each, some four per SM for the whole list:
             # every block pays for its histogram (zeroing, choosing the digits so far, adding it up)
@@ -150,9 +186,10 @@ def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) ->
             entry = {
                 "items": to_dev(items), "block_item": to_dev(np.asarray(block_item, dtype=np.int32)),
                 "block_part": to_dev(np.asarray(block_part, dtype=np.int32)), "parts": to_dev(np.asarray(parts, dtype=np.int32)),
-                "nblocks": len(block_item),
+                "nblocks": len(block_item), "dense": dense, "turn": 0,
                 "cand_v": torch.empty(max(room, 1), dtype=torch.float32, device=device), "cand_p": torch.empty(max(room, 1), dtype=torch.int32, device=device),
-                "ws": torch.zeros(len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
+                # one half per call in turn: a call clears the other for the next. (A recorded call clears its own.)
+                "ws": torch.zeros(2 * len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
             }
         if recorded:
             keep_with_graph(None, entry)
@@ -163,12 +200,18 @@ def _select(tensors, ks, mems, values: torch.Tensor, positions: torch.Tensor) ->
                 _many_cache.clear()
             _many_cache[key] = entry
     vp = ctypes.c_void_p
+    half = 2 * entry["ws"].numel()   # in bytes
+    turn, base = entry["turn"], entry["ws"].data_ptr()
     code = lib.psgd_topk_abs_many(
         vp(entry["items"].data_ptr()), len(tensors), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
-        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(entry["ws"].data_ptr()), vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()),
-        vp(values.data_ptr()), vp(positions.data_ptr()), stream,
+        vp(entry["parts"].data_ptr()), entry["nblocks"], vp(base + turn * half), vp(0 if recorded else base + (1 - turn) * half),
+        vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
     )
+    entry["turn"] = 1 - turn
+    if code != 0 and not recorded:
+        _many_cache.pop(key, None)   # who knows what is cleared
     native.check(code, "psgd_topk_abs_many")
+    return entry["dense"]
 
 
 _SEG_DTYPE = None

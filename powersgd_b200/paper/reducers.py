@@ -514,12 +514,16 @@ class TopKReducer(Reducer):
             ends, sizes = np.cumsum(sizes).tolist(), sizes.tolist()
         with self.timer("reduce.topk", verbosity=2):
             # selection, gather and the error-feedback write (memory = x with the taken entries
-            # zeroed) are one fused operation over the whole list: four launches on CUDA
-            values, positions = topk_abs_many(list(grad_in), sizes, list(memory_out))
+            # zeroed) are one fused operation over the whole list: four launches on CUDA, which write
+            # the output as well when there is nothing to gather
+            alone = self.n_workers == 1
+            values, positions = topk_abs_many(list(grad_in), sizes, list(memory_out), list(grad_out) if alone else None)
+        bits = n_bits(values) + n_bits(positions)
+        if alone:
+            return bits
         with self.timer("reduce.gather", verbosity=2):
             all_values = _gather_all(values, self.n_workers)
             all_positions = _gather_all(positions, self.n_workers)
-            bits = n_bits(values) + n_bits(positions)
         with self.timer("reduce.combine", verbosity=2):
             # zero fill + the scatter of every worker's pairs, in rank order: one launch on CUDA
             sparse_combine(_rows(all_values), _rows(all_positions), grad_out, ends, float(self.n_workers))
