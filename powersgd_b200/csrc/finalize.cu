@@ -12,6 +12,7 @@
 //     or        SGD with momentum / dampening / nesterov / weight decay applied to `param`
 // HBM traffic: read + write M, plus param / momentum when fused. The rank-(T*r) updates run on
 // FP32 FMAs from shared-memory panels (4x4 register micro-tiles).
+#include "psgd_async.cuh"
 #include "psgd_bounds.cuh"
 #include "psgd_comm.cuh"
 
@@ -247,7 +248,10 @@ constexpr int FIN_STRIP_KMAX = 32;
 // row by row (r values together), so neighbouring threads of the staging loop write to neighbouring
 // panel rows; at a pitch of 128 or 256 floats all of them would meet in one shared-memory bank.
 // With this, the division below and eight rows per warp from 16 factor columns on, 50257 x 1024 at rank
-// 16 x 2 half-iterations takes 475 us per pass instead of 499.
+// 16 x 2 half-iterations takes 475 us per pass instead of 499. Staged by asynchronous copies, all of them under way together
+// (a loop of loads and stores waits for each round): 3700 -> 2000 of the 11 000 cycles of a strip of 64 rows at rank 3 x 3, 5700
+// -> 3600 of 25 000 on ResNet-18 with the optimizer step; us per pass 96.4 -> 94.3 and, recorded, 105.5 -> 104, 50257 x 1024 433 -> 428
+// (the products' staging included).
 constexpr int FIN_PANEL_PAD = 4;
 constexpr int FIN_RPITCH = FIN_COLS + FIN_PANEL_PAD;
 __host__ __device__ constexpr int fin_panel_floats(int tile_rows) { return FIN_RPITCH + tile_rows + FIN_PANEL_PAD; }  // per factor column
@@ -284,7 +288,7 @@ __device__ __forceinline__ void fin_gather(const PsgdCommDev& c, int e1, long lo
 
 // ROWS: where the rank is a multiple of four and accesses take 16 bytes, the left panel lies row by row, as in memory: staged by 16-byte copies
 // without index arithmetic, read four values of a row at a time. Staging, 48 single loads per thread and strip at 32
-// factor columns before, was a sixth of such a strip's time and a quarter of its instructions. 50257 x 1024 at rank
+// factor columns then, was a sixth of such a strip's time and a quarter of its instructions. 50257 x 1024 at rank
 // 16 x 2: 467.6 -> 448.1 us per pass. Launches alone, before / now: 6 x 2048^2 at 8 x 2 88 / 87, 12 x 2 105 / 100, 16 x 2 118 / 110;
 // with 4-byte accesses 4 x 3000x1001 at 8 x 2 46.8 / 50.8, 16 x 2 59.3 / 62.5, with 8-byte ones 3 x 9000x650 75.9 / 77.8 and 97.4 /
 // 94.1, so those keep the other form. In the same kernel they are still 1 to 3 % slower per pass than in one without ROWS
@@ -381,21 +385,11 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
       const float* gl = a.rloc[h] + base;
       const float* gs = a.rsum[h] + base;
       const bool poll = last && !a.poll_left;
-      const bool wide = by_rows && ((uintptr_t)gl & 15u) == 0;
-      if (wide) {
-#pragma unroll 2
-        for (int e = 4 * tid; e < t.cols * r; e += 4 * FIN_THREADS) {
-          const float4 q = *reinterpret_cast<const float4*>(gl + e);
-          const int lc = fin_div(e, r, magic), j = e - lc * r;
-          float* dst = sRl + (h * r + j) * FIN_RPITCH + fin_panel_pos<VEC>(lc);
-          dst[0] = q.x; dst[FIN_RPITCH] = q.y; dst[2 * FIN_RPITCH] = q.z; dst[3 * FIN_RPITCH] = q.w;
-        }
-      }
-      for (int e = tid; !wide && e < t.cols * r; e += FIN_THREADS) {
+      for (int e = tid; e < t.cols * r; e += FIN_THREADS) {
         const int lc = fin_div(e, r, magic), j = e - lc * r;
         const int pos = fin_panel_pos<VEC>(lc);
-        sRl[(h * r + j) * FIN_RPITCH + pos] = gl[e];
-        if (!SAME && !poll && gs != gl) sRs[(h * r + j) * FIN_RPITCH + pos] = gs[e];
+        psgd_copy4(sRl + (h * r + j) * FIN_RPITCH + pos, gl + e);
+        if (!SAME && !poll && gs != gl) psgd_copy4(sRs + (h * r + j) * FIN_RPITCH + pos, gs + e);
       }
       if (poll) {
         const bool writer = t.row0 == 0;
@@ -417,17 +411,15 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
       if (by_rows) {
         float* dst = sLl + h * tile_rows * r;
         if (((uintptr_t)gl & 15u) == 0) {
-#pragma unroll 4
-          for (int e = 4 * tid; e < t.rows * r; e += 4 * FIN_THREADS) *reinterpret_cast<float4*>(dst + e) = *reinterpret_cast<const float4*>(gl + e);
+          for (int e = 4 * tid; e < t.rows * r; e += 4 * FIN_THREADS) psgd_copy16(dst + e, gl + e);
         } else {
-#pragma unroll 4
-          for (int e = tid; e < t.rows * r; e += FIN_THREADS) dst[e] = gl[e];
+          for (int e = tid; e < t.rows * r; e += FIN_THREADS) psgd_copy4(dst + e, gl + e);
         }
       }
       for (int e = tid; !by_rows && e < t.rows * r; e += FIN_THREADS) {
         const int lr = fin_div(e, r, magic), j = e - lr * r;
-        sLl[(h * r + j) * lp + lr] = gl[e];
-        if (!SAME && !poll && gs != gl) sLs[(h * r + j) * lp + lr] = gs[e];
+        psgd_copy4(sLl + (h * r + j) * lp + lr, gl + e);
+        if (!SAME && !poll && gs != gl) psgd_copy4(sLs + (h * r + j) * lp + lr, gs + e);
       }
       if (poll) {
         const bool writer = t.col0 == 0;
@@ -443,6 +435,7 @@ __device__ __forceinline__ void finalize_strip_tile(const FinalizeArgs& a, const
     }
   }
   if (gather) psgd_comm_close_epoch(*a.comm, e1);  // (CTA barrier inside) this strip has read its words
+  psgd_copies_wait();
   __syncthreads();
 
   for (int rc = 0; rc < t.rows; rc += CHUNK) {

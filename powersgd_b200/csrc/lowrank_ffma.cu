@@ -18,6 +18,7 @@
 // Tiles that cover the same output rows (NT: row blocks of one column block; NN: column
 // blocks of one row block) write partial sums to a scratch arena; the tile that arrives last
 // (arrival counter) adds them in a fixed order, so the result does not depend on scheduling.
+#include "psgd_async.cuh"
 #include "psgd_bounds.cuh"
 #include "psgd_comm.cuh"
 
@@ -175,10 +176,16 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
     }
     // stage the chunk's rows of P-hat (zero padded to RT columns)
     const float* pin = a.in + mt.p_off + (long long)(t.row0 + rb) * r;
-    for (int e = tid; e < rows * RT; e += GEMM_THREADS) {
-      const int row = e / RT, k = e % RT;
-      sP[e] = (k < r) ? pin[row * r + k] : 0.f;
+    if (RT >= 4 && r == RT && ((uintptr_t)pin & 15u) == 0) {
+      for (int e = 4 * tid; e < rows * RT; e += 4 * GEMM_THREADS) psgd_copy16(sP + e, pin + e);
+    } else {
+      for (int e = tid; e < rows * RT; e += GEMM_THREADS) {
+        const int row = e / RT, k = e % RT;
+        if (k < r) psgd_copy4(sP + e, pin + row * r + k);
+        else sP[e] = 0.f;
+      }
     }
+    psgd_copies_wait();
     __syncthreads();
 
     auto use = [&](const float (&v)[UR][4], int i0) {
@@ -326,7 +333,9 @@ __device__ __forceinline__ float warp_sums(float (&v)[N], int lane) {
 // reads its 4 columns x RT values as RT 16-byte words: read straight from global memory they cost more
 // load instructions than the gradient itself), and the loop over 128-column chunks keeps two chunks
 // of the gradient under way. ResNet-18 at rank 2 (45 MB) 18.8 -> 16.1 us, 3 x 1001x777 + 2 x 515x2049 at rank 3
-// 15.2 -> 12.1 us; tiles of 512 / 256 columns instead: 19.1 / 21.3 us on ResNet-18.
+// 15.2 -> 12.1 us; tiles of 512 / 256 columns instead: 19.1 / 21.3 us on ResNet-18. The staging itself, as a loop of loads and
+// stores with a division for each value, took 2600 of a tile's some 10 000 cycles on ResNet-18, 4100 of 13 500 at rank 3 and, with
+// five CTAs per SM at it, 8200 of 17 000 on the LSTM model; by asynchronous copies column by column 1550, 1700 and 4700.
 template <int RT, int VEC, int RPW>
 __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& t, const PsgdMat& mt, float* sQ, float* sSum) {
   const int r = mt.r, m = mt.m;
@@ -365,22 +374,32 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
 
   // element (column lc of the tile, k): chunk of 128 columns, then word of 4 floats, then lane
   const float* qin = a.in + mt.q_off + (long long)t.col0 * r;   // written by the launch before: plain loads
-  for (int e = tid; e < t.cols * r; e += GEMM_THREADS) {
-    const int lc = e / r, k = e - lc * r, b = lc & 127;
+  auto place = [&](int lc, int k) {   // in sQ
+    const int b = lc & 127;
     const int ln = VEC == 4 ? b >> 2 : VEC == 2 ? (b & 63) >> 1 : b & 31;
     const int c = VEC == 4 ? b & 3 : VEC == 2 ? (b & 1) + 2 * (b >> 6) : b >> 5;
     const int f = c * RT + k;
-    sQ[(((lc >> 7) * RT + (f >> 2)) * 32 + ln) * 4 + (f & 3)] = qin[e];
-  }
-  if (r < RT || (t.cols & 127) != 0) {
-    // the padding the loop reads: columns beyond the tile in its last chunk, values beyond the rank
-    const int chunks = (t.cols + 127) >> 7;
-    for (int e = tid; e < chunks * 128 * RT; e += GEMM_THREADS) {
-      const int word = e >> 7, ln = (e >> 2) & 31, f = (word % RT) * 4 + (e & 3);
-      const int c = f / RT, k = f % RT;
-      if (k >= r || (word / RT) * 128 + lane_col<VEC>(ln, c) >= t.cols) sQ[e] = 0.f;
+    return sQ + (((lc >> 7) * RT + (f >> 2)) * 32 + ln) * 4 + (f & 3);
+  };
+  // the values of a column lie together in both: copies of up to 16 bytes where the alignment allows them. Zeros for what the loop
+  // reads besides: columns beyond the tile in its last chunk, values beyond the rank
+  constexpr int W = RT >= 4 ? 4 : RT;
+  const bool wide = RT > 1 && r == RT && ((uintptr_t)qin & (4 * W - 1)) == 0;
+  if (wide) {
+    for (int e = tid; e < t.cols * (RT / W); e += GEMM_THREADS) {
+      const int lc = e / (RT / W), k = e % (RT / W) * W;
+      if (W == 4) psgd_copy16(place(lc, k), qin + e * W);
+      else psgd_copy8(place(lc, k), qin + e * W);
     }
   }
+  for (int lc = (wide ? t.cols : 0) + tid; lc < ((t.cols + 127) & ~127); lc += GEMM_THREADS) {
+#pragma unroll
+    for (int k = 0; k < RT; ++k) {
+      if (lc < t.cols && k < r) psgd_copy4(place(lc, k), qin + lc * r + k);
+      else *place(lc, k) = 0.f;
+    }
+  }
+  psgd_copies_wait();
   __syncthreads();
 
   const float4* q4 = reinterpret_cast<const float4*>(sQ) + lane;

@@ -63,3 +63,17 @@ __device__ __forceinline__ void psgd_bulk_load(void* dst, const void* src, uint3
                "l"(src), "r"(bytes), "r"(psgd_smem_u32(bar))
                : "memory");
 }
+
+// Copies of 4, 8 or 16 bytes of global memory into shared memory that need no registers while they are under way: a loop of them has
+// all its copies in flight, where a loop of loads and stores (which the compiler must take for overlapping)
+// waits for each. Everybody who reads the copies waits for their own and passes a barrier.
+__device__ __forceinline__ void psgd_copy4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(psgd_smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void psgd_copy8(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(psgd_smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void psgd_copy16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(psgd_smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void psgd_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
