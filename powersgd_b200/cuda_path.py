@@ -81,9 +81,13 @@ def _ptr_array(tensors: Sequence[torch.Tensor]):
 
 def _split_even(total: int, max_chunk: int, multiple: int) -> List[Tuple[int, int]]:
     """Cut [0, total) into near-equal chunks of at most `max_chunk`, starts on `multiple`."""
-    if total <= max_chunk:
+    return _split_parts(total, -(-total // max_chunk), multiple)
+
+
+def _split_parts(total: int, parts: int, multiple: int) -> List[Tuple[int, int]]:
+    """Cut [0, total) into at most `parts` near-equal chunks, starts on `multiple`."""
+    if parts <= 1:
         return [(0, total)]
-    parts = -(-total // max_chunk)
     size = -(-total // parts)
     size = -(-size // multiple) * multiple
     out, start = [], 0
@@ -138,8 +142,9 @@ class TilePlan:
         # epilogue, short enough that a small model still fills the GPU, and such that the last
         # wave of CTAs is nearly full (the block scheduler runs TC_CTAS_PER_SM per SM at a time)
         tc_mats = [self.plan.groups[gi] for (gi, _p, _i), f in zip(self.mats, tc_flags) if f]
-        tc_k_nt = self._pick_tc_k(tc_mats, transposed=True)
-        tc_k_nn = self._pick_tc_k(tc_mats, transposed=False)
+        tc_k_nt, tail_nt = self._tc_extents(tc_mats, transposed=True)
+        tc_k_nn, tail_nn = self._tc_extents(tc_mats, transposed=False)
+        tc_nt = tc_nn = 0   # output blocks so far
         self._pick_nt_rows([self.plan.groups[gi] for (gi, _p, _i), f in zip(self.mats, tc_flags) if not f])
         for mi, (gi, _pos, _idx) in enumerate(self.mats):
             g = self.plan.groups[gi]
@@ -149,14 +154,17 @@ class TilePlan:
             else:
                 fin["f"].append((mi, g.n, self.fin_rows, g.m, 128, v))
             if tc_flags[mi]:
-                row_blocks = _split_even(g.n, tc_k_nt, 32)
+                row_blocks, col_blocks = _split_even(g.n, tc_k_nt, 32), _split_even(g.m, tc_k_nn, 32)
                 for c0 in range(0, g.m, 128):
+                    if tail_nt:
+                        row_blocks, tc_nt = _split_parts(g.n, tail_nt.get(tc_nt, _split_count(g.n, tc_k_nt, 32)), 32), tc_nt + 1
                     for si, (r0, rows) in enumerate(row_blocks):
                         nt["tc"].append((mi, r0, rows, c0, min(128, g.m - c0), si, len(row_blocks), ticket, tc_slots, v, (0, 0)))
                     ticket += 1
                     tc_slots += len(row_blocks)
-                col_blocks = _split_even(g.m, tc_k_nn, 32)
                 for r0 in range(0, g.n, 128):
+                    if tail_nn:
+                        col_blocks, tc_nn = _split_parts(g.m, tail_nn.get(tc_nn, _split_count(g.m, tc_k_nn, 32)), 32), tc_nn + 1
                     for si, (c0, cols) in enumerate(col_blocks):
                         nn["tc"].append((mi, r0, min(128, g.n - r0), c0, cols, si, len(col_blocks), ticket, tc_slots, v, (0, 0)))
                     ticket += 1
@@ -241,6 +249,41 @@ class TilePlan:
     # prologue + epilogue of a tile (~4 us), in units of streamed K rows (~0.03 us each): measured
     # as rounds x (overhead + rows) over tile extents 512 ... 4096 on 4 x 4096^2
     TC_TILE_OVERHEAD_ROWS = 136
+
+    # The same for lists of one to three rounds, template ranks up to 8 and above, from rounds of 176 to 2720 rows: 50257 x 1024 at rank 16,
+    # 1408 and 704 rows 57.5 / 68.4 us, 352 rows 88.7; GPT-2 medium at rank 4, 1456 / 2712 / 5416 tiles 252.5 / 282.6 / 328 us.
+    TC_ROUND_OVERHEAD_ROWS = (236, 330)
+
+    def _tc_extents(self, groups, transposed: bool) -> Tuple[int, Dict[int, int]]:
+        """K extent of the tiles, and how many tiles the last output blocks of 128 (by number, in the order of `build`) are cut in if
+        not by that. In lists of one to three rounds of resident CTAs what does not fill the last round is cut finer, so that it
+        does: 50257 x 1024 at rank 16, P = M Q: 393 blocks in 393 tiles 74 us, in 786 80 (the extent that fills its rounds best), 296 whole
+        ones and 97 in three 68. Above, the scheduler evens rounds out by itself (GPT-2 medium, five to eight rounds: 286 -> 277 us for
+        one product, 253 -> 269 for the other)."""
+        slots = 148 * self.TC_CTAS_PER_SM
+        k = self._pick_tc_k(groups, transposed)
+        blocks = [((g.n if transposed else g.m), -(-(g.m if transposed else g.n) // 128)) for g in groups]   # of (length, number)
+        if not slots < sum(number * _split_count(length, k, 32) for length, number in blocks) <= 3 * slots or os.environ.get("PSGD_B200_TC_K"):
+            return k, {}
+        overhead, longest = self.TC_ROUND_OVERHEAD_ROWS[self.rp_tc > 8], max(length for length, _number in blocks)
+        work, best = sum(length * number for length, number in blocks), None
+        for pieces in range(1, 9):
+            k = -(-longest // pieces)
+            tiles = sum(number * _split_count(length, k, 32) for length, number in blocks)
+            rounds, rest = divmod(tiles, slots)
+            cost = rounds * (overhead + work / tiles) + (overhead + k / (slots // rest) if rest else 0)
+            if best is None or cost < best[0]:
+                best = (cost, k, rest)
+        _cost, k, rest = best
+        finer, at, tail = slots // rest if rest else 1, sum(number for _length, number in blocks), {}
+        for length, number in reversed(blocks):
+            parts = _split_count(length, k, 32)
+            for _ in range(number):
+                if finer == 1 or rest <= 0:
+                    return k, tail
+                at, rest = at - 1, rest - parts
+                tail[at] = _split_count(length, max(128, -(-length // (parts * finer))), 32)
+        return k, tail
 
     def _pick_tc_k(self, groups, transposed: bool) -> int:
         if not groups:
