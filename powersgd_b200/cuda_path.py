@@ -194,7 +194,9 @@ class TilePlan:
         return {
             "nt": {k: arr(v) for k, v in nt.items()},
             "nn": {k: arr(v) for k, v in nn.items()},
-            "fin": {k: self._grids(v) if v else arr(v) for k, v in fin.items()},
+            # last rows first: some of what the product before has read last is still in the L2 cache. us per pass, first rows first / last
+            # rows first: LSTM step 212.7 / 210.9, ResNet-18's recorded step 103.2 / 102.6, 50257 x 1024 at rank 16 427.7 / 426.2
+            "fin": {k: self._grids(v)[::-1].copy() if v else arr(v) for k, v in fin.items()},
         }
 
     @staticmethod
