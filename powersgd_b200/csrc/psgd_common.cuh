@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <tuple>
 #include "psgd_types.h"
 
 #define PSGD_API extern "C" __attribute__((visibility("default")))
@@ -120,17 +121,21 @@ static inline int psgd_allow_shared(const void* kernel, size_t bytes, unsigned l
   return 0;
 }
 
+// Launches of the calling thread are written down here while it is not null, besides being made (psgd_host.cpp, psgd_tape_begin).
+struct PsgdTape;
+extern thread_local PsgdTape* psgd_tape_now;
+void psgd_tape_add(const void* kernel, int grid, int block, size_t smem, int early, int cluster, int count, const void* const* args,
+                   const size_t* sizes);
+
 // `early` != 0: the kernel contains the wait above and the launch directly before it in `stream` is
 // one of this library's.
-template <typename... Params, typename... Args>
-static inline int psgd_launch_clusters(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int early,
-                                       int cluster, Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
+static inline void psgd_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs, int grid, int block, size_t smem, cudaStream_t stream,
+                                      int early, int cluster) {
+  cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attrs[2];
   int n = 0;
   if (early) {
     attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -144,7 +149,22 @@ static inline int psgd_launch_clusters(void (*kernel)(Params...), int grid, int 
   }
   cfg.attrs = attrs;
   cfg.numAttrs = n;
+}
+template <typename... Params, typename... Args>
+static inline int psgd_launch_clusters(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, int early,
+                                       int cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attrs[2];
+  psgd_launch_config(cfg, attrs, grid, block, smem, stream, early, cluster);
   PSGD_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+  if (psgd_tape_now != nullptr) {
+    const std::tuple<Params...> held(static_cast<Params>(args)...);
+    std::apply([&](const auto&... arg) {
+      const void* at[] = {(const void*)&arg...};
+      const size_t sizes[] = {sizeof(arg)...};
+      psgd_tape_add((const void*)kernel, grid, block, smem, early, cluster, (int)sizeof...(arg), at, sizes);
+    }, held);
+  }
   return 0;
 }
 template <typename... Params, typename... Args>

@@ -4,10 +4,10 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <memory>
 #include <mutex>
 #include <vector>
-
-#define PSGD_API extern "C" __attribute__((visibility("default")))
+#include "psgd_common.cuh"
 
 static thread_local char g_last_error[1024] = "";
 
@@ -63,6 +63,51 @@ PSGD_API int psgd_capture_mode(int* mode) {
 PSGD_API int psgd_stream_wait(cudaStream_t stream) {
   const cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) { psgd_set_error("cudaStreamSynchronize: %s", cudaGetErrorString(e)); return (int)e; }
+  return 0;
+}
+
+// ---- launches written down and made again ---------------------------------------------------------
+// An eager step repeats the launches of the step before it with the same arguments. Each through its own entry point and a foreign
+// function call with some fifteen converted arguments took 4.3 us of the host; one call that makes them all takes half.
+struct PsgdTape {
+  struct Launch {
+    const void* kernel;
+    int grid, block, early, cluster;
+    size_t smem;
+    std::vector<std::unique_ptr<max_align_t[]>> held;   // copies of the arguments
+    std::vector<void*> args;
+  };
+  std::vector<Launch> launches;
+};
+thread_local PsgdTape* psgd_tape_now = nullptr;
+
+void psgd_tape_add(const void* kernel, int grid, int block, size_t smem, int early, int cluster, int count, const void* const* args,
+                   const size_t* sizes) {
+  PsgdTape::Launch l = {kernel, grid, block, early, cluster, smem, {}, {}};
+  for (int i = 0; i < count; ++i) {
+    l.held.emplace_back(new max_align_t[sizes[i] / sizeof(max_align_t) + 1]);
+    memcpy(l.held.back().get(), args[i], sizes[i]);
+    l.args.push_back(l.held.back().get());
+  }
+  psgd_tape_now->launches.push_back(std::move(l));
+}
+
+// Writes down the launches that this thread makes through psgd_launch from here to psgd_tape_end, which returns their number.
+PSGD_API void* psgd_tape_begin() { return psgd_tape_now = new PsgdTape; }
+PSGD_API int psgd_tape_end() {
+  const int count = psgd_tape_now ? (int)psgd_tape_now->launches.size() : 0;
+  psgd_tape_now = nullptr;
+  return count;
+}
+PSGD_API void psgd_tape_free(void* tape) { delete (PsgdTape*)tape; }
+// Makes them again, on `stream`. Returns a CUDA error code.
+PSGD_API int psgd_tape_replay(const void* tape, cudaStream_t stream) {
+  for (const PsgdTape::Launch& l : ((const PsgdTape*)tape)->launches) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attrs[2];
+    psgd_launch_config(cfg, attrs, l.grid, l.block, l.smem, stream, l.early, l.cluster);
+    PSGD_CUDA_OK(cudaLaunchKernelExC(&cfg, l.kernel, const_cast<void**>(l.args.data())));
+  }
   return 0;
 }
 

@@ -416,6 +416,26 @@ class _Recordable:
             self._stream = before
 
 
+class _Tape:
+    """Launches written down by the library, to be made again by one call of it. Only their arguments are kept."""
+
+    def __init__(self, lib, body):
+        self._lib = lib
+        self._launches = lib.psgd_tape_begin()
+        try:
+            body()
+        finally:
+            self.count = lib.psgd_tape_end()
+
+    def __del__(self):
+        self._lib.psgd_tape_free(self._launches)
+
+    def __call__(self, stream: ctypes.c_void_p) -> None:
+        code = self._lib.psgd_tape_replay(self._launches, stream)
+        if code != 0:
+            native.check(code, "psgd_tape_replay")
+
+
 class NativeCompressor(_Recordable):
     """Runs `BasicPowerSGD.aggregate` on the GPU with the in-tree kernels."""
 
@@ -423,10 +443,10 @@ class NativeCompressor(_Recordable):
     _orth_clusters: Dict[str, bool] = {}
     _orth_by_rule: Dict[str, bool] = {}
 
-    # Rows of a list from which on one launch is the rule. Below, a replayed step gains 0 to 4 us of 30 to 45 at ranks 1 to 4 (two launches /
-    # one: 784x256 34.8 / 30.7, 4 x 256^2 33.0 / 33.1 at rank 2); such steps keep the number of launches that they
-    # report, except behind an orthonormalisation ahead of time (`begin_step`: a recorded training step 101.2 / 98.2 us).
-    ORTH_CLUSTER_ROWS = 2048
+    # Elements of a list from which on one launch is the rule. Below, a replayed step gains 3 to 4 us of 31 to 35 (two launches / one:
+    # 784x256 at rank 2 34.8 / 30.7); steps that small keep the number of launches that they report, except behind an
+    # orthonormalisation ahead of time (`begin_step`: a recorded training step 101.2 / 98.2 us).
+    ORTH_CLUSTER_ELEMS = 1 << 18
 
     def __init__(self, core):
         # the owner holds this object, not the other way round: both then go when the owner is dropped, and
@@ -471,8 +491,7 @@ class NativeCompressor(_Recordable):
             if world_size() == 1:
                 members = max((g.batch for g in self.plan.groups if g.r == 1), default=1)
                 self._orth_clusters[s] = bool(self.lib.psgd_orth_takes_clusters(self.tiles.max_r, longest, members, max(self.T - 1, 0)))
-                rows = sum((g.n if s == "p" else g.m) * g.batch for g in self.plan.groups)
-                self._orth_by_rule[s] = self._orth_clusters[s] and rows >= self.ORTH_CLUSTER_ROWS
+                self._orth_by_rule[s] = self._orth_clusters[s] and self.tiles.total_elems >= self.ORTH_CLUSTER_ELEMS
         # scratch of the orthonormalisation: partial sums per chunk; per unit (`_orth_rinv`) the leading
         # rows of the factor as they came in, which R falls back on when a column has to be replaced
         part_doubles = int(self.lib.psgd_orth_part_doubles(self.tiles.max_r, max(self.T - 1, 0)))
@@ -480,8 +499,7 @@ class NativeCompressor(_Recordable):
         self._orth_part = torch.zeros(max(max(self.n_chunks.values()), 1) * part_doubles, device=self.device, dtype=torch.float64)
         self._orth_rinv = torch.zeros(max_units * 2 * rt * rt, device=self.device, dtype=torch.float32)
         self._key = None
-        self._tape: Optional[list] = None
-        self._tapes: Dict[Tuple, list] = {}
+        self._tapes: Dict[Tuple, _Tape] = {}
         self._out_arena: Optional[torch.Tensor] = None
         self._hyper_dev = _to_device(self._default_hyper(), self.device)
         self.launches = 0  # kernels launched by the last aggregate()
@@ -703,15 +721,12 @@ class NativeCompressor(_Recordable):
 
     # -- launches --------------------------------------------------------------------------
     def _call(self, name: str, *args) -> None:
-        """One launch of the library on the current stream, counted, and written down while a step is
-        being recorded (see `_taped`)."""
+        """One launch of the library on the current stream, counted."""
         fn = getattr(self.lib, name)
         self._stream = _stream_ptr()
         native.check(fn(*args, self._stream), name)
         launched = 2 if name == "psgd_orth_launch" and not args[-1] & 4 else 1   # orthonormalisation: Gram matrices, then their use
         self.launches += launched
-        if self._tape is not None:
-            self._tape.append((fn, name, args, launched))
 
     def _taped(self, key: Tuple, body, inside: bool = False) -> None:
         """Run `body`, which issues the launches of a step; from the second step of its kind on repeat
@@ -732,21 +747,16 @@ class NativeCompressor(_Recordable):
         key = key + (self.core._ps_buffer.data_ptr(), self.core._qs_buffer.data_ptr())
         tape = self._tapes.get(key)
         if tape is None:
-            self._tape = []
-            try:
-                body()
+            before = self.launches
+            tape = _Tape(self.lib, body)
+            if tape.count == self.launches - before:   # (all of them went through the library's one way of launching)
                 if len(self._tapes) >= 16:   # recordings with tables of their own bring keys of their own
                     self._tapes.clear()
-                self._tapes[key] = self._tape
-            finally:
-                self._tape = None
+                self._tapes[key] = tape
             return
         self._stream = stream
-        for fn, name, args, launched in tape:
-            code = fn(*args, stream)
-            if code != 0:
-                native.check(code, name)
-            self.launches += launched
+        tape(stream)
+        self.launches += tape.count
 
     def _owned(self) -> tuple:
         """Everything a step addresses besides the caller's tensors; the next binding replaces the tables and
@@ -1118,6 +1128,7 @@ class NativeFlatAllReduce(_Recordable):
         self._keep_inputs = False
         self._nvls = None     # in-switch all-reduce object (parallel/nvls.py)
         self._nvls_failed = False
+        self._tapes: Dict[Tuple, _Tape] = {}   # of one worker's launch, see NativeCompressor._taped
 
     def check(self) -> None:
         """Raise `PowerSGDCommTimeout` if a bounded wait of an earlier launch gave up."""
@@ -1173,6 +1184,7 @@ class NativeFlatAllReduce(_Recordable):
         self._views = views
         self._hyper_dev = _to_device(NativeCompressor._default_hyper(), device)
         self._key = key
+        self._tapes.clear()
         self._choose_path(total, world_size(), device)
 
     def _choose_path(self, total: int, workers: int, device: torch.device) -> None:
@@ -1292,7 +1304,15 @@ class NativeFlatAllReduce(_Recordable):
             return
         self._stream = stream
         if self.path == "local":
-            self._launch(4 if sgd else 3, hyper_dev, 1.0, early, stream=stream)
+            key = (sgd, early, self._keep_inputs, hyper_dev.data_ptr())
+            tape = self._tapes.get(key)
+            if tape is not None:
+                tape(stream)
+                self.launches += 1
+                return
+            if len(self._tapes) >= 16:
+                self._tapes.clear()
+            self._tapes[key] = _Tape(self.lib, lambda: self._launch(4 if sgd else 3, hyper_dev, 1.0, early, stream=stream))
         elif self.path == "bulk":
             self._launch(0, hyper_dev, float(workers), stream=stream)
             code = self.lib.psgd_bulk_allreduce_launch(self.comm.ptr, ctypes.c_longlong(self.n_pad), workers, _stream_ptr())

@@ -21,6 +21,14 @@ def declare(lib) -> None:
 
     lib.psgd_stream_wait.restype = i32
     lib.psgd_stream_wait.argtypes = [vp]
+    lib.psgd_tape_begin.restype = vp
+    lib.psgd_tape_begin.argtypes = []
+    lib.psgd_tape_end.restype = i32
+    lib.psgd_tape_end.argtypes = []
+    lib.psgd_tape_free.restype = None
+    lib.psgd_tape_free.argtypes = [vp]
+    lib.psgd_tape_replay.restype = i32
+    lib.psgd_tape_replay.argtypes = [vp, vp]
     lib.psgd_graph_retain.restype = i32
     lib.psgd_graph_retain.argtypes = [C.c_longlong, vp]
     lib.psgd_graph_released.restype = i32

@@ -144,10 +144,9 @@ def _as_matrix(t: torch.Tensor) -> torch.Tensor:
 
 
 def _split_by_dim(grad_in, grad_out, memory_out):
-    vectors, matrices = [], []
-    for trio in zip(grad_in, grad_out, memory_out):
-        (vectors if trio[0].ndimension() <= 1 else matrices).append(trio)
-    return vectors, matrices
+    trios = list(zip(grad_in, grad_out, memory_out))
+    flat = [t.dim() <= 1 for t in grad_in]
+    return [x for x, f in zip(trios, flat) if f], [x for x, f in zip(trios, flat) if not f]
 
 
 class Reducer:
@@ -218,7 +217,8 @@ class _LowRankBase(Reducer):
         return self._native, fresh
 
     def _rank1_bits(self, vectors) -> int:
-        return 8 * sum(t.nelement() * t.element_size() for t, _, _ in vectors)
+        """Of float32 vectors."""
+        return 32 * int(np.frombuffer(scan.sizes([t for t, _, _ in vectors]), dtype=np.uint64).sum()) if vectors else 0
 
     def _views(self, matrices):
         sizes = []

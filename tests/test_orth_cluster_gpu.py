@@ -71,15 +71,15 @@ def test_rank_one_groups(members):
 
 
 def test_rule():
-    """Short lists keep two launches, as do units too long for a cluster and groups with too many members."""
+    """Small models keep two launches, as do units too long for a cluster and groups with too many members."""
     def rule(shapes, rank, iters=2):
         nat = NativeCompressor(BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=rank, num_iters_per_step=iters), backend="native"))
         return nat._orth_by_rule["p"], nat._orth_by_rule["q"]
 
-    assert rule([(2048, 64)], 2) == (True, False)
-    assert rule([(40, 2048)], 2) == (False, True)
+    assert rule([(512, 512)], 2) == (True, True)
+    assert rule([(512, 511)], 2) == (False, False)
     assert rule([(50257, 2048)], 4) == (False, True)
     assert rule([(4096, 2048)], 8) == (False, True)
-    assert rule([(64, 64)] * 700, 1) == (False, False)
-    assert rule([(64, 64)] * 700, 1, iters=1) == (False, False)   # 700 x 64 rows in one unit
+    assert rule([(64, 512)] * 700, 1) == (False, False)
+    assert rule([(16, 512)] * 700, 1, iters=1) == (True, False)   # 700 x 16 and 700 x 512 rows in one unit
     assert rule([(2048, 2048)], 32) == (False, False)
