@@ -78,11 +78,15 @@ __device__ __forceinline__ bool product_tile_ok(const PsgdTile& t, const PsgdMat
 
 template <int RT>
 __host__ __device__ constexpr int nt_max_rows() { return RT <= 16 ? NT_MAX_ROWS : NT_MAX_ROWS / 2; }
-// Staging buffer of an NT tile: rows of P-hat, later (up to rank 8, 32 KiB) one sum per warp, so that
-// the warps' sums are added by all threads at once instead of one warp after another.
+// Staging buffer of an NT tile: rows of P-hat, later the sums of the warps, [warp][column of a lane x RT][32 lanes + 1], all eight
+// warps' up to rank 8, four above.
+template <int RT>
+__host__ __device__ constexpr int nt_sum_warps() { return RT <= 8 ? GEMM_WARPS : GEMM_WARPS / 2; }
+constexpr int NT_SUM_PITCH = 33;   // words: neither lanes nor values of a lane meet in one bank
 template <int RT>
 __host__ __device__ constexpr int nt_stage_floats() {
-  return RT <= 8 && GEMM_WARPS * NT_TILE_COLS > nt_max_rows<RT>() ? GEMM_WARPS * NT_TILE_COLS * RT : nt_max_rows<RT>() * RT;
+  const int sums = (nt_sum_warps<RT>() * 4 * RT * NT_SUM_PITCH + 3) / 4 * 4, rows = nt_max_rows<RT>() * RT;
+  return sums > rows ? sums : rows;
 }
 
 // A lane owns 4 of the 128 columns of a column block; which ones depends on the access width:
@@ -94,6 +98,12 @@ __device__ __forceinline__ int lane_col(int lane, int c) {
   if (VEC == 2) return (c < 2) ? 2 * lane + c : 64 + 2 * lane + (c - 2);
   return lane + 32 * c;
 }
+
+// The lane that owns column lc, and which of its columns that is.
+template <int VEC>
+__device__ __forceinline__ int col_lane(int lc) { return VEC == 4 ? lc >> 2 : VEC == 2 ? (lc & 63) >> 1 : lc & 31; }
+template <int VEC>
+__device__ __forceinline__ int col_of_lane(int lc) { return VEC == 4 ? lc & 3 : VEC == 2 ? (lc & 1) + 2 * (lc >> 6) : lc >> 5; }
 
 // v[0..3] = the lane's four columns of the row at `rowp` (column block starting at c0, valid up
 // to cend); zero where the row or the column does not exist.
@@ -212,37 +222,43 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   }
   __syncthreads();
 
-  // deterministic cross-warp sum: warps are added in index order
-  if (RT <= 8) {
-    float* mine = sP + warp * NT_TILE_COLS * RT;
+  // Sum over the warps, in a fixed order. A warp's values lie lane by lane, so that neither their stores nor the loads of a thread that
+  // adds up one (column, k) meet in one bank: written in the order of the result, [column][k], 16 or 32 lanes did, and above rank 8, where
+  // one warp after another added to it, the sum was three quarters of a tile: 39 500 of 52 000 cycles on 4 x 1024x1001 at rank 16, 75 000
+  // of 134 000 on 3 x 9000x650 at rank 11, 4700 of 13 000 on 4 x 1001x1024 at rank 5; now 2900, 3000 and 1100.
+  // The launches: 34.8 -> 12.6 us, 137 -> 60, 9.7 -> 7.7.
+  constexpr int SUMS = nt_sum_warps<RT>(), PER_WARP = 4 * RT * NT_SUM_PITCH;
+  auto slot = [&](int w, int c, int k) { return sP + w * PER_WARP + (c * RT + k) * NT_SUM_PITCH; };
+  if (SUMS < GEMM_WARPS) {
+    if (warp >= SUMS) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int k = 0; k < RT; ++k) slot(warp - SUMS, c, k)[lane] = acc[c][k];
+    }
+    __syncthreads();
+    if (warp < SUMS) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int k = 0; k < RT; ++k) slot(warp, c, k)[lane] += acc[c][k];   // (its own places: nobody else reads them yet)
+    }
+  } else {
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int k = 0; k < RT; ++k) mine[lane_col<VEC>(lane, c) * RT + k] = acc[c][k];
-    __syncthreads();
-    for (int e = tid; e < NT_TILE_COLS * RT; e += GEMM_THREADS) {
-      float s = sP[e];
-#pragma unroll
-      for (int w = 1; w < GEMM_WARPS; ++w) s += sP[w * NT_TILE_COLS * RT + e];
-      sSum[e] = s;
-    }
-    __syncthreads();
-  } else {
-    for (int w = 0; w < GEMM_WARPS; ++w) {
-      if (warp == w) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int lc = lane_col<VEC>(lane, c);
-#pragma unroll
-          for (int k = 0; k < RT; ++k) {
-            if (w == 0) sSum[lc * RT + k] = acc[c][k];
-            else sSum[lc * RT + k] += acc[c][k];
-          }
-        }
-      }
-      __syncthreads();
-    }
+      for (int k = 0; k < RT; ++k) slot(warp, c, k)[lane] = acc[c][k];
   }
+  __syncthreads();
+#pragma unroll 1
+  for (int e = tid; e < NT_TILE_COLS * RT; e += GEMM_THREADS) {
+    const float* of = slot(0, col_of_lane<VEC>(e / RT), e % RT) + col_lane<VEC>(e / RT);
+    float s = of[0];
+#pragma unroll
+    for (int w = 1; w < SUMS; ++w) s += of[w * PER_WARP];
+    sSum[e] = s;
+  }
+  __syncthreads();
 
   constexpr int tile_elems = NT_TILE_COLS * RT;
   bool owner = true;  // does this CTA write the output rows?
@@ -376,8 +392,7 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
   const float* qin = a.in + mt.q_off + (long long)t.col0 * r;   // written by the launch before: plain loads
   auto place = [&](int lc, int k) {   // in sQ
     const int b = lc & 127;
-    const int ln = VEC == 4 ? b >> 2 : VEC == 2 ? (b & 63) >> 1 : b & 31;
-    const int c = VEC == 4 ? b & 3 : VEC == 2 ? (b & 1) + 2 * (b >> 6) : b >> 5;
+    const int ln = col_lane<VEC>(b), c = col_of_lane<VEC>(b);
     const int f = c * RT + k;
     return sQ + (((lc >> 7) * RT + (f >> 2)) * 32 + ln) * 4 + (f & 3);
   };
@@ -426,10 +441,15 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
     }
   }
 
-  if (RPW * RT <= 32) {
-    const float s = warp_sums<RPW * RT>(acc, lane);
-    constexpr int SPAN = 32 / (RPW * RT);   // lanes that hold the same sum
-    if (lane % SPAN == 0) sSum[rbase * RT + lane / SPAN] = s;
+  constexpr int N = RPW * RT < 32 ? RPW * RT : 32;   // values added up at a time
+#pragma unroll
+  for (int first = 0; first < RPW * RT; first += N) {
+    float part[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) part[i] = acc[first + i];
+    const float s = warp_sums<N>(part, lane);
+    constexpr int SPAN = 32 / N;   // lanes that hold the same sum
+    if (lane % SPAN == 0) sSum[rbase * RT + first + lane / SPAN] = s;
   }
   __syncthreads();
 
@@ -478,8 +498,16 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
   }
 }
 
-template <int RT, int RPW>
-__global__ void __launch_bounds__(GEMM_THREADS) psgd_gemm_nn_kernel(GemmArgs a) {
+// Rows of a warp: 64 sums at most in registers. Every row more spreads the rows of Q-hat that a tile stages, as many bytes as 32 rows
+// of its part of the matrix at rank 16, over more of them: 4 x 1024x1001 at rank 16, two rows / four 19.1 / 13.9 us, 3 x 9000x650 at rank
+// 11 69.8 / 62.2.
+template <int RT>
+__host__ __device__ constexpr int nn_rows_per_warp() { return RT <= 16 ? 4 : 2; }
+// PER_SM: CTAs of an SM that registers have to allow. More registers let more of a tile's loads run ahead, which is what a launch of at most
+// two tiles per SM needs; with more tiles a third CTA does more: us per pass, two / three, 3 x 1001x777 + 2 x 515x2049 at rank
+// 3 x 3 (198 tiles) 89.4 / 94.1, ResNet-18's recorded step (443) 105.6 / 102.2, LSTM step (1532) 212.7 / 212.0.
+template <int RT, int RPW, int PER_SM>
+__global__ void __launch_bounds__(GEMM_THREADS, PER_SM) psgd_gemm_nn_kernel(GemmArgs a) {
   extern __shared__ __align__(16) float smem[];   // staged rows of Q-hat
   __shared__ float sSum[GEMM_WARPS * RPW * RT];
   psgd_launch_dependents();
@@ -523,9 +551,10 @@ static int launch_nt(const GemmArgs& a, int ntiles, int early, cudaStream_t stre
 
 template <int RT>
 static int launch_nn(const GemmArgs& a, int ntiles, int early, cudaStream_t stream) {
-  constexpr int RPW = RT <= 8 ? 4 : (RT == 16 ? 2 : 1);
+  constexpr int RPW = nn_rows_per_warp<RT>();
   const size_t smem = (size_t)nn_max_cols<RT>() * RT * sizeof(float);
-  return psgd_launch(psgd_gemm_nn_kernel<RT, RPW>, ntiles, GEMM_THREADS, smem, stream, early, a);
+  if (RT >= 8 || ntiles <= 2 * 148) return psgd_launch(psgd_gemm_nn_kernel<RT, RPW, 2>, ntiles, GEMM_THREADS, smem, stream, early, a);
+  return psgd_launch(psgd_gemm_nn_kernel<RT, RPW, RT >= 8 ? 2 : 3>, ntiles, GEMM_THREADS, smem, stream, early, a);
 }
 
 #define PSGD_DISPATCH_RT(FN)                                   \
@@ -539,7 +568,7 @@ static int launch_nn(const GemmArgs& a, int ntiles, int early, cudaStream_t stre
 // Rows handled by one NN tile for the template rank that `max_r` selects (the planner needs it).
 PSGD_API int psgd_gemm_nn_tile_rows(int max_r) {
   const int rt = max_r <= 1 ? 1 : max_r <= 2 ? 2 : max_r <= 4 ? 4 : max_r <= 8 ? 8 : max_r <= 16 ? 16 : 32;
-  return GEMM_WARPS * (rt <= 8 ? 4 : (rt == 16 ? 2 : 1));
+  return GEMM_WARPS * (rt <= 16 ? nn_rows_per_warp<16>() : nn_rows_per_warp<32>());
 }
 // Most columns of an NN tile (a multiple of 128).
 PSGD_API int psgd_gemm_nn_max_cols(int max_r) { return max_r <= 8 ? 1024 : max_r <= 16 ? nn_max_cols<16>() : nn_max_cols<32>(); }
