@@ -604,12 +604,13 @@ class NativeCompressor(_Recordable):
         # tensor-core (TMA + tcgen05) path: matrices TMA can address and that are worth it
         mode = os.environ.get("PSGD_B200_GEMM", "auto")
         hbm_bound = self.tiles.total_elems * 4 > (96 << 20)
+        few = self.tiles.total_elems <= self.TC_FEW_ELEMS.get(self.tiles.rt, 0) and all(g.n <= 2048 and g.m <= 4096 for g in self.plan.groups)
         tc = []
         maps = np.zeros((len(self.tiles.mats), 256), dtype=np.uint8)
         for mi, (gi, _pos, idx) in enumerate(self.tiles.mats):
             g = self.plan.groups[gi]
             ok = vec[mi] == 4 and g.n >= 128 and g.m >= 128 and mode != "ffma"
-            ok = ok and (mode == "tc" or hbm_bound or self.tiles.max_r >= 8)
+            ok = ok and (mode == "tc" or hbm_bound or (self.tiles.max_r >= 8 and not few))
             if ok:
                 buf = (ctypes.c_ubyte * 256)()
                 code = self.lib.psgd_tma_encode_matrix(buf, ctypes.c_void_p(grads[idx].data_ptr()), g.n, g.m)
@@ -640,6 +641,14 @@ class NativeCompressor(_Recordable):
         self._out_views = out_views
         self._tapes.clear()
         self._key = key
+
+    # Elements up to which the products of a list at template rank 8 and 16 stay on the CUDA cores, where a tile has less to set up
+    # and to wait for. us per pass, tensor cores / CUDA cores, at 8 x 1, 8 x 2, 16 x 1, 16 x 2: 4 x 512^2 36.8 / 33.6, 53.6 / 46.1, 42.9 / 41.2,
+    # 68.1 / 60.6; 16 x 512^2 64 / 60, 84 / 74, 71 / 69, 103 / 93; 4 x 1024^2 65 / 63, 82 / 77, 71 / 74, 101 / 95; 8 x 1024^2 85 / 80, 107 / 105, 94 / 101,
+    # 130 / 139; 16 x 1024^2 133 / 132, 168 / 174, 150 / 164, 196 / 220. Sums of more than 2048 rows make many tiles of M^T P whose
+    # hand-over costs more than they save: 1 x 4096x1024 65 / 66, 83 / 90, 72 / 77, 101 / 112; 12000x512 76 / 78, 101 / 113, 90 / 96, 126 / 138; rows
+    # of more than 4096 make many of M Q: 512x12000 76 / 74, 104 / 102, 90 / 92, 135 / 135; 1024x8192 86 / 83, 114 / 113, 99 / 103, 143 / 148.
+    TC_FEW_ELEMS = {8: 1 << 23, 16: 1 << 22}
 
     # Share of elements accessed by 16 bytes from which on the decompression takes the form for those (csrc/finalize.cu, ROWS):
     # 94 % loses 3 % at 16 factor columns, 98 % loses nothing.
