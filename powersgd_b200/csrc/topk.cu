@@ -143,8 +143,8 @@ PSGD_API int psgd_topk_abs(const float* x, long long n, long long k, int* worksp
 // per SM serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: 68 us by three histogram passes and a
 // compaction, 54 us by lists. With one worker launch 2 writes the dense output beside the memory (TopkItem::out), so that nothing
 // is left to combine, every launch starts beside the end of the one before, and the workspace is cleared by the call
-// before: the pass of the reducer 86 -> 55 us, of which 12 go to launch 1 (45 MB from HBM and as many additions in shared
-// memory), 27 to launch 2 (135 MB), 8 to launch 3 and 2 to launch 4.
+// before: the pass of the reducer 86 -> 55 us; with as many blocks as run at a time, three per SM, in launch 2 too, 51.5, of which 12 go
+// to launch 1 (45 MB from HBM and as many additions in shared memory), 22 to launch 2 (135 MB), 8 to launch 3 and 2 to launch 4.
 namespace {
 
 struct TopkItem {
@@ -359,7 +359,7 @@ __device__ __forceinline__ float tk_dense(float v) { return __fadd_rn(0.f, v); }
 // Launch 2: what lies above the leading digit is taken, what lies in it is listed; or the second histogram.
 // cand_v / cand_p: lists of candidates. ws_next: workspace of the call after this one, cleared here (a clearing of its own costs
 // a call 3.5 us), or null.
-__global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_split_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
+__global__ void __launch_bounds__(TK_THREADS, 3) psgd_topk_many_split_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                            const int* __restrict__ block_part, const int* __restrict__ item_parts,
                                                                            int* __restrict__ ws_all, int* __restrict__ ws_next,
                                                                            float* __restrict__ values, int* __restrict__ positions,
@@ -453,7 +453,8 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   int* ws = ws_all + (long long)it * TK_WS_INTS;
   const int* counters = ws + TK_BINS0 + TK_BINS1 + TK_BINS2;
   int* sh = bins_sh.c;
-  for (int b = threadIdx.x; b < TK_BINS1 + TK_BINS2; b += TK_THREADS) sh[b] = 0;
+  if (block_part[blockIdx.x] == 0)
+    for (int b = threadIdx.x; b < TK_BINS1 + TK_BINS2; b += TK_THREADS) sh[b] = 0;
   psgd_wait_for_predecessor();
   if (threadIdx.x == 0) {
     pick.prefix = (unsigned)counters[TK_PREFIX];
