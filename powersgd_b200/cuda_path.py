@@ -155,16 +155,19 @@ class TilePlan:
                 fin["f"].append((mi, g.n, self.fin_rows, g.m, 128, v))
             if tc_flags[mi]:
                 row_blocks, col_blocks = _split_even(g.n, tc_k_nt, 32), _split_even(g.m, tc_k_nn, 32)
+                whole_rows, whole_cols = row_blocks, col_blocks
                 for c0 in range(0, g.m, 128):
                     if tail_nt:
-                        row_blocks, tc_nt = _split_parts(g.n, tail_nt.get(tc_nt, _split_count(g.n, tc_k_nt, 32)), 32), tc_nt + 1
+                        row_blocks = _split_parts(g.n, tail_nt[tc_nt], 32) if tc_nt in tail_nt else whole_rows
+                        tc_nt += 1
                     for si, (r0, rows) in enumerate(row_blocks):
                         nt["tc"].append((mi, r0, rows, c0, min(128, g.m - c0), si, len(row_blocks), ticket, tc_slots, v, (0, 0)))
                     ticket += 1
                     tc_slots += len(row_blocks)
                 for r0 in range(0, g.n, 128):
                     if tail_nn:
-                        col_blocks, tc_nn = _split_parts(g.m, tail_nn.get(tc_nn, _split_count(g.m, tc_k_nn, 32)), 32), tc_nn + 1
+                        col_blocks = _split_parts(g.m, tail_nn[tc_nn], 32) if tc_nn in tail_nn else whole_cols
+                        tc_nn += 1
                     for si, (c0, cols) in enumerate(col_blocks):
                         nn["tc"].append((mi, r0, min(128, g.n - r0), c0, cols, si, len(col_blocks), ticket, tc_slots, v, (0, 0)))
                     ticket += 1
@@ -697,6 +700,9 @@ class NativeCompressor(_Recordable):
         """Product tile lists of the early bucket ("fA") and of everything else ("fB")."""
         early_mats = [mi for mi, (_gi, _pos, idx) in enumerate(self.tiles.mats) if idx in self._early_bucket]
         for name in ("nt", "nn"):
+            if not early_mats:
+                self._tiles_dev[name].update(fA=(None, 0), fB=self._tiles_dev[name]["f"])
+                continue
             arr = self._tile_arrays[name]["f"]
             mask = np.isin(arr["mat"], early_mats) if len(arr) else np.zeros(0, dtype=bool)
             for key, sub in (("fA", arr[mask]), ("fB", arr[~mask])):
