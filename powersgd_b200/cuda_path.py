@@ -255,9 +255,9 @@ class TilePlan:
     # as rounds x (overhead + rows) over tile extents 512 ... 4096 on 4 x 4096^2
     TC_TILE_OVERHEAD_ROWS = 136
 
-    # The same for lists of one to three rounds, template ranks up to 8 and above, from rounds of 176 to 2720 rows: 50257 x 1024 at rank 16,
-    # 1408 and 704 rows 57.5 / 68.4 us, 352 rows 88.7; GPT-2 medium at rank 4, 1456 / 2712 / 5416 tiles 252.5 / 282.6 / 328 us.
-    TC_ROUND_OVERHEAD_ROWS = (236, 330)
+    # The same above rank 8 for lists of one to three rounds, from rounds of 352 to 1408 rows: 50257 x 1024 at rank 16, 1408 and
+    # 704 rows 57.5 / 68.4 us, 352 rows 88.7.
+    TC_ROUND_OVERHEAD_ROWS = 330
 
     def _tc_extents(self, groups, transposed: bool) -> Tuple[int, Dict[int, int]]:
         """K extent of the tiles, and how many tiles the last output blocks of 128 (by number, in the order of `build`) are cut in if
@@ -268,9 +268,11 @@ class TilePlan:
         slots = 148 * self.TC_CTAS_PER_SM
         k = self._pick_tc_k(groups, transposed)
         blocks = [((g.n if transposed else g.m), -(-(g.m if transposed else g.n) // 128)) for g in groups]   # of (length, number)
-        if not slots < sum(number * _split_count(length, k, 32) for length, number in blocks) <= 3 * slots or os.environ.get("PSGD_B200_TC_K"):
+        # (above rank 8: at 8 two half-iterations leave directions of nearly equal size, where another order of a sum shows in later steps)
+        if (self.rp_tc <= 8 or os.environ.get("PSGD_B200_TC_K")
+                or not slots < sum(number * _split_count(length, k, 32) for length, number in blocks) <= 3 * slots):
             return k, {}
-        overhead, longest = self.TC_ROUND_OVERHEAD_ROWS[self.rp_tc > 8], max(length for length, _number in blocks)
+        overhead, longest = self.TC_ROUND_OVERHEAD_ROWS, max(length for length, _number in blocks)
         work, best = sum(length * number for length, number in blocks), None
         for pieces in range(1, 9):
             k = -(-longest // pieces)
@@ -607,13 +609,12 @@ class NativeCompressor(_Recordable):
         # tensor-core (TMA + tcgen05) path: matrices TMA can address and that are worth it
         mode = os.environ.get("PSGD_B200_GEMM", "auto")
         hbm_bound = self.tiles.total_elems * 4 > (96 << 20)
-        few = self.tiles.total_elems <= self.TC_FEW_ELEMS.get(self.tiles.rt, 0) and all(g.n <= 2048 and g.m <= 4096 for g in self.plan.groups)
         tc = []
         maps = np.zeros((len(self.tiles.mats), 256), dtype=np.uint8)
         for mi, (gi, _pos, idx) in enumerate(self.tiles.mats):
             g = self.plan.groups[gi]
             ok = vec[mi] == 4 and g.n >= 128 and g.m >= 128 and mode != "ffma"
-            ok = ok and (mode == "tc" or hbm_bound or (self.tiles.max_r >= 8 and not few))
+            ok = ok and (mode == "tc" or hbm_bound or self.tiles.max_r >= 8)
             if ok:
                 buf = (ctypes.c_ubyte * 256)()
                 code = self.lib.psgd_tma_encode_matrix(buf, ctypes.c_void_p(grads[idx].data_ptr()), g.n, g.m)
@@ -644,14 +645,6 @@ class NativeCompressor(_Recordable):
         self._out_views = out_views
         self._tapes.clear()
         self._key = key
-
-    # Elements up to which the products of a list at template rank 8 and 16 stay on the CUDA cores, where a tile has less to set up
-    # and to wait for. us per pass, tensor cores / CUDA cores, at 8 x 1, 8 x 2, 16 x 1, 16 x 2: 4 x 512^2 36.8 / 33.6, 53.6 / 46.1, 42.9 / 41.2,
-    # 68.1 / 60.6; 16 x 512^2 64 / 60, 84 / 74, 71 / 69, 103 / 93; 4 x 1024^2 65 / 63, 82 / 77, 71 / 74, 101 / 95; 8 x 1024^2 85 / 80, 107 / 105, 94 / 101,
-    # 130 / 139; 16 x 1024^2 133 / 132, 168 / 174, 150 / 164, 196 / 220. Sums of more than 2048 rows make many tiles of M^T P whose
-    # hand-over costs more than they save: 1 x 4096x1024 65 / 66, 83 / 90, 72 / 77, 101 / 112; 12000x512 76 / 78, 101 / 113, 90 / 96, 126 / 138; rows
-    # of more than 4096 make many of M Q: 512x12000 76 / 74, 104 / 102, 90 / 92, 135 / 135; 1024x8192 86 / 83, 114 / 113, 99 / 103, 143 / 148.
-    TC_FEW_ELEMS = {8: 1 << 23, 16: 1 << 22}
 
     # Share of elements accessed by 16 bytes from which on the decompression takes the form for those (csrc/finalize.cu, ROWS):
     # 94 % loses 3 % at 16 factor columns, 98 % loses nothing.

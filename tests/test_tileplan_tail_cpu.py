@@ -6,8 +6,8 @@ from powersgd_b200.plan import CompressionPlan
 native = pytest.importorskip("powersgd_b200.ops.native")
 
 
-@pytest.mark.parametrize("shapes,rank", [([(50257, 1024)], 16), ([(38016, 256)], 4), ([(37889, 1000)], 8), ([(20000, 640)] * 4, 8),
-                                         ([(4096, 4096)] * 4, 4), ([(512, 38000)], 4), ([(24000, 1500), (130, 40004), (9000, 132)], 11)])
+@pytest.mark.parametrize("shapes,rank", [([(50257, 1024)], 16), ([(38016, 256)], 9), ([(37889, 1000)], 11), ([(20000, 640)] * 4, 8),
+                                         ([(4096, 4096)] * 4, 4), ([(512, 38000)], 32), ([(24000, 1500), (130, 40004), (9000, 132)], 11)])
 def test_every_sum_is_covered_once_and_the_last_round_is_full(shapes, rank):
     from powersgd_b200.cuda_path import TilePlan
 
@@ -33,7 +33,7 @@ def test_every_sum_is_covered_once_and_the_last_round_is_full(shapes, rank):
         count = len(arrays[name]["tc"])
         blocks = sum(g.batch * -(-(g.m if name == "nt" else g.n) // 128) for g in plan.groups)
         assert len(by_ticket) == blocks
-        if slots < blocks <= 1.5 * slots:   # the rest of the blocks has room to be cut at least in two
+        if rank > 8 and slots < blocks <= 1.5 * slots:   # the rest of the blocks has room to be cut at least in two
             last = arrays[name]["tc"][-1]
             g = plan.groups[tiles.mats[int(last["mat"])][0]]
             assert count > blocks and int(last[size]) <= (g.n if name == "nt" else g.m) / 2 + 32
