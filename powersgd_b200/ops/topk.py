@@ -148,7 +148,8 @@ def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tens
     lib = native.lib()
     device = tensors[0].device
     stream = _current_stream()
-    key = (device, stream.value, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks), scan.addresses(outs))
+    key = (device, stream.value, scan.addresses(tensors), scan.addresses(mems), scan.sizes(tensors), tuple(ks), scan.addresses(outs),
+           None if outs is None else scan.sizes(outs))   # (an output of another length is not written by these launches)
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
     recorded = is_recorded(stream)

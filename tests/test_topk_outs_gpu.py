@@ -65,3 +65,17 @@ def test_outputs_where_others_are_read():
         for b, v, p in zip(before, values.split(ks), positions.split(ks)):
             assert torch.equal(v, b[p.long()])
     topk._many_cache.clear()
+
+
+def test_another_length_at_the_same_address():
+    """A view that is as long as the tensor, then longer and shorter ones that begin where it does, on the tables that the first has left."""
+    topk._many_cache.clear()
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x, room = torch.randn(30000, generator=g, device="cuda"), torch.empty(32000, device="cuda")
+    for length in (30000, 31000, 29000, 30000):
+        room.fill_(float("nan"))
+        values, positions = topk.topk_abs_many([x], [700], None, [room[:length]])
+        want, inside = torch.zeros(length, device="cuda"), positions < length
+        want.index_add_(0, positions[inside].long(), values[inside])
+        assert torch.equal(room[:length], want) and room[length:].isnan().all()
+    topk._many_cache.clear()
