@@ -165,7 +165,7 @@ constexpr int TK_SHORT = 1, TK_LONG = 2;   // TK_WAY: by the list of candidates,
 // Block-wide: walks `bins` (<= 2048, TK_THREADS threads x 4 bins) from the top until `remain` entries are
 // covered; returns the bin in *bin_out and the number to take inside it in *remain_io. `scan`: one
 // int per warp.
-__device__ void tk_choose_block(const int* __restrict__ hist, int bins, long long* remain_io, int* bin_out, int* scan) {
+__device__ void tk_choose_block(const int* hist, int bins, long long* remain_io, int* bin_out, int* scan) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   // thread t owns bins [4t, 4t + 4), counted from the TOP: bin index bins - 1 - j
   int c[4], local = 0;
@@ -361,7 +361,7 @@ __device__ __forceinline__ float tk_dense(float v) { return __fadd_rn(0.f, v); }
 // a call 3.5 us), or null.
 __global__ void __launch_bounds__(TK_THREADS, 3) psgd_topk_many_split_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                            const int* __restrict__ block_part, const int* __restrict__ item_parts,
-                                                                           int* __restrict__ ws_all, int* __restrict__ ws_next,
+                                                                           int* ws_all, int* __restrict__ ws_next,
                                                                            float* __restrict__ values, int* __restrict__ positions,
                                                                            float* __restrict__ cand_v, int* __restrict__ cand_p) {
   __shared__ SplitScratch sh;
@@ -423,25 +423,26 @@ __global__ void __launch_bounds__(TK_THREADS, 3) psgd_topk_many_split_kernel(con
 
 // f(value, index) for every entry of a list from `from` on (block-wide), eight loads of a thread under way.
 template <class F>
-__device__ __forceinline__ void tk_walk(const float* __restrict__ list, int from, int n, F f) {
+__device__ __forceinline__ void tk_walk(const float* list, int from, int n, F f) {
   for (int first = from + threadIdx.x; first < n; first += 8 * TK_THREADS) {
     float v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      if (first + u * TK_THREADS < n) v[u] = list[first + u * TK_THREADS];
+      if (first + u * TK_THREADS < n) v[u] = __ldcg(list + first + u * TK_THREADS);
 #pragma unroll
     for (int u = 0; u < 8; ++u)
       if (first + u * TK_THREADS < n) f(v[u], first + u * TK_THREADS);
   }
 }
 
-// Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram. One block walks a list alone,
+// Launch 3: the threshold among a tensor's candidates, by its first block; or the third histogram. The launch may start while the one
+// before still writes the list and the workspace: no read-only loads of them, here or in launch 4. One block walks a list alone,
 // three times over, so nothing but the loads under way hides a latency: the first 4096 entries stay in registers.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                             const int* __restrict__ block_part, const int* __restrict__ item_parts,
-                                                                            int* __restrict__ ws_all, float* __restrict__ values,
-                                                                            int* __restrict__ positions, const float* __restrict__ cand_v,
-                                                                            const int* __restrict__ cand_p) {
+                                                                            int* ws_all, float* __restrict__ values,
+                                                                            int* __restrict__ positions, const float* cand_v,
+                                                                            const int* cand_p) {
   __shared__ Bins bins_sh;
   __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
   constexpr int OWN = 8;
   float own[OWN];
 #pragma unroll
-  for (int u = 0; u < OWN; ++u) own[u] = (int)threadIdx.x + u * TK_THREADS < n ? cv[threadIdx.x + u * TK_THREADS] : 0.f;
+  for (int u = 0; u < OWN; ++u) own[u] = (int)threadIdx.x + u * TK_THREADS < n ? __ldcg(cv + threadIdx.x + u * TK_THREADS) : 0.f;
   auto walk = [&](auto f) {
 #pragma unroll
     for (int u = 0; u < OWN; ++u)
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
       slot = base_equal + eq;
     }
     if (slot >= item.k) return;
-    const int p = cp[e];
+    const int p = __ldcg(cp + e);
     val[slot] = v;
     pos[slot] = p;
     if (item.memory) item.memory[p] = 0.f;
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_refine_kernel(const
 // Launch 4: takes the k entries of a tensor with too many candidates.
 __global__ void __launch_bounds__(TK_THREADS) psgd_topk_many_compact_kernel(const TopkItem* __restrict__ items, const int* __restrict__ block_item,
                                                                              const int* __restrict__ block_part, const int* __restrict__ item_parts,
-                                                                             int* __restrict__ ws_all, float* __restrict__ values,
+                                                                             int* ws_all, float* __restrict__ values,
                                                                              int* __restrict__ positions) {
   __shared__ int scan[TK_THREADS / 32];
   __shared__ Pick pick;

@@ -49,3 +49,27 @@ def test_a_wait_that_ran_out_is_not_put_down_to_the_tensor_cores():
     assert "tensor-core" not in str(caught.value)
     Word.value = 0
     nat.check()
+
+
+def test_launches_that_may_start_early_promise_nothing_about_what_they_wait_for():
+    """A `const __restrict__` parameter may be read through the cache for data that nobody writes while the kernel runs, which does
+    not hold for what the launch before it writes. Tables that no launch writes may be declared so."""
+    import os
+    import re
+
+    import powersgd_b200
+
+    folder = os.path.join(os.path.dirname(powersgd_b200.__file__), "csrc")
+    tables, waiting = {"items", "block_item", "block_part", "item_parts"}, 0
+    for name in sorted(f for f in os.listdir(folder) if f.endswith(".cu")):
+        with open(os.path.join(folder, name)) as fp:
+            text = fp.read()
+        kernels = list(re.finditer(r"__global__[^;{]*?(\w+_kernel)\(([^{;]*)\)\s*\{", text))
+        for kernel, after in zip(kernels, kernels[1:] + [None]):
+            body = text[kernel.end() : after.start() if after else len(text)].split("\n}\n")[0]
+            if "psgd_wait_for_predecessor" not in body:
+                continue
+            waiting += 1
+            promised = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", kernel.group(2)))
+            assert promised <= tables, (name, kernel.group(1), promised - tables)
+    assert waiting >= 10, waiting
