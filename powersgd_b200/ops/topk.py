@@ -153,7 +153,8 @@ def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tens
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
     recorded = is_recorded(stream)
-    entry = None if recorded else _many_cache.get(key)
+    # (taken out until the call is complete: whatever breaks it off may leave the half of the workspace uncleared that the next one counts in)
+    entry = None if recorded else _many_cache.pop(key, None)
     if entry is None:
         release_finished()
         dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64),
@@ -197,12 +198,8 @@ def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tens
             }
         if recorded:
             keep_with_graph(None, entry)
-        else:
-            # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
-            # valid for whatever tensors present the same addresses again, so no tensor is kept alive
-            if len(_many_cache) >= MOST_LISTS:
-                _many_cache.clear()
-            _many_cache[key] = entry
+        elif len(_many_cache) >= MOST_LISTS:
+            _many_cache.clear()
     vp = ctypes.c_void_p
     half = 2 * entry["ws"].numel()   # in bytes
     turn, base = entry["turn"], entry["ws"].data_ptr()
@@ -211,10 +208,12 @@ def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tens
         vp(entry["parts"].data_ptr()), entry["nblocks"], vp(base + turn * half), vp(0 if recorded else base + (1 - turn) * half),
         vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
     )
-    entry["turn"] = 1 - turn
-    if code != 0 and not recorded:
-        _many_cache.pop(key, None)   # who knows what is cleared
     native.check(code, "psgd_topk_abs_many")
+    if not recorded:
+        # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
+        # valid for whatever tensors present the same addresses again, so no tensor is kept alive
+        entry["turn"] = 1 - turn
+        _many_cache[key] = entry
     return entry["dense"]
 
 

@@ -35,3 +35,25 @@ def test_an_output_of_another_length_at_the_same_address(fake):
     assert not _select(x, [room])
     assert _select(x, [room[:100]])
     assert not _select(x, None)
+
+
+def test_a_call_that_breaks_off_leaves_no_workspace_behind(fake):
+    """A call counts in one half of its workspace and clears the other for the next; the halves change places with its last line."""
+    halves = []
+
+    def launch(*args):
+        halves.append((args[6].value, args[7].value))   # counted in, cleared
+        if len(halves) == 3:
+            raise KeyboardInterrupt   # as the interpreter raises it behind a foreign call, whose launches have been made
+        return 0
+
+    fake.launch, x = launch, torch.randn(100)
+    _select(x, None)
+    _select(x, None)
+    assert halves[1] == halves[0][::-1]
+    with pytest.raises(KeyboardInterrupt):
+        _select(x, None)
+    assert not topk._many_cache   # the next call brings a workspace of zeros
+    _select(x, None)
+    (entry,) = topk._many_cache.values()
+    assert entry["turn"] == 1
