@@ -1316,11 +1316,14 @@ class NativeFlatAllReduce(_Recordable):
             tape = self._tapes.get(key)
             if tape is not None:
                 tape(stream)
-                self.launches += 1
+                self.launches += tape.count
                 return
-            if len(self._tapes) >= 16:
-                self._tapes.clear()
-            self._tapes[key] = _Tape(self.lib, lambda: self._launch(4 if sgd else 3, hyper_dev, 1.0, early, stream=stream))
+            before = self.launches
+            tape = _Tape(self.lib, lambda: self._launch(4 if sgd else 3, hyper_dev, 1.0, early, stream=stream))
+            if tape.count == self.launches - before:   # (it went through the library's one way of launching)
+                if len(self._tapes) >= 16:
+                    self._tapes.clear()
+                self._tapes[key] = tape
         elif self.path == "bulk":
             self._launch(0, hyper_dev, float(workers), stream=stream)
             code = self.lib.psgd_bulk_allreduce_launch(self.comm.ptr, ctypes.c_longlong(self.n_pad), workers, _stream_ptr())
