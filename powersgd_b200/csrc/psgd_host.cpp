@@ -6,6 +6,7 @@
 #include <string.h>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <vector>
 #include "psgd_common.cuh"
 
@@ -78,26 +79,33 @@ struct PsgdTape {
     std::vector<void*> args;
   };
   std::vector<Launch> launches;
+  bool complete = true;
 };
 thread_local PsgdTape* psgd_tape_now = nullptr;
 
 void psgd_tape_add(const void* kernel, int grid, int block, size_t smem, int early, int cluster, int count, const void* const* args,
                    const size_t* sizes) {
-  PsgdTape::Launch l = {kernel, grid, block, early, cluster, smem, {}, {}};
-  for (int i = 0; i < count; ++i) {
-    l.held.emplace_back(new max_align_t[sizes[i] / sizeof(max_align_t) + 1]);
-    memcpy(l.held.back().get(), args[i], sizes[i]);
-    l.args.push_back(l.held.back().get());
+  PsgdTape& tape = *psgd_tape_now;
+  try {
+    PsgdTape::Launch l = {kernel, grid, block, early, cluster, smem, {}, {}};
+    for (int i = 0; i < count; ++i) {
+      l.held.emplace_back(new max_align_t[sizes[i] / sizeof(max_align_t) + 1]);
+      memcpy(l.held.back().get(), args[i], sizes[i]);
+      l.args.push_back(l.held.back().get());
+    }
+    tape.launches.push_back(std::move(l));
+  } catch (const std::bad_alloc&) {   // the launch itself has been made: the callers of the library get no exception from it
+    tape.complete = false;
   }
-  psgd_tape_now->launches.push_back(std::move(l));
 }
 
-// Writes down the launches that this thread makes through psgd_launch from here to psgd_tape_end, which returns their number.
-PSGD_API void* psgd_tape_begin() { return psgd_tape_now = new PsgdTape; }
+// Writes down the launches that this thread makes through psgd_launch from here to psgd_tape_end, which returns their number; -1
+// if there was no memory for all of them. Null if there is none at all.
+PSGD_API void* psgd_tape_begin() { return psgd_tape_now = new (std::nothrow) PsgdTape; }
 PSGD_API int psgd_tape_end() {
-  const int count = psgd_tape_now ? (int)psgd_tape_now->launches.size() : 0;
+  const PsgdTape* tape = psgd_tape_now;
   psgd_tape_now = nullptr;
-  return count;
+  return tape && tape->complete ? (int)tape->launches.size() : -1;
 }
 PSGD_API void psgd_tape_free(void* tape) { delete (PsgdTape*)tape; }
 // Makes them again, on `stream`. Returns a CUDA error code.

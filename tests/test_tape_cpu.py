@@ -46,3 +46,65 @@ def test_a_flat_launch_is_repeated_only_if_it_was_written_down(written, monkeypa
         flat._run(buf, 1, sgd=True)
     assert (flat.lib.made, flat.lib.repeated) == ((1, 2) if written else (3, 0))
     assert flat.launches == 3
+
+
+MEMORY = r"""
+#include <stdlib.h>
+#include <new>
+bool full = false;
+void* operator new(size_t n) {
+  void* p = full ? nullptr : malloc(n);
+  if (p == nullptr) throw std::bad_alloc();
+  return p;
+}
+void* operator new[](size_t n) { return operator new(n); }
+void operator delete(void* p) noexcept { free(p); }
+void operator delete[](void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
+void operator delete[](void* p, size_t) noexcept { free(p); }
+"""
+HARNESS = r"""
+#include "psgd_host.cpp"
+extern bool full;
+int main() {
+  const long long value = 7;
+  const void* args[] = {&value};
+  const size_t sizes[] = {sizeof(value)};
+  void* tape = psgd_tape_begin();
+  psgd_tape_add(nullptr, 1, 32, 0, 0, 1, 1, args, sizes);
+  psgd_tape_add(nullptr, 1, 32, 0, 0, 1, 1, args, sizes);
+  if (psgd_tape_end() != 2) return 1;
+  psgd_tape_free(tape);
+  tape = psgd_tape_begin();
+  psgd_tape_add(nullptr, 1, 32, 0, 0, 1, 1, args, sizes);
+  full = true;
+  psgd_tape_add(nullptr, 1, 32, 0, 0, 1, 1, args, sizes);
+  full = false;
+  if (psgd_tape_end() != -1) return 2;
+  psgd_tape_free(tape);
+  full = true;
+  tape = psgd_tape_begin();
+  const int count = psgd_tape_end();
+  full = false;
+  if (tape != nullptr || count != -1) return 3;
+  psgd_tape_free(tape);
+  return 0;
+}
+"""
+
+
+def test_a_record_without_memory_is_no_exception(tmp_path):
+    """The library is called through C entries, which no exception may leave: the record says that it is not complete."""
+    import subprocess
+
+    from powersgd_b200.csrc import build
+
+    try:
+        nvcc = build._nvcc()
+    except RuntimeError:
+        pytest.skip("no CUDA compiler")
+    sources, program = [tmp_path / "tape.cu", tmp_path / "memory.cpp"], str(tmp_path / "tape")
+    for path, text in zip(sources, (HARNESS, MEMORY)):
+        path.write_text(text)
+    subprocess.run([nvcc, *build.ARCH, "-std=c++17", "-I", build.HERE, *map(str, sources), "-o", program], check=True)
+    assert subprocess.run([program]).returncode == 0
