@@ -220,6 +220,10 @@ class _LowRankBase(Reducer):
         """Of float32 vectors."""
         return 32 * int(np.frombuffer(scan.sizes([t for t, _, _ in vectors]), dtype=np.uint64).sum()) if vectors else 0
 
+    def _reduce_vectors(self, drv, vectors, early: bool = False) -> None:
+        with self.timer("reduce.rank1", verbosity=2):
+            drv.reduce_vectors(vectors, early)
+
     def _views(self, matrices):
         sizes = []
         for tensor, _, _ in matrices:
@@ -262,13 +266,12 @@ class RankKReducer(_LowRankBase):
                 for i in range(len(matrices)):
                     self.set_random(drv.core.q_view(i))
         alone = self.n_workers == 1   # nothing to wait for: the vectors beside the end of the matrices
-        with self.timer("reduce.rank1", verbosity=2):
-            if not alone:
-                drv.reduce_vectors(vectors)
+        if not alone:
+            self._reduce_vectors(drv, vectors)
         with self.timer("reduce.lowrank", verbosity=2):
             drv.rank_k(matrices)
-            if alone:
-                drv.reduce_vectors(vectors, early=True)
+        if alone:
+            self._reduce_vectors(drv, vectors, early=True)
         self._native_launches_last = drv.launches
         return n_bits(self.p_memory) + n_bits(self.q_memory) + self._rank1_bits(vectors)
 
@@ -335,13 +338,12 @@ class HalfRankKReducer(_LowRankBase):
             for i in range(len(matrices)):
                 self.set_random(drv.core.q_view(i))
         alone = self.n_workers == 1   # nothing to wait for: the vectors beside the end of the matrices
-        with self.timer("reduce.rank1", verbosity=2):
-            if not alone:
-                drv.reduce_vectors(vectors)
+        if not alone:
+            self._reduce_vectors(drv, vectors)
         with self.timer("reduce.lowrank", verbosity=2):
             drv.half_rank_k(matrices, compute_p)
-            if alone:
-                drv.reduce_vectors(vectors, early=True)
+        if alone:
+            self._reduce_vectors(drv, vectors, early=True)
         self._native_launches_last = drv.launches
         return n_bits(self.p_memory if compute_p else self.q_memory) + self._rank1_bits(vectors)
 
@@ -515,18 +517,18 @@ class TopKReducer(Reducer):
         with self.timer("reduce.topk", verbosity=2):
             # selection, gather and the error-feedback write (memory = x with the taken entries
             # zeroed) are one fused operation over the whole list: four launches on CUDA, which write
-            # the output as well when there is nothing to gather
+            # the output as well when there is nothing to gather (the phases below are then empty, but timed all the same)
             alone = self.n_workers == 1
             values, positions = topk_abs_many(list(grad_in), sizes, list(memory_out), list(grad_out) if alone else None)
         bits = n_bits(values) + n_bits(positions)
-        if alone:
-            return bits
         with self.timer("reduce.gather", verbosity=2):
-            all_values = _gather_all(values, self.n_workers)
-            all_positions = _gather_all(positions, self.n_workers)
+            if not alone:
+                all_values = _gather_all(values, self.n_workers)
+                all_positions = _gather_all(positions, self.n_workers)
         with self.timer("reduce.combine", verbosity=2):
             # zero fill + the scatter of every worker's pairs, in rank order: one launch on CUDA
-            sparse_combine(_rows(all_values), _rows(all_positions), grad_out, ends, float(self.n_workers))
+            if not alone:
+                sparse_combine(_rows(all_values), _rows(all_positions), grad_out, ends, float(self.n_workers))
         return bits
 
 
