@@ -145,7 +145,7 @@ def _as_matrix(t: torch.Tensor) -> torch.Tensor:
 
 def _split_by_dim(grad_in, grad_out, memory_out):
     trios = list(zip(grad_in, grad_out, memory_out))
-    flat = [t.dim() <= 1 for t in grad_in]
+    flat = [t.dim() <= 1 for t, _, _ in trios]
     return [x for x, f in zip(trios, flat) if f], [x for x, f in zip(trios, flat) if not f]
 
 

@@ -48,3 +48,17 @@ def test_rank_k_times_the_vectors(kind, monkeypatch):
     vector, matrix = [(torch.zeros(5),) * 3], [(torch.zeros(4, 4),) * 3]
     red._reduce_native(vector, matrix)
     assert sorted(calls) == [("matrices", "reduce.lowrank"), ("vectors", "reduce.rank1")]
+
+
+@pytest.mark.parametrize("kind", [R.RankKReducer, R.HalfRankKReducer])
+def test_rank_k_takes_iterators(kind):
+    """The lists are walked once."""
+    def reduced(wrap):
+        g = torch.Generator().manual_seed(3)
+        grads = [torch.randn(s, generator=g) for s in ((8, 6), (5,), (3, 4, 2))]
+        outs, mems = [torch.zeros_like(x) for x in grads], [torch.zeros_like(x) for x in grads]
+        bits = kind(7, "cpu", _Phases(), rank=2).reduce(wrap(grads), wrap(outs), wrap(mems))
+        return bits, outs + mems
+
+    (bits, listed), (walked_bits, walked) = reduced(list), reduced(iter)
+    assert bits == walked_bits and all(torch.equal(a, b) for a, b in zip(listed, walked))
