@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import heapq
 import os
 import weakref
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -251,6 +252,8 @@ class TilePlan:
             tiles(rows, 256)
 
     TC_CTAS_PER_SM = 2
+    TC_CHAIN = 512         # rows that a product kernel adds up in the tensor core at a time
+    TC_MAX_EXTENT = 8192   # rows of a tile; from some thousand on its overhead does not count any more
     # prologue + epilogue of a tile (~4 us), in units of streamed K rows (~0.03 us each): measured
     # as rounds x (overhead + rows) over tile extents 512 ... 4096 on 4 x 4096^2
     TC_TILE_OVERHEAD_ROWS = 136
@@ -264,33 +267,98 @@ class TilePlan:
         not by that. In lists of one to three rounds of resident CTAs what does not fill the last round is cut finer, so that it
         does: 50257 x 1024 at rank 16, P = M Q: 393 blocks in 393 tiles 74 us, in 786 80 (the extent that fills its rounds best), 296 whole
         ones and 97 in three 68. Above, the scheduler evens rounds out by itself (GPT-2 medium, five to eight rounds: 286 -> 277 us for
-        one product, 253 -> 269 for the other)."""
+        one product, 253 -> 269 for the other). A plan is taken for the time at which its last CTA ends, the tiles handed out in
+        their order to the first place that is free, and only where that is 3 % earlier than with the extent of `_pick_tc_k`:
+        matrices of different lengths have tiles of different lengths, and a few long ones among them keep their places alone. Nor
+        may it cost precision (`_tc_error`): 2 x 25718x460 at rank 16, M Q, 3.1e-6 from 64 bits in sums of 460, 1.8e-6 in sums of 232."""
         slots = 148 * self.TC_CTAS_PER_SM
-        k = self._pick_tc_k(groups, transposed)
+        plain = self._pick_tc_k(groups, transposed)
         blocks = [((g.n if transposed else g.m), -(-(g.m if transposed else g.n) // 128)) for g in groups]   # of (length, number)
         # (above rank 8: at 8 two half-iterations leave directions of nearly equal size, where another order of a sum shows in later steps)
         if (self.rp_tc <= 8 or os.environ.get("PSGD_B200_TC_K")
-                or not slots < sum(number * _split_count(length, k, 32) for length, number in blocks) <= 3 * slots):
-            return k, {}
-        overhead, longest = self.TC_ROUND_OVERHEAD_ROWS, max(length for length, _number in blocks)
-        work, best = sum(length * number for length, number in blocks), None
-        for pieces in range(1, 9):
-            k = -(-longest // pieces)
+                or not slots < sum(number * _split_count(length, plain, 32) for length, number in blocks) <= 3 * slots):
+            return plain, {}
+        lengths, work = {length for length, _number in blocks}, sum(length * number for length, number in blocks)
+        error = lambda k: [self._tc_error(length, k) for length in lengths]  # noqa: E731
+        longest, usual, best = max(lengths), error(plain), (plain, {})
+        end = 0.97 * self._tc_end(self._tc_runs(blocks, plain, {}), float("inf"))
+        pieces = -(-longest // self.TC_MAX_EXTENT)
+        for k in [plain] + [-(-longest // p) for p in range(pieces, pieces + 8)]:
             tiles = sum(number * _split_count(length, k, 32) for length, number in blocks)
-            rounds, rest = divmod(tiles, slots)
-            cost = rounds * (overhead + work / tiles) + (overhead + k / (slots // rest) if rest else 0)
-            if best is None or cost < best[0]:
-                best = (cost, k, rest)
-        _cost, k, rest = best
+            if work + tiles * self.TC_ROUND_OVERHEAD_ROWS >= end * slots or any(e > before for e, before in zip(error(k), usual)):
+                continue
+            tail = self._tc_tail(blocks, k, tiles)
+            earlier = self._tc_end(self._tc_runs(blocks, k, tail), end)
+            if earlier < end:
+                best, end = (k, tail), earlier
+        return best
+
+    def _tc_error(self, length: int, k: int) -> int:
+        """Grows with the error of sums of `length` in tiles of an extent of `k`. The tensor core truncates as it adds, so a chain of n terms,
+        the sum of which grows as the root of n, is off by the 3/2th power of n; chains are added up rounded, their errors independent."""
+        def of(tile: int) -> int:
+            whole, rest = divmod(tile, self.TC_CHAIN)
+            return whole * self.TC_CHAIN ** 3 + rest ** 3
+
+        tiles = _split_count(length, k, 32)
+        size = length if tiles == 1 else _split_even(length, k, 32)[0][1]
+        return (tiles - 1) * of(size) + of(length - (tiles - 1) * size)
+
+    def _tc_tail(self, blocks: Sequence[Tuple[int, int]], k: int, tiles: int) -> Dict[int, int]:
+        """The output blocks whose tiles would make up the last round of `tiles` at an extent of `k`, and in how many tiles they fill it."""
+        slots = 148 * self.TC_CTAS_PER_SM
+        rest = tiles % slots
         finer, at, tail = slots // rest if rest else 1, sum(number for _length, number in blocks), {}
         for length, number in reversed(blocks):
+            if finer == 1 or rest <= 0:
+                break
             parts = _split_count(length, k, 32)
-            for _ in range(number):
-                if finer == 1 or rest <= 0:
-                    return k, tail
-                at, rest = at - 1, rest - parts
-                tail[at] = _split_count(length, max(128, -(-length // (parts * finer))), 32)
-        return k, tail
+            number = min(number, -(-rest // parts))
+            at, rest = at - number, rest - number * parts
+            tail.update(dict.fromkeys(range(at, at + number), _split_count(length, max(128, -(-length // (parts * finer))), 32)))
+        return tail
+
+    def _tc_runs(self, blocks: Sequence[Tuple[int, int]], k: int, tail: Dict[int, int]) -> List[Tuple[int, int]]:
+        """What the tiles of a plan take, in rows, and how many of them do, in their order (but for the last tiles of the blocks of a
+        matrix, which are counted behind the others)."""
+        runs, at, overhead = [], 0, self.TC_ROUND_OVERHEAD_ROWS
+
+        def add(length: int, parts: int, number: int) -> None:
+            size = -(-length // (32 * parts)) * 32 if parts > 1 else length   # (as `_split_parts`)
+            whole, rest = divmod(length, size)
+            runs.append((overhead + size, whole * number))
+            if rest:
+                runs.append((overhead + rest, number))
+
+        first = min(tail, default=sum(number for _length, number in blocks))   # of the blocks that are cut finer, all behind it
+        for length, number in blocks:
+            usual = min(max(first - at, 0), number)
+            if usual:
+                add(length, -(-length // k), usual)
+            if usual < number:   # (alike within a matrix)
+                add(length, tail[at + usual], number - usual)
+            at += number
+        return runs
+
+    def _tc_end(self, runs: Sequence[Tuple[int, int]], limit: float) -> float:
+        """When the last CTA ends, in rows; `limit` if that is not before it."""
+        free, ends = {0: 148 * self.TC_CTAS_PER_SM}, [0]   # how many places are free from when on; a heap of these times
+        for t, number in runs:
+            while number:
+                first = ends[0]
+                end, taken = first + t, min(number, free[first])
+                if end >= limit:
+                    return limit
+                number -= taken
+                free[first] -= taken
+                if not free[first]:
+                    del free[heapq.heappop(ends)]
+                if end in free:
+                    free[end] += taken
+                else:
+                    free[end] = taken
+                    heapq.heappush(ends, end)
+        return max(ends)
 
     def _pick_tc_k(self, groups, transposed: bool) -> int:
         if not groups:
@@ -304,10 +372,14 @@ class TilePlan:
             k_len, out_len = (g.n, g.m) if transposed else (g.m, g.n)
             extents[k_len] = extents.get(k_len, 0) + -(-out_len // 128)
         longest = max(extents)
-        for k in range(256, max(256, min(8192, -(-longest // 32) * 32)) + 1, 32):
-            tiles = sum(blocks * _split_count(k_len, k, 32) for k_len, blocks in extents.items())
-            waves = -(-tiles // slots)
-            score = tiles / (waves * slots) * k / (k + self.TC_TILE_OVERHEAD_ROWS)
+        ks = np.arange(256, max(256, min(self.TC_MAX_EXTENT, -(-longest // 32) * 32)) + 1, 32)
+        tiles = 0
+        for k_len, blocks in extents.items():   # (`_split_count` of all of them)
+            size = -(-k_len // -(-k_len // ks))
+            tiles = tiles + blocks * -(-k_len // (-(-size // 32) * 32))
+        waves = -(-tiles // slots)
+        scores = tiles / (waves * slots) * ks / (ks + self.TC_TILE_OVERHEAD_ROWS)
+        for k, score in zip(ks.tolist(), scores.tolist()):
             if score > best_score + 1e-9:
                 best, best_score = k, score
         return best
