@@ -78,14 +78,17 @@ __device__ __forceinline__ bool product_tile_ok(const PsgdTile& t, const PsgdMat
 
 template <int RT>
 __host__ __device__ constexpr int nt_max_rows() { return RT <= 16 ? NT_MAX_ROWS : NT_MAX_ROWS / 2; }
-// Staging buffer of an NT tile: rows of P-hat, later the sums of the warps, [warp][column of a lane x RT][32 lanes + 1], all eight
+// Staging buffer of an NT tile: rows of P-hat, later the sums of the warps, [warp][column of a lane x RT][32 lanes, padded], all eight
 // warps' up to rank 8, four above.
 template <int RT>
 __host__ __device__ constexpr int nt_sum_warps() { return RT <= 8 ? GEMM_WARPS : GEMM_WARPS / 2; }
-constexpr int NT_SUM_PITCH = 33;   // words: neither lanes nor values of a lane meet in one bank
+// Words from one value of the lanes to the next. 32 results in a row, [column][RT], belong to 32 / (VEC x RT) lanes, one behind the
+// other, and to VEC x RT values of theirs: so far apart, they all lie in banks of their own.
+template <int RT, int VEC>
+__host__ __device__ constexpr int nt_sum_pitch() { return 32 + (VEC * RT >= 32 ? 1 : 32 / (VEC * RT) % 32); }
 template <int RT>
 __host__ __device__ constexpr int nt_stage_floats() {
-  const int sums = (nt_sum_warps<RT>() * 4 * RT * NT_SUM_PITCH + 3) / 4 * 4, rows = nt_max_rows<RT>() * RT;
+  const int sums = nt_sum_warps<RT>() * 4 * RT * nt_sum_pitch<RT, RT == 1 ? 2 : 1>(), rows = nt_max_rows<RT>() * RT;
   return sums > rows ? sums : rows;
 }
 
@@ -101,9 +104,22 @@ __device__ __forceinline__ int lane_col(int lane, int c) {
 
 // The lane that owns column lc, and which of its columns that is.
 template <int VEC>
-__device__ __forceinline__ int col_lane(int lc) { return VEC == 4 ? lc >> 2 : VEC == 2 ? (lc & 63) >> 1 : lc & 31; }
+__host__ __device__ constexpr int col_lane(int lc) { return VEC == 4 ? lc >> 2 : VEC == 2 ? (lc & 63) >> 1 : lc & 31; }
 template <int VEC>
-__device__ __forceinline__ int col_of_lane(int lc) { return VEC == 4 ? lc & 3 : VEC == 2 ? (lc & 1) + 2 * (lc >> 6) : lc >> 5; }
+__host__ __device__ constexpr int col_of_lane(int lc) { return VEC == 4 ? lc & 3 : VEC == 2 ? (lc & 1) + 2 * (lc >> 6) : lc >> 5; }
+
+// Where value k of column lc lies among a warp's sums.
+template <int RT, int VEC>
+__host__ __device__ constexpr int nt_sum_at(int lc, int k) { return (col_of_lane<VEC>(lc) * RT + k) * nt_sum_pitch<RT, VEC>() + col_lane<VEC>(lc); }
+template <int RT, int VEC>
+__host__ __device__ constexpr bool nt_sums_in_banks_of_their_own() {
+  for (int first = 0; first < NT_TILE_COLS * RT; first += 32) {
+    unsigned banks = 0;
+    for (int e = first; e < first + 32; ++e) banks |= 1u << (nt_sum_at<RT, VEC>(e / RT, e % RT) & 31);
+    if (banks != ~0u) return false;
+  }
+  return true;
+}
 
 // v[0..3] = the lane's four columns of the row at `rowp` (column block starting at c0, valid up
 // to cend); zero where the row or the column does not exist.
@@ -225,10 +241,14 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   // Sum over the warps, in a fixed order. A warp's values lie lane by lane, so that neither their stores nor the loads of a thread that
   // adds up one (column, k) meet in one bank: written in the order of the result, [column][k], 16 or 32 lanes did, and above rank 8, where
   // one warp after another added to it, the sum was three quarters of a tile: 39 500 of 52 000 cycles on 4 x 1024x1001 at rank 16, 75 000
-  // of 134 000 on 3 x 9000x650 at rank 11, 4700 of 13 000 on 4 x 1001x1024 at rank 5; now 2900, 3000 and 1100.
-  // The launches: 34.8 -> 12.6 us, 137 -> 60, 9.7 -> 7.7.
-  constexpr int SUMS = nt_sum_warps<RT>(), PER_WARP = 4 * RT * NT_SUM_PITCH;
-  auto slot = [&](int w, int c, int k) { return sP + w * PER_WARP + (c * RT + k) * NT_SUM_PITCH; };
+  // of 134 000 on 3 x 9000x650 at rank 11, 4700 of 13 000 on 4 x 1001x1024 at rank 5; then 2900, 3000 and 1100.
+  // The launches: 34.8 -> 12.6 us, 137 -> 60, 9.7 -> 7.7. With one pitch of 33 words for all, the loads still met, two to four to a bank
+  // where VEC * RT < 32: launches alone, in the order of the result / 33 words / now, 4 x 1024x1001 at rank 8 9.8 / 10.4 / 9.6, 3 x 1001x777 +
+  // 2 x 515x2049 at rank 8 12.3 / 12.4 / 11.9, rank 3 9.3 / 9.9 / 9.5, 4 x 1024x1002 at rank 5 10.0 / 9.2 / 9.0.
+  constexpr int SUMS = nt_sum_warps<RT>(), PITCH = nt_sum_pitch<RT, VEC>(), PER_WARP = 4 * RT * PITCH;
+  static_assert(SUMS * PER_WARP <= nt_stage_floats<RT>(), "the widest pitch has room");
+  static_assert(nt_sums_in_banks_of_their_own<RT, VEC>(), "32 results in a row are added up by a warp");
+  auto slot = [&](int w, int c, int k) { return sP + w * PER_WARP + (c * RT + k) * PITCH; };
   if (SUMS < GEMM_WARPS) {
     if (warp >= SUMS) {
 #pragma unroll
@@ -252,7 +272,7 @@ __device__ __forceinline__ void gemm_nt_tile(const GemmArgs& a, const PsgdTile& 
   __syncthreads();
 #pragma unroll 1
   for (int e = tid; e < NT_TILE_COLS * RT; e += GEMM_THREADS) {
-    const float* of = slot(0, col_of_lane<VEC>(e / RT), e % RT) + col_lane<VEC>(e / RT);
+    const float* of = sP + nt_sum_at<RT, VEC>(e / RT, e % RT);
     float s = of[0];
 #pragma unroll
     for (int w = 1; w < SUMS; ++w) s += of[w * PER_WARP];
