@@ -107,7 +107,10 @@ PSGD_API int psgd_tape_end() {
   psgd_tape_now = nullptr;
   return tape && tape->complete ? (int)tape->launches.size() : -1;
 }
-PSGD_API void psgd_tape_free(void* tape) { delete (PsgdTape*)tape; }
+PSGD_API void psgd_tape_free(void* tape) {
+  if (tape == psgd_tape_now) psgd_tape_now = nullptr;   // (dropped while it is being written)
+  delete (PsgdTape*)tape;
+}
 // Makes them again, on `stream`. Returns a CUDA error code.
 PSGD_API int psgd_tape_replay(const void* tape, cudaStream_t stream) {
   for (const PsgdTape::Launch& l : ((const PsgdTape*)tape)->launches) {

@@ -497,9 +497,9 @@ class _Tape:
     """Launches written down by the library, to be made again by one call of it. Only their arguments are kept."""
 
     def __init__(self, lib, body):
-        self._lib = lib
-        self._launches = lib.psgd_tape_begin()
-        try:
+        self._lib, self._launches = lib, None
+        try:   # (an interrupt may come anywhere)
+            self._launches = lib.psgd_tape_begin()
             body()
         finally:
             self.count = lib.psgd_tape_end()

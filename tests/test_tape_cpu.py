@@ -88,6 +88,8 @@ int main() {
   full = false;
   if (tape != nullptr || count != -1) return 3;
   psgd_tape_free(tape);
+  psgd_tape_free(psgd_tape_begin());   // dropped before its end: nothing is written into it any more
+  if (psgd_tape_now != nullptr) return 4;
   return 0;
 }
 """
@@ -108,3 +110,25 @@ def test_a_record_without_memory_is_no_exception(tmp_path):
         path.write_text(text)
     subprocess.run([nvcc, *build.ARCH, "-std=c++17", "-I", build.HERE, *map(str, sources), "-o", program], check=True)
     assert subprocess.run([program]).returncode == 0
+
+
+def test_an_interrupt_ends_the_record():
+    """Wherever it comes, later launches of the thread are not written down."""
+    class Lib:
+        open = False
+
+        def psgd_tape_begin(self):
+            self.open = True
+            raise KeyboardInterrupt   # as the interpreter raises it behind the call
+
+        def psgd_tape_end(self):
+            self.open = False
+            return -1
+
+        def psgd_tape_free(self, tape):
+            pass
+
+    lib = Lib()
+    with pytest.raises(KeyboardInterrupt):
+        cuda_path._Tape(lib, lambda: None)
+    assert not lib.open
