@@ -156,6 +156,8 @@ class PowerSGD(Aggregator):
             return self._allreduce.aggregate(gradients)
         lowrank, plain = self._split(gradients)
         updates = self._powersgd.aggregate(lowrank)
+        if type(self._allreduce) is not AllReduce or type(self._powersgd) is not BasicPowerSGD:   # a program's own parts
+            return self._merge(updates, self._allreduce.aggregate(plain))
         native = self._powersgd._native
         return self._merge(updates, self._allreduce._aggregate(plain, early=self._powersgd._ran_native and native._chained()))
 

@@ -243,3 +243,21 @@ def test_dense_layout_helpers():
     v = like_strided(flat, cl)
     assert v.shape == cl.shape and v.stride() == cl.stride() and v.data_ptr() == flat.data_ptr()
     assert v[0, 1, 0, 0] == 1 and v[0, 0, 0, 1] == 4  # channel is the fastest dimension
+
+
+def test_parts_of_a_programs_own():
+    """Aggregators in the place of the parts are asked through their one method."""
+    from powersgd_b200.aggregators import Aggregator
+
+    class Negated(Aggregator):
+        def aggregate(self, gradients):
+            return [-g for g in gradients]
+
+    params = [torch.zeros(20, 30), torch.zeros(7)]
+    grads = [torch.randn(20, 30), torch.randn(7)]
+    for name in ("_allreduce", "_powersgd"):
+        agg = PowerSGD(params, Config(rank=1, start_compressing_after_num_steps=0))
+        setattr(agg, name, Negated())
+        out = agg.aggregate([g.clone() for g in grads])
+        kept = 1 if name == "_allreduce" else 0
+        assert torch.equal(out[kept], -grads[kept])
