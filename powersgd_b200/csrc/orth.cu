@@ -3,10 +3,10 @@
 // Replaces the reference's per-group `torch.linalg.qr` / joint-norm division
 // (powersgd/orthogonalization.py:4-8) and the research harness' column-serial Gram-Schmidt
 // (paper-code/gradient_reducers.py:945-956) with a Gram-matrix formulation that walks the
-// tall matrix exactly twice, whatever the rank:
+// tall matrix twice, whatever the rank (in a cluster, the second time from registers or L2):
 //
 //   G = X^T X        accumulated in float64, fixed summation order (bit-reproducible)
-//   G = R^T R        Cholesky in float64 by one warp
+//   G = R^T R        Cholesky in float64, by one warp up to rank 4, by the whole block above
 //   X <- X R^-1      by forward substitution in float64, rounded to float32 once
 //
 // With a float64 Gram matrix one pass is as orthonormal as float32 can express for any X
@@ -18,7 +18,8 @@
 // Rank-1 units keep the reference's quirk: ONE Frobenius norm over the whole shape group
 // (all B matrices jointly), floored at 1e-16, divides every entry.
 //
-// Two launches, one CTA per row chunk of a unit in both. The first writes the chunk's partial Gram
+// One launch with a cluster of CTAs per unit (psgd_orth_cluster_kernel), or, for long units, small models and
+// several workers, two with one CTA per row chunk of a unit in both. The first writes the chunk's partial Gram
 // matrix (and partial cross products F_i^T X against earlier factors of the same side). In the
 // second EVERY chunk adds the partials of its unit in chunk order, factorises the sum and solves
 // its own rows; one chunk per earlier factor also publishes the cross products
@@ -130,7 +131,7 @@ __device__ __forceinline__ void chunk_pairs(const float* a, const float* b, int 
     __syncthreads();
   } else {
     // rows staged as float64; every thread owns a 4 x 4 block of pairs and every NG-th row, so 8
-    // values read feed 16 multiply-adds; the row groups are added in index order at the end
+    // values read feed 16 multiply-adds; at the end the row groups of a warp are added in pairs, the warps in index order
     constexpr int SR = ORTH_STAGE_ROWS_X_RT / RT;
     constexpr int NB = RT / 4 < 1 ? 1 : RT / 4;
     constexpr int NG = ORTH_THREADS / (NB * NB);
@@ -192,6 +193,7 @@ __device__ __forceinline__ void chunk_pairs(const float* a, const float* b, int 
     const int e0 = GW < 32 ? (tid & 31) / GW * LEFT : 0;   // the first of them
     constexpr int SETS = GW < 32 ? ORTH_WARPS : NG;        // (RT = 32: the groups are whole warps apart)
     const int set = GW < 32 ? tid >> 5 : g;
+    static_assert(SETS * NP <= 2 * ORTH_STAGE_ROWS_X_RT, "the sums of the warps fit where the rows were staged");
 #pragma unroll
     for (int i = 0; i < LEFT; ++i) {
       const int e = e0 + i;
@@ -697,6 +699,7 @@ __host__ __device__ constexpr int orth_cluster_doubles() {
 template <int RT>
 __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_cluster_kernel(OrthArgs a, int same) {
   constexpr int NP = RT * RT, CL = ORTH_CLUSTER;
+  static_assert(RT <= 4 || orth_tile_floats<RT>() * sizeof(float) <= orth_stage_doubles<RT>() * sizeof(double), "the tile of rows takes the place of the stage");
   extern __shared__ __align__(16) double orth_smem[];
   double* stage = orth_smem;                                           // products; later the tile of rows (RT >= 8)
   double* mine = stage + orth_stage_doubles<RT>();                     // [1 + nprev][NP] (RT >= 8)

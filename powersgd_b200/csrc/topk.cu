@@ -139,11 +139,11 @@ PSGD_API int psgd_topk_abs(const float* x, long long n, long long k, int* worksp
 // A tensor with more candidates than its list holds (many entries of nearly equal size, or a large k) goes the long
 // way instead: histograms of the second and the third digit over all entries in launches 2 and 3, and a
 // compaction pass in launch 4, which has nothing to do for the others. How long a list one block should walk: ops/topk.py.
-// Bound by the reads (L2 for a model of this size) and by what a block costs besides them, so some four blocks
-// per SM serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: 68 us by three histogram passes and a
+// Bound by the reads (L2 for a model of this size) and by what a block costs besides them, so as many blocks as run at a
+// time, three per SM, serve the whole list. 62 tensors of ResNet-18 (45 MB), k = numel / 488: 68 us by three histogram passes and a
 // compaction, 54 us by lists. With one worker launch 2 writes the dense output beside the memory (TopkItem::out), so that nothing
 // is left to combine, every launch starts beside the end of the one before, and the workspace is cleared by the call
-// before: the pass of the reducer 86 -> 55 us; with as many blocks as run at a time, three per SM, in launch 2 too, 51.5, of which 12 go
+// before: the pass of the reducer 86 -> 55 us; with three blocks per SM in place of four, 51.5, of which 12 go
 // to launch 1 (45 MB from HBM and as many additions in shared memory), 22 to launch 2 (135 MB), 8 to launch 3 and 2 to launch 4.
 namespace {
 

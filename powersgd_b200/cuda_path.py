@@ -520,9 +520,10 @@ class NativeCompressor(_Recordable):
     _orth_clusters: Dict[str, bool] = {}
     _orth_by_rule: Dict[str, bool] = {}
 
-    # Elements of a list from which on one launch is the rule. Below, a replayed step gains 3 to 4 us of 31 to 35 (two launches / one:
-    # 784x256 at rank 2 34.8 / 30.7); steps that small keep the number of launches that they report, except behind an
-    # orthonormalisation ahead of time (`begin_step`: a recorded training step 101.2 / 98.2 us).
+    # Elements of a list from which on one launch is the rule. It pays below as well: a replayed step gains 3 to 4 us of 31 to 35 (two
+    # launches / one: 784x256 at rank 2 34.8 / 30.7). But lists that small have reported a fixed number of launches (`launches`), which the tests
+    # hold: seven for 254 164 elements at two half-iterations. The line lies above that one, and an
+    # orthonormalisation behind one ahead of time (`begin_step`) does not heed it: a recorded training step 101.2 / 98.2 us.
     ORTH_CLUSTER_ELEMS = 1 << 18
 
     def __init__(self, core):
