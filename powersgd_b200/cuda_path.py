@@ -258,9 +258,10 @@ class TilePlan:
     # as rounds x (overhead + rows) over tile extents 512 ... 4096 on 4 x 4096^2
     TC_TILE_OVERHEAD_ROWS = 136
 
-    # The same above rank 8 for lists of one to three rounds, from rounds of 352 to 1408 rows: 50257 x 1024 at rank 16, 1408 and
-    # 704 rows 57.5 / 68.4 us, 352 rows 88.7.
-    TC_ROUND_OVERHEAD_ROWS = 330
+    # The same above rank 8 for lists of one to three rounds. Of 330 (from rounds of 352 to 1408 rows alone) to 900, 500 tells best which
+    # plans are faster: over 71 products of random lists at rank 11 to 32 that it changes they take 0.87 of the time with the extent of
+    # `_pick_tc_k`, at worst 1.03; plans less than a tenth better by it were 9 % slower to 6 % faster.
+    TC_ROUND_OVERHEAD_ROWS = 500
 
     def _tc_extents(self, groups, transposed: bool) -> Tuple[int, Dict[int, int]]:
         """K extent of the tiles, and how many tiles the last output blocks of 128 (by number, in the order of `build`) are cut in if
@@ -268,7 +269,7 @@ class TilePlan:
         does: 50257 x 1024 at rank 16, P = M Q: 393 blocks in 393 tiles 74 us, in 786 80 (the extent that fills its rounds best), 296 whole
         ones and 97 in three 68. Above, the scheduler evens rounds out by itself (GPT-2 medium, five to eight rounds: 286 -> 277 us for
         one product, 253 -> 269 for the other). A plan is taken for the time at which its last CTA ends, the tiles handed out in
-        their order to the first place that is free, and only where that is 3 % earlier than with the extent of `_pick_tc_k`:
+        their order to the first place that is free, and only where that is a tenth earlier than with the extent of `_pick_tc_k`:
         matrices of different lengths have tiles of different lengths, and a few long ones among them keep their places alone. Nor
         may it cost precision (`_tc_error`): 2 x 25718x460 at rank 16, M Q, 3.1e-6 from 64 bits in sums of 460, 1.8e-6 in sums of 232."""
         slots = 148 * self.TC_CTAS_PER_SM
@@ -281,7 +282,7 @@ class TilePlan:
         lengths, work = {length for length, _number in blocks}, sum(length * number for length, number in blocks)
         error = lambda k: [self._tc_error(length, k) for length in lengths]  # noqa: E731
         longest, usual, best = max(lengths), error(plain), (plain, {})
-        end = 0.97 * self._tc_end(self._tc_runs(blocks, plain, {}), float("inf"))
+        end = 0.9 * self._tc_end(self._tc_runs(blocks, plain, {}), float("inf"))
         pieces = -(-longest // self.TC_MAX_EXTENT)
         for k in [plain] + [-(-longest // p) for p in range(pieces, pieces + 8)]:
             tiles = sum(number * _split_count(length, k, 32) for length, number in blocks)
