@@ -916,12 +916,38 @@ __global__ void __launch_bounds__(ORTH_THREADS) psgd_orth_cluster_kernel(OrthArg
 }
 
 template <int RT>
-static int orth_cluster_launch(const OrthArgs& a, int nunits, int same, int early, cudaStream_t stream) {
-  const size_t smem = (size_t)orth_cluster_doubles<RT>() * sizeof(double);
-  if (smem > 48 * 1024) {
-    static unsigned long long devices = 0;   // per instantiation
-    if (const int code = psgd_allow_shared((const void*)psgd_orth_cluster_kernel<RT>, smem, devices)) return code;
+static int orth_cluster_smem(size_t& smem) {
+  smem = (size_t)orth_cluster_doubles<RT>() * sizeof(double);
+  static unsigned long long devices = 0;   // per instantiation
+  return smem > 48 * 1024 ? psgd_allow_shared((const void*)psgd_orth_cluster_kernel<RT>, smem, devices) : 0;
+}
+
+// Clusters that run at a time on the current device; 0 if it does not say.
+template <int RT>
+static int orth_clusters_at_a_time() {
+  static int known[64] = {};   // by device, one more than that
+  int device = 0, n = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 0;
+  int* at = known + device;
+  const int before = __atomic_load_n(at, __ATOMIC_RELAXED);
+  if (before > 0) return before - 1;
+  size_t smem;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attrs[2];
+  if (orth_cluster_smem<RT>(smem) != 0) return 0;
+  psgd_launch_config(cfg, attrs, 1024 * ORTH_CLUSTER, ORTH_THREADS, smem, nullptr, 0, ORTH_CLUSTER);
+  if (cudaOccupancyMaxActiveClusters(&n, psgd_orth_cluster_kernel<RT>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
   }
+  __atomic_store_n(at, n + 1, __ATOMIC_RELAXED);
+  return n;
+}
+
+template <int RT>
+static int orth_cluster_launch(const OrthArgs& a, int nunits, int same, int early, cudaStream_t stream) {
+  size_t smem;
+  if (const int code = orth_cluster_smem<RT>(smem)) return code;
   return psgd_launch_clusters(psgd_orth_cluster_kernel<RT>, nunits * ORTH_CLUSTER, ORTH_THREADS, smem, stream, early, ORTH_CLUSTER, a, same);
 }
 
@@ -960,16 +986,28 @@ PSGD_API int psgd_orth_chunk_rows(int max_r, long long longest) {
     default: return orth_chunk_rows<32>(longest);
   }
 }
-// Whether one launch with a cluster per unit is the faster one for a list whose longest unit has `longest` rows in at most `subs`
-// sub-matrices, with `nprev` earlier factors. A cluster has eight SMs for a unit however long it is, the two launches have
-// one per chunk. us, two launches / one, 1 and 24 units: rank 1, 4096 rows 3.9 / 2.4 and 4.8 / 2.8, 16384 4.3 / 2.7 and 5.9 / 3.2, 24000
-// 4.3 / 4.9; rank 2, 4096 4.7 / 3.0 and 5.9 / 3.4, 12288 5.0 / 4.4 and 6.3 / 5.5, 24000 5.1 / 7.1; rank 4, 1024 5.7 / 3.3 and 6.7 / 3.6, 12288
-// 6.3 / 5.5 and 10.4 / 6.9, 16384 6.4 / 6.8; rank 8, 1024 6.5 / 5.0 and 8.3 / 5.8, 2048 6.7 / 5.5 and 7.9 / 6.7, 4096 6.9 / 7.6 and 11.4 / 9.4;
-// rank 16, 1024 8.5 / 7.7 and 10.2 / 9.5, 2048 9.0 / 9.5 and 15.1 / 12.4.
-PSGD_API int psgd_orth_takes_clusters(int max_r, long long longest, int subs, int nprev) {
+// Whether one launch with a cluster per unit is the faster one for a list of `units` units, `rows` rows in all, whose longest unit has
+// `longest` rows in at most `subs` sub-matrices, with `nprev` earlier factors. A cluster has eight SMs for a unit however long it
+// is, the two launches have one per chunk. us, two launches / one, 1 and 24 units: rank 1, 4096 rows 3.9 / 2.4 and 4.8 / 2.8, 16384 4.3 / 2.7 and
+// 5.9 / 3.2, 24000 4.3 / 4.9; rank 2, 4096 4.7 / 3.0 and 5.9 / 3.4, 12288 5.0 / 4.4 and 6.3 / 5.5, 24000 5.1 / 7.1; rank 4, 1024 5.7 / 3.3 and 6.7 /
+// 3.6, 12288 6.3 / 5.5 and 10.4 / 6.9, 16384 6.4 / 6.8; rank 8, 1024 6.5 / 5.0 and 8.3 / 5.8, 2048 6.7 / 5.5 and 7.9 / 6.7, 4096 6.9 / 7.6 and 11.4 /
+// 9.4; rank 16, 1024 8.5 / 7.7 and 10.2 / 9.5, 2048 9.0 / 9.5 and 15.1 / 12.4.
+// Some 46 clusters run at a time up to rank 2 and 30 above; what is beyond them waits for a round of its own, while the two launches
+// spread over all SMs. 64 rows, rank 2, 46, 60 and 400 units 4.0 / 3.2, 4.2 / 5.9, 4.8 / 27; rank 4, 30, 34 and 400 units 4.7 / 3.7, 4.8 / 6.6,
+// 6.6 / 46; rank 16, 30, 34 and 400 units 9.0 / 7.9, 8.5 / 13.7, 13 / 99. Only where the rows bound both do more rounds pay: 60 units of 8192 rows at rank 1
+// 7.7 / 5.7, 2 10.4 / 7.9, 4 16.6 / 10.2; of 4096 5.0 / 5.4, 6.6 / 6.7 and 10.2 / 8.6 (74 units 10.5 / 12.3).
+PSGD_API int psgd_orth_takes_clusters(int max_r, long long longest, int subs, int nprev, int units, long long rows) {
   const int rt = psgd_orth_template_rank(max_r);
   if (rt > 16 || nprev >= ORTH_CLUSTER || (subs > 1 && (subs + ORTH_CLUSTER - 1) / ORTH_CLUSTER * nprev > ORTH_CLUSTER_SUBS)) return 0;
-  return longest <= (rt == 1 ? 16384 : rt <= 4 ? 12288 : rt == 8 ? 3072 : 1536);
+  if (longest > (rt == 1 ? 16384 : rt <= 4 ? 12288 : rt == 8 ? 3072 : 1536)) return 0;
+  if (rt <= 4 && rows >= 8192ll * units) return 1;
+  switch (rt) {
+    case 1: return units <= orth_clusters_at_a_time<1>();
+    case 2: return units <= orth_clusters_at_a_time<2>();
+    case 4: return units <= orth_clusters_at_a_time<4>();
+    case 8: return units <= orth_clusters_at_a_time<8>();
+    default: return units <= orth_clusters_at_a_time<16>();
+  }
 }
 // Scratch per chunk (doubles) for `nprev` earlier factors; per unit: 2 * RT*RT floats (`head`).
 PSGD_API int psgd_orth_part_doubles(int max_r, int nprev) {

@@ -569,7 +569,8 @@ class NativeCompressor(_Recordable):
             self.n_units[s], self.n_chunks[s] = len(units), len(chunks)
             if world_size() == 1:
                 members = max((g.batch for g in self.plan.groups if g.r == 1), default=1)
-                self._orth_clusters[s] = bool(self.lib.psgd_orth_takes_clusters(self.tiles.max_r, longest, members, max(self.T - 1, 0)))
+                rows = sum((g.n if s == "p" else g.m) * g.batch for g in self.plan.groups)
+                self._orth_clusters[s] = bool(self.lib.psgd_orth_takes_clusters(self.tiles.max_r, longest, members, max(self.T - 1, 0), len(units), rows))
                 self._orth_by_rule[s] = self._orth_clusters[s] and self.tiles.total_elems >= self.ORTH_CLUSTER_ELEMS
         # scratch of the orthonormalisation: partial sums per chunk; per unit (`_orth_rinv`) the leading
         # rows of the factor as they came in, which R falls back on when a column has to be replaced

@@ -83,7 +83,7 @@ _OPTIONAL = {
     "psgd_finalize_strip_rows": (i32, [i32, i32]),
     "psgd_orth_template_rank": (i32, [i32]),
     "psgd_orth_chunk_rows": (i32, [i32, i64]),
-    "psgd_orth_takes_clusters": (i32, [i32, i64, i32, i32]),
+    "psgd_orth_takes_clusters": (i32, [i32, i64, i32, i32, i32, i64]),
     "psgd_orth_part_doubles": (i32, [i32, i32]),
     "psgd_finalize_tc_max_k": (i32, []),
     "psgd_finalize_tc_launch": (i32, [vp, vp, i32, vp, vp, i32, i32, vp, vp, vp, vp, f32, i32, vp, vp]),

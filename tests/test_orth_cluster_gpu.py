@@ -83,3 +83,16 @@ def test_rule():
     assert rule([(64, 512)] * 700, 1) == (False, False)
     assert rule([(16, 512)] * 700, 1, iters=1) == (True, False)   # 700 x 16 and 700 x 512 rows in one unit
     assert rule([(2048, 2048)], 32) == (False, False)
+
+
+def test_rule_by_the_number_of_units():
+    """More units than run at a time take two launches, but for long ones."""
+    def rule(shapes, rank):
+        nat = NativeCompressor(BasicPowerSGD([torch.zeros(s, device="cuda") for s in shapes], BasicConfig(rank=rank, num_iters_per_step=2), backend="native"))
+        return nat._orth_by_rule["p"], nat._orth_by_rule["q"], nat._orth_clusters["p"]
+
+    for rank in (2, 3, 8, 16):
+        assert rule([(128, 512)] * 20, rank) == (True, True, True)
+        assert rule([(128, 512)] * 100, rank) == (False, False, False)
+    assert rule([(8192, 64)] * 60, 4) == (True, False, True)
+    assert rule([(128, 512)] * 100, 1) == (True, False, True)   # one unit, of 12 800 and of 51 200 rows
