@@ -372,6 +372,10 @@ __device__ __forceinline__ float warp_sums(float (&v)[N], int lane) {
 // 15.2 -> 12.1 us; tiles of 512 / 256 columns instead: 19.1 / 21.3 us on ResNet-18. The staging itself, as a loop of loads and
 // stores with a division for each value, took 2600 of a tile's some 10 000 cycles on ResNet-18, 4100 of 13 500 at rank 3 and, with
 // five CTAs per SM at it, 8200 of 17 000 on the LSTM model; by asynchronous copies column by column 1550, 1700 and 4700.
+// All CTAs of a column part copy the same rows of Q-hat at the same time. Up to rank 8 they do it by way of L1: launches alone, loads
+// and stores / copies by L2 / by L1, 4 x 8192x512 at rank 4 11.7 / 16.3 / 11.3 us, 16000x1000 13.2 / 18.0 / 11.2, 4 x 1024^2 5.4 / 5.6 / 4.6; at rank 8
+// 4 x 8192x512 20.1 / 23.4 / 21.3, 10000x1001 24.1 / 19.7 / 13.5, 64 x 512^2 20.4 / 20.3 / 20.7. At rank 16 and 32 by L2: 64 x 512^2
+// 43.7 / 30.6 / 32.7 and 173 / 108 / 111, 4 x 8192x512 43.5 / 34.3 / 31.5 and 170 / 110 / 112.
 template <int RT, int VEC, int RPW>
 __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& t, const PsgdMat& mt, float* sQ, float* sSum) {
   const int r = mt.r, m = mt.m;
@@ -423,7 +427,8 @@ __device__ __forceinline__ void gemm_nn_tile(const GemmArgs& a, const PsgdTile& 
   if (wide) {
     for (int e = tid; e < t.cols * (RT / W); e += GEMM_THREADS) {
       const int lc = e / (RT / W), k = e % (RT / W) * W;
-      if (W == 4) psgd_copy16(place(lc, k), qin + e * W);
+      if (W == 4 && RT <= 8) psgd_copy16_shared(place(lc, k), qin + e * W);
+      else if (W == 4) psgd_copy16(place(lc, k), qin + e * W);
       else psgd_copy8(place(lc, k), qin + e * W);
     }
   }

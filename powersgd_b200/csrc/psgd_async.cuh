@@ -76,4 +76,8 @@ __device__ __forceinline__ void psgd_copy8(float* dst, const float* src) {
 __device__ __forceinline__ void psgd_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(psgd_smem_u32(dst)), "l"(src) : "memory");
 }
+// The same by way of L1, for what many CTAs of an SM copy: by way of L2 alone they all meet on its few lines.
+__device__ __forceinline__ void psgd_copy16_shared(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(psgd_smem_u32(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void psgd_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }

@@ -32,3 +32,20 @@ def test_products_against_float64(rank, lead, monkeypatch):
             taken, size = left @ (right.T @ basis), left.abs() @ (right.abs().T @ basis.abs())
             bound = (grp.m + 2 * r) * 2.0 ** -24 * (m.abs() @ basis.abs() + size)
             assert ((p(nat.h_loc[1]) - (m @ basis - taken)).abs() <= bound + 1e-30).all(), (shapes[idx], "M Q")
+
+
+@pytest.mark.parametrize("rank", [1, 2, 3, 4, 8])
+def test_product_of_more_tiles_than_run_at_a_time(rank, monkeypatch):
+    """M Q of a tall matrix: some 470 tiles of 32 rows, which all copy the same rows of Q-hat."""
+    monkeypatch.setenv("PSGD_B200_GEMM", "ffma")
+    g = torch.Generator(device="cuda").manual_seed(rank)
+    m = torch.randn(15001, 132, generator=g, device="cuda")
+    core = BasicPowerSGD([torch.zeros_like(m)], BasicConfig(rank=rank, num_iters_per_step=1), backend="native")
+    core.aggregate([m.clone()])             # left factor first ...
+    core.aggregate([m.clone()])             # ... right factor now: one M Q
+    nat = core._native
+    assert len(nat._tile_arrays["nn"]["f"]) > 3 * 148
+    q = nat.h_in[0][: 132 * rank].view(132, rank).double()
+    p = nat.h_loc[0][: 15001 * rank].view(15001, rank).double()
+    m = m.double()
+    assert ((p - m @ q).abs() <= 132 * 2.0 ** -24 * (m.abs() @ q.abs()) + 1e-30).all()
