@@ -153,9 +153,9 @@ def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tens
     # a recorded call gets tables and counters of its own: the cache may drop an entry at any time, and a
     # replay may run beside an eager call on the same tensors
     recorded = is_recorded(stream)
-    # (taken out until the call is complete: whatever breaks it off may leave the half of the workspace uncleared that the next one counts in)
-    entry = None if recorded else _many_cache.pop(key, None)
-    if entry is None:
+    entry = None if recorded else _many_cache.get(key)
+    # (open: a call was broken off, and the half of the workspace that the next one counts in may not be cleared)
+    if entry is None or entry["open"]:
         release_finished()
         dtype = np.dtype([("x", np.uint64), ("memory", np.uint64), ("n", np.int64), ("k", np.int64), ("out_off", np.int64),
                           ("cand_off", np.int64), ("cap", np.int64), ("out", np.uint64)])
@@ -191,29 +191,30 @@ def _select(tensors, ks, mems, outs, values: torch.Tensor, positions: torch.Tens
             entry = {
                 "items": to_dev(items), "block_item": to_dev(np.asarray(block_item, dtype=np.int32)),
                 "block_part": to_dev(np.asarray(block_part, dtype=np.int32)), "parts": to_dev(np.asarray(parts, dtype=np.int32)),
-                "nblocks": len(block_item), "dense": dense, "turn": 0,
+                "nblocks": len(block_item), "dense": dense, "turn": 0, "open": False,
                 "cand_v": torch.empty(max(room, 1), dtype=torch.float32, device=device), "cand_p": torch.empty(max(room, 1), dtype=torch.int32, device=device),
                 # one half per call in turn: a call clears the other for the next. (A recorded call clears its own.)
                 "ws": torch.zeros(2 * len(tensors) * int(lib.psgd_topk_workspace_ints()), dtype=torch.int32, device=device),
             }
         if recorded:
             keep_with_graph(None, entry)
-        elif len(_many_cache) >= MOST_LISTS:
-            _many_cache.clear()
+        else:
+            # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
+            # valid for whatever tensors present the same addresses again, so no tensor is kept alive
+            if len(_many_cache) >= MOST_LISTS:
+                _many_cache.clear()
+            _many_cache[key] = entry
     vp = ctypes.c_void_p
     half = 2 * entry["ws"].numel()   # in bytes
     turn, base = entry["turn"], entry["ws"].data_ptr()
+    entry["open"] = True
     code = lib.psgd_topk_abs_many(
         vp(entry["items"].data_ptr()), len(tensors), vp(entry["block_item"].data_ptr()), vp(entry["block_part"].data_ptr()),
         vp(entry["parts"].data_ptr()), entry["nblocks"], vp(base + turn * half), vp(0 if recorded else base + (1 - turn) * half),
         vp(entry["cand_v"].data_ptr()), vp(entry["cand_p"].data_ptr()), vp(values.data_ptr()), vp(positions.data_ptr()), stream,
     )
     native.check(code, "psgd_topk_abs_many")
-    if not recorded:
-        # the tables hold addresses and lengths only, and the key is exactly those: an entry stays
-        # valid for whatever tensors present the same addresses again, so no tensor is kept alive
-        entry["turn"] = 1 - turn
-        _many_cache[key] = entry
+    entry["turn"], entry["open"] = 1 - turn, False
     return entry["dense"]
 
 

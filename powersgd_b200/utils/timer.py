@@ -12,11 +12,24 @@ from __future__ import annotations
 
 import json
 import time
-from contextlib import contextmanager
+from contextlib import ContextDecorator, contextmanager
 from typing import Callable, Dict, List, Optional, Tuple
 
 import numpy as np
 import torch
+
+
+class _Untimed(ContextDecorator):
+    """The phases that a timer leaves out: nothing is entered (a generator for each costs more than a small step's checks)."""
+
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_UNTIMED = _Untimed()
 
 
 class Timer:
@@ -45,11 +58,11 @@ class Timer:
         self.totals[label] = self.totals.get(label, 0.0) + (end - start)
         self.call_counts[label] = self.call_counts.get(label, 0) + 1
 
-    @contextmanager
     def __call__(self, label: str, epoch: float = -1.0, verbosity: int = 1):
-        if verbosity > self.verbosity_level:
-            yield
-            return
+        return _UNTIMED if verbosity > self.verbosity_level else self._timed(label, epoch)
+
+    @contextmanager
+    def _timed(self, label: str, epoch: float):
         self._sync()
         start = time.perf_counter()
         yield

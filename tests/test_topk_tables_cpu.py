@@ -53,7 +53,7 @@ def test_a_call_that_breaks_off_leaves_no_workspace_behind(fake):
     assert halves[1] == halves[0][::-1]
     with pytest.raises(KeyboardInterrupt):
         _select(x, None)
-    assert not topk._many_cache   # the next call brings a workspace of zeros
-    _select(x, None)
+    (broken,) = topk._many_cache.values()
+    _select(x, None)   # a workspace of zeros
     (entry,) = topk._many_cache.values()
-    assert entry["turn"] == 1
+    assert entry["ws"] is not broken["ws"] and entry["turn"] == 1 and not entry["open"]
