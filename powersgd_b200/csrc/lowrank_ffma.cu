@@ -530,7 +530,9 @@ template <int RT>
 __host__ __device__ constexpr int nn_rows_per_warp() { return RT <= 16 ? 4 : 2; }
 // PER_SM: CTAs of an SM that registers have to allow. More registers let more of a tile's loads run ahead, which is what a launch of at most
 // two tiles per SM needs; with more tiles a third CTA does more: us per pass, two / three, 3 x 1001x777 + 2 x 515x2049 at rank
-// 3 x 3 (198 tiles) 89.4 / 94.1, ResNet-18's recorded step (443) 105.6 / 102.2, LSTM step (1532) 212.7 / 212.0.
+// 3 x 3 (198 tiles) 89.4 / 94.1, ResNet-18's recorded step (443) 105.6 / 102.2, LSTM step (1532) 212.7 / 212.0. At rank 1 a fourth one, where
+// that saves a round; launches alone, three / four, 6 x 512x4608 (480 tiles) 10.5 / 9.2, 16000x1000 (500) 7.5 / 6.8, 4 x 4000x650 (500) 6.6 / 6.9, 2 x
+// 16000x1000 (1000) 23.2 / 21.9; where it saves none, 10000x1001 (313) 6.0 / 9.2, 40 x 512^2 (640) 5.9 / 6.3.
 template <int RT, int RPW, int PER_SM>
 __global__ void __launch_bounds__(GEMM_THREADS, PER_SM) psgd_gemm_nn_kernel(GemmArgs a) {
   extern __shared__ __align__(16) float smem[];   // staged rows of Q-hat
@@ -579,6 +581,7 @@ static int launch_nn(const GemmArgs& a, int ntiles, int early, cudaStream_t stre
   constexpr int RPW = nn_rows_per_warp<RT>();
   const size_t smem = (size_t)nn_max_cols<RT>() * RT * sizeof(float);
   if (RT >= 8 || ntiles <= 2 * 148) return psgd_launch(psgd_gemm_nn_kernel<RT, RPW, 2>, ntiles, GEMM_THREADS, smem, stream, early, a);
+  if (RT == 1 && psgd_ceil_div(ntiles, 4 * 148) < psgd_ceil_div(ntiles, 3 * 148)) return psgd_launch(psgd_gemm_nn_kernel<RT, RPW, RT == 1 ? 4 : 2>, ntiles, GEMM_THREADS, smem, stream, early, a);
   return psgd_launch(psgd_gemm_nn_kernel<RT, RPW, RT >= 8 ? 2 : 3>, ntiles, GEMM_THREADS, smem, stream, early, a);
 }
 
